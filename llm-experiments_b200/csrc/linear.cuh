@@ -6,12 +6,15 @@
 namespace b2kv {
 namespace lin {
 
-// x * sigmoid(1.702 x) of the clamped gate times the clamped up part plus one; silu(gate) * up.
+// x * sigmoid(1.702 x) of the clamped gate times the clamped up part plus one; silu(gate) * up.  Results are rounded to bf16, so
+// the quotients are __fdividef's (2 ulp of fp32): the operator's division is a branch to a subroutine per element, and an
+// epilogue thread has 128 of them one after the other per tile (2975 rows, K = 2048, 10880 gated columns beside 3648 plain ones:
+// 259 us with it, 176 without; the experts' 17850 rows x 2816 gated columns: 417 and 282).
 __device__ __forceinline__ float glu(int kind, float g, float u, float limit) {
-    if (kind == B2KV_SEG_GLU_SILU) return g / (1.0f + __expf(-g)) * u;
+    if (kind == B2KV_SEG_GLU_SILU) return __fdividef(g, 1.0f + __expf(-g)) * u;
     g = fminf(g, limit);
     u = fminf(fmaxf(u, -limit), limit);
-    return g / (1.0f + __expf(-1.702f * g)) * (u + 1.0f);
+    return __fdividef(g, 1.0f + __expf(-1.702f * g)) * (u + 1.0f);
 }
 
 // Kinds whose columns are (gate, up) pairs; kinds whose output is fp32.
