@@ -6,13 +6,16 @@
 //   o_t  = S^T (q_t P_t) + sum_{s <= t} A_ts v_s,   A_ts = sum_d q_td k_sd prod_{s < r <= t} alpha_rd
 //   S   <- diag(P_last) S + sum_s (k_s R_s) v_s^T
 //
-// Two kernels.  What does not depend on the state is made for many chunks at once (gla_prepare_kernel): one CTA per chunk and
+// Three kernels.  What does not depend on the state is made for many chunks at once (gla_prepare_kernel): one CTA per chunk and
 // head, thread = two key channels; A's products of decays are carried along exactly instead of being taken apart into factors that
 // could overflow, and its entries are summed over the channels 32 at a time.  The result is a record per chunk and head that is
 // byte for byte what the second kernel wants in shared memory.  Records are made a slice of the segments at a time, small enough
 // to stay in L2.
 //
-// gla_state_kernel has one CTA per (head, segment) and walks the chunks in order:
+// gla_state_kernel has one CTA per (64 value columns of a head, segment) and walks the chunks in order.  Nothing in the recurrence
+// connects value columns, and a chunk is a chain of dependent products, so what counts is how few warps share an SM's tensor pipe:
+// one per scheduler here (with a whole head's 256 columns on one SM a prompt of 2048 tokens kept 8 SMs busy: two prompts of 1750 tokens, 8 heads of
+// 128 x 256, took 402 us and take 170).
 //   * every warp owns 16 value columns of the state, transposed, as accumulators of mma.m16n8k16: the state never
 //     leaves registers between the first and the last chunk.  As an A operand of the first product the accumulators need no
 //     shuffle.  A step of the recurrence is sixteen tokens deep, one k-step of this instruction; larger tiles would have to
@@ -20,8 +23,9 @@
 //     copies and waits several times as long as these products.
 //   * fp32 operands (q P, k R, A and the state) are split into two bf16 halves, x = hi + lo, and lo * lo is dropped; v is
 //     exact.  Accumulation, decay and state are fp32.
-//   * o goes through shared memory so that the warps can take whole rows for the head's norm and the gate.
-//   * copies run ahead through a ring: records with one bulk copy each, rows of v and gate with TMA.  A thread of the first warp
+//   * the three split products of o have accumulators of their own: a third of the chain.
+//   * o leaves in fp32 for the workspace; gla_finish_kernel applies the head's norm, which needs whole rows, and the gate.
+//   * copies run ahead through a ring: records with one bulk copy each, rows of v with TMA.  A thread of the first warp
 //     asks for them when everybody has left the chunk before (a warp of its own would take registers from all others).
 // Every wait is bounded; a thread whose wait ran out goes on without waiting (so that nobody is left at a barrier) and reports.
 #include <algorithm>
@@ -37,11 +41,12 @@ namespace {
 constexpr int kChunk = 16;
 constexpr int kPairs = kChunk * (kChunk + 1) / 2;  // entries of A on and below the diagonal
 constexpr int kSlab = 16;                          // value columns per state warp
-constexpr int kMaxWarps = 16;                      // state warps
+constexpr int kWarps = 4;                          // state warps of a CTA
+constexpr int kMaxVdim = 256;
 constexpr int kBox = 32;                           // value columns per copy of v: two warps' slabs
 constexpr int kMaxRing = 6;
-constexpr int kSmemLimit = 220 * 1024;
-constexpr size_t kSliceBytes = 64u << 20;  // records of a slice, at most (but at least kMinSlice chunks per segment)
+constexpr int kSmemLimit = 109 * 1024;     // two CTAs per SM
+constexpr size_t kSliceBytes = 96u << 20;  // records and o of a slice, at most (but at least kMinSlice chunks per segment)
 constexpr int kMinSlice = 8;
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
@@ -202,37 +207,32 @@ __global__ void __launch_bounds__(kD16 <= 4 ? 32 : 8 * kD16) gla_prepare_kernel(
     for (int i = tid; i < static_cast<int>(sizeof(R) / 16); i += kThreads) dst[i] = reinterpret_cast<const uint4*>(&out)[i];
 }
 
-// One place of the ring: the record, then v in boxes of 32 columns (64-byte swizzle), then the gate's rows.
-struct RowPlan {
-    int boxes, v, gate, stride, bytes;
-    __host__ __device__ RowPlan(int record, int vdim) {
-        boxes = (vdim + kBox - 1) / kBox;
-        v = (record + 1023) / 1024 * 1024;
-        gate = v + boxes * kChunk * kBox * 2;
-        stride = (gate + kChunk * vdim * 2 + 1023) / 1024 * 1024;
-        bytes = record + kChunk * (boxes * kBox + vdim) * 2;
-    }
-};
+// o of a token and head: row ((segment * count + chunk - first) * kChunk + token) * H + head of vdim floats behind the records.
+__host__ __device__ inline int64_t record_count(const b2kv_gla_args& a, const Slice& slice) {
+    return static_cast<int64_t>(a.n_segments) * a.H * slice.count;
+}
+
+// One place of the ring: the record, then the CTA's part of v in boxes of 32 columns (64-byte swizzle).
+constexpr int kBoxBytes = kChunk * kBox * 2;
+__host__ __device__ constexpr int v_offset(int record) { return (record + 1023) / 1024 * 1024; }
+__host__ __device__ constexpr int place_bytes(int record) { return v_offset(record) + kWarps * kSlab / kBox * kBoxBytes; }
 
 struct Shared {
-    alignas(16) float norm[kSlab * kMaxWarps];
-    alignas(8) uint64_t full[kMaxRing];
-    uint64_t o_ready[2];  // o of an even / odd chunk is in shared memory: one arrival per warp
+    alignas(8) uint64_t full[kMaxRing], empty[kMaxRing];
 };
 
 template <int kD16>
-__global__ void __launch_bounds__(32 * kMaxWarps, 1) gla_state_kernel(
-    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_gate, const __grid_constant__ b2kv_gla_args a,
-    const Slice slice, int n_warps, int n_ring, int lanes_per_token, int32_t* dev_status) {
+__global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_constant__ CUtensorMap tm_v,
+                                                                  const __grid_constant__ b2kv_gla_args a, const Slice slice,
+                                                                  int parts, int n_ring, int32_t* dev_status) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ Shared sm;
     using R = Record<kD16>;
-    const RowPlan plan(sizeof(R), a.vdim);
-    const int ldo = kSlab * n_warps + 4;  // row pitch of o
+    constexpr int kStride = place_bytes(sizeof(R)), kV = v_offset(sizeof(R));
     // (an offset, not a rounded pointer: the compiler has to see that all of this is shared memory)
     uint8_t* const ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    float* const s_o = reinterpret_cast<float*>(ring + n_ring * plan.stride);  // [2][kChunk][ldo]
-    const int h = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int h = static_cast<int>(blockIdx.x) / parts, part = static_cast<int>(blockIdx.x) % parts;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     grid_launch_dependents();
     if (tid == 0) grid_dependency_wait();
@@ -241,25 +241,31 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gla_state_kernel(
     if (!segment_place(a, blockIdx.y, sg)) return;  // (reported by the other kernel)
     const int chunks = min((sg.n + kChunk - 1) / kChunk - slice.first, slice.count);
     if (chunks <= 0) return;
-    for (int i = tid; i < a.vdim; i += blockDim.x) sm.norm[i] = a.norm[i];
+    const int v0 = (part * kWarps + warp) * kSlab;  // this warp's first value column
+    const int left = a.vdim - part * kWarps * kSlab;
+    const int n_warps = min(kWarps, (left + kSlab - 1) / kSlab), boxes = (min(left, kWarps * kSlab) + kBox - 1) / kBox;
     if (tid == 0) {
-        for (int i = 0; i < kMaxRing; ++i) mbar_init(&sm.full[i], 1);
-        for (int i = 0; i < 2; ++i) mbar_init(&sm.o_ready[i], n_warps);
+        for (int i = 0; i < kMaxRing; ++i) {
+            mbar_init(&sm.full[i], 1);
+            mbar_init(&sm.empty[i], n_warps);
+        }
         fence_mbar_init();
     }
     __syncthreads();
+    if (warp >= n_warps) return;  // (there are no barriers of the whole CTA from here on)
     bool ok = true;
     const int row0 = sg.row0 + slice.first * kChunk, rows_left = sg.n - slice.first * kChunk;
 
     const R* const records = reinterpret_cast<const R*>(a.workspace) + (static_cast<int64_t>(blockIdx.y) * a.H + h) * slice.count;
+    float* const o_rows = reinterpret_cast<float*>(reinterpret_cast<R*>(a.workspace) + record_count(a, slice)) +
+                          (static_cast<int64_t>(blockIdx.y) * slice.count * kChunk * a.H + h) * a.vdim;
     auto request = [&](int ci, int slot) {
-        uint8_t* const dst = ring + slot * plan.stride;
+        uint8_t* const dst = ring + slot * kStride;
         uint64_t* const bar = &sm.full[slot];
-        mbar_arrive_expect_tx(bar, plan.bytes);
+        mbar_arrive_expect_tx(bar, sizeof(R) + boxes * kBoxBytes);
         bulk_g2s(dst, records + ci, sizeof(R), bar);
-        for (int b = 0; b < plan.boxes; ++b)
-            tma_load_2d(dst + plan.v + b * kChunk * kBox * 2, &tm_v, bar, a.v_col + h * a.vdim + b * kBox, row0 + ci * kChunk);
-        tma_load_2d(dst + plan.gate, &tm_gate, bar, a.g_col + h * a.vdim, row0 + ci * kChunk);
+        for (int b = 0; b < boxes; ++b)
+            tma_load_2d(dst + kV + b * kBoxBytes, &tm_v, bar, a.v_col + h * a.vdim + part * kWarps * kSlab + b * kBox, row0 + ci * kChunk);
     };
     if (tid == 0)
         for (int i = 0; i < min(n_ring, chunks); ++i) request(i, i);
@@ -274,7 +280,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gla_state_kernel(
         for (int j = 0; j < 2 * kD16; ++j)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int v = warp * kSlab + row + (e >> 1) * 8, d = j * 8 + col + (e & 1);
+                const int v = v0 + row + (e >> 1) * 8, d = j * 8 + col + (e & 1);
                 fn(c[j][e], static_cast<int64_t>(d) * a.vdim + v, v < a.vdim && d < a.dim);
             }
     };
@@ -284,21 +290,19 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gla_state_kernel(
     // ldmatrix row addresses: [token][channel] tiles as they lie (tokens 0-7 | 8-15 outermost), and transposed
     const int plain_t = r8 + 8 * (mat >> 1), plain_c = 8 * (mat & 1);
     const int trans_t = r8 + 8 * (mat & 1), trans_c = 8 * (mat >> 1);
-    const float inv_vdim = 1.0f / static_cast<float>(a.vdim);
-    const int group = lane / lanes_per_token, sub = lane % lanes_per_token, groups = 32 / lanes_per_token;
     int slot = 0;
     uint32_t phase = 0;
     for (int ci = 0; ci < chunks; ++ci) {
-        const uint8_t* const place = ring + slot * plan.stride;
+        const uint8_t* const place = ring + slot * kStride;
         const R& b = *reinterpret_cast<const R*>(place);
         ok = ok && mbar_wait(&sm.full[slot], phase);
         // this warp's half of a box of v: rows of 64 bytes, 16-byte pieces exchanged by row
-        const uint32_t v_addr = smem_u32(place + plan.v + (warp >> 1) * kChunk * kBox * 2 + plain_t * 64) +
+        const uint32_t v_addr = smem_u32(place + kV + (warp >> 1) * kBoxBytes + plain_t * 64) +
                                 (((2 * (warp & 1) + (plain_c >> 3)) ^ ((plain_t >> 1) & 3)) << 4);
         const uint32_t q_addr = smem_u32(&b.q_hi[plain_t][plain_c]), k_addr = smem_u32(&b.k_hi[trans_t][trans_c]);
         constexpr uint32_t kLo = sizeof(b.q_hi);  // from a matrix of leading halves to that of what they leave
         uint32_t vf[4], x[2][4], z[2][4];
-        float o[2][4];
+        float o[2][4], oa[2][4], ob[2][4];  // products of leading halves; those with the low half of q and of the state
         ldsm4t(vf, v_addr);
         {
             ldsm4(x[1], smem_u32(&b.a_hi[plain_t][plain_c]));
@@ -307,11 +311,11 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gla_state_kernel(
             ldsm4(z[0], q_addr + kLo);
 #pragma unroll
             for (int n = 0; n < 2; ++n) {
-                o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-                mma16816(o[n], vf, x[1][2 * n], x[1][2 * n + 1]);
-            }
 #pragma unroll
-            for (int n = 0; n < 2; ++n) mma16816(o[n], vf, z[1][2 * n], z[1][2 * n + 1]);
+                for (int e = 0; e < 4; ++e) o[n][e] = oa[n][e] = ob[n][e] = 0.f;
+                mma16816(o[n], vf, x[1][2 * n], x[1][2 * n + 1]);
+                mma16816(oa[n], vf, z[1][2 * n], z[1][2 * n + 1]);
+            }
         }
 #pragma unroll
         for (int kk = 0; kk < kD16; ++kk) {
@@ -329,19 +333,19 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gla_state_kernel(
 #pragma unroll
             for (int n = 0; n < 2; ++n) mma16816(o[n], s_hi, hi[2 * n], hi[2 * n + 1]);
 #pragma unroll
-            for (int n = 0; n < 2; ++n) mma16816(o[n], s_hi, lo[2 * n], lo[2 * n + 1]);
+            for (int n = 0; n < 2; ++n) mma16816(oa[n], s_hi, lo[2 * n], lo[2 * n + 1]);
 #pragma unroll
-            for (int n = 0; n < 2; ++n) mma16816(o[n], s_lo, hi[2 * n], hi[2 * n + 1]);
+            for (int n = 0; n < 2; ++n) mma16816(ob[n], s_lo, hi[2 * n], hi[2 * n + 1]);
         }
         ldsm4t(x[0], k_addr);
         ldsm4t(z[0], k_addr + kLo);
-        float* const so = s_o + (ci & 1) * kChunk * ldo;
 #pragma unroll
         for (int n = 0; n < 2; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) so[(n * 8 + col + (e & 1)) * ldo + warp * kSlab + row + (e >> 1) * 8] = o[n][e];
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.o_ready[ci & 1]);
+            for (int e = 0; e < 4; ++e) {
+                const int t = ci * kChunk + n * 8 + col + (e & 1), v = v0 + row + (e >> 1) * 8;
+                if (v < a.vdim && t < rows_left) o_rows[static_cast<int64_t>(t) * a.H * a.vdim + v] = o[n][e] + (oa[n][e] + ob[n][e]);
+            }
 #pragma unroll
         for (int kk = 0; kk < kD16; ++kk) {
             if (kk + 1 < kD16) {
@@ -359,44 +363,15 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gla_state_kernel(
 #pragma unroll
             for (int u = 0; u < 2; ++u) mma16816(c[2 * kk + u], vf, lo[2 * u], lo[2 * u + 1]);
         }
-        // All warps have stored their part of o, so they have left the chunk before: its place in the ring is free, and so is the
-        // other buffer of o.  Nobody waits for the others' updates here: the warps drift apart and keep the tensor pipe busy.
-        ok = ok && mbar_wait(&sm.o_ready[ci & 1], (ci >> 1) & 1);
         __syncwarp();
-        if (tid == 0 && ci > 0 && ci - 1 + n_ring < chunks) request(ci - 1 + n_ring, slot == 0 ? n_ring - 1 : slot - 1);
-        // whole rows of o: lanes_per_token lanes with eight values each
-        for (int t0 = warp * groups; t0 < kChunk; t0 += n_warps * groups) {
-            const int t = t0 + group;
-            const bool mine = sub * 8 < a.vdim && t < kChunk && ci * kChunk + t < rows_left;
-            const float* const src = so + t * ldo + sub * 8;
-            float sum = 0.f;
-            if (mine) {
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const float4 f = *reinterpret_cast<const float4*>(src + half * 4);
-                    sum = fmaf(f.x, f.x, fmaf(f.y, f.y, fmaf(f.z, f.z, fmaf(f.w, f.w, sum))));
-                }
-            }
-            for (int off = lanes_per_token / 2; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-            if (mine) {
-                const float scale = rsqrtf(fmaf(sum, inv_vdim, a.eps));
-                const uint8_t* const gate = place + plan.gate + (t * a.vdim + sub * 8) * 2;
-                __nv_bfloat16* const dst = static_cast<__nv_bfloat16*>(a.out) + (static_cast<int64_t>(row0) + ci * kChunk + t) * a.ld_out +
-                                           static_cast<int64_t>(h) * a.vdim + sub * 8;
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const float4 f = *reinterpret_cast<const float4*>(src + half * 4);
-                    const float4 n = *reinterpret_cast<const float4*>(&sm.norm[sub * 8 + half * 4]);
-                    const uint2 g = *reinterpret_cast<const uint2*>(gate + half * 8);
-                    uint2 out;
-                    out.x = tc::pack_bf16(f.x * scale * n.x * silu_fast(__uint_as_float(g.x << 16)),
-                                          f.y * scale * n.y * silu_fast(__uint_as_float(g.x & 0xffff0000u)));
-                    out.y = tc::pack_bf16(f.z * scale * n.z * silu_fast(__uint_as_float(g.y << 16)),
-                                          f.w * scale * n.w * silu_fast(__uint_as_float(g.y & 0xffff0000u)));
-                    *reinterpret_cast<uint2*>(dst + half * 4) = out;
-                }
-            }
+        if (lane == 0) mbar_arrive(&sm.empty[slot]);
+        // the place of the chunk before is free when the last warp has left it (one chunk behind: nobody waits long)
+        if (tid == 0 && ci > 0 && ci - 1 + n_ring < chunks) {
+            const int before = slot == 0 ? n_ring - 1 : slot - 1;
+            ok = ok && mbar_wait(&sm.empty[before], (ci - 1) / n_ring & 1);
+            request(ci - 1 + n_ring, before);
         }
+        __syncwarp();
         if (++slot == n_ring) slot = 0, phase ^= 1;
     }
     each_state([&](float& x, int64_t at, bool live) {
@@ -408,6 +383,44 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gla_state_kernel(
             for (int i = max(0, chunks - n_ring); i < chunks; ++i) mbar_wait(&sm.full[i % n_ring], (i / n_ring) & 1);
         report_status(dev_status, B2KV_DEV_WAIT_TIMEOUT);
     }
+}
+
+// The heads' norm and the gate: one warp per (token, head), eight value columns per lane.
+constexpr int kFinishWarps = 8;
+template <typename R>
+__global__ void __launch_bounds__(32 * kFinishWarps) gla_finish_kernel(const __grid_constant__ b2kv_gla_args a, const Slice slice) {
+    const int lane = threadIdx.x & 31, at = static_cast<int>(blockIdx.x) * kFinishWarps + (threadIdx.x >> 5);
+    const int t = at / a.H, h = at % a.H, c = lane * 8;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    b2kv_row_segment sg;
+    if (!segment_place(a, blockIdx.y, sg)) return;
+    if (t >= slice.count * kChunk || slice.first * kChunk + t >= sg.n) return;
+    const int64_t row = static_cast<int64_t>(sg.row0) + slice.first * kChunk + t;
+    const float* const src = reinterpret_cast<const float*>(reinterpret_cast<const R*>(a.workspace) + record_count(a, slice)) +
+                             ((static_cast<int64_t>(blockIdx.y) * slice.count * kChunk + t) * a.H + h) * a.vdim + c;
+    const bool mine = c < a.vdim;
+    float f[8], sum = 0.f;
+    uint4 gate = make_uint4(0u, 0u, 0u, 0u);
+    if (mine) {
+        *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(src);
+        *reinterpret_cast<float4*>(f + 4) = *reinterpret_cast<const float4*>(src + 4);
+        gate = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.y) + row * a.ld_y + a.g_col + h * a.vdim + c);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum = fmaf(f[i], f[i], sum);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    if (!mine) return;
+    const float scale = rsqrtf(fmaf(sum, 1.0f / static_cast<float>(a.vdim), a.eps));
+    const uint32_t g[4] = {gate.x, gate.y, gate.z, gate.w};
+    uint32_t out[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        out[i] = tc::pack_bf16(f[2 * i] * scale * __ldg(a.norm + c + 2 * i) * silu_fast(__uint_as_float(g[i] << 16)),
+                               f[2 * i + 1] * scale * __ldg(a.norm + c + 2 * i + 1) * silu_fast(__uint_as_float(g[i] & 0xffff0000u)));
+    *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(a.out) + row * a.ld_out + static_cast<int64_t>(h) * a.vdim + c) =
+        make_uint4(out[0], out[1], out[2], out[3]);
 }
 
 // Row-major bf16 matrix, boxes of kChunk rows.
@@ -426,25 +439,25 @@ int record_bytes(int dim) {
     return static_cast<int>(dim <= 32 ? sizeof(Record<2>) : (dim <= 64 ? sizeof(Record<4>) : sizeof(Record<8>)));
 }
 
-int slice_chunks(int H, int dim, int n_segments, int max_n) {
+size_t chunk_bytes(int H, int dim, int vdim) {
+    return (static_cast<size_t>(record_bytes(dim)) + kChunk * static_cast<size_t>(vdim) * sizeof(float)) * H;
+}
+
+int slice_chunks(int H, int dim, int vdim, int n_segments, int max_n) {
     const int chunks = (max_n + kChunk - 1) / kChunk;
-    const size_t per_chunk = static_cast<size_t>(record_bytes(dim)) * H * n_segments;
-    const int fit = static_cast<int>(std::min<size_t>(kSliceBytes / per_chunk, 1u << 20));
+    const int fit = static_cast<int>(std::min<size_t>(kSliceBytes / (chunk_bytes(H, dim, vdim) * n_segments), 1u << 20));
     return std::min(chunks, std::max(kMinSlice, fit));
 }
 
 template <int kD16>
 int launch_chunked(const b2kv_gla_args& a, int32_t* dev_status, void* stream) {
-    const int n_warps = (a.vdim + kSlab - 1) / kSlab;
-    const RowPlan plan(sizeof(Record<kD16>), a.vdim);
-    const int fixed = 1024 + 2 * kChunk * (kSlab * n_warps + 4) * static_cast<int>(sizeof(float));
-    const int n_ring = std::min(kMaxRing, (kSmemLimit - fixed) / plan.stride);
-    const size_t smem = fixed + static_cast<size_t>(n_ring) * plan.stride;
-    CUtensorMap tv, tg;
+    using R = Record<kD16>;
+    const int parts = (a.vdim + kWarps * kSlab - 1) / (kWarps * kSlab);
+    const int n_ring = std::min(kMaxRing, (kSmemLimit - 1024) / place_bytes(sizeof(R)));
+    const size_t smem = 1024 + static_cast<size_t>(n_ring) * place_bytes(sizeof(R));
+    CUtensorMap tv;
     const int64_t cols = std::max(a.v_col, a.g_col) + static_cast<int64_t>(a.H) * a.vdim;
-    if (!make_map(&tv, a.y, a.rows, cols, a.ld_y, kBox, CU_TENSOR_MAP_SWIZZLE_64B) ||
-        !make_map(&tg, a.y, a.rows, cols, a.ld_y, a.vdim, CU_TENSOR_MAP_SWIZZLE_NONE))
-        return B2KV_ERR_UNSUPPORTED;
+    if (!make_map(&tv, a.y, a.rows, cols, a.ld_y, kBox, CU_TENSOR_MAP_SWIZZLE_64B)) return B2KV_ERR_UNSUPPORTED;
     static int configured[64] = {0};
     int dev = 0;
     B2KV_CUDA_TRY(cudaGetDevice(&dev));
@@ -454,22 +467,23 @@ int launch_chunked(const b2kv_gla_args& a, int32_t* dev_status, void* stream) {
         B2KV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
         configured[dev] = static_cast<int>(smem);
     }
-    int lanes = 2;  // lanes per row of o, eight values each: a power of two
-    while (lanes * 8 < a.vdim) lanes *= 2;
     const int chunks = (a.max_n + kChunk - 1) / kChunk;
-    Slice slice{0, slice_chunks(a.H, a.dim, a.n_segments, a.max_n)};
+    Slice slice{0, slice_chunks(a.H, a.dim, a.vdim, a.n_segments, a.max_n)};
     for (; slice.first < chunks; slice.first += slice.count) {
         const unsigned here = static_cast<unsigned>(std::min(slice.count, chunks - slice.first));
         OverlapLaunch prep(dim3(here, a.H, a.n_segments), kD16 <= 4 ? 32 : 8 * kD16, 0, stream);
         B2KV_CUDA_TRY(cudaLaunchKernelEx(&prep.cfg, gla_prepare_kernel<kD16>, a, slice, dev_status));
-        OverlapLaunch walk(dim3(a.H, a.n_segments), 32 * n_warps, smem, stream);
-        B2KV_CUDA_TRY(cudaLaunchKernelEx(&walk.cfg, kernel, tv, tg, a, slice, n_warps, n_ring, lanes, dev_status));
+        OverlapLaunch walk(dim3(a.H * parts, a.n_segments), 32 * kWarps, smem, stream);
+        B2KV_CUDA_TRY(cudaLaunchKernelEx(&walk.cfg, kernel, tv, a, slice, parts, n_ring, dev_status));
+        const unsigned pairs = here * kChunk * static_cast<unsigned>(a.H);
+        OverlapLaunch finish(dim3((pairs + kFinishWarps - 1) / kFinishWarps, a.n_segments), 32 * kFinishWarps, 0, stream);
+        B2KV_CUDA_TRY(cudaLaunchKernelEx(&finish.cfg, gla_finish_kernel<R>, a, slice));
     }
     return B2KV_OK;
 }
 
 bool chunked_sizes(int dim, int vdim, int dtype) {
-    return dtype == B2KV_DTYPE_BF16 && dim > 0 && dim % 8 == 0 && dim <= 128 && vdim > 0 && vdim % 8 == 0 && vdim <= kSlab * kMaxWarps;
+    return dtype == B2KV_DTYPE_BF16 && dim > 0 && dim % 8 == 0 && dim <= 128 && vdim > 0 && vdim % 8 == 0 && vdim <= kMaxVdim;
 }
 
 }  // namespace
@@ -477,7 +491,7 @@ bool chunked_sizes(int dim, int vdim, int dtype) {
 
 size_t gla_chunked_workspace(int H, int dim, int vdim, int n_segments, int max_n, int dtype) {
     if (!gla::chunked_sizes(dim, vdim, dtype)) return 0;
-    return static_cast<size_t>(gla::slice_chunks(H, dim, n_segments, max_n)) * gla::record_bytes(dim) * H * n_segments;
+    return static_cast<size_t>(gla::slice_chunks(H, dim, vdim, n_segments, max_n)) * gla::chunk_bytes(H, dim, vdim) * n_segments;
 }
 
 int gla_chunked(const b2kv_gla_args& a, int32_t* dev_status, void* stream) {
