@@ -1,5 +1,4 @@
-// b2kv_linear: argument checks, the choice of the kernel, and the CUDA-core kernel for fp32 and for shapes that the
-// tensor-core kernels do not take, and the one for few input features (64 x 64 output tiles, 16 input features per step, 4 x 4 outputs per thread, fp32
+// b2kv_linear: argument checks, the choice of the kernel, the CUDA-core kernel for shapes and alignments that the others do not take, and the one for few input features (64 x 64 output tiles, 16 input features per step, 4 x 4 outputs per thread, fp32
 // accumulation).
 #include "linear.cuh"
 
@@ -7,16 +6,6 @@ namespace b2kv {
 namespace lin {
 
 constexpr int kTile = 64, kStep = 16, kThreads = 256;
-
-// Exact exponential for the fp32 path; the bf16 paths round the result to 8 bits anyway.
-template <typename T>
-__device__ __forceinline__ float glu_value(int kind, float g, float u, float limit) {
-    if (sizeof(T) == 2) return glu(kind, g, u, limit);
-    if (kind == B2KV_SEG_GLU_SILU) return g / (1.0f + expf(-g)) * u;
-    g = fminf(g, limit);
-    u = fminf(fmaxf(u, -limit), limit);
-    return g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
-}
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) linear_simt_kernel(const b2kv_linear_args a) {
@@ -68,31 +57,7 @@ __global__ void __launch_bounds__(kThreads) linear_simt_kernel(const b2kv_linear
         for (int j = 0; j < 4; j += 2) {  // pairs of columns: boundaries of segments are even
             const int c = col0 + tx * 4 + j;
             if (c >= a.N) break;
-            const int s = segment_of(a, c);
-            const b2kv_segment& sg = a.seg[s];
-            const int local = c - segment_first(a, s);
-            const int64_t base = out_row * sg.ld + static_cast<int64_t>(g) * (a.group_rows ? 0 : sg.group);
-            if (a.bias != nullptr) {
-                acc[i][j] += a.bias[c];
-                if (c + 1 < a.N) acc[i][j + 1] += a.bias[c + 1];
-            }
-            if (is_pair(sg.kind)) {
-                static_cast<T*>(sg.out)[base + local / 2] =
-                    Elt<T>::from_float(glu_value<T>(sg.kind, acc[i][j], acc[i][j + 1], a.limit));
-                continue;
-            }
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                if (c + e >= a.N) break;
-                float v = sizeof(T) == 4 && sg.kind == B2KV_SEG_DECAY ? decay_exact(acc[i][j + e], a.limit)
-                                                                      : single(sg.kind, acc[i][j + e], a.limit);
-                if (is_f32(sg.kind)) {
-                    if (a.residual != nullptr && sg.kind == B2KV_SEG_F32) v += a.residual[out_row * a.ld_residual + local + e];
-                    static_cast<float*>(sg.out)[base + local + e] = v;
-                } else {
-                    static_cast<T*>(sg.out)[base + local + e] = Elt<T>::from_float(v);
-                }
-            }
+            finish_pair<T>(a, g, out_row, c, acc[i][j], acc[i][j + 1]);
         }
     }
 }
@@ -231,6 +196,10 @@ extern "C" int b2kv_linear(const b2kv_linear_args* args, int32_t* dev_status, vo
         } else {
             rc = linear_tiled_tc(a, dev_status, stream);
         }
+        if (rc != B2KV_ERR_UNSUPPORTED) return rc;
+    }
+    if (a.path == 0 && a.dtype == B2KV_DTYPE_F32) {
+        const int rc = linear_f32(a, stream);
         if (rc != B2KV_ERR_UNSUPPORTED) return rc;
     }
     return lin::launch_simt(a, stream);

@@ -56,7 +56,50 @@ __device__ __forceinline__ int segment_of(const b2kv_linear_args& a, int c) {
 
 __device__ __forceinline__ int segment_first(const b2kv_linear_args& a, int s) { return s == 0 ? 0 : a.seg[s - 1].end; }
 
+// Exact exponential for the fp32 path; the bf16 paths round the result to 8 bits anyway.
+template <typename T>
+__device__ __forceinline__ float glu_value(int kind, float g, float u, float limit) {
+    if (sizeof(T) == 2) return glu(kind, g, u, limit);
+    if (kind == B2KV_SEG_GLU_SILU) return g / (1.0f + expf(-g)) * u;
+    g = fminf(g, limit);
+    u = fminf(fmaxf(u, -limit), limit);
+    return g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
+}
+
+// The outputs of columns c and c + 1 (c even) of one row, from the sums of their products.
+template <typename T>
+__device__ __forceinline__ void finish_pair(const b2kv_linear_args& a, int g, int64_t out_row, int c, float v0, float v1) {
+    const int s = segment_of(a, c);
+    const b2kv_segment& sg = a.seg[s];
+    const int local = c - segment_first(a, s);
+    const int64_t base = out_row * sg.ld + static_cast<int64_t>(g) * (a.group_rows ? 0 : sg.group);
+    const bool second = c + 1 < a.N;
+    if (a.bias != nullptr) {
+        v0 += a.bias[c];
+        if (second) v1 += a.bias[c + 1];
+    }
+    if (is_pair(sg.kind)) {
+        static_cast<T*>(sg.out)[base + local / 2] = Elt<T>::from_float(glu_value<T>(sg.kind, v0, v1, a.limit));
+        return;
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        if (e == 1 && !second) break;
+        float v = e ? v1 : v0;
+        v = sizeof(T) == 4 && sg.kind == B2KV_SEG_DECAY ? decay_exact(v, a.limit) : single(sg.kind, v, a.limit);
+        if (is_f32(sg.kind)) {
+            if (a.residual != nullptr && sg.kind == B2KV_SEG_F32) v += a.residual[out_row * a.ld_residual + local + e];
+            static_cast<float*>(sg.out)[base + local + e] = v;
+        } else {
+            static_cast<T*>(sg.out)[base + local + e] = Elt<T>::from_float(v);
+        }
+    }
+}
+
 }  // namespace lin
+
+// fp32 on the CUDA cores; B2KV_ERR_UNSUPPORTED where rows are not made of 16-byte pieces.
+int linear_f32(const b2kv_linear_args& a, void* stream);  // linear_f32.cu
 
 // bf16 kernels on the tensor cores; B2KV_ERR_UNSUPPORTED when the shape is not one they take.
 int linear_rows_tc(const b2kv_linear_args& a, int32_t* dev_status, void* stream);   // linear_rows.cu

@@ -1,0 +1,291 @@
+// b2kv_linear in fp32 on the CUDA cores, two kernels.  Sums are fp32 multiply-adds, so what bounds them is that pipe (72 TFLOP/s
+// over the chip at 1.9 GHz) for many rows and the weights' bytes for few.  693 rows, 3072 x 768 weights: 441 us with linear_simt_kernel
+// (one read of shared memory per two multiply-adds, 132 CTAs, nothing ahead of its use), 158 here; 6 rows, 768 x 4096: 128 and 14.
+//
+// linear_f32_tile_kernel: 64 x 128 outputs per CTA of 128 threads, 8 x 8 per thread: 64 multiply-adds for every four 16-byte reads
+// of shared memory, so the pipe and not the reads is what is busy.  Steps of 16 input features through two buffers; the next
+// step's global reads are in flight (in registers) under the products of this one.  A product whose tiles leave SMs idle has its
+// input features cut into up to eight ranges, one per CTA of a cluster; the partial sums meet in distributed shared memory, where
+// every CTA adds up its share of the tile's rows in the order of the ranges (results do not depend on timing).
+//
+// linear_f32_rows_kernel: up to 16 rows (a decode step, the wanted logits).  A thread keeps four neighbouring columns of every row;
+// the warps of a CTA and the CTAs of a cluster share the input features, so w is read once, 512 bytes per warp at a time.
+#include <algorithm>
+
+#include "linear.cuh"
+
+namespace b2kv {
+namespace linf32 {
+
+constexpr int kBM = 64, kBN = 128, kStep = 16, kThreads = 128;
+constexpr int kLdX = kBM + 4, kLdT = kBN + 4;
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peer_address(const void* local, uint32_t rank) {
+    uint32_t addr;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(local)), "r"(rank));
+    return addr;
+}
+__device__ __forceinline__ float2 peer_load2(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+
+// Rows of a CTA's group, and where its operands start.
+struct Operands {
+    const float *x, *w;
+    int first, n_rows;
+};
+__device__ __forceinline__ Operands operands(const b2kv_linear_args& a, int g) {
+    Operands o{static_cast<const float*>(a.x), static_cast<const float*>(a.w) + static_cast<int64_t>(g) * a.group_w, 0, a.rows};
+    if (a.group_rows != nullptr) {
+        o.first = a.group_rows[g];
+        o.n_rows = a.group_rows[g + 1] - o.first;
+        o.x += static_cast<int64_t>(o.first) * a.ld_x;
+    } else {
+        o.x += static_cast<int64_t>(g) * a.group_x;
+    }
+    return o;
+}
+
+__global__ void __launch_bounds__(kThreads, 3) linear_f32_tile_kernel(const __grid_constant__ b2kv_linear_args a, int splits) {
+    struct Ring {
+        float x[2][kStep][kLdX], w[2][kStep][kBN];
+    };
+    __shared__ union {
+        Ring ring;
+        float tile[kBM][kLdT];
+    } sm;
+    grid_dependency_wait();
+    const int g = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const Operands op = operands(a, g);
+    const int split = splits > 1 ? static_cast<int>(cluster_rank()) : 0;
+    const int row0 = blockIdx.y * kBM, col0 = static_cast<int>(blockIdx.x) / splits * kBN;
+    if (row0 >= op.n_rows) return;  // (all CTAs of a cluster)
+    const int steps = (a.K + kStep - 1) / kStep;
+    const int k_first = static_cast<int>(static_cast<long long>(steps) * split / splits) * kStep;
+    const int k_end = min(static_cast<int>(static_cast<long long>(steps) * (split + 1) / splits) * kStep, a.K);
+
+    // x: a warp reads one 16-byte piece of 32 rows (the same pieces of the other rows next); w: whole rows of 128 columns
+    float4 xr[2], wr[4];
+    auto read = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int r = row0 + lane + 32 * i, k = k0 + warp * 4;
+            xr[i] = r < op.n_rows && k < k_end ? *reinterpret_cast<const float4*>(op.x + static_cast<int64_t>(r) * a.ld_x + k)
+                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int k = k0 + warp + 4 * i, c = col0 + lane * 4;
+            wr[i] = k < k_end && c < a.N ? __ldg(reinterpret_cast<const float4*>(op.w + static_cast<int64_t>(k) * a.ld_w + c))
+                                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    auto write = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            float* const dst = &sm.ring.x[buf][warp * 4][lane + 32 * i];
+            dst[0] = xr[i].x, dst[kLdX] = xr[i].y, dst[2 * kLdX] = xr[i].z, dst[3 * kLdX] = xr[i].w;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(&sm.ring.w[buf][warp + 4 * i][lane * 4]) = wr[i];
+    };
+    // a warp has 32 rows x 64 columns, a thread rows r, r + 16 .. + 3 and columns c, c + 32 .. + 3 of them
+    const int tr = (warp & 1) * 32 + (lane >> 3) * 4, tc = (warp >> 1) * 64 + (lane & 7) * 4;
+    float acc[8][8] = {};
+    read(k_first);
+    write(0);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = k_first; k0 < k_end; k0 += kStep, buf ^= 1) {
+        const bool more = k0 + kStep < k_end;
+        if (more) read(k0 + kStep);
+#pragma unroll
+        for (int k = 0; k < kStep; ++k) {
+            const float4 x0 = *reinterpret_cast<const float4*>(&sm.ring.x[buf][k][tr]);
+            const float4 x1 = *reinterpret_cast<const float4*>(&sm.ring.x[buf][k][tr + 16]);
+            const float4 w0 = *reinterpret_cast<const float4*>(&sm.ring.w[buf][k][tc]);
+            const float4 w1 = *reinterpret_cast<const float4*>(&sm.ring.w[buf][k][tc + 32]);
+            const float xv[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+            const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(xv[i], wv[j], acc[i][j]);
+        }
+        if (more) write(buf ^ 1);
+        __syncthreads();
+    }
+    grid_launch_dependents();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; j += 4)
+            *reinterpret_cast<float4*>(&sm.tile[tr + (i & 3) + (i >> 2) * 16][tc + j * 8]) =
+                make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+    if (splits > 1) cluster_sync();
+    else __syncthreads();
+    const int c = (tid & 63) * 2, share = kBM / splits;
+    uint32_t peer[8];
+#pragma unroll
+    for (int s = 0; s < 8; ++s) peer[s] = s < splits ? peer_address(&sm.tile[0][c], s) : 0u;
+    const bool live = col0 + c < a.N;
+    for (int r = split * share + (tid >> 6); r < (split + 1) * share; r += 2) {
+        if (!live || row0 + r >= op.n_rows) break;
+        float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            if (s >= splits) break;
+            const float2 p = peer_load2(peer[s] + r * kLdT * 4);
+            v.x += p.x, v.y += p.y;
+        }
+        lin::finish_pair<float>(a, g, op.first + row0 + r, col0 + c, v.x, v.y);
+    }
+    __syncwarp();
+    if (splits > 1) cluster_sync();  // the peers have read this CTA's part
+}
+
+constexpr int kRowsThreads = 256, kRowsCols = 128, kChunkK = 128;
+
+template <int kR>
+__global__ void __launch_bounds__(kRowsThreads) linear_f32_rows_kernel(const __grid_constant__ b2kv_linear_args a, int splits) {
+    constexpr int kWarps = kRowsThreads / 32;
+    __shared__ float4 xs[kChunkK][kR / 4];
+    __shared__ float4 part[kWarps / 2][kR][kRowsCols / 4];
+    grid_dependency_wait();
+    const int g = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const Operands op = operands(a, g);
+    const int split = splits > 1 ? static_cast<int>(cluster_rank()) : 0;
+    const int c0 = static_cast<int>(blockIdx.x) / splits * kRowsCols, c = c0 + lane * 4;
+    if (op.n_rows <= 0) return;
+    const int chunks = (a.K + kChunkK - 1) / kChunkK;
+    const int k_first = static_cast<int>(static_cast<long long>(chunks) * split / splits) * kChunkK;
+    const int k_end = min(static_cast<int>(static_cast<long long>(chunks) * (split + 1) / splits) * kChunkK, a.K);
+    float4 acc[kR];
+#pragma unroll
+    for (int r = 0; r < kR; ++r) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+    constexpr int kMine = kChunkK / kWarps;  // input features of a chunk per warp: neighbours, so that w is read in long runs
+    for (int k0 = k_first; k0 < k_end; k0 += kChunkK) {
+        float4 wv[kMine];
+#pragma unroll
+        for (int i = 0; i < kMine; ++i) {
+            const int k = k0 + warp * kMine + i;
+            wv[i] = k < k_end && c < a.N ? __ldg(reinterpret_cast<const float4*>(op.w + static_cast<int64_t>(k) * a.ld_w + c))
+                                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncthreads();
+        for (int i = tid; i < kChunkK * kR; i += kRowsThreads) {
+            const int r = i / kChunkK, k = i % kChunkK;
+            reinterpret_cast<float*>(xs[k])[r] = r < op.n_rows && k0 + k < k_end ? op.x[static_cast<int64_t>(r) * a.ld_x + k0 + k] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kMine; ++i) {
+#pragma unroll
+            for (int q = 0; q < kR / 4; ++q) {
+                const float4 xq = xs[warp * kMine + i][q];
+                const float xv[4] = {xq.x, xq.y, xq.z, xq.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float4& s = acc[q * 4 + e];
+                    s.x = fmaf(xv[e], wv[i].x, s.x), s.y = fmaf(xv[e], wv[i].y, s.y);
+                    s.z = fmaf(xv[e], wv[i].z, s.z), s.w = fmaf(xv[e], wv[i].w, s.w);
+                }
+            }
+        }
+    }
+    grid_launch_dependents();
+    // the warps' sums, halves of them at a time, then the ranges' (in order)
+#pragma unroll
+    for (int half = kWarps / 2; half > 0; half >>= 1) {
+        __syncthreads();
+        if (warp >= half && warp < 2 * half) {
+#pragma unroll
+            for (int r = 0; r < kR; ++r) part[warp - half][r][lane] = acc[r];
+        }
+        __syncthreads();
+        if (warp < half) {
+#pragma unroll
+            for (int r = 0; r < kR; ++r) {
+                const float4 p = part[warp][r][lane];
+                acc[r].x += p.x, acc[r].y += p.y, acc[r].z += p.z, acc[r].w += p.w;
+            }
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int r = 0; r < kR; ++r) part[0][r][lane] = acc[r];
+    }
+    if (splits > 1) cluster_sync();
+    else __syncthreads();
+    const int cp = (tid & 63) * 2;
+    for (int r = (tid >> 6) * splits + split; r < min(kR, op.n_rows); r += kRowsThreads / 64 * splits) {
+        if (c0 + cp >= a.N) break;
+        float2 v = make_float2(0.f, 0.f);
+        for (int s = 0; s < splits; ++s) {
+            const float2 p = peer_load2(peer_address(&part[0][r][0], s) + cp * 4);
+            v.x += p.x, v.y += p.y;
+        }
+        lin::finish_pair<float>(a, g, op.first + r, c0 + cp, v.x, v.y);
+    }
+    __syncwarp();
+    if (splits > 1) cluster_sync();
+}
+
+}  // namespace linf32
+
+int linear_f32(const b2kv_linear_args& a, void* stream) {
+    using namespace linf32;
+    if (a.dtype != B2KV_DTYPE_F32) return B2KV_ERR_UNSUPPORTED;
+    // 16-byte pieces of rows of x and w; outputs and the residual have no rule
+    if (!aligned16(a.x) || !aligned16(a.w) || a.K % 4 || a.N % 4 || a.ld_x % 4 || a.ld_w % 4 || a.group_x % 4 || a.group_w % 4)
+        return B2KV_ERR_UNSUPPORTED;
+    const int max_rows = a.group_rows ? a.max_group_rows : a.rows, sms = device_sm_count();
+    const long long tiles_n = (a.N + kBN - 1) / kBN;
+    int splits = 1;
+    auto forced = [](int by_shape) {  // the knob of the tensor-core kernel for few rows
+        int s = 1;
+        while (s < 8 && s * 2 <= tune_get("matmul_splits")) s *= 2;
+        return tune_get("matmul_splits") > 0 ? s : by_shape;
+    };
+    if (max_rows <= 16) {
+        // ranges of at least one chunk, two CTAs per SM at most
+        const long long tiles = tiles_n * a.groups;
+        while (splits < 8 && tiles * splits * 2 <= 2 * sms && splits * 2 * kChunkK <= a.K) splits *= 2;
+        splits = forced(splits);
+        if (tiles_n * splits > 0x7fffffffLL || a.groups > 65535) return B2KV_ERR_UNSUPPORTED;
+        OverlapLaunch launch(dim3(static_cast<unsigned>(tiles_n * splits), 1, a.groups), kRowsThreads, 0, stream, splits);
+        B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg,
+                                         max_rows <= 4 ? linear_f32_rows_kernel<4>
+                                                       : (max_rows <= 8 ? linear_f32_rows_kernel<8> : linear_f32_rows_kernel<16>),
+                                         a, splits));
+        return B2KV_OK;
+    }
+    const long long tiles_m = (max_rows + kBM - 1) / kBM, tiles = tiles_n * tiles_m * a.groups;
+    // The work of the fullest SM, in CTAs of whole input features; a range keeps eight steps at least.  (With rows grouped by
+    // expert most of the tiles that max_group_rows allows for are empty: no ranges.)
+    double best = 1e30;
+    for (int s = 1; s <= 8 && !(s > 1 && a.group_rows); s *= 2) {
+        if (s > 1 && a.K < 8 * kStep * s) break;
+        const double cost = static_cast<double>((tiles * s + sms - 1) / sms) / s + 0.02 * (s - 1);
+        if (cost < 0.95 * best) best = cost, splits = s;
+    }
+    splits = forced(splits);
+    if (tiles_m > 65535 || a.groups > 65535 || tiles_n * splits > 0x7fffffffLL) return B2KV_ERR_UNSUPPORTED;
+    OverlapLaunch launch(dim3(static_cast<unsigned>(tiles_n * splits), static_cast<unsigned>(tiles_m), a.groups), kThreads, 0, stream, splits);
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, linear_f32_tile_kernel, a, splits));
+    return B2KV_OK;
+}
+
+}  // namespace b2kv

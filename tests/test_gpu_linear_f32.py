@@ -1,0 +1,101 @@
+"""fp32 products on the CUDA cores (the choice left open) against float64: few rows and tiles, their edges, ranges of input features,
+every kind of segment, groups."""
+import numpy as np
+import pytest
+import torch
+
+from tests.kv_util import make_ctx
+from tests.test_gpu_linear import close, glu, rnd, run, wrap
+
+pytestmark = pytest.mark.gpu
+
+F32 = torch.float32
+
+
+def bounded(got, x, w, add=0.0):
+    """Each of the K products and sums rounds once, a residual's once more: at most (K + 1) * 2^-24 of the sum of magnitudes, in any order."""
+    want, size = x.double() @ w.double() + add, x.double().abs() @ w.double().abs() + abs(add)
+    assert ((got.double() - want).abs() <= (x.shape[1] + 1) * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("rows", [1, 4, 5, 8, 9, 16, 17, 63, 64, 65, 200])
+@pytest.mark.parametrize("K,cols", [(4, (4, 0)), (36, (64, 68)), (128, (128, 4)), (260, (96, 164)), (2052, (32, 100)), (1040, (2048, 32))])
+def test_store_and_residual(pkg, rows, K, cols):
+    from llm_experiments_b200 import projection as proj
+
+    ctx, (a, b) = make_ctx(pkg), cols
+    x, w = rnd((rows, K + 8), F32, 1)[:, 4:4 + K], rnd((K, a + b + 4), F32, 2, K ** -0.5)[:, :a + b]
+    out = torch.full((rows + 1, a + 5), 7.0, dtype=F32, device="cuda")
+    res = rnd((rows, b + 3), F32, 3)
+    keep = res.clone()
+    segments = [proj.OutputSegment(a, proj.SEG_STORE, wrap(pkg, out[:, :a]))]
+    if b:
+        segments.append(proj.OutputSegment(a + b, proj.SEG_F32, wrap(pkg, res)))
+    run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), K, segments, residual=wrap(pkg, res) if b else None)
+    bounded(out[:rows, :a], x, w[:, :a])
+    bounded(res[:, :b], x, w[:, a:], keep[:, :b].double())
+    assert (out[rows] == 7).all() and (out[:, a:] == 7).all() and torch.equal(res[:, b:], keep[:, b:])
+
+
+@pytest.mark.parametrize("splits", [1, 2, 4, 8])
+@pytest.mark.parametrize("rows,K", [(3, 2048), (16, 1000), (70, 1040), (64, 64)])
+def test_ranges_of_input_features(pkg, rows, K, splits):
+    """Any number of ranges, also more than there are steps."""
+    from llm_experiments_b200 import _native
+    from llm_experiments_b200 import projection as proj
+
+    ctx = make_ctx(pkg)
+    x, w, bias = rnd((rows, K), F32, 4), rnd((K, 132), F32, 5, K ** -0.5), rnd((132,), F32, 6)
+    out = torch.empty((rows, 132), dtype=F32, device="cuda")
+    _native.tune("matmul_splits", splits)
+    try:
+        run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), K, [proj.OutputSegment(132, proj.SEG_STORE, wrap(pkg, out))],
+            bias=pkg.gpu.GPUBuffer1D(buffer=bias, shape=(132,), size=132))
+    finally:
+        _native.tune("matmul_splits", 0)
+    bounded(out, x, w, bias.double())
+
+
+@pytest.mark.parametrize("rows", [6, 90])
+@pytest.mark.parametrize("kind", ["SEG_GLU_SILU", "SEG_GLU_CLAMP", "SEG_RELU2", "SEG_SOFTCAP", "SEG_DECAY"])
+def test_kinds(pkg, rows, kind):
+    from llm_experiments_b200 import projection as proj
+
+    ctx, code, K, n, limit = make_ctx(pkg), getattr(proj, kind), 256, 136, 1.5
+    x, w = rnd((rows, K), F32, 7), rnd((K, n), F32, 8, 2 * K ** -0.5)
+    prod = x.double() @ w.double()
+    pair = kind.startswith("SEG_GLU")
+    want = glu(code, prod[:, ::2], prod[:, 1::2], limit, proj) if pair else dict(
+        SEG_RELU2=prod.clamp(min=0) ** 2, SEG_SOFTCAP=limit * torch.tanh(prod / limit),
+        SEG_DECAY=torch.exp(torch.nn.functional.logsigmoid(prod) / limit))[kind]
+    out = torch.full((rows + 1, want.shape[1] + 1), 7.0, dtype=F32, device="cuda")
+    run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), K, [proj.OutputSegment(n, code, wrap(pkg, out[:, :-1]))], limit=limit)
+    close(out[:rows, :-1], want, F32)
+    assert (out[rows] == 7).all() and (out[:, -1] == 7).all()
+
+
+@pytest.mark.parametrize("counts", [(3, 0, 16, 1), (0, 130, 64, 1, 0)])
+def test_rows_of_experts(pkg, counts):
+    from llm_experiments_b200 import projection as proj
+
+    ctx, K, n = make_ctx(pkg), 132, 140
+    offs = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    x, w = rnd((sum(counts), K), F32, 9), rnd((len(counts) * K, n), F32, 10, K ** -0.5)
+    out = torch.empty((sum(counts), n), dtype=F32, device="cuda")
+    run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), K, [proj.OutputSegment(n, proj.SEG_STORE, wrap(pkg, out))], groups=len(counts),
+        group_w=K * n, group_rows=torch.from_numpy(offs).cuda(), max_group_rows=max(counts))
+    for e in range(len(counts)):
+        bounded(out[offs[e]:offs[e + 1]], x[offs[e]:offs[e + 1]], w[e * K:(e + 1) * K])
+
+
+@pytest.mark.parametrize("rows", [2, 40])
+def test_heads(pkg, rows):
+    from llm_experiments_b200 import projection as proj
+
+    ctx, heads, k, n = make_ctx(pkg), 3, 20, 132
+    x, w = rnd((rows, heads * k), F32, 11), rnd((heads * k, n), F32, 12, k ** -0.5)
+    out = torch.empty((rows, heads * n), dtype=F32, device="cuda")
+    run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), k, [proj.OutputSegment(n, proj.SEG_STORE, wrap(pkg, out), group=n)], groups=heads,
+        group_x=k, group_w=k * n)
+    for h in range(heads):
+        bounded(out[:, h * n:(h + 1) * n], x[:, h * k:(h + 1) * k], w[h * k:(h + 1) * k])
