@@ -167,6 +167,10 @@ extern "C" int b2kv_gla(const b2kv_gla_args* args, int32_t* dev_status, void* st
         const int rc = gla_chunked(a, dev_status, stream);
         if (rc != B2KV_ERR_UNSUPPORTED || a.path == 2) return rc;
     }
+    if (a.path == 0 && a.max_n > 1) {  // (a single token reads and writes its state once either way)
+        const int rc = gla_run_f32(a, dev_status, stream);
+        if (rc != B2KV_ERR_UNSUPPORTED) return rc;
+    }
     return a.dtype == B2KV_DTYPE_F32 ? gla::launch_step<float>(a, dev_status, stream)
                                      : gla::launch_step<__nv_bfloat16>(a, dev_status, stream);
 }

@@ -11,6 +11,9 @@ namespace b2kv {
 int gla_chunked(const b2kv_gla_args& a, int32_t* dev_status, void* stream);
 size_t gla_chunked_workspace(int H, int dim, int vdim, int n_segments, int max_n, int dtype);  // 0: no such form
 
+// fp32 runs with the state in registers; B2KV_ERR_UNSUPPORTED where rows are not made of 16-byte pieces.
+int gla_run_f32(const b2kv_gla_args& a, int32_t* dev_status, void* stream);  // gla_run.cu
+
 namespace gla {
 
 __device__ __forceinline__ float silu(float g) { return g / (1.0f + expf(-g)); }

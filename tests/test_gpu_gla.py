@@ -109,6 +109,22 @@ def test_whole_sequences(pkg, path, dtype, heads, dim, vdim, n):
     assert torch.isnan(state[0]).all()
 
 
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 4, 4), (3, 12, 36), (1, 32, 32), (2, 36, 20), (2, 64, 128), (1, 128, 68)])
+@pytest.mark.parametrize("lens", [(2,), (7, 1, 8), (9, 17, 33), (100, 24, 25)])
+def test_fp32_runs_with_the_state_in_registers(pkg, heads, dim, vdim, lens):
+    """Lengths around the eight tokens of a step and the ring of three, several runs at a time, continued once."""
+    layer = Layer(pkg, heads, dim, vdim, 4.0, F32, seed=sum(lens))
+    state, pos = layer.states(len(lens)), np.concatenate([np.arange(n) for n in lens])
+    segments, rows, last = [(sum(lens[:i]), n, len(lens) - 1 - i) for i, n in enumerate(lens)], sum(lens), {}
+    for again in (0, 1):
+        y, al = layer.rows(rows)
+        got = layer.run(y, al, segments, pos + again * np.repeat(lens, lens), state, 0)
+        for r0, n, slot in segments:
+            want, last[slot] = layer.want(y[r0:r0 + n], al[r0:r0 + n], last.get(slot))
+            close(got[r0:r0 + n], want, F32, (r0, n, again))
+            state_close(state[slot], last[slot])
+
+
 @pytest.mark.parametrize("path,dtype,heads,dim,vdim", [(STEP, F32, 3, 5, 7), (CHUNK, BF, 5, 56, 40), (0, BF, 2, 128, 128), (0, BF, 2, 64, 64)])
 def test_portions_carry_the_state(pkg, path, dtype, heads, dim, vdim):
     """Any cut gives the outputs of the whole, with two sequences in unequal portions per call and the rows of a call in any
