@@ -8,18 +8,21 @@
 //
 //     a * b  ~  a_hi * b_hi + a_hi * b_lo + a_lo * b_hi        (the dropped a_lo * b_lo is below 2^-16 relative)
 //
-//   * a first kernel writes the hi and lo halves of Q, K and V into a scratch buffer ([B*N, H*D] bfloat16 each);
-//   * one CTA per (sequence, head, 128 query rows).  Warp 4 loads the Q tile and, step by step, a 128-key K tile
-//     and V tile (hi and lo: 64 KB each at head_dim 128, so the rings hold one step) with TMA tiled loads into
-//     128-byte-swizzled shared memory; warp 5 issues S = Q K^T (3 x head_dim/16 tcgen05.mma, both operands in
+//   * a first kernel writes the hi and lo halves of Q, K and V into a scratch buffer ([B*N, H*D] bfloat16 each) and, when the
+//     prompt goes to a contiguous cache, the K / V rows to their places there: they pass through its registers anyway (B = 2,
+//     N = 1000, H = 12, D = 64: three launches of it and the copy kernel behind the attention were 20 of 53 us);
+//   * one CTA per (sequence, head, 128 query rows), two CTAs per SM at head_dim 64.  Warp 8 loads the Q tile and, step by step, a
+//     128-key K tile and V tile (hi and lo: 64 KB each at head_dim 128, so the rings hold one step) with TMA tiled loads into
+//     128-byte-swizzled shared memory; warp 9 issues S = Q K^T (3 x head_dim/16 tcgen05.mma, both operands in
 //     shared memory) and O += P V (3 x 8, P read from tensor memory, V an MN-major shared-memory operand);
-//   * warps 0 - 3: thread = query row = TMEM lane.  Scores in registers, running maximum and sum in the log2
-//     domain in fp32, O rescaled only when the maximum has grown by more than 2^8, P written back as hi and lo
-//     halves (packed bfloat16) over the score buffer: hi in columns 0 - 63, lo in columns 64 - 127;
+//   * warps 0 - 7: two threads per query row = TMEM lane, one for each half of a step's keys.  QK^T, softmax and PV of the one
+//     query tile follow one another, and only another CTA fills the gaps: with half a row per thread two CTAs fit the registers
+//     (B = 8, N = 2048, H = 12, D = 64: 443 us with four warps and one CTA per SM, 250 so; N = 4096, H = 8, B = 4: 408 and 286;
+//     one CTA per SM at D = 128, B = 2, N = 4096, H = 16: 506 and 454).  Scores in registers, the row's maximum exchanged through shared memory, running maximum
+//     and sum in the log2 domain in fp32, O rescaled only when the maximum has grown by more than 2^8, P written back as hi and
+//     lo halves (packed bfloat16) over the score buffer: hi in columns 0 - 63, lo in columns 64 - 127;
 //   * epilogue O / max(l, 1e-8) as fp32, L and M as the reference writes them (:762-768).
 //
-// The K / V rows of the prompt reach a cache (fp32 like the prompt) through the copy kernel of append.cu behind the
-// attention: the tiles in shared memory are bfloat16 halves, not the rows themselves.
 // Tensor memory: S / P columns 0 - 127, O columns 128 - 255.  Every mbarrier wait is bounded.
 #include <math.h>
 
@@ -38,7 +41,8 @@ using namespace tc;
 constexpr int kTileM = 128;
 constexpr int kBlockN = 128;
 constexpr int kHalfTileBytes = 128 * 128;  // 128 rows x 64 bf16
-constexpr int kThreads = 192;              // 4 softmax warps, copy warp, MMA warp
+constexpr int kSoftmaxWarps = 8, kCopyWarp = 8, kMmaWarp = 9;
+constexpr int kThreads = 320;
 constexpr int kTmemCols = 256;
 constexpr int kColS = 0, kColO = 128;
 constexpr float kRescaleThreshold = 8.0f;
@@ -50,29 +54,43 @@ struct SharedStorage {
     alignas(1024) uint8_t k[2][kTileBytes];
     alignas(1024) uint8_t v[2][kTileBytes];
     alignas(8) uint64_t q_full, k_full, k_empty, v_full, v_empty, s_full, p_ready, o_done;
+    float exchange[2][2][kTileM];  // [parity of the step][half of the keys][row]: maxima; sums at the end
     uint32_t tmem_base;
     volatile int abort_flag;
 };
 
-// x -> (bf16(x), bf16(x - bf16(x))), four elements per thread.
-__global__ void __launch_bounds__(256) split_kernel(const float4* __restrict__ x, uint2* __restrict__ hi, uint2* __restrict__ lo,
-                                                    int64_t n4) {
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n4) return;
-    const float4 a = x[i];
-    const __nv_bfloat16 h0 = __float2bfloat16_rn(a.x), h1 = __float2bfloat16_rn(a.y), h2 = __float2bfloat16_rn(a.z),
-                        h3 = __float2bfloat16_rn(a.w);
-    uint2 ph, pl;
-    ph.x = pack_bf16(__bfloat162float(h0), __bfloat162float(h1));
-    ph.y = pack_bf16(__bfloat162float(h2), __bfloat162float(h3));
-    pl.x = pack_bf16(a.x - __bfloat162float(h0), a.y - __bfloat162float(h1));
-    pl.y = pack_bf16(a.z - __bfloat162float(h2), a.w - __bfloat162float(h3));
-    hi[i] = ph;
-    lo[i] = pl;
+// x -> (bf16(x), bf16(x - bf16(x))) of one row of Q, K or V (grid: rows, 3), and of K and V a copy in the cache.
+struct SplitArgs {
+    const float* src[3];
+    __nv_bfloat16 *hi[3], *lo[3];
+    float* cache[3];  // null: none
+    int64_t stride_b, stride_t, stride_h;
+    int N, E, D;
+};
+__global__ void __launch_bounds__(256) split_kernel(const __grid_constant__ SplitArgs a) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int which = blockIdx.y;
+    const int64_t row = blockIdx.x;
+    const float4* const x = reinterpret_cast<const float4*>(a.src[which] + row * a.E);
+    uint2* const hi = reinterpret_cast<uint2*>(a.hi[which] + row * a.E);
+    uint2* const lo = reinterpret_cast<uint2*>(a.lo[which] + row * a.E);
+    float* const cache = a.cache[which] == nullptr ? nullptr : a.cache[which] + row / a.N * a.stride_b + row % a.N * a.stride_t;
+    for (int i = threadIdx.x; i < a.E / 4; i += blockDim.x) {
+        const float4 v = x[i];
+        const uint32_t h0 = pack_bf16(v.x, v.y), h1 = pack_bf16(v.z, v.w);
+        hi[i] = make_uint2(h0, h1);
+        lo[i] = make_uint2(pack_bf16(v.x - __uint_as_float(h0 << 16), v.y - __uint_as_float(h0 & 0xffff0000u)),
+                           pack_bf16(v.z - __uint_as_float(h1 << 16), v.w - __uint_as_float(h1 & 0xffff0000u)));
+        if (cache != nullptr) {
+            const int h = i * 4 / a.D, d = i * 4 - h * a.D;
+            *reinterpret_cast<float4*>(cache + h * a.stride_h + d) = v;
+        }
+    }
 }
 
 template <int kD>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads, kD == 64 ? 2 : 1)
 prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_constant__ CUtensorMap tm_ql,
                       const __grid_constant__ CUtensorMap tm_kh, const __grid_constant__ CUtensorMap tm_kl,
                       const __grid_constant__ CUtensorMap tm_vh, const __grid_constant__ CUtensorMap tm_vl,
@@ -108,12 +126,12 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
         mbar_init(&sm.v_full, 1);
         mbar_init(&sm.v_empty, 1);
         mbar_init(&sm.s_full, 1);
-        mbar_init(&sm.p_ready, 4);
+        mbar_init(&sm.p_ready, kSoftmaxWarps);
         mbar_init(&sm.o_done, 1);
         sm.abort_flag = 0;
         fence_mbar_init();
     }
-    if (warp == 5) {
+    if (warp == kMmaWarp) {
         tmem_alloc(&sm.tmem_base, kTmemCols);
         tmem_relinquish();
     }
@@ -122,10 +140,11 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
     tc_fence_after();
     const uint32_t tmem = sm.tmem_base;
 
-    if (warp == 4) {
+    if (warp == kCopyWarp) {
         // ------------------------------ TMA producer ------------------------------
         if (lane == 0) {
             const int x0 = h * kD;
+            grid_dependency_wait();  // the halves are the kernel before this one's; all else here follows from them
             mbar_arrive_expect_tx(&sm.q_full, 2 * kTileBytes);
 #pragma unroll
             for (int hf = 0; hf < kHalves; ++hf) {
@@ -155,7 +174,7 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
             if (!ok) sm.abort_flag = 1;
         }
         __syncwarp();
-    } else if (warp == 5) {
+    } else if (warp == kMmaWarp) {
         // ------------------------------ MMA issuer ------------------------------
         if (lane == 0) {
             constexpr uint32_t idesc_qk = instr_desc(0, 0, kBlockN);  // S[128 x 128 keys]
@@ -216,33 +235,40 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
         }
         __syncwarp();
     } else {
-        // ------------------------------ softmax: thread = query row ------------------------------
-        const int row = threadIdx.x;  // row inside the tile, also the TMEM lane
-        const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
+        // ------------------------------ softmax: two threads per query row ------------------------------
+        const int row = threadIdx.x & (kTileM - 1), half = warp >> 2;  // row inside the tile = TMEM lane; half of the keys
+        const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const uint32_t s_tmem = tmem + lane_base + kColS;
-        const uint32_t o_tmem = tmem + lane_base + kColO;
+        const uint32_t o_tmem = tmem + lane_base + kColO + half * (kD / 2);
         const float c = p.q_prescale;  // log2(e) / sqrt(D)
         float m_used = -INFINITY, m_run = -INFINITY, l = 0.f;
-        bool ok = true;
-        for (int j = 0; j < n && ok; ++j) {
-            ok = mbar_wait(&sm.s_full, j & 1);
-            if (!ok) break;
+        bool ok = true;  // (a thread whose wait ran out goes on without waiting: its partners wait for it at the named barrier)
+        for (int j = 0; j < n; ++j) {
+            ok = ok && mbar_wait(&sm.s_full, j & 1);
+            __syncwarp();
             tc_fence_after();
-            uint32_t r[128];
-            tmem_ld128(s_tmem, r);
+            uint32_t r[64];
+            tmem_ld32(s_tmem + half * 64, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+            tmem_ld32(s_tmem + half * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
             tmem_wait_ld();
             if (j == rb) {
 #pragma unroll
-                for (int i = 0; i < 128; ++i)
-                    if (i > row) r[i] = 0xff800000u;  // -inf: key after the query
+                for (int i = 0; i < 64; ++i)
+                    if (half * 64 + i > row) r[i] = 0xff800000u;  // -inf: key after the query
             }
-            float mxs[8];
+            float mxs[4];
 #pragma unroll
-            for (int a = 0; a < 8; ++a) mxs[a] = __uint_as_float(r[a]);
+            for (int a = 0; a < 4; ++a) mxs[a] = __uint_as_float(r[a]);
 #pragma unroll
-            for (int i = 8; i < 128; ++i) mxs[i & 7] = fmaxf(mxs[i & 7], __uint_as_float(r[i]));
-            const float mx = fmaxf(fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])),
-                                   fmaxf(fmaxf(mxs[4], mxs[5]), fmaxf(mxs[6], mxs[7])));
+            for (int i = 4; i < 64; ++i) mxs[i & 3] = fmaxf(mxs[i & 3], __uint_as_float(r[i]));
+            float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3]));
+            sm.exchange[j & 1][half][row] = mx;
+            // the four warps of the row's quarter pair up: both halves' scores are in registers behind this barrier as well,
+            // so that either may write over the score columns
+            tc_fence_before();
+            named_barrier_sync<64>(1 + (warp & 3));
+            tc_fence_after();
+            mx = fmaxf(mx, sm.exchange[j & 1][half ^ 1][row]);
             m_run = fmaxf(m_run, mx * c);
             float factor = 1.f;
             bool need = false;
@@ -254,41 +280,38 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
                 need = true;
             }
             // P = exp2(s*c - m_used) in fp32, written as hi + lo: packed hi pairs over columns 0 - 63 of the score
-            // buffer, packed lo pairs over columns 64 - 127 (every score is in registers by now)
-            float sums[8];
-#pragma unroll
-            for (int a = 0; a < 8; ++a) sums[a] = 0.f;
+            // buffer, packed lo pairs over columns 64 - 127
+            float sums[4] = {0.f, 0.f, 0.f, 0.f};
             const float neg_m = -m_used;
 #pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {
+            for (int cc = 0; cc < 2; ++cc) {
                 uint32_t ph[16], pl[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const float p0 = ex2(fmaf(__uint_as_float(r[cc * 32 + 2 * i]), c, neg_m));
                     const float p1 = ex2(fmaf(__uint_as_float(r[cc * 32 + 2 * i + 1]), c, neg_m));
-                    sums[(2 * i) & 7] += p0;
-                    sums[(2 * i + 1) & 7] += p1;
+                    sums[(2 * i) & 3] += p0;
+                    sums[(2 * i + 1) & 3] += p1;
                     const uint32_t hi = pack_bf16(p0, p1);
                     ph[i] = hi;
                     pl[i] = pack_bf16(p0 - __uint_as_float(hi << 16), p1 - __uint_as_float(hi & 0xffff0000u));
                 }
-                tmem_st16(s_tmem + cc * 16, ph);
-                tmem_st16(s_tmem + 64 + cc * 16, pl);
+                tmem_st16(s_tmem + half * 32 + cc * 16, ph);
+                tmem_st16(s_tmem + 64 + half * 32 + cc * 16, pl);
             }
-            l = l * factor + (((sums[0] + sums[1]) + (sums[2] + sums[3])) + ((sums[4] + sums[5]) + (sums[6] + sums[7])));
+            l = l * factor + ((sums[0] + sums[1]) + (sums[2] + sums[3]));
             if (__any_sync(0xffffffffu, need)) {
-                ok = mbar_wait(&sm.o_done, (j - 1) & 1);
-                if (ok) {
-                    tc_fence_after();
+                ok = ok && mbar_wait(&sm.o_done, (j - 1) & 1);
+                __syncwarp();
+                tc_fence_after();
 #pragma unroll 1
-                    for (int cc = 0; cc < kD / 32; ++cc) {
-                        uint32_t o[32];
-                        tmem_ld32(o_tmem + cc * 32, o);
-                        tmem_wait_ld();
+                for (int cc = 0; cc < kD / 32; ++cc) {
+                    uint32_t o[16];
+                    tmem_ld16(o_tmem + cc * 16, o);
+                    tmem_wait_ld();
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
-                        tmem_st32(o_tmem + cc * 32, o);
-                    }
+                    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
+                    tmem_st16(o_tmem + cc * 16, o);
                 }
             }
             tmem_wait_st();
@@ -296,16 +319,20 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.p_ready);
         }
+        sm.exchange[n & 1][half][row] = l;
         // every PV is waited for in order here or by nobody, so the parity names the last one
-        if (ok) ok = mbar_wait(&sm.o_done, (n - 1) & 1);
-        if (ok) {
+        ok = ok && mbar_wait(&sm.o_done, (n - 1) & 1);
+        named_barrier_sync<64>(1 + (warp & 3));
+        l += sm.exchange[n & 1][half ^ 1][row];
+        if (__all_sync(0xffffffffu, ok)) {
             tc_fence_after();
             const int grow = q0 + row;
             const float inv = 1.f / fmaxf(l, 1e-8f);
             const int E = p.H * kD;
-            float* Og = static_cast<float*>(p.O) + (static_cast<size_t>(b) * p.N + grow) * E + static_cast<size_t>(h) * kD;
+            float* Og = static_cast<float*>(p.O) + (static_cast<size_t>(b) * p.N + grow) * E + static_cast<size_t>(h) * kD +
+                        half * (kD / 2);
 #pragma unroll 1
-            for (int cc = 0; cc < kD / 32; ++cc) {
+            for (int cc = 0; cc < kD / 64; ++cc) {
                 uint32_t o[32];
                 tmem_ld32(o_tmem + cc * 32, o);
                 tmem_wait_ld();
@@ -320,8 +347,9 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
                         *reinterpret_cast<float4*>(Og + cc * 32 + v4 * 4) = w;
                     }
                 }
+                __syncwarp();
             }
-            if (grow < p.N) {
+            if (grow < p.N && half == 0) {
                 const size_t sidx = (static_cast<size_t>(b) * p.N + grow) * p.H + h;
                 if (p.L) p.L[sidx] = l * ex2(m_used - m_run);
                 if (p.M) p.M[sidx] = m_run * 0.6931471805599453f;
@@ -334,7 +362,7 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
     // common exit: every warp arrives here, then the allocating warp releases the tensor memory
     tc_fence_before();
     __syncthreads();
-    if (warp == 5) {
+    if (warp == kMmaWarp) {
         tc_fence_after();
         tmem_dealloc(tmem, kTmemCols);
     }
@@ -378,15 +406,18 @@ static int launch_prefill_tc_f32(const PrefillParams& p_in, void* scratch, void*
     CUtensorMap tm[6];
     for (int i = 0; i < 6; ++i)
         if (!tcf::make_map(&tm[i], half[i], p.B, p.N, E)) return B2KV_ERR_UNSUPPORTED;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const long long rows = static_cast<long long>(p.B) * p.N;
+    if (rows > 0x7fffffffLL) return B2KV_ERR_UNSUPPORTED;
+    tcf::SplitArgs split{};
     const void* src[3] = {p.Q, p.K, p.V};
-    const int64_t n4 = static_cast<int64_t>(elems / 4);
+    void* cache[3] = {nullptr, p.k_cache, p.v_cache};
     for (int i = 0; i < 3; ++i) {
-        tcf::split_kernel<<<static_cast<unsigned>((n4 + 255) / 256), 256, 0, s>>>(
-            static_cast<const float4*>(src[i]), reinterpret_cast<uint2*>(half[2 * i]), reinterpret_cast<uint2*>(half[2 * i + 1]),
-            n4);
-        B2KV_CUDA_TRY(cudaGetLastError());
+        split.src[i] = static_cast<const float*>(src[i]);
+        split.hi[i] = half[2 * i], split.lo[i] = half[2 * i + 1];
+        split.cache[i] = static_cast<float*>(cache[i]);
     }
+    split.stride_b = p.stride_b, split.stride_t = p.stride_t, split.stride_h = p.stride_h;
+    split.N = p.N, split.E = E, split.D = kD;
     constexpr size_t smem = sizeof(tcf::SharedStorage<kD>) + 1024;
     auto kernel = tcf::prefill_tc_f32_kernel<kD>;
     static bool configured[64] = {false};
@@ -397,8 +428,10 @@ static int launch_prefill_tc_f32(const PrefillParams& p_in, void* scratch, void*
         B2KV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
         configured[dev] = true;
     }
-    kernel<<<static_cast<unsigned>(ctas), tcf::kThreads, smem, s>>>(tm[0], tm[1], tm[2], tm[3], tm[4], tm[5], p);
-    B2KV_CUDA_TRY(cudaGetLastError());
+    OverlapLaunch first(dim3(static_cast<unsigned>(rows), 3), std::min(256, (E / 4 + 31) / 32 * 32), 0, stream);
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&first.cfg, tcf::split_kernel, split));
+    OverlapLaunch launch(static_cast<unsigned>(ctas), tcf::kThreads, smem, stream);
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, kernel, tm[0], tm[1], tm[2], tm[3], tm[4], tm[5], p));
     return B2KV_OK;
 }
 
