@@ -4,7 +4,8 @@
 // written once per run instead of once per token.  A lane owns two value columns and every eighth group of four key channels; the
 // decays, keys and queries of eight tokens at a time come through a ring in shared memory, ahead of their use.  What bounds it is
 // the issue of three multiply-adds per element of the state; gla_step_kernel, one CTA per head with the state streamed through L2
-// for every token, took 939 us for runs of up to 400 tokens (6 heads, 64 x 128), this one 100.
+// for every token, took 939 us for runs of up to 400 tokens (6 heads, 64 x 128), this one 80 (100 with
+// the tokens one after the other: eight at a time, their sums over the lanes run side by side).
 // o goes to the output rows as it is (they are fp32); gla_norm_kernel applies the head's norm and the gate there.
 #include "gla.cuh"
 
@@ -79,29 +80,51 @@ __global__ void __launch_bounds__(32 * kWarps) gla_run_kernel(const __grid_const
         request(step + kRing - 1);
         const Stage& st = ring[step % kRing];
         const int n = min(kTok, sg.n - step * kTok);
-#pragma unroll 4
-        for (int t = 0; t < kTok; ++t) {
-            if (t >= n) break;
+        // one token: the state moves on; this lane's part of o
+        auto token = [&](int t) {
             const float2 v = reinterpret_cast<const float2*>(st.v[t])[warp * 4 + (lane & 3)];
-            float2 o = make_float2(0.f, 0.f);
+            float2 o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] = make_float2(0.f, 0.f);
 #pragma unroll
             for (int j = 0; j < kGroups; ++j) {
                 const float4 al = st.alpha[t][j * 8 + dg], kk = st.k[t][j * 8 + dg], qq = st.q[t][j * 8 + dg];
                 const float av[4] = {al.x, al.y, al.z, al.w}, kv[4] = {kk.x, kk.y, kk.z, kk.w}, qv[4] = {qq.x, qq.y, qq.z, qq.w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const float2 sc = s[j][e];
-                    s[j][e] = __ffma2_rn(sc, make_float2(av[e], av[e]), __fmul2_rn(make_float2(kv[e], kv[e]), v));
+                    s[j][e] = __ffma2_rn(s[j][e], make_float2(av[e], av[e]), __fmul2_rn(make_float2(kv[e], kv[e]), v));
                     const float q = qv[e] * a.q_scale;
-                    o = __ffma2_rn(make_float2(q, q), s[j][e], o);
+                    o[e] = __ffma2_rn(make_float2(q, q), s[j][e], o[e]);
                 }
             }
+            return __fadd2_rn(__fadd2_rn(o[0], o[1]), __fadd2_rn(o[2], o[3]));
+        };
+        auto other = [](float2 x, int off) {
+            return make_float2(__shfl_xor_sync(0xffffffffu, x.x, off), __shfl_xor_sync(0xffffffffu, x.y, off));
+        };
+        if (n == kTok) {
+            // The tokens' parts of o are summed over the eight lanes that share the key channels by halving: a lane hands on what
+            // the other half of the lanes sums up, and is left with one token (lane bits 4, 3, 2 = token bits 2, 1, 0).
+            float2 o[kTok];
 #pragma unroll
-            for (int off = 4; off < 32; off <<= 1) {
-                o.x += __shfl_xor_sync(0xffffffffu, o.x, off);
-                o.y += __shfl_xor_sync(0xffffffffu, o.y, off);
+            for (int t = 0; t < kTok; ++t) o[t] = token(t);
+#pragma unroll
+            for (int half = kTok / 2; half > 0; half >>= 1) {
+                const bool up = lane & (half * 4);
+#pragma unroll
+                for (int t = 0; t < half; ++t) {
+                    const float2 mine = up ? o[t + half] : o[t], theirs = up ? o[t] : o[t + half];
+                    o[t] = __fadd2_rn(mine, other(theirs, half * 4));
+                }
             }
-            if (dg == 0 && live) *reinterpret_cast<float2*>(out + static_cast<int64_t>(step * kTok + t) * a.ld_out) = o;
+            if (live) *reinterpret_cast<float2*>(out + static_cast<int64_t>(step * kTok + dg) * a.ld_out) = o[0];
+        } else {
+            for (int t = 0; t < n; ++t) {
+                float2 o = token(t);
+#pragma unroll
+                for (int off = 4; off < 32; off <<= 1) o = __fadd2_rn(o, other(o, off));
+                if (dg == 0 && live) *reinterpret_cast<float2*>(out + static_cast<int64_t>(step * kTok + t) * a.ld_out) = o;
+            }
         }
     }
     if (!live) return;
