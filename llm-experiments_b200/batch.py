@@ -32,15 +32,23 @@ def validate_buffer_shape_2d(buffer: GPUBuffer2D, expected_shape: Tuple[int, int
         raise ValueError(f"{name} shape mismatch: got {buffer.shape}, expected {expected_shape}")
 
 
+def _current_handle(device: torch.device) -> int:
+    """The raw handle of torch's current stream.  (A stream object for it costs 2 us, three times per step of a decoding loop
+    whose kernels take less than ten.)"""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
+
+
 def batch_begin(ctx: GPUContext, enable_profiling: bool = False) -> None:
     """Opens a batch on torch's current stream (reference: gpu_ops.py:226-250).  With
     ``enable_profiling`` every operation of the batch is wrapped in an NVTX range named after the
     reference function and bracketed by CUDA events; ``batch_commit`` then synchronises and adds
     the durations to ``ctx.perf_monitor`` (the reference stores the flag, gpu_ops.py:245-250, and
     leaves the recording to the caller, gpu_device.py:569-608)."""
-    stream = torch.cuda.current_stream(ctx.device)
+    stream, handle = ctx.stream, _current_handle(ctx.device)
+    if stream is None or stream.cuda_stream != handle:
+        stream = ctx.stream = torch.cuda.current_stream(ctx.device)
     ctx.batch_state = BatchState(encoder=stream, retained_buffers=[], enable_profiling=enable_profiling,
-                                 operation_count=0)
+                                 operation_count=0, stream_handle=handle)
 
 
 def batch_op_begin(ctx: GPUContext) -> int:
@@ -53,11 +61,11 @@ def batch_op_begin(ctx: GPUContext) -> int:
         raise RuntimeError(f"Batch operation limit ({max_ops}) exceeded. Call batch_commit() to flush operations.")
     # The kernels go to the batch's stream; the few torch operations beside them (length counters) go to
     # torch's current stream.  They are ordered only when the two are the same stream.
-    if torch.cuda.current_stream(ctx.device) != state.encoder:
+    if _current_handle(ctx.device) != state.stream_handle:
         raise RuntimeError("The current CUDA stream changed since batch_begin; commit the batch and begin a new one "
                            "on the new stream")
     state.operation_count += 1
-    return state.encoder.cuda_stream
+    return state.stream_handle
 
 
 def reference_op(name: str):

@@ -132,7 +132,8 @@ def state_set_lengths(state: SequenceState, lens: Sequence[int]) -> None:
     if len(lens) != state.batch_size or min(lens) < 0 or max(lens) > state.max_seq_len:
         raise ValueError(f"lengths must be {state.batch_size} values in [0, {state.max_seq_len}]")
     state.lengths = [int(v) for v in lens]
-    state.seq_lens.copy_(torch.tensor(state.lengths, dtype=torch.int32), non_blocking=False)
+    # in stream order, like the steps themselves: waiting for it here would wait for every step still running
+    state.seq_lens.copy_(torch.tensor(state.lengths, dtype=torch.int32), non_blocking=True)
     state._sync_upper_bound()
 
 

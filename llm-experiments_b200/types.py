@@ -75,6 +75,7 @@ class BatchState:
     retained_buffers: List[Any] = field(default_factory=list)
     enable_profiling: bool = False
     operation_count: int = 0
+    stream_handle: Optional[int] = None  # of the encoder
 
 
 @dataclass
@@ -117,6 +118,7 @@ class GPUContext:
     perf_monitor: Optional[PerfMonitor] = None  # filled by batches opened with enable_profiling
     prefill_workspace: Optional[torch.Tensor] = None  # scratch of flash_attention for fp32 prompts, grown on demand
     recurrent_workspace: Optional[torch.Tensor] = None  # scratch of recurrent layers over prompt portions, grown on demand
+    stream: Optional[Any] = None  # the stream of the last batch, taken again while it is the current one
 
 
 @dataclass
