@@ -57,7 +57,7 @@ struct GemmParams {
     __nv_bfloat16* out;             // [M, N]
     int M, N, K;
     int gelu;
-    int tiles_m, tiles_n;
+    int tiles_m, tiles_n, tile_cols;
     int32_t* dev_status;  // optional status word: receives B2KV_DEV_WAIT_TIMEOUT when a bounded wait ran out
 };
 
@@ -66,7 +66,7 @@ constexpr int kMaxGroups = 1024;
 struct SegParams {
     b2kv_linear_args a;
     int M, N, K;
-    int tiles_m, tiles_n;
+    int tiles_m, tiles_n, tile_cols;
     int32_t* dev_status;
 };
 
@@ -75,14 +75,18 @@ struct Tile {
     int row0, row_end, tn, k_row0;
 };
 
-// First row tile of every group (and behind the last one), for tiles of tile_rows rows; in shared memory, empty for
-// parameters without groups.
+// First row tile of every group (and behind the last one), for tiles of tile_rows rows, and the epilogue warps' pieces of fp32 outputs;
+// in shared memory, empty for parameters without segments.
+constexpr int kSlabLd = 36;  // words per row of a warp's 32 x 32 piece: no bank conflicts by 16-byte pieces, written or read
 template <typename P>
 struct GroupTable {};
 template <>
 struct GroupTable<SegParams> {
+    alignas(16) uint32_t slab[4 * 32 * kSlabLd];
     int first[kMaxGroups + 1];
 };
+__device__ __forceinline__ uint32_t* slab_of(GroupTable<SegParams>& table, int quarter) { return table.slab + quarter * (32 * kSlabLd); }
+__device__ __forceinline__ uint32_t* slab_of(GroupTable<GemmParams>&, int) { return nullptr; }
 
 struct SharedStorage {
     alignas(1024) uint8_t stage[kStages][kStageBytes];
@@ -163,8 +167,8 @@ __device__ __forceinline__ Tile find_tile(int t, const SegParams& p, const Group
     return {p.a.group_rows[lo] + within % rows_here * tile_rows, p.a.group_rows[lo + 1], within / rows_here, lo * p.K};
 }
 
-__device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_addr, int grow, int row_end, int col_base);
-__device__ __forceinline__ void epilogue_rows(const SegParams& p, uint32_t t_addr, int grow, int row_end, int col_base);
+__device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_addr, int grow, int row_end, int col_base, uint32_t* slab);
+__device__ __forceinline__ void epilogue_rows(const SegParams& p, uint32_t t_addr, int grow, int row_end, int col_base, uint32_t* slab);
 
 template <typename P>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -174,7 +178,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     extern __shared__ uint8_t smem_raw[];
     SharedStorage& sm = *reinterpret_cast<SharedStorage*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_tiles = setup_tiles(p, table, kBM);
     const int n_k = (p.K + kBK - 1) / kBK;
 
     if (threadIdx.x == 0) {
@@ -194,9 +197,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         tmem_relinquish();
     }
     tc_fence_before();
+    grid_dependency_wait();  // what comes before hides behind the kernel ahead
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sm.tmem_base;
+    const int n_tiles = setup_tiles(p, table, kBM), spans = (p.tile_cols + 63) / 64;
 
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
@@ -209,21 +214,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                     const int s = it % kStages;
                     ok = mbar_wait(&sm.empty[s], ((it / kStages) & 1) ^ 1);
                     if (!ok) break;
-                    mbar_arrive_expect_tx(&sm.full[s], kStageBytes);
+                    mbar_arrive_expect_tx(&sm.full[s], kABytes + spans * kWSpanBytes);
                     tma_load_2d(sm.stage[s], &tm_a, &sm.full[s], kb * kBK, tl.row0);
-#pragma unroll
-                    for (int sp = 0; sp < kBN / 64; ++sp)
-                        tma_load_2d(sm.stage[s] + kABytes + sp * kWSpanBytes, &tm_w, &sm.full[s], tl.tn * kBN + sp * 64,
+                    for (int sp = 0; sp < spans; ++sp)
+                        tma_load_2d(sm.stage[s] + kABytes + sp * kWSpanBytes, &tm_w, &sm.full[s], tl.tn * p.tile_cols + sp * 64,
                                     tl.k_row0 + kb * kBK);
                 }
             }
+            grid_launch_dependents();  // the next kernel sets up under the last products and outputs
             if (!ok) sm.abort_flag = 1;
         }
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
         if (lane == 0) {
-            constexpr uint32_t idesc = instr_desc(0, 1, kBN);  // A K-major, W MN-major, N = 256
+            const uint32_t idesc = instr_desc(0, 1, p.tile_cols);  // A K-major, W MN-major
             bool ok = true;
             uint32_t it = 0, local = 0;  // stages consumed; tiles done by this CTA
             for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++local) {
@@ -266,7 +271,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             ok = mbar_wait(&sm.acc_full[buf], (local >> 1) & 1);
             if (!ok) break;
             tc_fence_after();
-            epilogue_rows(p, tmem + lane_base + buf * kBN, tl.row0 + row, tl.row_end, tl.tn * kBN);
+            epilogue_rows(p, tmem + lane_base + buf * kBN, tl.row0 + row, tl.row_end, tl.tn * p.tile_cols, slab_of(table, quarter));
             // this warp has read its lanes of the accumulator: hand it back to the MMA issuer
             tc_fence_before();
             __syncwarp();
@@ -293,6 +298,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
 // the same again in TMA writes, which holds its tensor pipe at 80 %.  The copies of both CTAs complete on
 // the leader's barriers, one thread of the leader issues the MMAs and commits to the barriers of both CTAs,
 // and each CTA's epilogue warps drain their own 128 lanes of the accumulator.  No multicast load is used.
+// A tile has 256 columns, or fewer where that saves more of the last wave than it costs (tile_cols, chosen by launch): the copies
+// stay whole spans of 64 columns, the MMAs read what the tile has.
 // The ring holds 128 input features per stage in three stages by default (the issuing thread then waits,
 // fences and commits once per eight MMAs; 4 - 5 % faster than 64 features in six stages).
 // ---------------------------------------------------------------------------------------------------
@@ -372,10 +379,10 @@ __device__ __forceinline__ void mma_ss_pair(uint32_t d_tmem, uint64_t a_desc, ui
 
 // Epilogue of one accumulator for one warp: thread = output row `grow` (TMEM lane of `t_addr`; rows from row_end on are
 // not stored), columns [col_base, col_base + 256) clipped to N.
-__device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_addr, int grow, int row_end, int col_base) {
+__device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_addr, int grow, int row_end, int col_base, uint32_t*) {
     const size_t row_off = static_cast<size_t>(grow) * p.N;
 #pragma unroll 1
-    for (int c = 0; c < kBN / 32; ++c) {
+    for (int c = 0; c < p.tile_cols / 32; ++c) {
         const int col0 = col_base + c * 32;
         if (col0 >= p.N) break;  // the same for every thread of the CTA
         uint32_t acc[32];
@@ -422,90 +429,90 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_ad
     }
 }
 
-// The same for segments (32 columns never straddle a boundary).
-__device__ __forceinline__ void epilogue_rows(const SegParams& p, uint32_t t_addr, int grow, int row_end, int col_base) {
-    const bool live = grow < row_end;
+// The same for segments (32 columns never straddle a boundary).  fp32 outputs go through shared memory, so that the warp reads the
+// residual and writes the outputs as whole pieces of rows: with every lane on a row of its own a 16-byte access touches 32 lines
+// (2975 rows x 2048 columns with a residual, 2048 input features: 34 us, 29 so; without one 30 and 28).
+// What happens to a column is chosen outside the loops over columns, so that the columns' exponentials run side by side.
+__device__ __forceinline__ void epilogue_rows(const SegParams& p, uint32_t t_addr, int grow, int row_end, int col_base, uint32_t* slab) {
+    const int lane = threadIdx.x & 31, row0 = grow - lane, rows = min(32, row_end - row0);  // (not positive: nothing to store)
+    const auto f = [](uint32_t v) { return __uint_as_float(v); };
+    const auto u = [](float v) { return __float_as_uint(v); };
 #pragma unroll 1
-    for (int c = 0; c < kBN / 32; ++c) {
-        const int col0 = col_base + c * 32;
-        if (col0 >= p.N) break;
+    for (int c = 0; c < p.tile_cols / 32; ++c) {
+        const int col0 = col_base + c * 32, n_cols = min(32, p.N - col0);
+        if (n_cols <= 0 || rows <= 0) break;  // the same for the whole warp
         uint32_t acc[32];
-        __syncwarp();  // lanes past row_end skipped the stores of the columns before
+        __syncwarp();  // everybody has read the columns before
         tmem_ld32(t_addr + c * 32, acc);
         const int s = lin::segment_of(p.a, col0);
         const b2kv_segment& sg = p.a.seg[s];
-        const int local = col0 - lin::segment_first(p.a, s);
+        const int local = col0 - lin::segment_first(p.a, s), kind = sg.kind;
+        const bool f32 = lin::is_f32(kind);
+        // fp32: lane = four columns (lane & 7) of the rows lane >> 3, + 4, ..; the residual is on its way before the sums are here
+        const int c4 = (lane & 7) * 4, r4 = lane >> 3;
+        float4 add[8];
+        if (f32) {
+            const bool with = p.a.residual != nullptr && kind == B2KV_SEG_F32 && c4 < n_cols;
+            const float* const res = with ? p.a.residual + static_cast<int64_t>(row0 + r4) * p.a.ld_residual + local + c4 : nullptr;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                add[i] = with && r4 + 4 * i < rows ? *reinterpret_cast<const float4*>(res + 4 * i * p.a.ld_residual) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
         tmem_wait_ld();
-        if (!live) continue;
-        const int64_t row = grow;
         if (p.a.bias != nullptr) {
 #pragma unroll
             for (int v = 0; v < 8; ++v) {
-                if (col0 + v * 4 >= p.N) break;  // (columns come in fours)
+                if (v * 4 >= n_cols) break;  // (columns come in fours)
                 const float4 b = __ldg(reinterpret_cast<const float4*>(p.a.bias + col0 + v * 4));
-                acc[v * 4 + 0] = __float_as_uint(__uint_as_float(acc[v * 4 + 0]) + b.x);
-                acc[v * 4 + 1] = __float_as_uint(__uint_as_float(acc[v * 4 + 1]) + b.y);
-                acc[v * 4 + 2] = __float_as_uint(__uint_as_float(acc[v * 4 + 2]) + b.z);
-                acc[v * 4 + 3] = __float_as_uint(__uint_as_float(acc[v * 4 + 3]) + b.w);
+                acc[v * 4 + 0] = u(f(acc[v * 4 + 0]) + b.x), acc[v * 4 + 1] = u(f(acc[v * 4 + 1]) + b.y);
+                acc[v * 4 + 2] = u(f(acc[v * 4 + 2]) + b.z), acc[v * 4 + 3] = u(f(acc[v * 4 + 3]) + b.w);
             }
         }
-        if (sg.kind == B2KV_SEG_RELU2) {
+        if (f32) {
+            if (kind == B2KV_SEG_DECAY) {
+                const float inv_tau = 1.0f / p.a.limit;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(lin::single(B2KV_SEG_RELU2, __uint_as_float(acc[i]), 0.f));
-        } else if (sg.kind == B2KV_SEG_DECAY) {
-            const float inv_tau = 1.0f / p.a.limit;
+                for (int i = 0; i < 32; ++i) acc[i] = u(lin::decay(f(acc[i]), inv_tau));
+            } else if (kind == B2KV_SEG_SOFTCAP) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(lin::decay(__uint_as_float(acc[i]), inv_tau));
-        } else if (sg.kind == B2KV_SEG_SOFTCAP) {
+                for (int i = 0; i < 32; ++i) acc[i] = u(lin::single(B2KV_SEG_SOFTCAP, f(acc[i]), p.a.limit));
+            }
+            uint4* const mine = reinterpret_cast<uint4*>(slab + lane * kSlabLd);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(lin::single(B2KV_SEG_SOFTCAP, __uint_as_float(acc[i]), p.a.limit));
+            for (int v = 0; v < 8; ++v) mine[v] = make_uint4(acc[v * 4], acc[v * 4 + 1], acc[v * 4 + 2], acc[v * 4 + 3]);
+            __syncwarp();
+            float* const out = static_cast<float*>(sg.out) + static_cast<int64_t>(row0 + r4) * sg.ld + local + c4;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (r4 + 4 * i >= rows || c4 >= n_cols) break;
+                const float4 v = *reinterpret_cast<const float4*>(slab + (r4 + 4 * i) * kSlabLd + c4);
+                *reinterpret_cast<float4*>(out + 4 * i * sg.ld) = make_float4(v.x + add[i].x, v.y + add[i].y, v.z + add[i].z, v.w + add[i].w);
+            }
+            continue;
         }
-        if (lin::is_f32(sg.kind)) {
-            float* out = static_cast<float*>(sg.out) + row * sg.ld + local;
-            const float* res = p.a.residual && sg.kind == B2KV_SEG_F32 ? p.a.residual + row * p.a.ld_residual + local : nullptr;
-            float4 add[8];
+        const bool pair = lin::is_pair(kind);
+        if (kind == B2KV_SEG_GLU_SILU) {
 #pragma unroll
-            for (int v = 0; v < 8; ++v)
-                add[v] = (res != nullptr && col0 + v * 4 < p.N) ? *reinterpret_cast<const float4*>(res + v * 4)
-                                                                : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int i = 0; i < 16; ++i) acc[i] = u(lin::glu(B2KV_SEG_GLU_SILU, f(acc[2 * i]), f(acc[2 * i + 1]), p.a.limit));
+        } else if (pair) {
 #pragma unroll
-            for (int v = 0; v < 8; ++v) {
-                if (col0 + v * 4 >= p.N) break;
-                float4 o;
-                o.x = __uint_as_float(acc[v * 4 + 0]) + add[v].x, o.y = __uint_as_float(acc[v * 4 + 1]) + add[v].y;
-                o.z = __uint_as_float(acc[v * 4 + 2]) + add[v].z, o.w = __uint_as_float(acc[v * 4 + 3]) + add[v].w;
-                *reinterpret_cast<float4*>(out + v * 4) = o;
-            }
-        } else if (!lin::is_pair(sg.kind)) {
-            __nv_bfloat16* out = static_cast<__nv_bfloat16*>(sg.out) + row * sg.ld + local;
+            for (int i = 0; i < 16; ++i) acc[i] = u(lin::glu(B2KV_SEG_GLU_CLAMP, f(acc[2 * i]), f(acc[2 * i + 1]), p.a.limit));
+        } else if (kind == B2KV_SEG_RELU2) {
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                if (col0 + v * 8 >= p.N) break;
-                uint4 w;
-                w.x = pack_bf16(__uint_as_float(acc[v * 8 + 0]), __uint_as_float(acc[v * 8 + 1]));
-                w.y = pack_bf16(__uint_as_float(acc[v * 8 + 2]), __uint_as_float(acc[v * 8 + 3]));
-                w.z = pack_bf16(__uint_as_float(acc[v * 8 + 4]), __uint_as_float(acc[v * 8 + 5]));
-                w.w = pack_bf16(__uint_as_float(acc[v * 8 + 6]), __uint_as_float(acc[v * 8 + 7]));
-                *reinterpret_cast<uint4*>(out + v * 8) = w;
-            }
-        } else {
-            __nv_bfloat16* out = static_cast<__nv_bfloat16*>(sg.out) + row * sg.ld + local / 2;
-            float z[16];
+            for (int i = 0; i < 32; ++i) acc[i] = u(lin::single(B2KV_SEG_RELU2, f(acc[i]), 0.f));
+        }
+        if (lane >= rows) continue;
+        const int n_out = pair ? n_cols / 2 : n_cols;
+        __nv_bfloat16* const out = static_cast<__nv_bfloat16*>(sg.out) + static_cast<int64_t>(grow) * sg.ld + (pair ? local / 2 : local);
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-                z[i] = lin::glu(sg.kind, __uint_as_float(acc[2 * i]), __uint_as_float(acc[2 * i + 1]), p.a.limit);
-#pragma unroll
-            for (int v = 0; v < 2; ++v) {
-                if (col0 + v * 16 >= p.N) break;
-                uint4 w;
-                w.x = pack_bf16(z[v * 8 + 0], z[v * 8 + 1]);
-                w.y = pack_bf16(z[v * 8 + 2], z[v * 8 + 3]);
-                w.z = pack_bf16(z[v * 8 + 4], z[v * 8 + 5]);
-                w.w = pack_bf16(z[v * 8 + 6], z[v * 8 + 7]);
-                *reinterpret_cast<uint4*>(out + v * 8) = w;
-            }
+        for (int v = 0; v < 4; ++v) {
+            if (v * 8 >= n_out) break;
+            *reinterpret_cast<uint4*>(out + v * 8) =
+                make_uint4(pack_bf16(f(acc[v * 8]), f(acc[v * 8 + 1])), pack_bf16(f(acc[v * 8 + 2]), f(acc[v * 8 + 3])),
+                           pack_bf16(f(acc[v * 8 + 4]), f(acc[v * 8 + 5])), pack_bf16(f(acc[v * 8 + 6]), f(acc[v * 8 + 7])));
         }
     }
+    __syncwarp();
 }
 
 template <int kBKP, int kStagesP, typename P>
@@ -515,12 +522,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     __shared__ GroupTable<P> table;
     extern __shared__ uint8_t smem_raw[];
     using Smem = PairStorage<kBKP, kStagesP>;
-    constexpr int kABytesP = Smem::kABytesP, kWSpanP = Smem::kWSpanP, kStageBytesP = Smem::kStageBytesP;
+    constexpr int kABytesP = Smem::kABytesP, kWSpanP = Smem::kWSpanP;
     Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = static_cast<int>(cluster_ctarank());  // 0 = leader
     const int cid = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
-    const int n_tiles = setup_tiles(p, table, 2 * kBM);  // tiles of 256 rows x 256 columns
     const int n_k = (p.K + kBKP - 1) / kBKP;
 
     if (threadIdx.x == 0) {
@@ -540,10 +546,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         tmem_relinquish_pair();
     }
     tc_fence_before();
+    grid_dependency_wait();  // what comes before hides behind the kernel ahead
     __syncthreads();
     cluster_sync_all();  // the peer's barriers are initialised before anything is sent to them
     tc_fence_after();
     const uint32_t tmem = sm.tmem_base;
+    const int n_tiles = setup_tiles(p, table, 2 * kBM);  // tiles of 256 rows x tile_cols columns
+    const int spans = p.tile_cols > 128 ? 2 : 1;         // of this CTA's half of them
 
     if (warp == 0) {
         // ------------------------------ TMA producer (both CTAs) ------------------------------
@@ -556,25 +565,25 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     const int s = it % kStagesP;
                     ok = mbar_wait(&sm.empty[s], ((it / kStagesP) & 1) ^ 1);
                     if (!ok) break;
-                    if (r == 0) mbar_arrive_expect_tx(&sm.full[s], 2 * kStageBytesP);
+                    if (r == 0) mbar_arrive_expect_tx(&sm.full[s], 2 * (kABytesP + spans * kWSpanP));
                     const uint32_t lead_full = map_to_cta(&sm.full[s], 0);
 #pragma unroll
                     for (int ks = 0; ks < kBKP / 64; ++ks)  // 64 input features (one swizzle span) per box of A
                         tma_load_2d_pair(sm.stage[s] + ks * (kBM * 128), &tm_a, lead_full, kb * kBKP + ks * 64,
                                          tl.row0 + r * kBM);
-#pragma unroll
-                    for (int sp = 0; sp < 2; ++sp)
+                    for (int sp = 0; sp < spans; ++sp)
                         tma_load_2d_pair(sm.stage[s] + kABytesP + sp * kWSpanP, &tm_w, lead_full,
-                                         tl.tn * kBN + r * (kBN / 2) + sp * 64, tl.k_row0 + kb * kBKP);
+                                         tl.tn * p.tile_cols + r * (p.tile_cols / 2) + sp * 64, tl.k_row0 + kb * kBKP);
                 }
             }
+            grid_launch_dependents();  // the next kernel sets up under the last products and outputs
             if (!ok) sm.abort_flag = 1;
         }
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------ MMA issuer (leader CTA only) ------------------------------
         if (lane == 0 && r == 0) {
-            constexpr uint32_t idesc = instr_desc_pair(0, 1, kBN);  // M = 256 over the pair, N = 256
+            const uint32_t idesc = instr_desc_pair(0, 1, p.tile_cols);  // M = 256 over the pair
             bool ok = true;
             uint32_t it = 0, local = 0;
             for (int t = cid; t < n_tiles && ok; t += n_clusters, ++local) {
@@ -617,7 +626,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             ok = mbar_wait(&sm.acc_full[buf], (local >> 1) & 1);
             if (!ok) break;
             tc_fence_after();
-            epilogue_rows(p, tmem + lane_base + buf * kBN, tl.row0 + r * kBM + row, tl.row_end, tl.tn * kBN);
+            epilogue_rows(p, tmem + lane_base + buf * kBN, tl.row0 + r * kBM + row, tl.row_end, tl.tn * p.tile_cols, slab_of(table, quarter));
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_cta(&sm.acc_empty[buf], 0));
@@ -654,13 +663,27 @@ static bool make_map(CUtensorMap* map, const void* base, int64_t rows, int cols,
 // Chooses the form and launches it.  max_tiles_m: row tiles of kBM rows at most; tall: whether 256-row tiles pay.
 template <typename P>
 static int launch(P p, const void* a, int64_t a_rows, int64_t lda, const void* w, int64_t w_rows, int64_t ldw, long long max_tiles_m,
-                  long long max_tiles_m_pair, bool tall, void* stream) {
+                  long long max_tiles_m_pair, bool tall, bool by_groups, void* stream) {
     const long long tiles_n = (static_cast<long long>(p.N) + kBN - 1) / kBN;
     if (max_tiles_m * tiles_n > 0x3fffffffLL) return B2KV_ERR_UNSUPPORTED;
     CUtensorMap ta, tw;
     if (!make_map(&ta, a, a_rows, p.K, lda, kBM) || !make_map(&tw, w, w_rows, p.N, ldw, kBK)) return B2KV_ERR_UNSUPPORTED;
     p.tiles_m = static_cast<int>(max_tiles_m);
-    p.tiles_n = static_cast<int>(tiles_n);
+    // Columns of a tile: what keeps waves times width least.  3548 rows x 2048 columns are 112 tiles of 256 x 256, two waves on 74
+    // pairs with half of the second empty, or 140 tiles of 224, two narrower waves (2048 / 8192 input features: 36 / 114 us, and
+    // 32 / 94); 200 rows x 2048 columns are 16 tiles of 128 x 256 or 64 of 128 x 64 on 148 SMs (2048 input features: 21 us and 20).
+    // A tile costs about as much as 32 columns beside its products.  (With rows grouped by expert the number of tiles is only known
+    // on the device.)
+    auto choose_cols = [&](long long tiles_m, long long places) {
+        long long best = 0, best_n = tiles_n;
+        p.tile_cols = kBN;
+        for (int cols = kBN; cols >= 64 && !by_groups; cols -= 32) {
+            const long long n = (p.N + cols - 1) / cols, cost = (tiles_m * n + places - 1) / places * (cols + 32);
+            if (best == 0 || cost < best) best = cost, best_n = n, p.tile_cols = cols;
+        }
+        p.tiles_n = static_cast<int>(best_n);
+        return tiles_m * best_n;
+    };
     constexpr size_t smem = sizeof(SharedStorage) + 1024;
     using Pair64 = PairStorage<64, 6>;
     using Pair128 = PairStorage<128, 3>;
@@ -675,29 +698,15 @@ static int launch(P p, const void* a, int64_t a_rows, int64_t lda, const void* w
     int dev = 0;
     B2KV_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return B2KV_ERR_UNSUPPORTED;
-    auto pair_config = [&](cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, unsigned grid, size_t bytes) {
-        cfg = cudaLaunchConfig_t{};
-        cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(kThreads);
-        cfg.dynamicSmemBytes = bytes;
-        cfg.stream = static_cast<cudaStream_t>(stream);
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-    };
     if (!configured[dev]) {
         B2KV_CUDA_TRY(cudaFuncSetAttribute(single, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
         B2KV_CUDA_TRY(cudaFuncSetAttribute(pair64, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_pair)));
         B2KV_CUDA_TRY(cudaFuncSetAttribute(pair128, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_pair128)));
         B2KV_CUDA_TRY(cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev));
-        cudaLaunchConfig_t cfg;
-        cudaLaunchAttribute attr[1];
-        pair_config(cfg, attr, 2u * static_cast<unsigned>(sm_count[dev]), smem_pair);
+        OverlapLaunch most(2u * static_cast<unsigned>(sm_count[dev]), kThreads, smem_pair, stream, 2);
+        most.cfg.numAttrs = 1;  // the cluster
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, pair64, &cfg) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveClusters(&n, pair64, &most.cfg) != cudaSuccess) {
             (void)cudaGetLastError();
             n = 0;
         }
@@ -713,24 +722,18 @@ static int launch(P p, const void* a, int64_t a_rows, int64_t lda, const void* w
     const bool use_pair = max_clusters[dev] > 0 && (variant == 2 || variant == 3 || (variant == 0 && pairs_fill && tall));
     if (use_pair) {
         p.tiles_m = static_cast<int>(max_tiles_m_pair);
-        const long long clusters = std::min<long long>(max_tiles_m_pair * tiles_n, max_clusters[dev]);
-        cudaLaunchConfig_t cfg;
-        cudaLaunchAttribute attr[1];
-        if (variant != 2) {  // default: 128 input features per stage (half as many barrier round trips per flop)
-            CUtensorMap tw128;
-            if (!make_map(&tw128, w, w_rows, p.N, ldw, 128)) return B2KV_ERR_UNSUPPORTED;
-            pair_config(cfg, attr, static_cast<unsigned>(2 * clusters), smem_pair128);
-            B2KV_CUDA_TRY(cudaLaunchKernelEx(&cfg, pair128, ta, tw128, p));
-        } else {
-            pair_config(cfg, attr, static_cast<unsigned>(2 * clusters), smem_pair);
-            B2KV_CUDA_TRY(cudaLaunchKernelEx(&cfg, pair64, ta, tw, p));
-        }
-        B2KV_CUDA_TRY(cudaGetLastError());
+        const long long n_tiles = choose_cols(max_tiles_m_pair, max_clusters[dev]);
+        const long long clusters = std::min<long long>(n_tiles, max_clusters[dev]);
+        const bool wide = variant != 2;  // default: 128 input features per stage (half as many barrier round trips per flop)
+        CUtensorMap tw128;
+        if (wide && !make_map(&tw128, w, w_rows, p.N, ldw, 128)) return B2KV_ERR_UNSUPPORTED;
+        OverlapLaunch run(static_cast<unsigned>(2 * clusters), kThreads, wide ? smem_pair128 : smem_pair, stream, 2);
+        B2KV_CUDA_TRY(wide ? cudaLaunchKernelEx(&run.cfg, pair128, ta, tw128, p) : cudaLaunchKernelEx(&run.cfg, pair64, ta, tw, p));
         return B2KV_OK;
     }
-    const long long grid = std::min<long long>(max_tiles_m * tiles_n, sm_count[dev]);
-    single<<<static_cast<unsigned>(grid), kThreads, smem, static_cast<cudaStream_t>(stream)>>>(ta, tw, p);
-    B2KV_CUDA_TRY(cudaGetLastError());
+    const long long n_tiles = choose_cols(max_tiles_m, sm_count[dev]);
+    OverlapLaunch run(static_cast<unsigned>(std::min<long long>(n_tiles, sm_count[dev])), kThreads, smem, stream);
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&run.cfg, single, ta, tw, p));
     return B2KV_OK;
 }
 
@@ -750,8 +753,8 @@ extern "C" int b2kv_matmul(const void* a, const void* w, const void* bias, const
     if (!aligned16(a) || !aligned16(w) || !aligned16(out) || !aligned16(residual) || !aligned16(bias)) return B2KV_ERR_ALIGN;
     const long long tiles_m = (static_cast<long long>(M) + gemm::kBM - 1) / gemm::kBM;
     gemm::GemmParams p{static_cast<const __nv_bfloat16*>(bias), static_cast<const __nv_bfloat16*>(residual),
-                       static_cast<__nv_bfloat16*>(out), M, N, K, activation, 0, 0, dev_status};
-    return gemm::launch(p, a, M, K, w, K, N, tiles_m, (tiles_m + 1) / 2, M > 2 * gemm::kBM, stream);
+                       static_cast<__nv_bfloat16*>(out), M, N, K, activation, 0, 0, 0, dev_status};
+    return gemm::launch(p, a, M, K, w, K, N, tiles_m, (tiles_m + 1) / 2, M > 2 * gemm::kBM, false, stream);
 }
 
 // b2kv_linear with many rows: one product, or rows grouped by expert.
@@ -771,12 +774,12 @@ int b2kv::linear_tiled_tc(const b2kv_linear_args& a, int32_t* dev_status, void* 
     }
     if (a.bias && !aligned16(a.bias)) return B2KV_ERR_UNSUPPORTED;
     if (a.residual && (!aligned16(a.residual) || a.ld_residual % 4 != 0)) return B2KV_ERR_UNSUPPORTED;
-    gemm::SegParams p{a, a.rows, a.N, a.K, 0, 0, dev_status};
+    gemm::SegParams p{a, a.rows, a.N, a.K, 0, 0, 0, dev_status};
     // with groups the number of tiles is only known on the device: every group may end in a partly filled tile
     const long long part = grouped ? a.groups : 0;
     const long long tiles_m = (static_cast<long long>(a.rows) + gemm::kBM - 1) / gemm::kBM + part;
     const long long tiles_m_pair = (static_cast<long long>(a.rows) + 2 * gemm::kBM - 1) / (2 * gemm::kBM) + part;
     const bool tall = grouped ? a.rows / a.groups > 2 * gemm::kBM : a.rows > 2 * gemm::kBM;
     return gemm::launch(p, a.x, a.rows, a.ld_x, a.w, grouped ? static_cast<int64_t>(a.groups) * a.K : a.K, a.ld_w, tiles_m,
-                        tiles_m_pair, tall, stream);
+                        tiles_m_pair, tall, grouped, stream);
 }

@@ -1,0 +1,47 @@
+"""Tiled products whose output columns ask for every width of tile there is, by CTA pairs (300 rows) and by single CTAs (200 rows),
+against float64: the sizes fill the places of one wave at that width and no narrower one."""
+import pytest
+import torch
+
+from tests.kv_util import make_ctx
+from tests.test_gpu_linear import close, rnd, run, wrap
+
+pytestmark = pytest.mark.gpu
+
+BF = torch.bfloat16
+TILED = 3
+
+
+@pytest.mark.parametrize("cols", [64, 96, 128, 160, 192, 224, 256])
+@pytest.mark.parametrize("rows,tiles", [(300, 37), (200, 74)])
+def test_every_width(pkg, rows, tiles, cols):
+    from llm_experiments_b200 import projection as proj
+
+    ctx, K, n, a = make_ctx(pkg), 200, tiles * cols - 24, 32
+    x, w, res = rnd((rows, K), BF, 1), rnd((K, n), BF, 2, K ** -0.5), rnd((rows, n - a), torch.float32, 3)
+    head, body = torch.full((rows + 1, a), 7.0, dtype=BF, device="cuda"), torch.full((rows + 1, n - a), 7.0, device="cuda")
+    body[:rows] = res
+    run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), K, [proj.OutputSegment(a, proj.SEG_STORE, wrap(pkg, head)), proj.OutputSegment(n, proj.SEG_F32, wrap(pkg, body))],
+        residual=wrap(pkg, body), path=TILED)
+    want = x.double() @ w.double()
+    close(head[:rows], want[:, :a], BF)
+    close(body[:rows], want[:, a:] + res.double(), torch.float32)
+    assert (head[rows] == 7).all() and (body[rows] == 7).all()
+
+
+@pytest.mark.parametrize("cols", [64, 96, 160, 224])
+@pytest.mark.parametrize("rows,tiles", [(300, 37), (200, 74)])
+def test_matmul_with_everything_behind_it(pkg, rows, tiles, cols):
+    ctx, K, n = make_ctx(pkg), 72, tiles * cols - 24
+    ctx.config.check_device_status = True
+    x, w, res, bias = rnd((rows, K), BF, 4), rnd((K, n), BF, 5, K ** -0.5), rnd((rows, n), BF, 6), rnd((n,), BF, 7)
+    out = torch.full((rows + 1, n), 7.0, dtype=BF, device="cuda")
+    pkg.gpu.batch_begin(ctx)
+    from llm_experiments_b200 import projection
+
+    projection.matmul(ctx, wrap(pkg, x), wrap(pkg, w), wrap(pkg, out[:rows]), residual=wrap(pkg, res),
+                      bias=pkg.gpu.GPUBuffer1D(buffer=bias, shape=(n,), size=n), activation="gelu")
+    pkg.gpu.batch_commit(ctx)
+    z = x.double() @ w.double() + bias.double()
+    close(out[:rows], z * torch.sigmoid(1.702 * z) + res.double(), BF)
+    assert (out[rows] == 7).all()
