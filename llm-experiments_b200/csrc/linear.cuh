@@ -6,15 +6,18 @@
 namespace b2kv {
 namespace lin {
 
-// x * sigmoid(1.702 x) of the clamped gate times the clamped up part plus one; silu(gate) * up.  Results are rounded to bf16, so
-// the quotients are __fdividef's (2 ulp of fp32): the operator's division is a branch to a subroutine per element, and an
-// epilogue thread has 128 of them one after the other per tile (2975 rows, K = 2048, 10880 gated columns beside 3648 plain ones:
-// 259 us with it, 176 without; the experts' 17850 rows x 2816 gated columns: 417 and 282).
+// x * sigmoid(1.702 x) of the clamped gate times the clamped up part plus one; silu(gate) * up.  kDivide: with the operator's
+// division, a branch to a subroutine per element, which few rows do not notice; otherwise the quotients are __fdividef's (2 ulp of
+// fp32; results are rounded to bf16): an epilogue thread of a tiled product has 128 of them one after the other per tile (2975 rows,
+// K = 2048, 10880 gated columns beside 3648 plain ones: 259 us with the division, 176 without; the experts' 17850 rows x 2816 gated
+// columns: 417 and 282).
+template <bool kDivide = false>
 __device__ __forceinline__ float glu(int kind, float g, float u, float limit) {
-    if (kind == B2KV_SEG_GLU_SILU) return __fdividef(g, 1.0f + __expf(-g)) * u;
+    const auto quotient = [](float a, float b) { return kDivide ? a / b : __fdividef(a, b); };
+    if (kind == B2KV_SEG_GLU_SILU) return quotient(g, 1.0f + __expf(-g)) * u;
     g = fminf(g, limit);
     u = fminf(fmaxf(u, -limit), limit);
-    return __fdividef(g, 1.0f + __expf(-1.702f * g)) * (u + 1.0f);
+    return quotient(g, 1.0f + __expf(-1.702f * g)) * (u + 1.0f);
 }
 
 // Kinds whose columns are (gate, up) pairs; kinds whose output is fp32.
@@ -59,7 +62,7 @@ __device__ __forceinline__ int segment_first(const b2kv_linear_args& a, int s) {
 // Exact exponential for the fp32 path; the bf16 paths round the result to 8 bits anyway.
 template <typename T>
 __device__ __forceinline__ float glu_value(int kind, float g, float u, float limit) {
-    if (sizeof(T) == 2) return glu(kind, g, u, limit);
+    if (sizeof(T) == 2) return glu<true>(kind, g, u, limit);
     if (kind == B2KV_SEG_GLU_SILU) return g / (1.0f + expf(-g)) * u;
     g = fminf(g, limit);
     u = fminf(fmaxf(u, -limit), limit);
