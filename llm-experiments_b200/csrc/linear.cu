@@ -199,7 +199,9 @@ extern "C" int b2kv_linear(const b2kv_linear_args* args, int32_t* dev_status, vo
         if (rc != B2KV_ERR_UNSUPPORTED) return rc;
     }
     if (a.path == 0 && a.dtype == B2KV_DTYPE_F32) {
-        const int rc = linear_f32(a, stream);
+        // many rows: the tensor cores, unless there are too few input features to be worth the parts
+        int rc = a.rows > 16 && a.K >= 128 ? linear_f32_tc(a, dev_status, stream) : B2KV_ERR_UNSUPPORTED;
+        if (rc == B2KV_ERR_UNSUPPORTED) rc = linear_f32(a, stream);
         if (rc != B2KV_ERR_UNSUPPORTED) return rc;
     }
     return lin::launch_simt(a, stream);

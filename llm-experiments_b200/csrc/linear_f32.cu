@@ -1,4 +1,4 @@
-// b2kv_linear in fp32 on the CUDA cores, two kernels.  Sums are fp32 multiply-adds, so what bounds them is that pipe (72 TFLOP/s
+// b2kv_linear in fp32 on the CUDA cores (rows grouped by expert, few rows, few input features), two kernels.  Sums are fp32 multiply-adds, so what bounds them is that pipe (72 TFLOP/s
 // over the chip at 1.9 GHz) for many rows and the weights' bytes for few.  693 rows, 3072 x 768 weights: 441 us with linear_simt_kernel
 // (one read of shared memory per two multiply-adds, 132 CTAs, nothing ahead of its use), 158 here; 6 rows, 768 x 4096: 128 and 14.
 //

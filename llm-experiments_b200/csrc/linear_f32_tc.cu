@@ -1,0 +1,338 @@
+// b2kv_linear in fp32 for many rows on the tensor cores: every operand is split into three bf16 parts, x = h + m + l, which hold all
+// 24 bits, and a product is h h' + (h m' + m h') + (m m' + h l' + l h'); what is dropped is below 2^-24 of it.
+//
+// The tensor core adds in fp32 but truncates, so a long chain of accumulations would lean towards zero by more than fp32 sums err.
+// Therefore the leading products h h' are accumulated over kChain input features only; the partial sums are taken out of tensor memory
+// and added up in registers, rounded to nearest.  The other five products, 2^-8 of the first and less, stay in an accumulator of
+// their own until the end.  Measured against 64 bits, 2-norm of the error over that of the result: 6e-8 at 128 input features, 8e-8 at
+// 768, 1.1e-7 at 3072, where sums of fp32 multiply-adds in order are off by 2.0e-7, 5.0e-7 and 9.9e-7 (chains of 64 input features
+// gave 8e-8, 9e-8 and 1.1e-7, and no more speed).  693 rows, 768 -> 3072: 48 us against 127 of linear_f32_tile_kernel; 3072 -> 768:
+// 57 and 130; 60 rows, 768 -> 3072: 17 and 25.
+//
+//   * a CTA has 128 x 128 outputs; steps of 64 input features through two stages of 96 KB;
+//   * warps 8-15 read fp32 rows of x and w, a step ahead in registers, and write the parts as the operands the MMAs want: x K-major,
+//     w as it lies (MN-major), 128-byte swizzle;
+//   * a thread of warp 8 issues 24 tcgen05.mma per step: 6 x 64 clocks per 16 input features, a sixth of the tensor peak, which is
+//     four times what the CUDA cores have (a seventeenth warp for it would leave all others 96 registers);
+//   * warps 0-7 take the leading sums out (two accumulators in turn), thread = row and half of the columns;
+//   * a product whose tiles leave SMs idle has its input features cut into ranges, one per CTA of a cluster, whose sums meet in
+//     distributed shared memory, in order.
+//
+// A number that is not finite (or rounds to none in bf16) makes no parts: it sets a flag and the CTA computes its sums again
+// with plain multiply-adds.  Every wait is bounded; after one ran out nothing is stored and the status word is set.
+#include <algorithm>
+
+#include "linear.cuh"
+#include "tc_ptx.cuh"
+
+namespace b2kv {
+namespace linf32tc {
+
+using namespace tc;
+
+constexpr int kBM = 128, kBN = 128, kBK = 64, kStages = 2;
+constexpr int kChain = 32;                          // input features per leading sum
+constexpr int kSums = kBK / kChain;                 // leading sums per step
+constexpr int kPartBytes = 128 * kBK * 2;           // one part of x or of w: 16 KB
+constexpr int kStageBytes = 6 * kPartBytes;         // x: h, m, l; w: h, m, l
+constexpr int kSumWarps = 8, kSplitWarps = 8;
+constexpr int kThreads = 32 * (kSumWarps + kSplitWarps);  // 128 registers each
+constexpr int kLdT = kBN + 4;                       // words per row of the tile of sums (over the stages, once they are free)
+constexpr int kMaxSplits = 8;                       // ranges of input features
+constexpr int kTmemCols = 512;                      // leading sums 2 x 128, the others 128
+constexpr int kColRest = 2 * kBN;
+constexpr size_t kSmem = kStages * kStageBytes + 1024;
+static_assert(kBM * kLdT * 4 <= kStages * kStageBytes, "the tile of sums fits the stages");
+
+struct Shared {
+    alignas(8) uint64_t full[kStages], empty[kStages], sum_full[2], sum_empty[2], done;
+    uint32_t tmem_base;
+    volatile int odd, abort_flag;
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peer_address(uint32_t local, uint32_t rank) {
+    uint32_t addr;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local), "r"(rank));
+    return addr;
+}
+__device__ __forceinline__ float2 peer_load2(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ int peer_load1(uint32_t addr) {
+    int v;
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+// The three parts of four numbers, to `at` and one and two parts further on.  `check` becomes NaN where a number has no parts.
+__device__ __forceinline__ void split3(const float4& v, uint8_t* at, float2& check) {
+    const float2 minus = make_float2(-1.f, -1.f);
+    float2 r0 = make_float2(v.x, v.y), r1 = make_float2(v.z, v.w);
+#pragma unroll
+    for (int part = 0; part < 3; ++part) {
+        const uint32_t a = pack_bf16(r0.x, r0.y), b = pack_bf16(r1.x, r1.y);
+        *reinterpret_cast<uint2*>(at + part * kPartBytes) = make_uint2(a, b);
+        r0 = __ffma2_rn(make_float2(__uint_as_float(a << 16), __uint_as_float(a & 0xffff0000u)), minus, r0);
+        r1 = __ffma2_rn(make_float2(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u)), minus, r1);
+    }
+    const float2 none = make_float2(0.f, 0.f);
+    check = __ffma2_rn(r0, none, __ffma2_rn(r1, none, check));
+}
+
+__global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid_constant__ b2kv_linear_args a, int splits, int32_t* dev_status) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ Shared sm;
+    uint8_t* const ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = blockIdx.z;
+    if (tid == 0) {
+        for (int s = 0; s < kStages; ++s) {
+            mbar_init(&sm.full[s], kSplitWarps);
+            mbar_init(&sm.empty[s], 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&sm.sum_full[s], 1);
+            mbar_init(&sm.sum_empty[s], kSumWarps);
+        }
+        mbar_init(&sm.done, 1);
+        sm.odd = sm.abort_flag = 0;
+        fence_mbar_init();
+    }
+    if (warp == 0) {
+        tmem_alloc(&sm.tmem_base, kTmemCols);
+        tmem_relinquish();
+    }
+    grid_dependency_wait();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = sm.tmem_base;
+
+    const float* const x = static_cast<const float*>(a.x) + static_cast<int64_t>(g) * a.group_x;
+    const float* const w = static_cast<const float*>(a.w) + static_cast<int64_t>(g) * a.group_w;
+    const int split = splits > 1 ? static_cast<int>(cluster_rank()) : 0;
+    const int row0 = blockIdx.y * kBM, col0 = static_cast<int>(blockIdx.x) / splits * kBN;
+    const int all_steps = (a.K + kBK - 1) / kBK;
+    const int step0 = static_cast<int>(static_cast<long long>(all_steps) * split / splits);
+    const int steps = static_cast<int>(static_cast<long long>(all_steps) * (split + 1) / splits) - step0;
+    const int k_first = step0 * kBK, k_end = min(a.K, (step0 + steps) * kBK);
+
+    float acc[64];
+    if (warp < kSumWarps) {
+        // ------------------------------ sums: thread = row, half of the columns ------------------------------
+        const uint32_t t_lane = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + (warp >> 2) * 64;
+#pragma unroll
+        for (int j = 0; j < 64; ++j) acc[j] = 0.f;
+        auto add = [&](uint32_t at) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                uint32_t r[16];
+                tmem_ld16(at + q * 16, r);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) acc[q * 16 + j] += __uint_as_float(r[j]);
+            }
+        };
+        bool ok = true;
+        for (int c = 0; c < kSums * steps; ++c) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&sm.sum_full[c & 1], (c >> 1) & 1));
+            if (!ok) break;
+            tc_fence_after();
+            add(t_lane + (c & 1) * kBN);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.sum_empty[c & 1]);
+        }
+        if (ok && steps > 0) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&sm.done, 0));
+            tc_fence_after();
+            if (ok) add(t_lane + kColRest);
+        }
+        if (!ok) sm.abort_flag = 1;
+    } else {
+        // ------------------------------ parts of x and w ------------------------------
+        const int ct = tid - 32 * kSumWarps;
+        const int xc = (ct & 15) * 4, xr = ct >> 4;  // x: four input features of the rows xr, + 16, ..
+        const int wc = (ct & 31) * 4, wk = ct >> 5;  // w: four columns of the input features wk, + 8, ..
+        float4 xv[8], wv[8];
+        auto read_x = [&](int k0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int r = row0 + xr + 16 * i;
+                xv[i] = r < a.rows && k0 + xc < k_end ? *reinterpret_cast<const float4*>(x + static_cast<int64_t>(r) * a.ld_x + k0 + xc)
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        };
+        auto read_w = [&](int k0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int k = k0 + wk + 8 * i;
+                wv[i] = k < k_end && col0 + wc < a.N ? *reinterpret_cast<const float4*>(w + static_cast<int64_t>(k) * a.ld_w + col0 + wc)
+                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        };
+        // the products of step s, once all warps have written their parts
+        auto issue = [&](int s) {
+            constexpr uint32_t idesc = instr_desc(0, 1, kBN);
+            constexpr uint64_t kPart = kPartBytes >> 4;
+            const int st = s % kStages;
+            if (!mbar_wait(&sm.full[st], (s / kStages) & 1)) return false;
+            const uint64_t dx = smem_desc(smem_u32(ring + st * kStageBytes), 16, 1024);
+            const uint64_t dw = smem_desc(smem_u32(ring + st * kStageBytes + 3 * kPartBytes), kBK * 128, 1024);
+#pragma unroll
+            for (int part = 0; part < kSums; ++part) {
+                const int c = kSums * s + part;
+                if (!mbar_wait(&sm.sum_empty[c & 1], ((c >> 1) & 1) ^ 1)) return false;
+                tc_fence_after();
+#pragma unroll
+                for (int i = 0; i < kChain / 16; ++i) {  // 16 input features: 32 bytes of x's rows, 16 rows of w
+                    const int kk = part * (kChain / 16) + i;
+                    mma_ss(tmem + (c & 1) * kBN, dx + 2 * kk, dw + 128 * kk, idesc, i ? 1u : 0u);
+                }
+                mma_commit(&sm.sum_full[c & 1]);
+#pragma unroll
+                for (int i = 0; i < kChain / 16; ++i) {
+                    const int kk = part * (kChain / 16) + i;
+                    const uint64_t ax = dx + 2 * kk, bw = dw + 128 * kk;
+                    mma_ss(tmem + kColRest, ax, bw + 2 * kPart, idesc, (s | kk) ? 1u : 0u);
+                    mma_ss(tmem + kColRest, ax + 2 * kPart, bw, idesc, 1u);
+                    mma_ss(tmem + kColRest, ax + kPart, bw + kPart, idesc, 1u);
+                    mma_ss(tmem + kColRest, ax, bw + kPart, idesc, 1u);
+                    mma_ss(tmem + kColRest, ax + kPart, bw, idesc, 1u);
+                }
+            }
+            mma_commit(&sm.empty[st]);
+            return true;
+        };
+        float2 check = make_float2(0.f, 0.f);
+        if (steps > 0) read_x(k_first), read_w(k_first);
+        bool ok = true;
+        for (int s = 0; s < steps; ++s) {
+            const int st = s % kStages, next = k_first + (s + 1) * kBK;
+            ok = __all_sync(0xffffffffu, mbar_wait(&sm.empty[st], ((s / kStages) & 1) ^ 1));
+            if (!ok) break;
+            uint8_t* const px = ring + st * kStageBytes;
+            uint8_t* const pw = px + 3 * kPartBytes + (wc >> 6) * (kBK * 128);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int r = xr + 16 * i;
+                split3(xv[i], px + r * 128 + (((xc >> 3) ^ (r & 7)) << 4) + (xc & 7) * 2, check);
+            }
+            if (s + 1 < steps) read_x(next);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int k = wk + 8 * i;
+                split3(wv[i], pw + k * 128 + ((((wc & 63) >> 3) ^ (k & 7)) << 4) + (wc & 7) * 2, check);
+            }
+            if (s + 1 < steps) read_w(next);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.full[st]);
+            if (warp == kSumWarps) {
+                if (lane == 0) ok = issue(s);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+            }
+        }
+        if (warp == kSumWarps && lane == 0 && ok) mma_commit(&sm.done);
+        if (check.x != 0.f || check.y != 0.f) sm.odd = 1;  // (NaN)
+        if (!ok) sm.abort_flag = 1;
+    }
+    grid_launch_dependents();
+    tc_fence_before();
+    __syncthreads();  // all MMAs have completed (the sums' warps have seen it): the stages are free
+    float* const tile = reinterpret_cast<float*>(ring);
+    if (warp < kSumWarps) {
+        const int r = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 64;
+        float* const mine = tile + r * kLdT + c0;
+#pragma unroll
+        for (int j = 0; j < 64; j += 4) *reinterpret_cast<float4*>(mine + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+        if (sm.odd) {
+            const float* const row = x + static_cast<int64_t>(min(row0 + r, a.rows - 1)) * a.ld_x;
+            for (int j = 0; j < 64 && col0 + c0 + j < a.N; ++j) {
+                const float* const col = w + col0 + c0 + j;
+                float sum = 0.f;
+                for (int k = k_first; k < k_end; ++k) sum = fmaf(row[k], col[static_cast<int64_t>(k) * a.ld_w], sum);
+                mine[j] = sum;
+            }
+        }
+    }
+    __syncwarp();
+    if (splits > 1) cluster_sync();
+    else __syncthreads();
+    const int c = (tid & 63) * 2, share = (kBM + splits - 1) / splits;
+    bool complete = true;
+    for (int s = 0; s < splits; ++s) complete = complete && peer_load1(peer_address(smem_u32(const_cast<int*>(&sm.abort_flag)), s)) == 0;
+    if (complete && col0 + c < a.N) {
+        for (int r = split * share + (tid >> 6); r < min((split + 1) * share, kBM) && row0 + r < a.rows; r += kThreads / 64) {
+            float2 v = make_float2(0.f, 0.f);
+            for (int s = 0; s < splits; ++s) {
+                const float2 p = peer_load2(peer_address(smem_u32(tile + r * kLdT + c), s));
+                v.x += p.x, v.y += p.y;
+            }
+            lin::finish_pair<float>(a, g, row0 + r, col0 + c, v.x, v.y);
+        }
+    }
+    __syncwarp();
+    if (splits > 1) cluster_sync();  // the peers have read this CTA's part
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, kTmemCols);
+    }
+    if (tid == 0 && sm.abort_flag) report_status(dev_status, B2KV_DEV_WAIT_TIMEOUT);
+}
+
+}  // namespace linf32tc
+
+int linear_f32_tc(const b2kv_linear_args& a, int32_t* dev_status, void* stream) {
+    using namespace linf32tc;
+    if (a.dtype != B2KV_DTYPE_F32 || a.group_rows != nullptr) return B2KV_ERR_UNSUPPORTED;
+    if (!aligned16(a.x) || !aligned16(a.w) || a.K % 4 || a.N % 4 || a.ld_x % 4 || a.ld_w % 4 || a.group_x % 4 || a.group_w % 4)
+        return B2KV_ERR_UNSUPPORTED;
+    const long long tiles_m = (a.rows + kBM - 1) / kBM, tiles_n = (a.N + kBN - 1) / kBN, tiles = tiles_m * tiles_n * a.groups;
+    const int steps = (a.K + kBK - 1) / kBK;
+    static bool configured[64] = {false};
+    static int clusters[64][kMaxSplits + 1] = {{0}};  // that can be resident together, by size
+    int dev = 0;
+    B2KV_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return B2KV_ERR_UNSUPPORTED;
+    if (!configured[dev]) {
+        B2KV_CUDA_TRY(cudaFuncSetAttribute(linear_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem)));
+        clusters[dev][1] = device_sm_count();
+        for (int s = 2; s <= kMaxSplits; ++s) {
+            OverlapLaunch most(static_cast<unsigned>(s * device_sm_count()), kThreads, kSmem, stream, s);
+            most.cfg.numAttrs = 1;  // the cluster
+            if (cudaOccupancyMaxActiveClusters(&clusters[dev][s], linear_f32_tc_kernel, &most.cfg) != cudaSuccess) {
+                (void)cudaGetLastError();
+                clusters[dev][s] = 0;
+            }
+        }
+        configured[dev] = true;
+    }
+    // Ranges of input features: the steps of the fullest places, where a CTA costs about four steps beside its own and the meeting of
+    // a cluster two more.  (Clusters of four do not reach every SM: 36 of them are two waves.)
+    int splits = 1;
+    double best = 1e30;
+    for (int s = 1; s <= kMaxSplits && (s == 1 || steps >= 2 * s); ++s) {
+        if (clusters[dev][s] <= 0) continue;
+        const double cost = static_cast<double>((tiles + clusters[dev][s] - 1) / clusters[dev][s]) * ((steps + s - 1) / s + 4 + (s > 1 ? 2 : 0));
+        if (cost < best) best = cost, splits = s;
+    }
+    if (tune_get("matmul_splits") > 0) splits = std::min(tune_get("matmul_splits"), kMaxSplits);
+    if (tiles_m > 65535 || a.groups > 65535 || tiles_n * splits > 0x7fffffffLL) return B2KV_ERR_UNSUPPORTED;
+    OverlapLaunch launch(dim3(static_cast<unsigned>(tiles_n * splits), static_cast<unsigned>(tiles_m), a.groups), kThreads, kSmem, stream, splits);
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, linear_f32_tc_kernel, a, splits, dev_status));
+    return B2KV_OK;
+}
+
+}  // namespace b2kv

@@ -99,3 +99,22 @@ def test_heads(pkg, rows):
         group_x=k, group_w=k * n)
     for h in range(heads):
         bounded(out[:, h * n:(h + 1) * n], x[:, h * k:(h + 1) * k], w[h * k:(h + 1) * k])
+
+
+@pytest.mark.parametrize("K", [128, 1028])
+def test_numbers_that_have_no_parts(pkg, K):
+    """What is not finite, or rounds to nothing finite in bf16, in either operand: as with plain multiply-adds, and nowhere else."""
+    from llm_experiments_b200 import projection as proj
+
+    ctx, rows, n = make_ctx(pkg), 150, 200
+    x, w = rnd((rows, K), F32, 13), rnd((K, n), F32, 14)
+    x[3, 5], x[140, K - 1], w[11, 13], w[7, 190], x[9, 11] = float("inf"), float("nan"), 3.4e38, -float("inf"), 0.0
+    got = {}
+    for path in (0, 1):
+        got[path] = torch.empty((rows, n), dtype=F32, device="cuda")
+        run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), K, [proj.OutputSegment(n, proj.SEG_STORE, wrap(pkg, got[path]))], path=path)
+    assert torch.equal(got[0].isnan(), got[1].isnan()) and torch.equal(got[0].isinf(), got[1].isinf())
+    plain = torch.ones((rows, n), dtype=torch.bool, device="cuda")
+    plain[[3, 140]] = False
+    plain[:, [13, 190]] = False
+    torch.testing.assert_close(got[0][plain].double(), (x.double() @ w.double())[plain], rtol=1e-4, atol=1e-3)
