@@ -6,6 +6,8 @@
 
 #include <math.h>
 
+#include <algorithm>
+
 namespace b2kv {
 namespace {
 
@@ -204,6 +206,213 @@ __global__ void __launch_bounds__(kWarps * 32) gqa_decode_kernel(const GqaDecode
     }
 }
 
+// Runs of rows of one sequence in fp32 (prompt portions, which fp32 has no tensor-core form for): 32 rows of one head per CTA and 64
+// tokens at a time, keys and values read into shared memory once for all of the rows.  A thread has 4 rows x 4 tokens of the scores
+// and 4 rows x 4 columns (per 64) of the output, 64 multiply-adds for every eight 16-byte reads of shared memory; the 16 lanes of a
+// row group keep the rows' softmax among themselves.  gqa_decode_kernel reads every key and value again for every row and reduces
+// over the warp for every token: 174 us for 693 rows of three prompts (12 heads of 64, 4 of them for keys), against 100.
+// Rows of other sequences in the same 32 are taken in turn; a weight of zero is never multiplied with what a row must not see.
+constexpr int kRunRows = 32, kRunTokens = 64, kRunThreads = 128;
+
+template <int kD>  // dim and vdim, rounded up
+__global__ void __launch_bounds__(kRunThreads) gqa_run_f32_kernel(const __grid_constant__ GqaDecodeArgs a) {
+    constexpr int kLd = kD + 4, kLdP = kRunTokens + 4, kCols = kD / 64;
+    extern __shared__ float4 sm_run[];
+    float* const s_q = reinterpret_cast<float*>(sm_run);  // [rows][kLd]
+    float* const s_k = s_q + kRunRows * kLd;              // [tokens][kLd]
+    float* const s_v = s_k + kRunTokens * kLd;            // [tokens][kLd]
+    float* const s_p = s_v + kRunTokens * kLd;            // [rows][kLdP]
+    __shared__ int s_slot[kRunRows], s_pos[kRunRows];
+    const int h = blockIdx.x, i0 = static_cast<int>(blockIdx.y) * kRunRows, n_rows = min(kRunRows, a.rows - i0);
+    const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16, g = h / (a.H / a.G);
+    grid_launch_dependents();
+    grid_dependency_wait();
+    if (tid < kRunRows) {
+        int slot = -1, pos = -1;
+        if (tid < n_rows && !row_place(a.row_slot, a.row_pos, i0 + tid, a.n_slots, a.T_max, slot, pos)) {
+            report_status(a.dev_status, B2KV_DEV_BAD_POSITION);
+            slot = pos = -1;
+        }
+        s_slot[tid] = slot, s_pos[tid] = pos;
+    }
+    const float* const q = static_cast<const float*>(a.q) + i0 * a.ld_q + h * a.dim;
+    for (int i = tid; i < kRunRows * (kD / 4); i += kRunThreads) {
+        const int r = i / (kD / 4), c = i % (kD / 4) * 4;
+        *reinterpret_cast<float4*>(s_q + r * kLd + c) =
+            r < n_rows && c < a.dim ? *reinterpret_cast<const float4*>(q + r * a.ld_q + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    const float slope = a.slopes != nullptr ? a.slopes[h] : 0.f;
+    float m[4], l[4];
+    float4 acc[4][kCols];
+    int pos[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        m[i] = -INFINITY, l[i] = 0.f, pos[i] = s_pos[ty * 4 + i];
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) acc[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int first = 0; first < n_rows;) {
+        // the run: rows [first, end) of one sequence, which see tokens up to last, all of them those up to all
+        const int here = s_slot[first];
+        int end = first, last = -1, all = 0x7fffffff;
+        for (; end < n_rows && s_slot[end] == here; ++end) last = max(last, s_pos[end]), all = min(all, s_pos[end]);
+        const bool alone = first == 0 && end == kRunRows;
+        bool mine[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mine[i] = ty * 4 + i >= first && ty * 4 + i < end;
+        first = end;
+        if (here < 0) continue;
+        const int64_t base = static_cast<int64_t>(here) * a.T_max * a.G + g;
+        const float* const keys = static_cast<const float*>(a.k_cache) + base * a.dim;
+        const float* const values = static_cast<const float*>(a.v_cache) + base * a.vdim;
+        for (int t0 = 0; t0 <= last; t0 += kRunTokens) {
+            __syncthreads();
+#pragma unroll 4
+            for (int i = tid; i < kRunTokens * (kD / 4); i += kRunThreads) {
+                const int t = i / (kD / 4), c = i % (kD / 4) * 4;
+                const bool in = t0 + t <= last;
+                *reinterpret_cast<float4*>(s_k + t * kLd + c) =
+                    in && c < a.dim ? *reinterpret_cast<const float4*>(keys + static_cast<int64_t>(t0 + t) * a.G * a.dim + c)
+                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+                *reinterpret_cast<float4*>(s_v + t * kLd + c) =
+                    in && c < a.vdim ? *reinterpret_cast<const float4*>(values + static_cast<int64_t>(t0 + t) * a.G * a.vdim + c)
+                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            __syncthreads();
+            float s[4][4] = {};
+#pragma unroll 4
+            for (int c = 0; c < a.dim; c += 4) {
+                float4 qv[4], kv[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    qv[i] = *reinterpret_cast<const float4*>(s_q + (ty * 4 + i) * kLd + c);
+                    kv[i] = *reinterpret_cast<const float4*>(s_k + (tx + 16 * i) * kLd + c);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        s[i][j] = fmaf(qv[i].w, kv[j].w, fmaf(qv[i].z, kv[j].z, fmaf(qv[i].y, kv[j].y, fmaf(qv[i].x, kv[j].x, s[i][j]))));
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float mn = m[i];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int t = t0 + tx + 16 * j;
+                    s[i][j] = mine[i] && t <= pos[i] ? s[i][j] * a.scale - slope * static_cast<float>(pos[i] - t) : -INFINITY;
+                    mn = fmaxf(mn, s[i][j]);
+                }
+#pragma unroll
+                for (int off = 8; off > 0; off >>= 1) mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, off));
+                const float f = mn == m[i] ? 1.f : expf(m[i] - mn);
+                m[i] = mn;
+                l[i] *= f;
+#pragma unroll
+                for (int c = 0; c < kCols; ++c) acc[i][c].x *= f, acc[i][c].y *= f, acc[i][c].z *= f, acc[i][c].w *= f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int t = tx + 16 * j;
+                    const float p = mine[i] && t0 + t <= pos[i] ? expf(s[i][j] - mn) : 0.f;
+                    l[i] += p;
+                    s_p[(ty * 4 + i) * kLdP + t] = p;
+                }
+            }
+            __syncwarp();  // a row's weights are written and read by the same 16 lanes
+            if (alone && t0 + kRunTokens - 1 <= all) {
+                for (int t = 0; t < kRunTokens; t += 4) {
+                    float4 p[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(s_p + (ty * 4 + i) * kLdP + t);
+#pragma unroll
+                    for (int c = 0; c < kCols; ++c) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float4 v = *reinterpret_cast<const float4*>(s_v + (t + e) * kLd + c * 64 + tx * 4);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const float w = e == 0 ? p[i].x : (e == 1 ? p[i].y : (e == 2 ? p[i].z : p[i].w));
+                                acc[i][c].x = fmaf(w, v.x, acc[i][c].x), acc[i][c].y = fmaf(w, v.y, acc[i][c].y);
+                                acc[i][c].z = fmaf(w, v.z, acc[i][c].z), acc[i][c].w = fmaf(w, v.w, acc[i][c].w);
+                            }
+                        }
+                    }
+                }
+            } else {
+                // Tokens that not all rows see.  A weight of zero is no answer to a value that is not finite, so what a row must not
+                // see counts as zero itself.
+#pragma unroll 2
+                for (int t = 0; t < kRunTokens; t += 4) {
+                    if (t0 + t > last) break;
+                    float4 p[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(s_p + (ty * 4 + i) * kLdP + t);
+#pragma unroll
+                    for (int c = 0; c < kCols; ++c) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float4 v = *reinterpret_cast<const float4*>(s_v + (t + e) * kLd + c * 64 + tx * 4);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const bool sees = mine[i] && t0 + t + e <= pos[i];
+                                const float w = e == 0 ? p[i].x : (e == 1 ? p[i].y : (e == 2 ? p[i].z : p[i].w));
+                                acc[i][c].x = fmaf(w, sees ? v.x : 0.f, acc[i][c].x), acc[i][c].y = fmaf(w, sees ? v.y : 0.f, acc[i][c].y);
+                                acc[i][c].z = fmaf(w, sees ? v.z : 0.f, acc[i][c].z), acc[i][c].w = fmaf(w, sees ? v.w : 0.f, acc[i][c].w);
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    }
+    float* const out = static_cast<float*>(a.out) + i0 * a.ld_out + h * a.vdim;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], off);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (s_slot[ty * 4 + i] < 0) continue;
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) {
+            const float v[4] = {acc[i][c].x, acc[i][c].y, acc[i][c].z, acc[i][c].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int d = c * 64 + tx * 4 + e;
+                if (d < a.vdim) out[static_cast<int64_t>(ty * 4 + i) * a.ld_out + d] = v[e] / l[i];
+            }
+        }
+    }
+}
+
+template <int kD>
+int launch_runs(const GqaDecodeArgs& a, void* stream) {
+    constexpr size_t smem = ((kRunRows + 2 * kRunTokens) * (kD + 4) + kRunRows * (kRunTokens + 4)) * sizeof(float);
+    static bool configured[64] = {false};
+    int dev = 0;
+    B2KV_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return B2KV_ERR_UNSUPPORTED;
+    if (!configured[dev]) {
+        B2KV_CUDA_TRY(cudaFuncSetAttribute(gqa_run_f32_kernel<kD>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        configured[dev] = true;
+    }
+    OverlapLaunch launch(dim3(a.H, (a.rows + kRunRows - 1) / kRunRows), kRunThreads, smem, stream);
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, gqa_run_f32_kernel<kD>, a));
+    return B2KV_OK;
+}
+
+// Rows come in runs when there are several for every place; a decoding step has one per sequence at most, and a CTA would take
+// its sequences one after the other.
+int launch_runs_f32(const GqaDecodeArgs& a, void* stream) {
+    if (a.rows < 4 * a.n_slots || a.rows < 2 * kRunRows || (a.rows + kRunRows - 1) / kRunRows > 65535) return B2KV_ERR_UNSUPPORTED;
+    const int widest = std::max(a.dim, a.vdim);
+    if (widest > 128 || a.dim % 4 || a.vdim % 4 || a.ld_q % 4 || !aligned16(a.q) || !aligned16(a.k_cache) || !aligned16(a.v_cache))
+        return B2KV_ERR_UNSUPPORTED;
+    return widest <= 64 ? launch_runs<64>(a, stream) : launch_runs<128>(a, stream);
+}
+
 template <typename T>
 int launch_simt(const GqaDecodeArgs& a, void* stream) {
     const int widest = a.dim > a.vdim ? a.dim : a.vdim;
@@ -273,6 +482,10 @@ extern "C" int b2kv_gqa_decode(const void* q, int64_t ld_q, const void* k_cache,
     if (dtype == B2KV_DTYPE_BF16 && path != 1) {
         const int rc = gqa_decode_tc(a, workspace, workspace_bytes, stream);
         if (rc != B2KV_ERR_UNSUPPORTED || path == 2) return rc;
+    }
+    if (dtype == B2KV_DTYPE_F32 && path == 0) {
+        const int rc = launch_runs_f32(a, stream);
+        if (rc != B2KV_ERR_UNSUPPORTED) return rc;
     }
     return dtype == B2KV_DTYPE_F32 ? launch_simt<float>(a, stream) : launch_simt<__nv_bfloat16>(a, stream);
 }

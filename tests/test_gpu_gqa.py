@@ -149,6 +149,37 @@ def test_single_rows(pkg, path, dtype, heads, kv, dim, vdim, bias):
     assert (out[len(pos)] == 7).all() and (out[:, heads * vdim:] == 7).all()
 
 
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(3, 1, 4, 8), (4, 2, 64, 64), (2, 1, 72, 128), (2, 2, 128, 20)])
+@pytest.mark.parametrize("runs", [((0, 0, 65),), ((2, 0, 64), (0, 60, 7), (1, 199, 1), (2, 64, 31), (0, 0, 40)), ((1, 130, 96), (0, 3, 33))])
+def test_runs_of_rows_in_fp32(pkg, heads, kv, dim, vdim, runs):
+    """Prompt portions of 32-row tiles and their parts, several sequences in a tile, one of them twice; nothing that a row must not
+    see reaches it, not even what is no number."""
+    from llm_experiments_b200 import gqa
+    from llm_experiments_b200.latent import RowPlaces
+
+    ctx = make_ctx(pkg)
+    shape = gqa.GqaShape(heads, kv, dim, vdim, 1.3 * dim ** -0.5)
+    cache = make_cache(pkg, ctx, shape, 3, 240, F32)
+    slots, pos = [s for s, _, n in runs for _ in range(n)], [p + i for _, p, n in runs for i in range(n)]
+    ends = {s: max(p for t, p in zip(slots, pos) if t == s) for s in slots}
+    for t in cache_views(cache, shape):
+        for s in range(3):
+            t[s, ends.get(s, -1) + 1:] = float("nan")
+    cache_views(cache, shape)[1][slots[0], ends[slots[0]]] = float("inf")  # the last row of one sequence alone sees this value
+    y = rnd((len(pos), heads * dim + 16), F32, 7)
+    out = torch.full((len(pos) + 1, heads * vdim + 8), 7.0, dtype=F32, device="cuda")
+    slopes = gqa.geometric_slopes(heads).cuda()
+    places = RowPlaces(torch.tensor(slots, dtype=torch.int32, device="cuda"), torch.tensor(pos, dtype=torch.int32, device="cuda"))
+    in_batch(pkg, ctx, lambda: gqa.gqa_decode(ctx, wrap(pkg, y), shape, wrap1(pkg, slopes), places, cache, wrap(pkg, out[:len(pos)]), 240))
+    k, v = (np64(t) for t in cache_views(cache, shape))
+    want = reference(np64(y)[:, :heads * dim].reshape(len(pos), heads, dim), k, v, slots, pos, shape, bo.head_slopes(heads))
+    got = np64(out)[:len(pos), :heads * vdim]
+    finite = np.array([(s, p) != (slots[0], ends[slots[0]]) for s, p in zip(slots, pos)])
+    np.testing.assert_allclose(got[finite], want[finite], rtol=2e-5, atol=2e-5)
+    assert not np.isfinite(got[~finite]).any()
+    assert (out[len(pos)] == 7).all() and (out[:, heads * vdim:] == 7).all()
+
+
 @pytest.mark.parametrize("share", [1, 2, 3, 5, 16])
 def test_single_rows_in_shares(pkg, share):
     """However a row's tokens are cut into shares the result is the same; rows of one share sit beside rows of many."""
