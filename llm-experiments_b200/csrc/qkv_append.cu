@@ -53,6 +53,9 @@ constexpr int kFeat = 128;      // output features per CTA (MMA M)
 constexpr int kKTile = 128;
 constexpr int kMaxStagesP = 6;
 constexpr int kRingBytes = 200 * 1024;  // shared memory given to the ring; as many stages as fit
+// Several waves of tiles (the logits): two CTAs per SM, so that one streams while the other starts or ends (8 rows, 4096 x 32768: 72 us
+// with one, 66 so).
+constexpr int kRingBytesTwo = 112 * 1024;
 constexpr int kSmemBytes = 224 * 1024;  // ring and partials of a split tile together (227 KB less alignment and statics)
 constexpr int kWBytes = kKTile * kFeat * 2;  // two halves of 16 KB, see the descriptors below
 constexpr int kWHalf = kWBytes / 2;
@@ -461,7 +464,7 @@ extern "C" int b2kv_matmul_rows(const void* x, const void* w, const void* bias, 
     // a split tile keeps the partials of its own sequences behind the rings: [splits][Bn / splits][128] fp32
     const int recv_bytes = splits > 1 ? Bn * proj::kFeat * 4 : 0;
     const int stage_bytes = proj::kWBytes + 2 * Bn * 128;
-    const int ring_bytes = std::min(proj::kRingBytes, proj::kSmemBytes - recv_bytes);
+    const int ring_bytes = tiles > device_sm_count() ? proj::kRingBytesTwo : std::min(proj::kRingBytes, proj::kSmemBytes - recv_bytes);
     const int stages = std::max(2, std::min(proj::kMaxStagesP, ring_bytes / stage_bytes));
     const size_t smem = static_cast<size_t>(stages) * stage_bytes + recv_bytes + 1024;
     // one weight matrix: every tile is of kind 0 (plain rows of `out`); the cache fields are unused
