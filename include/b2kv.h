@@ -258,8 +258,8 @@ int b2kv_prefill(const void* Q, const void* K, const void* V, void* O, float* L,
  * relative), softmax and outputs stay fp32; results agree with the fp32 oracle within rtol 1e-4 and atol 3e-5
  * on outputs of order one (the SIMT kernel, which b2kv_prefill takes for fp32, holds atol 1e-5).  b2kv_prefill_workspace_bytes gives the scratch size, 0 where scratch buys nothing (bf16
  * prompts, other head_dims, prompts shorter than 128 tokens): the call then is b2kv_prefill.  The scratch needs no
- * initialisation and carries nothing between calls.  With a cache the K / V rows are written by a copy kernel behind the
- * attention.
+ * initialisation and carries nothing between calls.  With a cache the K / V rows are written by the kernel that
+ * splits them, ahead of the attention.
  */
 size_t b2kv_prefill_workspace_bytes(int B, int N, int H, int D, int dtype);
 int b2kv_prefill_ws(const void* Q, const void* K, const void* V, void* O, float* L, float* M, void* k_cache, void* v_cache,
@@ -401,7 +401,9 @@ int b2kv_layernorm_rows(const float* y, int64_t ld_y, const int32_t* row_index, 
  * x is [rows, K] with row pitch ld_x; w is [K, N] row-major with row pitch ld_w.  Group g (0 <= g < groups) reads
  * x + g * group_x and w + g * group_w and writes seg.out + g * seg.group: the heads of a per-head product.  With group_rows
  * (device, groups + 1 row offsets) group g instead owns rows group_rows[g] .. group_rows[g + 1] - 1 of x and of the outputs:
- * the experts of a mixture, whose rows are sorted by expert; no group has more than max_group_rows of them.
+ * the experts of a mixture, whose rows are sorted by expert; no group has more than max_group_rows of them.  With group_x_rows
+ * as well, the rows of x of group g start at group_x_rows[g] (runs of rows anywhere in a cache; x has x_rows rows), and
+ * group_w = 0 gives all groups one w: tiled kernel only.
  * Offsets and pitches are in elements.  Segment boundaries are even.  The product runs on the tensor cores for bf16 when
  * pitches, offsets and boundaries allow it (multiples of 8 elements; boundaries multiples of 32): at most 128 rows per
  * group stream the weights once, more go to the tiled kernel.  fp32 products of more than 16 rows and at least 128 input
@@ -434,6 +436,8 @@ typedef struct b2kv_linear_args {
     b2kv_segment seg[B2KV_MAX_SEGMENTS];
     int32_t rows, K, N, groups, max_group_rows, n_seg, dtype, path;
     float limit;
+    int32_t x_rows;              /* with group_x_rows: rows of x */
+    const int32_t* group_x_rows; /* with group_rows: first row of x of every group (device), or NULL: group_rows */
 } b2kv_linear_args;
 int b2kv_linear(const b2kv_linear_args* args, int32_t* dev_status, void* stream);
 

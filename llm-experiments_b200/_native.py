@@ -54,7 +54,7 @@ class LinearArgs(ctypes.Structure):
                 ("ld_w", _i64), ("group_w", _i64), ("ld_residual", _i64), ("seg", Segment * MAX_SEGMENTS),
                 ("rows", ctypes.c_int32), ("K", ctypes.c_int32), ("N", ctypes.c_int32), ("groups", ctypes.c_int32),
                 ("max_group_rows", ctypes.c_int32), ("n_seg", ctypes.c_int32), ("dtype", ctypes.c_int32),
-                ("path", ctypes.c_int32), ("limit", _f)]
+                ("path", ctypes.c_int32), ("limit", _f), ("x_rows", ctypes.c_int32), ("group_x_rows", _vp)]
 
 
 class GlaArgs(ctypes.Structure):

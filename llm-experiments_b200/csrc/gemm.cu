@@ -70,9 +70,9 @@ struct SegParams {
     int32_t* dev_status;
 };
 
-// Output tile: first row of A, row behind the last one that belongs to the tile's group, column tile, first row of W.
+// Output tile: first row, row behind the last one that belongs to the tile's group, column tile, first row of W, first row of A.
 struct Tile {
-    int row0, row_end, tn, k_row0;
+    int row0, row_end, tn, k_row0, a_row0;
 };
 
 // First row tile of every group (and behind the last one), for tiles of tile_rows rows, and the epilogue warps' pieces of fp32 outputs;
@@ -148,13 +148,13 @@ __device__ __forceinline__ int setup_tiles(const SegParams& p, GroupTable<SegPar
 __device__ __forceinline__ Tile find_tile(int t, const GemmParams& p, const GroupTable<GemmParams>&, int tile_rows) {
     int tm, tn;
     tile_coords(t, p, tm, tn);
-    return {tm * tile_rows, p.M, tn, 0};
+    return {tm * tile_rows, p.M, tn, 0, tm * tile_rows};
 }
 __device__ __forceinline__ Tile find_tile(int t, const SegParams& p, const GroupTable<SegParams>& table, int tile_rows) {
     if (p.a.group_rows == nullptr) {
         int tm, tn;
         tile_coords(t, p, tm, tn);
-        return {tm * tile_rows, p.M, tn, 0};
+        return {tm * tile_rows, p.M, tn, 0, tm * tile_rows};
     }
     int lo = 0, hi = p.a.groups - 1;  // the last group whose first tile is not behind t (so it has tiles)
     while (lo < hi) {
@@ -164,7 +164,9 @@ __device__ __forceinline__ Tile find_tile(int t, const SegParams& p, const Group
     }
     const int first = table.first[lo], rows_here = table.first[lo + 1] - first;
     const int within = t - first * p.tiles_n;  // row tiles run fastest: they share the group's columns of W
-    return {p.a.group_rows[lo] + within % rows_here * tile_rows, p.a.group_rows[lo + 1], within / rows_here, lo * p.K};
+    const int row0 = p.a.group_rows[lo], down = within % rows_here * tile_rows;
+    return {row0 + down, p.a.group_rows[lo + 1], within / rows_here, p.a.group_w == 0 ? 0 : lo * p.K,
+            (p.a.group_x_rows != nullptr ? p.a.group_x_rows[lo] : row0) + down};
 }
 
 __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_addr, int grow, int row_end, int col_base, uint32_t* slab);
@@ -215,7 +217,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                     ok = mbar_wait(&sm.empty[s], ((it / kStages) & 1) ^ 1);
                     if (!ok) break;
                     mbar_arrive_expect_tx(&sm.full[s], kABytes + spans * kWSpanBytes);
-                    tma_load_2d(sm.stage[s], &tm_a, &sm.full[s], kb * kBK, tl.row0);
+                    tma_load_2d(sm.stage[s], &tm_a, &sm.full[s], kb * kBK, tl.a_row0);
                     for (int sp = 0; sp < spans; ++sp)
                         tma_load_2d(sm.stage[s] + kABytes + sp * kWSpanBytes, &tm_w, &sm.full[s], tl.tn * p.tile_cols + sp * 64,
                                     tl.k_row0 + kb * kBK);
@@ -570,7 +572,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 #pragma unroll
                     for (int ks = 0; ks < kBKP / 64; ++ks)  // 64 input features (one swizzle span) per box of A
                         tma_load_2d_pair(sm.stage[s] + ks * (kBM * 128), &tm_a, lead_full, kb * kBKP + ks * 64,
-                                         tl.row0 + r * kBM);
+                                         tl.a_row0 + r * kBM);
                     for (int sp = 0; sp < spans; ++sp)
                         tma_load_2d_pair(sm.stage[s] + kABytesP + sp * kWSpanP, &tm_w, lead_full,
                                          tl.tn * p.tile_cols + r * (p.tile_cols / 2) + sp * 64, tl.k_row0 + kb * kBKP);
@@ -762,7 +764,7 @@ int b2kv::linear_tiled_tc(const b2kv_linear_args& a, int32_t* dev_status, void* 
     if (a.dtype != B2KV_DTYPE_BF16) return B2KV_ERR_UNSUPPORTED;
     const bool grouped = a.group_rows != nullptr;
     if (a.groups > 1 && !grouped) return B2KV_ERR_UNSUPPORTED;
-    if (grouped && (a.groups > gemm::kMaxGroups || a.group_w != static_cast<int64_t>(a.K) * a.ld_w)) return B2KV_ERR_UNSUPPORTED;
+    if (grouped && (a.groups > gemm::kMaxGroups || (a.group_w != static_cast<int64_t>(a.K) * a.ld_w && !(a.group_w == 0 && a.group_x_rows)))) return B2KV_ERR_UNSUPPORTED;
     if (!aligned16(a.x) || !aligned16(a.w) || a.ld_x % 8 || a.ld_w % 8 || a.ld_x < a.K || a.ld_w < a.N) return B2KV_ERR_UNSUPPORTED;
     int first = 0;
     for (int s = 0; s < a.n_seg; ++s) {  // 16-byte accesses in the epilogue; 32 columns lie in one segment
@@ -780,6 +782,6 @@ int b2kv::linear_tiled_tc(const b2kv_linear_args& a, int32_t* dev_status, void* 
     const long long tiles_m = (static_cast<long long>(a.rows) + gemm::kBM - 1) / gemm::kBM + part;
     const long long tiles_m_pair = (static_cast<long long>(a.rows) + 2 * gemm::kBM - 1) / (2 * gemm::kBM) + part;
     const bool tall = grouped ? a.rows / a.groups > 2 * gemm::kBM : a.rows > 2 * gemm::kBM;
-    return gemm::launch(p, a.x, a.rows, a.ld_x, a.w, grouped ? static_cast<int64_t>(a.groups) * a.K : a.K, a.ld_w, tiles_m,
+    return gemm::launch(p, a.x, a.group_x_rows ? a.x_rows : a.rows, a.ld_x, a.w, a.group_w ? static_cast<int64_t>(a.groups) * a.K : a.K, a.ld_w, tiles_m,
                         tiles_m_pair, tall, grouped, stream);
 }

@@ -175,6 +175,7 @@ extern "C" int b2kv_linear(const b2kv_linear_args* args, int32_t* dev_status, vo
     if (a.n_seg < 1 || a.n_seg > B2KV_MAX_SEGMENTS || a.seg[a.n_seg - 1].end != a.N) return B2KV_ERR_BAD_ARG;
     if (a.bias && a.groups > 1) return B2KV_ERR_BAD_ARG;
     if (a.group_rows && (a.max_group_rows <= 0 || a.max_group_rows > a.rows)) return B2KV_ERR_BAD_ARG;
+    if (a.group_x_rows && (!a.group_rows || a.x_rows <= 0)) return B2KV_ERR_BAD_ARG;
     int first = 0;
     for (int s = 0; s < a.n_seg; ++s) {
         const b2kv_segment& sg = a.seg[s];
@@ -183,6 +184,7 @@ extern "C" int b2kv_linear(const b2kv_linear_args* args, int32_t* dev_status, vo
         if ((sg.end & 1) && (s + 1 < a.n_seg || lin::is_pair(sg.kind))) return B2KV_ERR_BAD_ARG;
         first = sg.end;
     }
+    if (a.group_x_rows) return a.path == 0 || a.path == 3 ? linear_tiled_tc(a, dev_status, stream) : B2KV_ERR_UNSUPPORTED;
     if (a.path == 2) return linear_rows_tc(a, dev_status, stream);
     if (a.path == 3) return linear_tiled_tc(a, dev_status, stream);
     if (a.path == 4) return lin::launch_thin(a, stream);

@@ -325,7 +325,14 @@ def _attend_prompts(ctx, state: GigezenState, i: int, y: GPUBuffer2D, z: GPUBuff
     cols = w.k_cols + a.heads * a.vdim
     kv = state.rows(f"kv{cols}", plan.kv_rows, cols, state.dtype)
     latents = cache.layers[0].v_cache.buffer.view(-1, a.kv_rank)
-    for _, _, cache_row, visible, kv_row in plan.portions:
+    n = len(plan.portions)
+    together = plan.groups is not None and state.dtype == torch.bfloat16 and a.kv_rank % 8 == 0 and cols % 8 == 0 and n <= 1024
+    if together:
+        # all portions in one launch: a thousand rows alone leave most of the chip idle
+        linear(ctx, _b2(latents), w.expand, a.kv_rank, [OutputSegment(cols, SEG_STORE, _sub(kv, 0, plan.kv_rows))], groups=n, group_w=0,
+               group_rows=plan.groups[:n + 1], max_group_rows=max(p[3] for p in plan.portions), group_x_rows=plan.groups[n + 1:],
+               rows=plan.kv_rows)
+    for _, _, cache_row, visible, kv_row in () if together else plan.portions:
         linear(ctx, _b2(latents[cache_row:cache_row + visible]), w.expand, a.kv_rank,
                [OutputSegment(cols, SEG_STORE, _sub(kv, kv_row, visible))])
     latent.latent_prefill(ctx, y, _sub(kv, 0, plan.kv_rows, 0, a.heads * a.dim), _sub(kv, 0, plan.kv_rows, w.k_cols), a, plan,

@@ -100,6 +100,7 @@ class PromptPlan:
     table: Optional[torch.Tensor]  # int32 [portions, 6] on the device
     n_blocks: int
     kv_rows: int
+    groups: Optional[torch.Tensor] = None  # int32 on the device, groups_rows() of several portions that are expanded
 
     BLOCK = 256  # query rows of one block of the kernel
 
@@ -122,6 +123,13 @@ class PromptPlan:
             out += [row0, n, kv_row, cache_row, visible - n, first]
             first += (n + PromptPlan.BLOCK - 1) // PromptPlan.BLOCK
         return out
+
+    def groups_rows(self) -> list:
+        """Where the portions' expanded rows begin (and the last one's end), then the cache rows they are made from; nothing for a
+        single portion and for portions that are read in place."""
+        if self.kv_rows == 0 or len(self.portions) < 2:
+            return []
+        return [p[4] for p in self.portions] + [self.kv_rows] + [p[2] for p in self.portions]
 
 
 def prefill_supported(shape: LatentShape, dtype: torch.dtype) -> bool:

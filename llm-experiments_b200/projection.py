@@ -123,15 +123,17 @@ class OutputSegment:
 def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Sequence[OutputSegment],
            residual: Optional[GPUBuffer2D] = None, limit: float = 0.0, groups: int = 1, group_x: int = 0, group_w: int = 0,
            group_rows: Optional[torch.Tensor] = None, max_group_rows: int = 0, path: int = 0,
-           bias: Optional[GPUBuffer1D] = None) -> None:
+           bias: Optional[GPUBuffer1D] = None, group_x_rows: Optional[torch.Tensor] = None, rows: Optional[int] = None) -> None:
     """``x @ w`` (``+ bias``, fp32) with the output columns cut into segments, fp32 or bfloat16 storage, any sizes (``b2kv_linear``).
 
     ``x`` ``[rows, >= k]`` and ``w`` (rows of the weight matrix, ``[in, out]``) may be views with a row pitch.  With
     ``groups`` > 1, group g reads ``x`` from element ``g * group_x`` on and ``w`` from ``g * group_w`` on (the heads of a
     per-head product), or, with ``group_rows`` (int32 ``[groups + 1]`` on the device), rows ``group_rows[g] ..
-    group_rows[g + 1] - 1`` of ``x`` (the experts of a mixture; at most ``max_group_rows`` rows each).  ``path`` forces a
+    group_rows[g + 1] - 1`` of ``x`` (the experts of a mixture; at most ``max_group_rows`` rows each).  With
+    ``group_x_rows`` as well (int32 ``[groups]``), group g's rows of ``x`` start there, ``rows`` counts all groups' rows, and
+    ``group_w`` 0 is one matrix for all (tiled kernel).  ``path`` forces a
     kernel (1 CUDA cores, 2 weight streaming, 3 tiled, 4 few input features)."""
-    rows, n = x.shape[0], segments[-1].end
+    rows, n = x.shape[0] if group_x_rows is None else rows, segments[-1].end
     if rows <= 0 or k <= 0 or n <= 0:
         raise ValueError(f"linear: Invalid dimensions x=({rows}, {k}), w=({k}, {n})")
     if x.buffer.dtype != w.buffer.dtype or any(t.buffer.stride(1) != 1 for t in (x, w)):
@@ -158,5 +160,7 @@ def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Se
         a.bias = bias.buffer.data_ptr()
     if group_rows is not None:
         a.group_rows = group_rows.data_ptr()
+    if group_x_rows is not None:
+        a.group_x_rows, a.x_rows = group_x_rows.data_ptr(), x.shape[0]
     stream = batch_op_begin(ctx)
     _native.check(_native.lib.b2kv_linear(ctypes.byref(a), dev_status_ptr(ctx), stream))

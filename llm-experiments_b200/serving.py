@@ -204,11 +204,11 @@ def forward(ctx: GPUContext, state: SequenceState, entries: Sequence[Tuple[int, 
     plans = state.prompt_plans(spans) if spans else {}
     # one upload per step: ids, sequences, positions, wanted rows, lengths behind the step, runs of rows, prompt tables
     parts = [np.concatenate(ids), np.concatenate(slots), np.concatenate(pos), want, lens, np.ravel(runs[True]), np.ravel(runs[False])]
-    parts += [plan.rows() for plan in plans.values()]
+    parts += [plan.rows() for plan in plans.values()] + [plan.groups_rows() for plan in plans.values()]
     host = torch.from_numpy(np.concatenate([np.asarray(part, dtype=np.int32) for part in parts])).pin_memory()
     pieces = list(host.to(ctx.device, non_blocking=True).split([len(part) for part in parts]))
-    for plan, table in zip(plans.values(), pieces[7:]):
-        plan.table = table
+    for plan, table, groups in zip(plans.values(), pieces[7:], pieces[7 + len(plans):]):
+        plan.table, plan.groups = table, groups if len(groups) else None
     segments = [RowSegments(table, len(r), max(n for _, n, _ in r)) if r else None
                 for table, r in ((pieces[5], runs[True]), (pieces[6], runs[False]))]
     batch_begin(ctx)

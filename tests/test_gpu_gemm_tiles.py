@@ -45,3 +45,22 @@ def test_matmul_with_everything_behind_it(pkg, rows, tiles, cols):
     z = x.double() @ w.double() + bias.double()
     close(out[:rows], z * torch.sigmoid(1.702 * z) + res.double(), BF)
     assert (out[rows] == 7).all()
+
+
+@pytest.mark.parametrize("counts,starts", [((300, 1, 513), (700, 0, 40)), ((129, 128), (3, 3)), ((5, 0, 900, 17), (10, 20, 30, 931))])
+def test_runs_of_rows_anywhere_with_one_matrix(pkg, counts, starts):
+    """Groups whose rows of x start anywhere, also where others lie, or end with x."""
+    import numpy as np
+
+    from llm_experiments_b200 import projection as proj
+
+    ctx, K, n = make_ctx(pkg), 136, 520
+    x, w = rnd((948 if starts[-1] == 931 else 1100, K), BF, 8), rnd((K, n), BF, 9, K ** -0.5)
+    offs = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    out = torch.full((sum(counts) + 1, n), 7.0, dtype=BF, device="cuda")
+    run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), K, [proj.OutputSegment(n, proj.SEG_STORE, wrap(pkg, out[:-1]))], groups=len(counts), group_w=0,
+        group_rows=torch.from_numpy(offs).cuda(), max_group_rows=max(counts),
+        group_x_rows=torch.tensor(starts, dtype=torch.int32, device="cuda"), rows=sum(counts))
+    want = torch.cat([x[s:s + c].double() @ w.double() for s, c in zip(starts, counts)])
+    close(out[:-1], want, BF)
+    assert (out[-1] == 7).all()
