@@ -2,19 +2,20 @@
 // 24 bits, and a product is h h' + (h m' + m h') + (m m' + h l' + l h'); what is dropped is below 2^-24 of it.
 //
 // The tensor core adds in fp32 but truncates, so a long chain of accumulations would lean towards zero by more than fp32 sums err.
-// Therefore the leading products h h' are accumulated over kChain input features only; the partial sums are taken out of tensor memory
+// Therefore the leading products h h' are accumulated over the 64 input features of a step only; the partial sums are taken out of tensor memory
 // and added up in registers, rounded to nearest.  The other five products, 2^-8 of the first and less, stay in an accumulator of
-// their own until the end.  Measured against 64 bits, 2-norm of the error over that of the result: 6e-8 at 128 input features, 8e-8 at
-// 768, 1.1e-7 at 3072, where sums of fp32 multiply-adds in order are off by 2.0e-7, 5.0e-7 and 9.9e-7 (chains of 64 input features
-// gave 8e-8, 9e-8 and 1.1e-7, and no more speed).  693 rows, 768 -> 3072: 48 us against 127 of linear_f32_tile_kernel; 3072 -> 768:
-// 57 and 130; 60 rows, 768 -> 3072: 17 and 25.
+// their own until the end.  Measured against 64 bits, 2-norm of the error over that of the result: 8e-8 at 128 input features, 9e-8 at
+// 768, 1.1e-7 at 3072, where sums of fp32 multiply-adds in order are off by 2.0e-7, 5.0e-7 and 9.9e-7.  693 rows, 768 -> 3072: 38 us
+// against 127 of linear_f32_tile_kernel; 3072 -> 768: 42 and 130; 60 rows, 768 -> 3072: 15 and 25.
 //
 //   * a CTA has 128 x 128 outputs; steps of 64 input features through two stages of 96 KB;
 //   * warps 8-15 read fp32 rows of x and w, a step ahead in registers, and write the parts as the operands the MMAs want: x K-major,
 //     w as it lies (MN-major), 128-byte swizzle;
-//   * a thread of warp 8 issues 24 tcgen05.mma per step: 6 x 64 clocks per 16 input features, a sixth of the tensor peak, which is
-//     four times what the CUDA cores have (a seventeenth warp for it would leave all others 96 registers);
-//   * warps 0-7 take the leading sums out (two accumulators in turn), thread = row and half of the columns;
+//   * a thread of warp 0 issues 24 tcgen05.mma per step: 6 x 64 clocks per 16 input features, a sixth of the tensor peak, which is
+//     four times what the CUDA cores have.  Issuing takes as long as the products do, so it is not for the warps that make the parts
+//     (48 us with one of them), and a seventeenth warp would leave all others 96 registers (41 us, and spills);
+//   * warps 0-7 take the leading sums out (two accumulators in turn), thread = row and half of the columns, warp 0 always one step
+//     behind what it has issued;
 //   * a product whose tiles leave SMs idle has its input features cut into ranges, one per CTA of a cluster, whose sums meet in
 //     distributed shared memory, in order.
 //
@@ -31,8 +32,6 @@ namespace linf32tc {
 using namespace tc;
 
 constexpr int kBM = 128, kBN = 128, kBK = 64, kStages = 2;
-constexpr int kChain = 32;                          // input features per leading sum
-constexpr int kSums = kBK / kChain;                 // leading sums per step
 constexpr int kPartBytes = 128 * kBK * 2;           // one part of x or of w: 16 KB
 constexpr int kStageBytes = 6 * kPartBytes;         // x: h, m, l; w: h, m, l
 constexpr int kSumWarps = 8, kSplitWarps = 8;
@@ -135,23 +134,57 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
         for (int j = 0; j < 64; ++j) acc[j] = 0.f;
         auto add = [&](uint32_t at) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                uint32_t r[16];
-                tmem_ld16(at + q * 16, r);
+            for (int half = 0; half < 2; ++half) {
+                uint32_t r[32];
+                tmem_ld32(at + half * 32, r);
                 tmem_wait_ld();
 #pragma unroll
-                for (int j = 0; j < 16; ++j) acc[q * 16 + j] += __uint_as_float(r[j]);
+                for (int j = 0; j < 32; ++j) acc[half * 32 + j] += __uint_as_float(r[j]);
             }
         };
-        bool ok = true;
-        for (int c = 0; c < kSums * steps; ++c) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&sm.sum_full[c & 1], (c >> 1) & 1));
+        // the products of step s, once all parts are written and the sums of the step before last are taken out
+        auto issue = [&](int s) {
+            constexpr uint32_t idesc = instr_desc(0, 1, kBN);
+            constexpr uint64_t kPart = kPartBytes >> 4;
+            const int st = s % kStages;
+            if (!mbar_wait(&sm.full[st], (s / kStages) & 1) || !mbar_wait(&sm.sum_empty[s & 1], ((s >> 1) & 1) ^ 1)) return false;
+            tc_fence_after();
+            const uint64_t dx = smem_desc(smem_u32(ring + st * kStageBytes), 16, 1024);
+            const uint64_t dw = smem_desc(smem_u32(ring + st * kStageBytes + 3 * kPartBytes), kBK * 128, 1024);
+#pragma unroll
+            for (int kk = 0; kk < kBK / 16; ++kk)  // 16 input features: 32 bytes of x's rows, 16 rows of w
+                mma_ss(tmem + (s & 1) * kBN, dx + 2 * kk, dw + 128 * kk, idesc, kk ? 1u : 0u);
+            mma_commit(&sm.sum_full[s & 1]);
+#pragma unroll
+            for (int kk = 0; kk < kBK / 16; ++kk) {
+                const uint64_t ax = dx + 2 * kk, bw = dw + 128 * kk;
+                mma_ss(tmem + kColRest, ax, bw + 2 * kPart, idesc, (s | kk) ? 1u : 0u);
+                mma_ss(tmem + kColRest, ax + 2 * kPart, bw, idesc, 1u);
+                mma_ss(tmem + kColRest, ax + kPart, bw + kPart, idesc, 1u);
+                mma_ss(tmem + kColRest, ax, bw + kPart, idesc, 1u);
+                mma_ss(tmem + kColRest, ax + kPart, bw, idesc, 1u);
+            }
+            mma_commit(&sm.empty[st]);
+            if (s + 1 == steps) mma_commit(&sm.done);
+            return true;
+        };
+        auto issue_by_warp0 = [&](int s) {
+            if (warp != 0 || s >= steps) return true;
+            bool good = true;
+            if (lane == 0) good = issue(s);
+            return __all_sync(0xffffffffu, good) != 0;
+        };
+        bool ok = issue_by_warp0(0);
+        for (int s = 0; s < steps && ok; ++s) {
+            ok = issue_by_warp0(s + 1);
+            if (!ok) break;
+            ok = __all_sync(0xffffffffu, mbar_wait(&sm.sum_full[s & 1], (s >> 1) & 1));
             if (!ok) break;
             tc_fence_after();
-            add(t_lane + (c & 1) * kBN);
+            add(t_lane + (s & 1) * kBN);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.sum_empty[c & 1]);
+            if (lane == 0) mbar_arrive(&sm.sum_empty[s & 1]);
         }
         if (ok && steps > 0) {
             ok = __all_sync(0xffffffffu, mbar_wait(&sm.done, 0));
@@ -181,39 +214,6 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         };
-        // the products of step s, once all warps have written their parts
-        auto issue = [&](int s) {
-            constexpr uint32_t idesc = instr_desc(0, 1, kBN);
-            constexpr uint64_t kPart = kPartBytes >> 4;
-            const int st = s % kStages;
-            if (!mbar_wait(&sm.full[st], (s / kStages) & 1)) return false;
-            const uint64_t dx = smem_desc(smem_u32(ring + st * kStageBytes), 16, 1024);
-            const uint64_t dw = smem_desc(smem_u32(ring + st * kStageBytes + 3 * kPartBytes), kBK * 128, 1024);
-#pragma unroll
-            for (int part = 0; part < kSums; ++part) {
-                const int c = kSums * s + part;
-                if (!mbar_wait(&sm.sum_empty[c & 1], ((c >> 1) & 1) ^ 1)) return false;
-                tc_fence_after();
-#pragma unroll
-                for (int i = 0; i < kChain / 16; ++i) {  // 16 input features: 32 bytes of x's rows, 16 rows of w
-                    const int kk = part * (kChain / 16) + i;
-                    mma_ss(tmem + (c & 1) * kBN, dx + 2 * kk, dw + 128 * kk, idesc, i ? 1u : 0u);
-                }
-                mma_commit(&sm.sum_full[c & 1]);
-#pragma unroll
-                for (int i = 0; i < kChain / 16; ++i) {
-                    const int kk = part * (kChain / 16) + i;
-                    const uint64_t ax = dx + 2 * kk, bw = dw + 128 * kk;
-                    mma_ss(tmem + kColRest, ax, bw + 2 * kPart, idesc, (s | kk) ? 1u : 0u);
-                    mma_ss(tmem + kColRest, ax + 2 * kPart, bw, idesc, 1u);
-                    mma_ss(tmem + kColRest, ax + kPart, bw + kPart, idesc, 1u);
-                    mma_ss(tmem + kColRest, ax, bw + kPart, idesc, 1u);
-                    mma_ss(tmem + kColRest, ax + kPart, bw, idesc, 1u);
-                }
-            }
-            mma_commit(&sm.empty[st]);
-            return true;
-        };
         float2 check = make_float2(0.f, 0.f);
         if (steps > 0) read_x(k_first), read_w(k_first);
         bool ok = true;
@@ -238,13 +238,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.full[st]);
-            if (warp == kSumWarps) {
-                if (lane == 0) ok = issue(s);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-            }
         }
-        if (warp == kSumWarps && lane == 0 && ok) mma_commit(&sm.done);
         if (check.x != 0.f || check.y != 0.f) sm.odd = 1;  // (NaN)
         if (!ok) sm.abort_flag = 1;
     }
