@@ -206,13 +206,13 @@ __global__ void __launch_bounds__(kWarps * 32) gqa_decode_kernel(const GqaDecode
     }
 }
 
-// Runs of rows of one sequence in fp32 (prompt portions, which fp32 has no tensor-core form for): 32 rows of one head per CTA and 64
+// Runs of rows of one sequence in fp32 (prompt portions, which fp32 has no tensor-core form for): 16 rows of one head per CTA and 64
 // tokens at a time, keys and values read into shared memory once for all of the rows.  A thread has 4 rows x 4 tokens of the scores
 // and 4 rows x 4 columns (per 64) of the output, 64 multiply-adds for every eight 16-byte reads of shared memory; the 16 lanes of a
 // row group keep the rows' softmax among themselves.  gqa_decode_kernel reads every key and value again for every row and reduces
-// over the warp for every token: 174 us for 693 rows of three prompts (12 heads of 64, 4 of them for keys), against 100.
-// Rows of other sequences in the same 32 are taken in turn; a weight of zero is never multiplied with what a row must not see.
-constexpr int kRunRows = 32, kRunTokens = 64, kRunThreads = 128;
+// over the warp for every token: 174 us for 693 rows of three prompts (12 heads of 64, 4 of them for keys), against 90
+// (100 with 32 rows: half as many warps to hide one another's waits).  Rows of other sequences in the same 16 are taken in turn; a weight of zero is never multiplied with what a row must not see.
+constexpr int kRunRows = 16, kRunTokens = 64, kRunThreads = 64;
 
 template <int kD>  // dim and vdim, rounded up
 __global__ void __launch_bounds__(kRunThreads) gqa_run_f32_kernel(const __grid_constant__ GqaDecodeArgs a) {
@@ -406,7 +406,7 @@ int launch_runs(const GqaDecodeArgs& a, void* stream) {
 // Rows come in runs when there are several for every place; a decoding step has one per sequence at most, and a CTA would take
 // its sequences one after the other.
 int launch_runs_f32(const GqaDecodeArgs& a, void* stream) {
-    if (a.rows < 4 * a.n_slots || a.rows < 2 * kRunRows || (a.rows + kRunRows - 1) / kRunRows > 65535) return B2KV_ERR_UNSUPPORTED;
+    if (a.rows < 4 * a.n_slots || a.rows < 64 || (a.rows + kRunRows - 1) / kRunRows > 65535) return B2KV_ERR_UNSUPPORTED;
     const int widest = std::max(a.dim, a.vdim);
     if (widest > 128 || a.dim % 4 || a.vdim % 4 || a.ld_q % 4 || !aligned16(a.q) || !aligned16(a.k_cache) || !aligned16(a.v_cache))
         return B2KV_ERR_UNSUPPORTED;
