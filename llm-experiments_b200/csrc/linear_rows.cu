@@ -30,7 +30,9 @@ constexpr int kFeat = 128;   // output features per CTA (MMA M)
 constexpr int kKTile = 128;  // input features per stage
 constexpr int kMaxStages = 6;
 constexpr int kRingBytes = 200 * 1024;
-constexpr int kRingBytesTwo = 100 * 1024;  // two CTAs per SM, when there are several waves of them
+// Two CTAs per SM, when there are several waves of them: three stages for up to 16 rows (with two, as in 100 KB, a step of 64 rows
+// over 64 experts took 1444 us, 1424 so; with 112 KB the second CTA no longer fits and it took 1551).
+constexpr int kRingBytesTwo = 110 * 1024;
 constexpr int kSmemBytes = 224 * 1024;
 constexpr int kWBytes = kKTile * kFeat * 2;
 constexpr int kWHalf = kWBytes / 2;
@@ -48,6 +50,7 @@ struct Params {
     b2kv_linear_args a;
     int32_t* dev_status;
     int tiles_n, Bn, box_rows, stages, splits, split_shift;
+    int ring_bytes;
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -145,12 +148,12 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     }
     const int Bn = by_rows ? (n_rows + 15) / 16 * 16 : p.Bn;
     const uint32_t x_span = static_cast<uint32_t>(Bn) * 128u;  // Bn rows of one 64-feature span
-    const uint32_t x_span_max = static_cast<uint32_t>(p.Bn) * 128u;
-    uint8_t* const x_ring = w_ring + p.stages * kWBytes;
-    const int n_st = p.stages;
-    float* const recv = reinterpret_cast<float*>(x_ring + p.stages * 2 * x_span_max);
-    const int rows_per_cta = p.Bn >> p.split_shift;
     const uint32_t stage_bytes = kWBytes + 2 * x_span;
+    // (an expert's rows are often far fewer than there may be: more stages in the same ring)
+    const int n_st = by_rows ? min(kMaxStages, p.ring_bytes / static_cast<int>(stage_bytes)) : p.stages;
+    uint8_t* const x_ring = w_ring + n_st * kWBytes;
+    float* const recv = reinterpret_cast<float*>(w_ring + p.ring_bytes);
+    const int rows_per_cta = p.Bn >> p.split_shift;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kMaxStages; ++s) {
@@ -177,7 +180,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             tma_load_3d(w_ring + st * kWBytes + kWHalf, &tm_w, &sm.full[st], c0 + 64, k0, g);
         };
         auto load_x = [&](int st, int k0) {
-            uint8_t* dst = x_ring + st * 2 * x_span_max;
+            uint8_t* dst = x_ring + st * 2 * x_span;
             for (int r = 0; r < Bn; r += p.box_rows) {
                 tma_load_3d(dst + r * 128, &tm_x, &sm.full[st], k0, by_rows ? 0 : g, row0 + r);
                 tma_load_3d(dst + x_span + r * 128, &tm_x, &sm.full[st], k0 + 64, by_rows ? 0 : g, row0 + r);
@@ -217,7 +220,7 @@ linear_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 if (!ok) break;
                 tc_fence_after();
                 const uint64_t da = smem_desc(smem_u32(w_ring + st * kWBytes), kWHalf, 1024);
-                const uint64_t db = smem_desc(smem_u32(x_ring + st * 2 * x_span_max), 16, 1024);
+                const uint64_t db = smem_desc(smem_u32(x_ring + st * 2 * x_span), 16, 1024);
 #pragma unroll
                 for (int kk = 0; kk < kKTile / 16; ++kk) {
                     const uint32_t b_off = (kk >> 2) * x_span + (kk & 3) * 32;
@@ -383,7 +386,9 @@ int linear_rows_tc(const b2kv_linear_args& a, int32_t* dev_status, void* stream)
     const bool waves = tiles * p.splits > device_sm_count();
     const int ring = waves ? kRingBytesTwo : kRingBytes;
     p.stages = std::max(2, std::min(std::min(kMaxStages, std::max(n_k, 1)), std::min(ring, kSmemBytes - recv_bytes) / stage_bytes));
-    const size_t smem = static_cast<size_t>(p.stages) * stage_bytes + recv_bytes + 1024;
+    p.ring_bytes = p.stages * stage_bytes;
+    if (a.group_rows && waves) p.ring_bytes = std::max(p.ring_bytes, ring);
+    const size_t smem = static_cast<size_t>(p.ring_bytes) + recv_bytes + 1024;
     static int configured[64] = {0};
     int dev = 0;
     B2KV_CUDA_TRY(cudaGetDevice(&dev));
