@@ -211,7 +211,8 @@ __global__ void __launch_bounds__(kWarps * 32) gqa_decode_kernel(const GqaDecode
 // and 4 rows x 4 columns (per 64) of the output, 64 multiply-adds for every eight 16-byte reads of shared memory; the 16 lanes of a
 // row group keep the rows' softmax among themselves.  gqa_decode_kernel reads every key and value again for every row and reduces
 // over the warp for every token: 174 us for 693 rows of three prompts (12 heads of 64, 4 of them for keys), against 90
-// (100 with 32 rows: half as many warps to hide one another's waits).  Rows of other sequences in the same 16 are taken in turn; a weight of zero is never multiplied with what a row must not see.
+// (100 with 32 rows: half as many warps to hide one another's waits).
+// Rows of other sequences in the same 16 are taken in turn; a weight of zero is never multiplied with what a row must not see.
 constexpr int kRunRows = 16, kRunTokens = 64, kRunThreads = 64;
 
 template <int kD>  // dim and vdim, rounded up
