@@ -5,8 +5,8 @@
 // Therefore the leading products h h' are accumulated over the 64 input features of a step only; the partial sums are taken out of tensor memory
 // and added up in registers, rounded to nearest.  The other five products, 2^-8 of the first and less, stay in an accumulator of
 // their own until the end.  Measured against 64 bits, 2-norm of the error over that of the result: 8e-8 at 128 input features, 9e-8 at
-// 768, 1.1e-7 at 3072, where sums of fp32 multiply-adds in order are off by 2.0e-7, 5.0e-7 and 9.9e-7.  693 rows, 768 -> 3072: 38 us
-// against 127 of linear_f32_tile_kernel; 3072 -> 768: 42 and 130; 60 rows, 768 -> 3072: 15 and 25.
+// 768, 1.1e-7 at 3072, where sums of fp32 multiply-adds in order are off by 2.0e-7, 5.0e-7 and 9.9e-7.  693 rows, 768 -> 3072: 35 us
+// against 127 of linear_f32_tile_kernel; 3072 -> 768: 39 and 130; 60 rows, 768 -> 3072: 15 and 25.
 //
 //   * a CTA has 128 x 128 outputs; steps of 64 input features through two stages of 96 KB;
 //   * warps 8-15 read fp32 rows of x and w, a step ahead in registers, and write the parts as the operands the MMAs want: x K-major,
@@ -82,6 +82,7 @@ __device__ __forceinline__ void split3(const float4& v, uint8_t* at, float2& che
     for (int part = 0; part < 3; ++part) {
         const uint32_t a = pack_bf16(r0.x, r0.y), b = pack_bf16(r1.x, r1.y);
         *reinterpret_cast<uint2*>(at + part * kPartBytes) = make_uint2(a, b);
+        if (part == 2) break;  // (what is not finite is not a number by now: infinity less infinity)
         r0 = __ffma2_rn(make_float2(__uint_as_float(a << 16), __uint_as_float(a & 0xffff0000u)), minus, r0);
         r1 = __ffma2_rn(make_float2(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u)), minus, r1);
     }
@@ -198,7 +199,18 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
         const int xc = (ct & 15) * 4, xr = ct >> 4;  // x: four input features of the rows xr, + 16, ..
         const int wc = (ct & 31) * 4, wk = ct >> 5;  // w: four columns of the input features wk, + 8, ..
         float4 xv[8], wv[8];
+        // (whole tiles without a condition per piece: instructions are what the parts cost, 38 us for the first size above with one)
+        const bool rows_in = row0 + kBM <= a.rows, cols_in = col0 + kBN <= a.N;
+        const float* const xp = x + static_cast<int64_t>(row0 + xr) * a.ld_x + xc;
+        const float* const wp = w + static_cast<int64_t>(wk) * a.ld_w + col0 + wc;
+        const int64_t x_step = 16 * a.ld_x, w_step = 8 * a.ld_w;
         auto read_x = [&](int k0) {
+            if (rows_in && k0 + kBK <= k_end) {
+                const float* p = xp + k0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i, p += x_step) xv[i] = *reinterpret_cast<const float4*>(p);
+                return;
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int r = row0 + xr + 16 * i;
@@ -207,6 +219,12 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
             }
         };
         auto read_w = [&](int k0) {
+            if (cols_in && k0 + kBK <= k_end) {
+                const float* p = wp + static_cast<int64_t>(k0) * a.ld_w;
+#pragma unroll
+                for (int i = 0; i < 8; ++i, p += w_step) wv[i] = *reinterpret_cast<const float4*>(p);
+                return;
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int k = k0 + wk + 8 * i;
