@@ -136,9 +136,12 @@ static int launch_thin(const b2kv_linear_args& a, void* stream) {
         return B2KV_ERR_UNSUPPORTED;
     if (!aligned16(a.w) || !aligned16(sg.out) || a.ld_w % 2 || sg.ld % 2 || (a.residual && (!aligned16(a.residual) || a.ld_residual % 2)))
         return B2KV_ERR_UNSUPPORTED;
-    // few rows: enough CTAs to be quick; many: the columns of w are loaded once per tile of rows
-    const int row_tile = a.rows > 1024 ? kThinRows : 8;
-    const dim3 grid((a.N / 2 + kThinThreads - 1) / kThinThreads, (a.rows + row_tile - 1) / row_tile);
+    // few rows: enough CTAs to be quick; many: the columns of w are loaded once per tile of rows, unless that leaves less than six CTAs
+    // per SM (a row after the other is a chain: 3548 rows x 1024 columns 29 us in tiles of 64, 18 in tiles of 16)
+    int row_tile = a.rows > 1024 ? kThinRows : 8;
+    const long long cols = (a.N / 2 + kThinThreads - 1) / kThinThreads;
+    while (row_tile > 8 && cols * ((a.rows + row_tile - 1) / row_tile) < 6LL * device_sm_count()) row_tile /= 2;
+    const dim3 grid(static_cast<unsigned>(cols), (a.rows + row_tile - 1) / row_tile);
     if (grid.y > 65535u) return B2KV_ERR_UNSUPPORTED;
     OverlapLaunch launch(grid, kThinThreads, 0, stream);
     B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, a.K <= 16 ? linear_thin_kernel<16> : linear_thin_kernel<32>, a, row_tile));
