@@ -409,7 +409,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_ad
                 }
                 if (p.gelu) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) z[i] = __fdividef(z[i], 1.0f + __expf(-1.702f * z[i]));
+                    for (int i = 0; i < 8; ++i) z[i] = lin::quotient(z[i], 1.0f + __expf(-1.702f * z[i]));
                 }
                 if (p.residual != nullptr) {
                     const uint4 rv = *reinterpret_cast<const uint4*>(p.residual + row_off + col);

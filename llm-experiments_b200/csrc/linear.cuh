@@ -6,14 +6,24 @@
 namespace b2kv {
 namespace lin {
 
-// x * sigmoid(1.702 x) of the clamped gate times the clamped up part plus one; silu(gate) * up.  kDivide: with the operator's
-// division, a branch to a subroutine per element, which few rows do not notice; otherwise the quotients are __fdividef's (2 ulp of
-// fp32; results are rounded to bf16): an epilogue thread of a tiled product has 128 of them one after the other per tile (2975 rows,
-// K = 2048, 10880 gated columns beside 3648 plain ones: 259 us with the division, 176 without; the experts' 17850 rows x 2816 gated
-// columns: 417 and 282).
-template <bool kDivide = false>
+// a / b for b = 1 + exp(..), so from one on, infinity among it: the operator's quotient without its branch to a subroutine.  An
+// approximate reciprocal, one step of Newton's for it, and the remainder a - q b, exact in a fused multiply-add, put right what is missing
+// of the quotient (Markstein, IBM J. Res. Dev. 34, 1990).  Where the reciprocal would be a subnormal number b is scaled; where the
+// remainder is no number (a or b infinite) or nothing is missing the first quotient stands.  For 1 + __expf(-a) and
+// 1 + __expf(-1.702 a) it has the operator's bits for each of the 2^32 fp32 numbers a (tried).
+__device__ __forceinline__ float quotient(float a, float b) {
+    const float s = b > 0x1p100f ? 0x1p-64f : 1.0f;
+    b *= s;
+    float r = __fdividef(1.0f, b);
+    r = fmaf(fmaxf(fmaf(-b, r, 1.0f), -1.0f), r, r);  // (the maximum: 0 for the reciprocal of infinity)
+    const float q = a * r, left = fmaf(-q, b, a);
+    return (left != 0.0f && fabsf(left) < INFINITY ? fmaf(left, r, q) : q) * s;
+}
+
+// x * sigmoid(1.702 x) of the clamped gate times the clamped up part plus one; silu(gate) * up.  An epilogue thread of a tiled product
+// has 128 quotients one after the other per tile, whose latencies have to overlap (2975 rows, K = 2048, 10880
+// gated columns beside 3648 plain ones: 192 us with the operator's division, 150 so; the experts' 17850 rows x 2816 gated columns: 308 and 230).
 __device__ __forceinline__ float glu(int kind, float g, float u, float limit) {
-    const auto quotient = [](float a, float b) { return kDivide ? a / b : __fdividef(a, b); };
     if (kind == B2KV_SEG_GLU_SILU) return quotient(g, 1.0f + __expf(-g)) * u;
     g = fminf(g, limit);
     u = fminf(fmaxf(u, -limit), limit);
@@ -62,7 +72,7 @@ __device__ __forceinline__ int segment_first(const b2kv_linear_args& a, int s) {
 // Exact exponential for the fp32 path; the bf16 paths round the result to 8 bits anyway.
 template <typename T>
 __device__ __forceinline__ float glu_value(int kind, float g, float u, float limit) {
-    if (sizeof(T) == 2) return glu<true>(kind, g, u, limit);
+    if (sizeof(T) == 2) return glu(kind, g, u, limit);
     if (kind == B2KV_SEG_GLU_SILU) return g / (1.0f + expf(-g)) * u;
     g = fminf(g, limit);
     u = fminf(fmaxf(u, -limit), limit);

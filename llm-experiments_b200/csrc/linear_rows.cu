@@ -93,7 +93,7 @@ __device__ __forceinline__ void emit(const Place& pl, float (&v)[kN], const int6
             const float other = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
             const float g = odd ? other : v[j], u = odd ? v[j + 1] : other;
             const int64_t r = odd ? row[j + 1] : row[j];
-            const float z = lin::glu<true>(pl.kind, g, u, limit);
+            const float z = lin::glu(pl.kind, g, u, limit);
             if (r >= 0 && pl.live) out[r * pl.ld] = __float2bfloat16_rn(z);
         }
         return;

@@ -64,3 +64,39 @@ def test_runs_of_rows_anywhere_with_one_matrix(pkg, counts, starts):
     want = torch.cat([x[s:s + c].double() @ w.double() for s, c in zip(starts, counts)])
     close(out[:-1], want, BF)
     assert (out[-1] == 7).all()
+
+
+@pytest.mark.parametrize("kind", ["SEG_GLU_SILU", "SEG_GLU_CLAMP"])
+def test_gated_outputs_have_the_bits_of_the_product_for_few_rows(pkg, kind):
+    """Rows of the identity pick the weights as sums, the same in both kernels; gates of all sizes, up to where the denominator is no
+    normal number's reciprocal any more, and infinity."""
+    from llm_experiments_b200 import projection as proj
+
+    ctx, n = make_ctx(pkg), 4096
+    w = rnd((128, n), BF, 11, 30.0)
+    w[1, ::2], w[2, ::2] = torch.linspace(-88.5, -86, n // 2, device="cuda"), torch.linspace(-52, -50, n // 2, device="cuda")
+    w[1:3, 1::2] = 3e4
+    w[3, 0], w[4, 2], w[5, 4], w[6, 6] = float("inf"), -float("inf"), -3e38, 3e38
+    got = []
+    for path in (2, TILED):
+        got.append(torch.empty((128, n // 2), dtype=BF, device="cuda"))
+        run(pkg, ctx, wrap(pkg, torch.eye(128, dtype=BF, device="cuda")), wrap(pkg, w), 128,
+            [proj.OutputSegment(n, getattr(proj, kind), wrap(pkg, got[-1]))], limit=1e30, path=path)
+    assert torch.equal(got[0].view(torch.int16), got[1].view(torch.int16))
+    assert (got[1][1 if kind == "SEG_GLU_SILU" else 2] != 0).all()
+
+
+def test_gelu_where_the_denominator_is_large(pkg):
+    """z sigmoid(1.702 z) is a normal number of bf16 at z = -52; nothing of it is lost before the rounding."""
+    from llm_experiments_b200 import projection
+
+    ctx, n = make_ctx(pkg), 2048
+    z = torch.linspace(-52, 3, 200 * n, device="cuda").view(200, n).to(BF)
+    out = torch.empty((200, n), dtype=BF, device="cuda")
+    pkg.gpu.batch_begin(ctx)
+    projection.matmul(ctx, wrap(pkg, torch.eye(200, dtype=BF, device="cuda")), wrap(pkg, z), wrap(pkg, out), activation="gelu")
+    pkg.gpu.batch_commit(ctx)
+    want = z.double() * torch.sigmoid(1.702 * z.double())
+    seen = want.abs() > 1.2e-38
+    torch.testing.assert_close(out.double()[seen], want[seen], rtol=2.0 ** -8 + 2.0 ** -16, atol=0)  # bf16, and __expf of 90: 2^-16.5
+    assert seen.sum() > 200 * n * 0.95
