@@ -9,13 +9,13 @@
 // Three kernels.  What does not depend on the state is made for many chunks at once (gla_prepare_kernel): one CTA per chunk and
 // head, thread = two key channels; A's products of decays are carried along exactly instead of being taken apart into factors that
 // could overflow, and its entries are summed over the channels 32 at a time.  The result is a record per chunk and head that is
-// byte for byte what the second kernel wants in shared memory.  Records are made a slice of the segments at a time, small enough
-// to stay in L2.
+// byte for byte what the second kernel wants in shared memory.  Records are made a slice of the segments at a time, which bounds the
+// workspace.
 //
 // gla_state_kernel has one CTA per (64 value columns of a head, segment) and walks the chunks in order.  Nothing in the recurrence
 // connects value columns, and a chunk is a chain of dependent products, so what counts is how few warps share an SM's tensor pipe:
 // one per scheduler here (with a whole head's 256 columns on one SM a prompt of 2048 tokens kept 8 SMs busy: two prompts of 1750 tokens, 8 heads of
-// 128 x 256, took 402 us, then 170, and 125 with the keys in two parts).
+// 128 x 256, took 366 us, 181 so).
 //   * every warp owns 16 value columns of the state, transposed, as accumulators of mma.m16n8k16: the state never
 //     leaves registers between the first and the last chunk.  As an A operand of the first product the accumulators need no
 //     shuffle.  A step of the recurrence is sixteen tokens deep, one k-step of this instruction; larger tiles would have to
@@ -23,9 +23,8 @@
 //     copies and waits several times as long as these products.
 //   * fp32 operands (q P, k R, A and the state) are split into two bf16 halves, x = hi + lo, and lo * lo is dropped; v is
 //     exact.  Accumulation, decay and state are fp32.
-//   * where that leaves schedulers without a warp, the key channels of a head are shared by two CTAs: half the products per warp and
-//     chunk, which is what a chunk waits for (one after the other on one scheduler), against two parts of o to add up.
-//   * the three split products of o have accumulators of their own: a third of the chain.
+//   * the products of o are one chain per accumulator, in an order that no other sequence of the step has a say in; the products that
+//     move the state on are independent of it and are issued in between.
 //   * o leaves in fp32 for the workspace; gla_finish_kernel applies the head's norm, which needs whole rows, and the gate.
 //   * copies run ahead through a ring: records with one bulk copy each, rows of v with TMA.  A thread of the first warp
 //     asks for them when everybody has left the chunk before (a warp of its own would take registers from all others).
@@ -209,15 +208,9 @@ __global__ void __launch_bounds__(kD16 <= 4 ? 32 : 8 * kD16) gla_prepare_kernel(
     for (int i = tid; i < static_cast<int>(sizeof(R) / 16); i += kThreads) dst[i] = reinterpret_cast<const uint4*>(&out)[i];
 }
 
-// o of a token and head: row ((segment * count + chunk - first) * kChunk + token) * H + head of vdim floats behind the records, one
-// such plane per part of the key channels.
+// o of a token and head: row ((segment * count + chunk - first) * kChunk + token) * H + head of vdim floats behind the records.
 __host__ __device__ inline int64_t record_count(const b2kv_gla_args& a, const Slice& slice) {
     return static_cast<int64_t>(a.n_segments) * a.H * slice.count;
-}
-
-// Parts of the key channels: two while every warp still has a scheduler to itself.
-int key_parts(int H, int vdim, int n_segments) {
-    return 2LL * H * n_segments * ((vdim + kSlab - 1) / kSlab) <= 4LL * device_sm_count() ? 2 : 1;
 }
 
 // One place of the ring: the record, then the CTA's part of v in boxes of 32 columns (64-byte swizzle).
@@ -229,7 +222,7 @@ struct Shared {
     alignas(8) uint64_t full[kMaxRing], empty[kMaxRing];
 };
 
-template <int kD16, int kParts>
+template <int kD16>
 __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_constant__ CUtensorMap tm_v,
                                                                   const __grid_constant__ b2kv_gla_args a, const Slice slice,
                                                                   int parts, int n_ring, int32_t* dev_status) {
@@ -239,9 +232,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_
     constexpr int kStride = place_bytes(sizeof(R)), kV = v_offset(sizeof(R));
     // (an offset, not a rounded pointer: the compiler has to see that all of this is shared memory)
     uint8_t* const ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    constexpr int kKeys = kD16 / kParts;  // steps of 16 key channels of this CTA
-    const int key_part = static_cast<int>(blockIdx.x) % kParts, key0 = key_part * kKeys * 16;
-    const int h = static_cast<int>(blockIdx.x) / kParts / parts, part = static_cast<int>(blockIdx.x) / kParts % parts;
+    const int h = static_cast<int>(blockIdx.x) / parts, part = static_cast<int>(blockIdx.x) % parts;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     grid_launch_dependents();
@@ -268,7 +259,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_
 
     const R* const records = reinterpret_cast<const R*>(a.workspace) + (static_cast<int64_t>(blockIdx.y) * a.H + h) * slice.count;
     float* const o_rows = reinterpret_cast<float*>(reinterpret_cast<R*>(a.workspace) + record_count(a, slice)) +
-                          (((static_cast<int64_t>(key_part) * a.n_segments + blockIdx.y) * slice.count * kChunk) * a.H + h) * a.vdim;
+                          ((static_cast<int64_t>(blockIdx.y) * slice.count * kChunk) * a.H + h) * a.vdim;
     auto request = [&](int ci, int slot) {
         uint8_t* const dst = ring + slot * kStride;
         uint64_t* const bar = &sm.full[slot];
@@ -284,13 +275,13 @@ __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_
     const int row = lane >> 2, col = (lane & 3) * 2;  // place of this thread's first accumulator in a tile
     float* const state = a.state + (static_cast<int64_t>(sg.slot) * a.H + h) * a.dim * a.vdim;
     const bool fresh = slice.first == 0 && a.row_pos[sg.row0] == 0;
-    float c[2 * kKeys][4];  // [tile of 8 key channels]
+    float c[2 * kD16][4];  // [tile of 8 key channels]
     auto each_state = [&](auto&& fn) {
 #pragma unroll
-        for (int j = 0; j < 2 * kKeys; ++j)
+        for (int j = 0; j < 2 * kD16; ++j)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int v = v0 + row + (e >> 1) * 8, d = key0 + j * 8 + col + (e & 1);
+                const int v = v0 + row + (e >> 1) * 8, d = j * 8 + col + (e & 1);
                 fn(c[j][e], static_cast<int64_t>(d) * a.vdim + v, v < a.vdim && d < a.dim);
             }
     };
@@ -309,72 +300,61 @@ __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_
         // this warp's half of a box of v: rows of 64 bytes, 16-byte pieces exchanged by row
         const uint32_t v_addr = smem_u32(place + kV + (warp >> 1) * kBoxBytes + plain_t * 64) +
                                 (((2 * (warp & 1) + (plain_c >> 3)) ^ ((plain_t >> 1) & 3)) << 4);
-        const uint32_t q_addr = smem_u32(&b.q_hi[plain_t][key0 + plain_c]), k_addr = smem_u32(&b.k_hi[trans_t][key0 + trans_c]);
+        const uint32_t q_addr = smem_u32(&b.q_hi[plain_t][plain_c]), k_addr = smem_u32(&b.k_hi[trans_t][trans_c]);
         constexpr uint32_t kLo = sizeof(b.q_hi);  // from a matrix of leading halves to that of what they leave
-        uint32_t vf[4], x[2][4], z[2][4];
-        float o[2][4], oa[2][4], ob[2][4];  // products of leading halves; those with the low half of q and of the state
+        uint32_t vf[4], q_hi[2][4], q_lo[2][4], k_hi[2][4], k_lo[2][4];  // [step of 16 key channels, even or odd]
+        float o[2][4] = {};
+        auto load = [&](int kk) {
+            ldsm4(q_hi[kk & 1], q_addr + kk * 32);
+            ldsm4(q_lo[kk & 1], q_addr + kLo + kk * 32);
+            ldsm4t(k_hi[kk & 1], k_addr + kk * 32);
+            ldsm4t(k_lo[kk & 1], k_addr + kLo + kk * 32);
+        };
         ldsm4t(vf, v_addr);
         {
-            ldsm4(x[1], smem_u32(&b.a_hi[plain_t][plain_c]));
-            ldsm4(z[1], smem_u32(&b.a_lo[plain_t][plain_c]));
-            ldsm4(x[0], q_addr);
-            ldsm4(z[0], q_addr + kLo);
+            uint32_t a_hi[4], a_lo[4];
+            ldsm4(a_hi, smem_u32(&b.a_hi[plain_t][plain_c]));
+            ldsm4(a_lo, smem_u32(&b.a_lo[plain_t][plain_c]));
+            load(0);
 #pragma unroll
-            for (int n = 0; n < 2; ++n) {
+            for (int n = 0; n < 2; ++n) mma16816(o[n], vf, a_hi[2 * n], a_hi[2 * n + 1]);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) o[n][e] = oa[n][e] = ob[n][e] = 0.f;
-                if (kParts == 1 || key_part == 0) {
-                    mma16816(o[n], vf, x[1][2 * n], x[1][2 * n + 1]);
-                    mma16816(oa[n], vf, z[1][2 * n], z[1][2 * n + 1]);
-                }
-            }
+            for (int n = 0; n < 2; ++n) mma16816(o[n], vf, a_lo[2 * n], a_lo[2 * n + 1]);
         }
 #pragma unroll
-        for (int kk = 0; kk < kKeys; ++kk) {
-            if (kk + 1 < kKeys) {  // the next step's operands are on their way during this one's products
-                ldsm4(x[(kk + 1) & 1], q_addr + (kk + 1) * 32);
-                ldsm4(z[(kk + 1) & 1], q_addr + kLo + (kk + 1) * 32);
-            }
+        for (int kk = 0; kk < kD16; ++kk) {
+            if (kk + 1 < kD16) load(kk + 1);  // the next step's operands are on their way during this one's products
             uint32_t s_hi[4], s_lo[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float(&t)[4] = c[2 * kk + (e >> 1)];
                 split2(t[2 * (e & 1)], t[2 * (e & 1) + 1], s_hi[e], s_lo[e]);
             }
-            const uint32_t(&hi)[4] = x[kk & 1], (&lo)[4] = z[kk & 1];
 #pragma unroll
-            for (int n = 0; n < 2; ++n) mma16816(o[n], s_hi, hi[2 * n], hi[2 * n + 1]);
+            for (int u = 0; u < 2; ++u) {
+                const float2 d = *reinterpret_cast<const float2*>(&b.decay[(2 * kk + u) * 8 + col]);
+                float(&t)[4] = c[2 * kk + u];
+                t[0] *= d.x, t[1] *= d.y, t[2] *= d.x, t[3] *= d.y;
+            }
+            const uint32_t(&qh)[4] = q_hi[kk & 1], (&ql)[4] = q_lo[kk & 1], (&kh)[4] = k_hi[kk & 1], (&kl)[4] = k_lo[kk & 1];
 #pragma unroll
-            for (int n = 0; n < 2; ++n) mma16816(oa[n], s_hi, lo[2 * n], lo[2 * n + 1]);
+            for (int n = 0; n < 2; ++n) mma16816(o[n], s_hi, qh[2 * n], qh[2 * n + 1]);
 #pragma unroll
-            for (int n = 0; n < 2; ++n) mma16816(ob[n], s_lo, hi[2 * n], hi[2 * n + 1]);
+            for (int u = 0; u < 2; ++u) mma16816(c[2 * kk + u], vf, kh[2 * u], kh[2 * u + 1]);
+#pragma unroll
+            for (int n = 0; n < 2; ++n) mma16816(o[n], s_hi, ql[2 * n], ql[2 * n + 1]);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) mma16816(c[2 * kk + u], vf, kl[2 * u], kl[2 * u + 1]);
+#pragma unroll
+            for (int n = 0; n < 2; ++n) mma16816(o[n], s_lo, qh[2 * n], qh[2 * n + 1]);
         }
-        ldsm4t(x[0], k_addr);
-        ldsm4t(z[0], k_addr + kLo);
 #pragma unroll
         for (int n = 0; n < 2; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int t = ci * kChunk + n * 8 + col + (e & 1), v = v0 + row + (e >> 1) * 8;
-                if (v < a.vdim && t < rows_left) o_rows[static_cast<int64_t>(t) * a.H * a.vdim + v] = o[n][e] + (oa[n][e] + ob[n][e]);
+                if (v < a.vdim && t < rows_left) o_rows[static_cast<int64_t>(t) * a.H * a.vdim + v] = o[n][e];
             }
-#pragma unroll
-        for (int kk = 0; kk < kKeys; ++kk) {
-            if (kk + 1 < kKeys) {
-                ldsm4t(x[(kk + 1) & 1], k_addr + (kk + 1) * 32);
-                ldsm4t(z[(kk + 1) & 1], k_addr + kLo + (kk + 1) * 32);
-            }
-            const uint32_t(&hi)[4] = x[kk & 1], (&lo)[4] = z[kk & 1];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const float2 d = *reinterpret_cast<const float2*>(&b.decay[key0 + (2 * kk + u) * 8 + col]);
-                float(&t)[4] = c[2 * kk + u];
-                t[0] *= d.x, t[1] *= d.y, t[2] *= d.x, t[3] *= d.y;
-                mma16816(t, vf, hi[2 * u], hi[2 * u + 1]);
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) mma16816(c[2 * kk + u], vf, lo[2 * u], lo[2 * u + 1]);
-        }
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.empty[slot]);
         // the place of the chunk before is free when the last warp has left it (one chunk behind: nobody waits long)
@@ -400,7 +380,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_
 // The heads' norm and the gate: one warp per (token, head), eight value columns per lane.
 constexpr int kFinishWarps = 8;
 template <typename R>
-__global__ void __launch_bounds__(32 * kFinishWarps) gla_finish_kernel(const __grid_constant__ b2kv_gla_args a, const Slice slice, int key_parts) {
+__global__ void __launch_bounds__(32 * kFinishWarps) gla_finish_kernel(const __grid_constant__ b2kv_gla_args a, const Slice slice) {
     const int lane = threadIdx.x & 31, at = static_cast<int>(blockIdx.x) * kFinishWarps + (threadIdx.x >> 5);
     const int t = at / a.H, h = at % a.H, c = lane * 8;
     grid_launch_dependents();
@@ -417,17 +397,10 @@ __global__ void __launch_bounds__(32 * kFinishWarps) gla_finish_kernel(const __g
     if (mine) {
         *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(src);
         *reinterpret_cast<float4*>(f + 4) = *reinterpret_cast<const float4*>(src + 4);
-        if (key_parts > 1) {
-            const float* const other = src + static_cast<int64_t>(a.n_segments) * slice.count * kChunk * a.H * a.vdim;
-            float g[8];
-            *reinterpret_cast<float4*>(g) = *reinterpret_cast<const float4*>(other);
-            *reinterpret_cast<float4*>(g + 4) = *reinterpret_cast<const float4*>(other + 4);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] += g[i];
-        }
         gate = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.y) + row * a.ld_y + a.g_col + h * a.vdim + c);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) sum = fmaf(f[i], f[i], sum);
+        for (int i = 0; i < 8; i += 4)
+            sum = fmaf(f[i], f[i], fmaf(f[i + 1], f[i + 1], fmaf(f[i + 2], f[i + 2], fmaf(f[i + 3], f[i + 3], sum))));
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
@@ -459,13 +432,13 @@ int record_bytes(int dim) {
     return static_cast<int>(dim <= 32 ? sizeof(Record<2>) : (dim <= 64 ? sizeof(Record<4>) : sizeof(Record<8>)));
 }
 
-size_t chunk_bytes(int H, int dim, int vdim, int n_segments) {
-    return (static_cast<size_t>(record_bytes(dim)) + key_parts(H, vdim, n_segments) * kChunk * static_cast<size_t>(vdim) * sizeof(float)) * H;
+size_t chunk_bytes(int H, int dim, int vdim) {
+    return (static_cast<size_t>(record_bytes(dim)) + kChunk * static_cast<size_t>(vdim) * sizeof(float)) * H;
 }
 
 int slice_chunks(int H, int dim, int vdim, int n_segments, int max_n) {
     const int chunks = (max_n + kChunk - 1) / kChunk;
-    const int fit = static_cast<int>(std::min<size_t>(kSliceBytes / (chunk_bytes(H, dim, vdim, n_segments) * n_segments), 1u << 20));
+    const int fit = static_cast<int>(std::min<size_t>(kSliceBytes / (chunk_bytes(H, dim, vdim) * n_segments), 1u << 20));
     return std::min(chunks, std::max(kMinSlice, fit));
 }
 
@@ -478,15 +451,14 @@ int launch_chunked(const b2kv_gla_args& a, int32_t* dev_status, void* stream) {
     CUtensorMap tv;
     const int64_t cols = std::max(a.v_col, a.g_col) + static_cast<int64_t>(a.H) * a.vdim;
     if (!make_map(&tv, a.y, a.rows, cols, a.ld_y, kBox, CU_TENSOR_MAP_SWIZZLE_64B)) return B2KV_ERR_UNSUPPORTED;
-    const int keys = key_parts(a.H, a.vdim, a.n_segments);
-    static int configured[2][64] = {{0}};
+    static int configured[64] = {0};
     int dev = 0;
     B2KV_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return B2KV_ERR_UNSUPPORTED;
-    auto kernel = keys > 1 ? gla_state_kernel<kD16, 2> : gla_state_kernel<kD16, 1>;
-    if (configured[keys - 1][dev] < static_cast<int>(smem)) {
+    auto kernel = gla_state_kernel<kD16>;
+    if (configured[dev] < static_cast<int>(smem)) {
         B2KV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        configured[keys - 1][dev] = static_cast<int>(smem);
+        configured[dev] = static_cast<int>(smem);
     }
     const int chunks = (a.max_n + kChunk - 1) / kChunk;
     Slice slice{0, slice_chunks(a.H, a.dim, a.vdim, a.n_segments, a.max_n)};
@@ -494,11 +466,11 @@ int launch_chunked(const b2kv_gla_args& a, int32_t* dev_status, void* stream) {
         const unsigned here = static_cast<unsigned>(std::min(slice.count, chunks - slice.first));
         OverlapLaunch prep(dim3(here, a.H, a.n_segments), kD16 <= 4 ? 32 : 8 * kD16, 0, stream);
         B2KV_CUDA_TRY(cudaLaunchKernelEx(&prep.cfg, gla_prepare_kernel<kD16>, a, slice, dev_status));
-        OverlapLaunch walk(dim3(a.H * parts * keys, a.n_segments), 32 * kWarps, smem, stream);
+        OverlapLaunch walk(dim3(a.H * parts, a.n_segments), 32 * kWarps, smem, stream);
         B2KV_CUDA_TRY(cudaLaunchKernelEx(&walk.cfg, kernel, tv, a, slice, parts, n_ring, dev_status));
         const unsigned pairs = here * kChunk * static_cast<unsigned>(a.H);
         OverlapLaunch finish(dim3((pairs + kFinishWarps - 1) / kFinishWarps, a.n_segments), 32 * kFinishWarps, 0, stream);
-        B2KV_CUDA_TRY(cudaLaunchKernelEx(&finish.cfg, gla_finish_kernel<R>, a, slice, keys));
+        B2KV_CUDA_TRY(cudaLaunchKernelEx(&finish.cfg, gla_finish_kernel<R>, a, slice));
     }
     return B2KV_OK;
 }
@@ -512,7 +484,7 @@ bool chunked_sizes(int dim, int vdim, int dtype) {
 
 size_t gla_chunked_workspace(int H, int dim, int vdim, int n_segments, int max_n, int dtype) {
     if (!gla::chunked_sizes(dim, vdim, dtype)) return 0;
-    return static_cast<size_t>(gla::slice_chunks(H, dim, vdim, n_segments, max_n)) * gla::chunk_bytes(H, dim, vdim, n_segments) * n_segments;
+    return static_cast<size_t>(gla::slice_chunks(H, dim, vdim, n_segments, max_n)) * gla::chunk_bytes(H, dim, vdim) * n_segments;
 }
 
 int gla_chunked(const b2kv_gla_args& a, int32_t* dev_status, void* stream) {

@@ -125,6 +125,24 @@ def test_fp32_runs_with_the_state_in_registers(pkg, heads, dim, vdim, lens):
             state_close(state[slot], last[slot])
 
 
+@pytest.mark.parametrize("heads,dim,vdim", [(10, 24, 256), (10, 64, 248), (8, 128, 256)])
+def test_a_sequence_does_not_depend_on_its_company(pkg, heads, dim, vdim):
+    """Alone and among five others: the same bits, and those of the equations."""
+    layer = Layer(pkg, heads, dim, vdim, 4.0, BF, seed=11)
+    lens = (100, 17, 40, 33, 64, 16)
+    y, al = layer.rows(sum(lens))
+    segments, pos = [(sum(lens[:i]), n, i) for i, n in enumerate(lens)], np.concatenate([np.arange(n) for n in lens])
+    state = layer.states(len(lens))
+    got = layer.run(y, al, segments, pos, state, CHUNK)
+    for r0, n, slot in segments:
+        alone = layer.states(1)
+        assert np.array_equal(layer.run(y[r0:r0 + n], al[r0:r0 + n], [(0, n, 0)], range(n), alone, CHUNK), got[r0:r0 + n]), n
+        assert torch.equal(alone[0], state[slot]), n
+        want, last = layer.want(y[r0:r0 + n], al[r0:r0 + n])
+        close(got[r0:r0 + n], want, BF, n)
+        state_close(state[slot], last)
+
+
 @pytest.mark.parametrize("path,dtype,heads,dim,vdim", [(STEP, F32, 3, 5, 7), (CHUNK, BF, 5, 56, 40), (0, BF, 2, 128, 128), (0, BF, 2, 64, 64)])
 def test_portions_carry_the_state(pkg, path, dtype, heads, dim, vdim):
     """Any cut gives the outputs of the whole, with two sequences in unequal portions per call and the rows of a call in any
