@@ -482,9 +482,16 @@ bool chunked_sizes(int dim, int vdim, int dtype) {
 }  // namespace
 }  // namespace gla
 
+static size_t workspace_for(int H, int dim, int vdim, int n_segments, int max_n) {
+    return static_cast<size_t>(gla::slice_chunks(H, dim, vdim, n_segments, max_n)) * gla::chunk_bytes(H, dim, vdim) * n_segments;
+}
+
+// Enough for fewer segments as well: slices are of whole chunks of all segments, so that fewer segments may take a little more.
 size_t gla_chunked_workspace(int H, int dim, int vdim, int n_segments, int max_n, int dtype) {
     if (!gla::chunked_sizes(dim, vdim, dtype)) return 0;
-    return static_cast<size_t>(gla::slice_chunks(H, dim, vdim, n_segments, max_n)) * gla::chunk_bytes(H, dim, vdim) * n_segments;
+    size_t most = 0;
+    for (int n = 1; n <= n_segments; ++n) most = std::max(most, workspace_for(H, dim, vdim, n, max_n));
+    return most;
 }
 
 int gla_chunked(const b2kv_gla_args& a, int32_t* dev_status, void* stream) {
@@ -494,7 +501,7 @@ int gla_chunked(const b2kv_gla_args& a, int32_t* dev_status, void* stream) {
     if (!aligned16(a.y) || !aligned16(a.out) || a.ld_y % 8 || a.ld_out % 8 || a.v_col % 8 || a.g_col % 8) return B2KV_ERR_UNSUPPORTED;
     if (!aligned16(a.alpha) || a.ld_alpha % 2 || a.q_col % 2 || a.k_col % 2) return B2KV_ERR_UNSUPPORTED;  // pairs of channels
     if (!a.workspace || (reinterpret_cast<uintptr_t>(a.workspace) & 127) ||
-        a.workspace_bytes < gla_chunked_workspace(a.H, a.dim, a.vdim, a.n_segments, a.max_n, a.dtype))
+        a.workspace_bytes < workspace_for(a.H, a.dim, a.vdim, a.n_segments, a.max_n))
         return B2KV_ERR_WORKSPACE;
     if (a.dim <= 32) return launch_chunked<2>(a, dev_status, stream);
     if (a.dim <= 64) return launch_chunked<4>(a, dev_status, stream);

@@ -202,3 +202,11 @@ def test_decoder_state_and_graphed_step_checks(pkg, ctx):
         cache.current_len = 32
     with pytest.raises(ValueError, match="Cache is full"):
         model.decode_step(ctx, state, tok)
+
+
+@pytest.mark.parametrize("heads,dim,vdim,max_n", [(8, 64, 256, 100), (3, 128, 64, 1000), (16, 32, 256, 5000), (1, 128, 8, 40)])
+def test_a_recurrence_workspace_is_enough_for_fewer_segments(pkg, heads, dim, vdim, max_n):
+    """A program may ask for its workspace once, for the most segments and tokens of a step."""
+    size = lambda n, t: pkg._native.lib.b2kv_gla_workspace_bytes(heads, dim, vdim, n, t, pkg._native.DTYPE_BF16, 0)  # noqa: E731
+    sizes = [size(n, max_n) for n in range(1, 65)]
+    assert sizes == sorted(sizes) and 0 < size(7, max_n // 2) <= size(7, max_n)
