@@ -20,8 +20,8 @@ __device__ __forceinline__ void copy16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
-// kD: key channels, rounded up.
-template <int kD>
+// kD: key channels, rounded up; kPadded: there are fewer.
+template <int kD, bool kPadded>
 __global__ void __launch_bounds__(32 * kWarps) gla_run_kernel(const __grid_constant__ b2kv_gla_args a, int parts, int32_t* dev_status) {
     constexpr int kGroups = (kD + 31) / 32;  // groups of four key channels per lane
     struct Stage {
@@ -89,10 +89,12 @@ __global__ void __launch_bounds__(32 * kWarps) gla_run_kernel(const __grid_const
 #pragma unroll
             for (int j = 0; j < kGroups; ++j) {
                 const float4 al = st.alpha[t][j * 8 + dg], kk = st.k[t][j * 8 + dg], qq = st.q[t][j * 8 + dg];
+                // (a key of zero is no answer to a value that is not finite)
+                const float2 vj = kPadded && j * 32 + dg * 4 >= a.dim ? make_float2(0.f, 0.f) : v;
                 const float av[4] = {al.x, al.y, al.z, al.w}, kv[4] = {kk.x, kk.y, kk.z, kk.w}, qv[4] = {qq.x, qq.y, qq.z, qq.w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    s[j][e] = __ffma2_rn(s[j][e], make_float2(av[e], av[e]), __fmul2_rn(make_float2(kv[e], kv[e]), v));
+                    s[j][e] = __ffma2_rn(s[j][e], make_float2(av[e], av[e]), __fmul2_rn(make_float2(kv[e], kv[e]), vj));
                     const float q = qv[e] * a.q_scale;
                     o[e] = __ffma2_rn(make_float2(q, q), s[j][e], o[e]);
                 }
@@ -170,8 +172,13 @@ int gla_run_f32(const b2kv_gla_args& a, int32_t* dev_status, void* stream) {
     const long long ctas = static_cast<long long>(a.H) * parts, pairs = static_cast<long long>(a.max_n) * a.H;
     if (ctas > 0x7fffffffLL || pairs > 0x7fffffffLL - kNormWarps) return B2KV_ERR_UNSUPPORTED;
     OverlapLaunch run(dim3(static_cast<unsigned>(ctas), a.n_segments), 32 * kWarps, 0, stream);
-    B2KV_CUDA_TRY(cudaLaunchKernelEx(&run.cfg, a.dim <= 32 ? gla_run_kernel<32> : (a.dim <= 64 ? gla_run_kernel<64> : gla_run_kernel<128>), a,
-                                     parts, dev_status));
+    const auto kernel = a.dim < 32    ? gla_run_kernel<32, true>
+                        : a.dim == 32  ? gla_run_kernel<32, false>
+                        : a.dim < 64   ? gla_run_kernel<64, true>
+                        : a.dim == 64  ? gla_run_kernel<64, false>
+                        : a.dim < 128  ? gla_run_kernel<128, true>
+                                       : gla_run_kernel<128, false>;
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&run.cfg, kernel, a, parts, dev_status));
     OverlapLaunch norm(dim3(static_cast<unsigned>((pairs + kNormWarps - 1) / kNormWarps), a.n_segments), 32 * kNormWarps, 0, stream);
     B2KV_CUDA_TRY(cudaLaunchKernelEx(&norm.cfg, gla_norm_kernel, a));
     return B2KV_OK;

@@ -125,6 +125,24 @@ def test_fp32_runs_with_the_state_in_registers(pkg, heads, dim, vdim, lens):
             state_close(state[slot], last[slot])
 
 
+@pytest.mark.parametrize("dim,vdim", [(4, 8), (36, 20), (64, 64), (100, 36)])
+def test_fp32_values_that_are_not_finite(pkg, dim, vdim):
+    """An infinite value stays in its column of the state, whatever the key channels are rounded up to; the head's other columns are
+    divided by an infinite norm, in registers as token after token."""
+    layer = Layer(pkg, 2, dim, vdim, 4.0, F32, seed=13)
+    y, al = layer.rows(21)
+    y.abs_()
+    y[9, layer.cols[2] + 3] = float("inf")
+    got, state = {}, {}
+    for path in (0, STEP):
+        state[path] = layer.states(1)
+        got[path] = layer.run(y, al, [(0, 21, 0)], range(21), state[path], path)
+    assert np.array_equal(np.isnan(got[0]), np.isnan(got[STEP])) and np.isnan(got[0]).sum() == 12
+    assert torch.equal(state[0].isinf(), state[STEP].isinf()) and not state[0].isnan().any()
+    finite = ~np.isnan(got[0])
+    np.testing.assert_allclose(got[0][finite], got[STEP][finite], rtol=1e-5, atol=1e-6)
+
+
 @pytest.mark.parametrize("heads,dim,vdim", [(10, 24, 256), (10, 64, 248), (8, 128, 256)])
 def test_a_sequence_does_not_depend_on_its_company(pkg, heads, dim, vdim):
     """Alone and among five others: the same bits, and those of the equations."""
