@@ -98,17 +98,19 @@ route_kernel(const float* logits, int64_t ld, int rows, int experts, int groups,
 // loads before its first copy, took 38 us for 2975 rows of 4 KB and six choices, this one 25).
 constexpr int kPlanThreads = 128;
 
+template <bool kTable>  // the experts' first rows fit shared memory
 __global__ void __launch_bounds__(kPlanThreads)
 moe_plan_kernel(const int32_t* idx, int32_t* counts, int experts, int top, int32_t* offsets,
                 int32_t* slot, const uint8_t* h, int64_t pitch_h, uint8_t* sorted,
                 int64_t pitch_sorted, int row_bytes, bool vec) {
-    extern __shared__ int first[];  // [experts + 1]: row behind the last one of the experts before; then the places of the row's choices
-    int* const place = first + experts + 1;
+    extern __shared__ int sm_plan[];  // [experts + 1]: row behind the last one of the experts before; then the places of the row's choices
+    const int row = blockIdx.x, lane = threadIdx.x & 31;
+    int* const first = kTable ? sm_plan : offsets;  // (without a table one CTA writes them where they belong)
+    int* const place = kTable ? sm_plan + experts + 1 : slot + static_cast<int64_t>(row) * top;
     constexpr int kKeep = 4;
     grid_launch_dependents();
     if (threadIdx.x == 0) grid_dependency_wait();
     __syncthreads();
-    const int row = blockIdx.x, lane = threadIdx.x & 31;
     const uint8_t* src = h + static_cast<int64_t>(row) * pitch_h;
     uint4 keep[kKeep];
 #pragma unroll
@@ -118,7 +120,7 @@ moe_plan_kernel(const int32_t* idx, int32_t* counts, int experts, int top, int32
     }
     if (threadIdx.x < 32) {
         int base = 0;
-        for (int e0 = 0; e0 < experts; e0 += 32) {
+        for (int e0 = 0; e0 < experts && (kTable || row == 0); e0 += 32) {
             const int n = e0 + lane < experts ? counts[e0 + lane] : 0;
             int end = n;
 #pragma unroll
@@ -129,16 +131,24 @@ moe_plan_kernel(const int32_t* idx, int32_t* counts, int experts, int top, int32
             if (e0 + lane < experts) first[e0 + lane] = base + end - n;
             base += __shfl_sync(0xffffffffu, end, 31);
         }
-        if (lane == 0) first[experts] = base;
+        if (lane == 0 && (kTable || row == 0)) first[experts] = base;
         __syncwarp();
-        for (int k = lane; k < top; k += 32) {
+        for (int k = 0; k < top && !kTable; ++k) {
+            const int e = idx[static_cast<int64_t>(row) * top + k];
+            int before = 0;
+            for (int i = lane; i < e; i += 32) before += counts[i];
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) before += __shfl_xor_sync(0xffffffffu, before, off);
+            if (lane == 0) place[k] = before + atomicAdd(&counts[experts + e], 1);
+        }
+        for (int k = lane; k < top && kTable; k += 32) {
             const int e = idx[static_cast<int64_t>(row) * top + k];
             place[k] = first[e] + atomicAdd(&counts[experts + e], 1);
             slot[static_cast<int64_t>(row) * top + k] = place[k];
         }
     }
     __syncthreads();
-    if (row == 0)
+    if (row == 0 && kTable)
         for (int i = threadIdx.x; i <= experts; i += kPlanThreads) offsets[i] = first[i];
     if (!vec) {
         for (int k = 0; k < top; ++k)
@@ -239,10 +249,10 @@ extern "C" int b2kv_moe_plan(const int32_t* idx, int32_t* counts, int rows, int 
         return B2KV_ERR_BAD_ARG;
     if (static_cast<long long>(rows) * top > 0x7fffffffLL) return B2KV_ERR_UNSUPPORTED;
     const bool vec = (dim * es) % 16 == 0 && (ld_h * es) % 16 == 0 && (ld_sorted * es) % 16 == 0 && aligned16(h) && aligned16(sorted);
-    const size_t smem = (static_cast<size_t>(experts) + 1 + top) * sizeof(int);
-    if (smem > 48 * 1024) return B2KV_ERR_UNSUPPORTED;
-    OverlapLaunch launch(rows, kPlanThreads, smem, stream);
-    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, moe_plan_kernel, idx, counts, experts, top, offsets, slot,
+    const size_t bytes = (static_cast<size_t>(experts) + 1 + top) * sizeof(int);
+    const bool table = bytes <= 48 * 1024;
+    OverlapLaunch launch(rows, kPlanThreads, table ? bytes : 0, stream);
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, table ? moe_plan_kernel<true> : moe_plan_kernel<false>, idx, counts, experts, top, offsets, slot,
                                      static_cast<const uint8_t*>(h), ld_h * es, static_cast<uint8_t*>(sorted), ld_sorted * es,
                                      dim * es, vec));
     return B2KV_OK;

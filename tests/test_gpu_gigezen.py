@@ -215,3 +215,29 @@ def test_folder_trace_runner_and_command_line(pkg, tmp_path):
     assert res.returncode == 0, res.stderr
     model = registry.load_model(make_ctx(pkg), tmp_path, F32, max_tokens=7)
     assert res.stdout.split() == [",".join(map(str, generate.generate_text(model, [3, 5, 8], 4, temperature=0.0)))]
+
+
+@pytest.mark.parametrize("experts,width", [(13, 24), (1024, 2056), (13000, 24), (13000, 9)])
+def test_rows_sorted_by_any_number_of_experts(pkg, experts, width):
+    """Also by more than a table in shared memory holds: the places of an expert's rows begin where the expert before ends."""
+    from llm_experiments_b200 import moe
+    from llm_experiments_b200.serving import buffer2
+
+    ctx, rows, top = make_ctx(pkg), 37, 5
+    gen = torch.Generator(device="cuda").manual_seed(experts)
+    idx = torch.stack([torch.randperm(experts, generator=gen, device="cuda")[:top] for _ in range(rows)]).to(torch.int32)
+    idx[3, 0], idx[4, 1] = experts - 1, 0
+    h = torch.randn((rows, width), generator=gen, device="cuda").to(BF)
+    count = torch.bincount(idx.flatten().long(), minlength=experts).to(torch.int32)
+    i32 = lambda *shape: torch.full(shape, -1, dtype=torch.int32, device="cuda")  # noqa: E731
+    s = moe.MoeScratch(idx=idx, score=None, slot=i32(rows, top), counts=torch.cat([count, torch.zeros_like(count)]), offsets=i32(experts + 2),
+                       sorted_h=buffer2(torch.full((rows * top + 1, width), 7.0, dtype=BF, device="cuda")), m=None, y=None)
+    pkg.gpu.batch_begin(ctx)
+    moe.plan(ctx, buffer2(h), moe.RouterShape(experts=experts, top=top, groups=1, keep=1), s)
+    pkg.gpu.batch_commit(ctx)
+    ends = torch.cat([count.new_zeros(1), count.cumsum(0).to(torch.int32)])
+    assert torch.equal(s.offsets[:-1], ends) and s.offsets[-1] == -1
+    assert torch.equal(s.slot.flatten().sort().values, torch.arange(rows * top, device="cuda", dtype=torch.int32))
+    e = idx.long()
+    assert ((s.slot >= ends[e]) & (s.slot < ends[e + 1])).all()
+    assert torch.equal(s.sorted_h.buffer[s.slot.long()], h[:, None].expand(rows, top, width)) and (s.sorted_h.buffer[-1] == 7).all()
