@@ -53,9 +53,6 @@ constexpr int kFeat = 128;      // output features per CTA (MMA M)
 constexpr int kKTile = 128;
 constexpr int kMaxStagesP = 6;
 constexpr int kRingBytes = 200 * 1024;  // shared memory given to the ring; as many stages as fit
-// Several waves of tiles (the logits): two CTAs per SM, so that one streams while the other starts or ends (8 rows, 4096 x 32768: 72 us
-// with one, 66 so).
-constexpr int kRingBytesTwo = 112 * 1024;
 constexpr int kSmemBytes = 224 * 1024;  // ring and partials of a split tile together (227 KB less alignment and statics)
 constexpr int kWBytes = kKTile * kFeat * 2;  // two halves of 16 KB, see the descriptors below
 constexpr int kWHalf = kWBytes / 2;
@@ -112,6 +109,21 @@ __device__ __forceinline__ void peer_store_u32(uint32_t local, uint32_t rank, ui
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local), "r"(rank));
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
+
+constexpr int ring_stages(int Bn, int ring_bytes) {
+    const int fit = ring_bytes / (kWBytes + 2 * Bn * 128);
+    return fit < 2 ? 2 : (fit > kMaxStagesP ? kMaxStagesP : fit);
+}
+// Several waves of tiles (the logits): two CTAs per SM, so that one streams while the other starts or ends (8 rows, 4096 x 32768: 72 us
+// with one, 66 so), where two fit (with two stages; the rate does not fall before there are fewer than three on an SM): up to 80 rows.
+// From 81 on one CTA of the large ring has three stages, and of the small one two and no neighbour (96 / 128 rows: 54 / 57 us, and 65 / 69).
+constexpr int kRingBytesTwo = 112 * 1024;
+constexpr bool two_fit(int Bn) {
+    return 2 * (ring_stages(Bn, kRingBytesTwo) * (kWBytes + 2 * Bn * 128) + 1024 + static_cast<int>(sizeof(ProjShared)) + 1024) <= 228 * 1024;
+}
+constexpr int ring_bytes_of(int Bn, bool waves) { return waves && two_fit(Bn) ? kRingBytesTwo : kRingBytes; }
+static_assert(two_fit(16) && two_fit(80) && !two_fit(96), "two CTAs per SM up to 80 rows");
+static_assert(ring_stages(96, ring_bytes_of(96, true)) == 3 && ring_stages(128, ring_bytes_of(128, true)) == 3, "or one of three stages");
 
 // x * sigmoid(1.702 x), the reference's GELU (simple-llm/src/gpu/gpu_kernels.py:285-293).  The denominator is at
 // least one, so the approximate division (2 ulp, no slow path: sixteen of them run interleaved) is safe; it
@@ -428,7 +440,7 @@ extern "C" int b2kv_qkv_append(const void* x, const void* wq, const void* wk, co
         !proj::make_matrix_map(&tv, wv, E, E, w_box_rows) || !proj::make_matrix_map(&tx, x, B, E, Bn))
         return B2KV_ERR_UNSUPPORTED;
     const int stage_bytes = proj::kWBytes + 2 * Bn * 128;
-    const int stages = std::max(2, std::min(proj::kMaxStagesP, proj::kRingBytes / stage_bytes));
+    const int stages = proj::ring_stages(Bn, proj::kRingBytes);
     const size_t smem = static_cast<size_t>(stages) * stage_bytes + 1024;
     proj::ProjParams p{q_out, k_cache, v_cache, seq_pos, dev_status, stride_b, stride_t, stride_h, pos, B, Bn, E, H, D, T_max,
                        E, nullptr, nullptr, 0, stages, 1, 0};
@@ -464,8 +476,8 @@ extern "C" int b2kv_matmul_rows(const void* x, const void* w, const void* bias, 
     // a split tile keeps the partials of its own sequences behind the rings: [splits][Bn / splits][128] fp32
     const int recv_bytes = splits > 1 ? Bn * proj::kFeat * 4 : 0;
     const int stage_bytes = proj::kWBytes + 2 * Bn * 128;
-    const int ring_bytes = tiles > device_sm_count() ? proj::kRingBytesTwo : std::min(proj::kRingBytes, proj::kSmemBytes - recv_bytes);
-    const int stages = std::max(2, std::min(proj::kMaxStagesP, ring_bytes / stage_bytes));
+    const int ring_bytes = std::min(proj::ring_bytes_of(Bn, tiles > device_sm_count()), proj::kSmemBytes - recv_bytes);
+    const int stages = proj::ring_stages(Bn, ring_bytes);
     const size_t smem = static_cast<size_t>(stages) * stage_bytes + recv_bytes + 1024;
     // one weight matrix: every tile is of kind 0 (plain rows of `out`); the cache fields are unused
     proj::ProjParams p{out, nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0, B, Bn, N, 1, N, 1, K, residual, bias, activation,

@@ -109,6 +109,20 @@ def test_matmul_rows_vs_oracle(pkg, ctx, M, K, N, with_residual):
     np.testing.assert_allclose(U.to_f32(C), want.astype(np.float32), rtol=RTOL, atol=ATOL)
 
 
+@pytest.mark.parametrize("M", [1, 8, 33, 80, 81, 96, 128])
+@pytest.mark.parametrize("K", [128, 1152])
+def test_matmul_rows_with_more_tiles_than_sms(pkg, ctx, M, K):
+    """The logits' form: two CTAs per SM up to 80 rows, one with a longer ring beyond; as many input features as stages or more."""
+    N = 128 * (torch.cuda.get_device_properties(0).multi_processor_count + 3)
+    A, W, R = _bf16(ctx, (M, K), 41), _bf16(ctx, (K, N), 42, scale=K ** -0.5), _bf16(ctx, (M, N), 43)
+    C = torch.full((M + 1, N), 7.0, dtype=torch.bfloat16, device=ctx.device)
+    pkg.gpu.batch_begin(ctx)
+    pkg.gpu.matmul(ctx, U.buf2d(pkg, ctx, A), U.buf2d(pkg, ctx, W), U.buf2d(pkg, ctx, C[:M]), residual=U.buf2d(pkg, ctx, R))
+    pkg.gpu.batch_commit(ctx)
+    torch.testing.assert_close(C[:M].double(), A.double() @ W.double() + R.double(), rtol=RTOL, atol=ATOL)
+    assert (C[M] == 7).all()
+
+
 def test_matmul_with_bias_gelu_and_residual_like_the_mlp(pkg, ctx):
     """C = gelu(A @ W + b) + R, the reference's matmul -> bias_add -> gelu (-> residual_add) chain."""
     gpu = pkg.gpu
