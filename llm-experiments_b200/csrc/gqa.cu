@@ -404,10 +404,10 @@ int launch_runs(const GqaDecodeArgs& a, void* stream) {
     return B2KV_OK;
 }
 
-// Rows come in runs when there are several for every place; a decoding step has one per sequence at most, and a CTA would take
-// its sequences one after the other.
+// For rows that the caller says come in runs (a CTA takes the sequences of its 16 rows one after the other, so that single rows of
+// many sequences would be in line: 16 of them take as long as the one that sees most, times 16), and enough of them to fill CTAs.
 int launch_runs_f32(const GqaDecodeArgs& a, void* stream) {
-    if (a.rows < 4 * a.n_slots || a.rows < 64 || (a.rows + kRunRows - 1) / kRunRows > 65535) return B2KV_ERR_UNSUPPORTED;
+    if (a.rows < 64 || (a.rows + kRunRows - 1) / kRunRows > 65535) return B2KV_ERR_UNSUPPORTED;
     const int widest = std::max(a.dim, a.vdim);
     if (widest > 128 || a.dim % 4 || a.vdim % 4 || a.ld_q % 4 || !aligned16(a.q) || !aligned16(a.k_cache) || !aligned16(a.v_cache))
         return B2KV_ERR_UNSUPPORTED;
@@ -475,7 +475,7 @@ extern "C" int b2kv_gqa_decode(const void* q, int64_t ld_q, const void* k_cache,
     if (elt_bytes(dtype) == 0) return B2KV_ERR_UNSUPPORTED;
     if (!q || !k_cache || !v_cache || !out || !row_pos) return B2KV_ERR_BAD_ARG;
     if (n_slots <= 0 || T_max <= 0 || rows <= 0 || H <= 0 || G <= 0 || H % G != 0 || dim <= 0 || vdim <= 0 || span <= 0 ||
-        path < 0 || path > 2 || ld_q < static_cast<int64_t>(H) * dim || ld_out < static_cast<int64_t>(H) * vdim)
+        path < 0 || path > 3 || ld_q < static_cast<int64_t>(H) * dim || ld_out < static_cast<int64_t>(H) * vdim)
         return B2KV_ERR_BAD_ARG;
     const GqaDecodeArgs a{q, k_cache, v_cache, out, slopes, row_slot, row_pos, dev_status, ld_q, ld_out,
                           n_slots, T_max, rows, H, G, dim, vdim, span, scale};
@@ -484,7 +484,7 @@ extern "C" int b2kv_gqa_decode(const void* q, int64_t ld_q, const void* k_cache,
         const int rc = gqa_decode_tc(a, workspace, workspace_bytes, stream);
         if (rc != B2KV_ERR_UNSUPPORTED || path == 2) return rc;
     }
-    if (dtype == B2KV_DTYPE_F32 && path == 0) {
+    if (dtype == B2KV_DTYPE_F32 && path == 3) {
         const int rc = launch_runs_f32(a, stream);
         if (rc != B2KV_ERR_UNSUPPORTED) return rc;
     }

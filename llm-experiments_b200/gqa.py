@@ -20,6 +20,9 @@ from .latent import PromptPlan, RowPlaces
 from .types import GPUBuffer1D, GPUBuffer2D, GPUContext, KVCache
 
 
+RUNS = 3  # path of gqa_decode: rows of prompt portions
+
+
 @dataclass
 class GqaShape:
     """Sizes and constants of one grouped-query attention layer."""
@@ -63,7 +66,8 @@ def gqa_append(ctx: GPUContext, y: GPUBuffer2D, shape: GqaShape, places: RowPlac
 def gqa_decode(ctx: GPUContext, q: GPUBuffer2D, shape: GqaShape, slopes: Optional[GPUBuffer1D], places: RowPlaces, cache: KVCache,
                out: GPUBuffer2D, span: int, path: int = 0) -> None:
     """Attention of single rows: ``q`` as ``gqa_append`` leaves it, ``out`` ``[rows, >= heads * vdim]``.  ``span`` bounds the tokens
-    any row sees.  ``path`` forces a kernel (1 CUDA cores, 2 tensor cores)."""
+    any row sees.  ``path`` forces a kernel (1 CUDA cores, 2 tensor cores) or says that the rows are ``RUNS`` of neighbouring rows of
+    one sequence."""
     k, v = _caches(cache, shape)
     rows, dt = q.shape[0], dtype_code(q.buffer.dtype)
     nbytes = _native.lib.b2kv_gqa_decode_workspace_bytes(rows, shape.heads, shape.kv_heads, shape.vdim, span, dt) if path != 1 else 0

@@ -56,12 +56,14 @@ class RowSegments:
 
 @dataclass
 class Step:
-    """The rows of one step.  The first ``n_single`` belong to short entries, the rest to prompt portions."""
+    """The rows of one step.  The first ``n_single`` go row by row, the rest to the kernels of prompt portions.  Of the former the
+    first ``n_few`` belong to entries of at most ``SHORT_ENTRY`` tokens (the others to longer ones, where there is no prompt form)."""
 
     ids: torch.Tensor
     places: RowPlaces
     rows: int
     n_single: int
+    n_few: int
     span: int                        # bounds the tokens that a row of a short entry sees
     plans: Dict[int, PromptPlan]     # prompt portions, by the key the state's prompt_plans chose
     short: Optional[RowSegments]     # the short entries and
@@ -69,9 +71,10 @@ class Step:
     row_index: Optional[torch.Tensor]  # rows whose logits are wanted (None: all)
     n_out: int
 
-    def single_places(self) -> RowPlaces:
-        p = self.places
-        return RowPlaces(None if p.slot is None else p.slot[:self.n_single], p.pos[:self.n_single])
+    def single_places(self, r0: int = 0, r1: Optional[int] = None) -> RowPlaces:
+        """Of the rows ``r0 .. r1 - 1`` (default: all) that go row by row.  (Without a table of sequences all rows are asked for.)"""
+        p, r1 = self.places, self.n_single if r1 is None else r1
+        return RowPlaces(None if p.slot is None else p.slot[r0:r1], p.pos[r0:r1])
 
 
 @dataclass
@@ -156,7 +159,7 @@ def decode_step(ctx: GPUContext, state: SequenceState, token_ids: GPUBuffer1D, n
     if upper >= state.max_seq_len:
         raise ValueError(f"Cache is full: current_len={upper}, max_seq_len={state.max_seq_len}")
     B = state.batch_size
-    state.run(ctx, Step(ids=token_ids.buffer, places=RowPlaces(None, state.seq_lens), rows=B, n_single=B, span=upper + 1, plans={},
+    state.run(ctx, Step(ids=token_ids.buffer, places=RowPlaces(None, state.seq_lens), rows=B, n_single=B, n_few=B, span=upper + 1, plans={},
                         short=RowSegments(None, B, 1), long=None, row_index=None, n_out=B))
     if next_ids is not None:
         argmax(ctx, state.logits, next_ids)
@@ -180,14 +183,16 @@ def forward(ctx: GPUContext, state: SequenceState, entries: Sequence[Tuple[int, 
         if state.lengths[slot] + len(tokens) > state.max_seq_len:
             raise ValueError(f"Cache is full: current_len={state.lengths[slot]} + {len(tokens)}, max_seq_len={state.max_seq_len}")
     short = [len(t) <= SHORT_ENTRY or not state.prompt_form for _, t, _ in entries]
-    order = sorted(range(len(entries)), key=lambda j: not short[j])  # stable: short entries first
+    order = sorted(range(len(entries)), key=lambda j: len(entries[j][1]) > SHORT_ENTRY)  # stable: short entries first
     ids, slots, pos, first_row, spans, lens = [], [], [], {}, [], list(state.lengths)
     runs = {True: [], False: []}  # (first row, rows, sequence) of the short entries and of the prompt portions
-    T, n_single, span = 0, 0, 1
+    T, n_single, n_few, span = 0, 0, 0, 1
     for j in order:
         slot, tokens, _ = entries[j]
         first_row[j] = T
         start, n = lens[slot], len(tokens)
+        if n <= SHORT_ENTRY:
+            n_few += n
         if short[j]:
             n_single += n
             span = max(span, start + n)
@@ -212,7 +217,7 @@ def forward(ctx: GPUContext, state: SequenceState, entries: Sequence[Tuple[int, 
     segments = [RowSegments(table, len(r), max(n for _, n, _ in r)) if r else None
                 for table, r in ((pieces[5], runs[True]), (pieces[6], runs[False]))]
     batch_begin(ctx)
-    state.run(ctx, Step(ids=pieces[0], places=RowPlaces(pieces[1], pieces[2]), rows=T, n_single=n_single, span=span, plans=plans,
+    state.run(ctx, Step(ids=pieces[0], places=RowPlaces(pieces[1], pieces[2]), rows=T, n_single=n_single, n_few=n_few, span=span, plans=plans,
                         short=segments[0], long=segments[1], row_index=pieces[3], n_out=n_out))
     batch_commit(ctx)
     state.seq_lens.copy_(pieces[4])
