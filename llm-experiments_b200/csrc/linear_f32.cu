@@ -1,15 +1,16 @@
-// b2kv_linear in fp32 on the CUDA cores (rows grouped by expert, few rows, few input features), two kernels.  Sums are fp32 multiply-adds, so what bounds them is that pipe (72 TFLOP/s
-// over the chip at 1.9 GHz) for many rows and the weights' bytes for few.  693 rows, 3072 x 768 weights: 441 us with linear_simt_kernel
-// (one read of shared memory per two multiply-adds, 132 CTAs, nothing ahead of its use), 158 here; 6 rows, 768 x 4096: 128 and 14.
+// b2kv_linear in fp32 on the CUDA cores, two kernels: what linear_f32_tc_kernel does not take, as rows grouped by expert, few rows and few
+// input features.  Sums are fp32 multiply-adds, so what bounds them is that pipe (72 TFLOP/s over the chip at 1.9 GHz) for many rows and
+// the weights' bytes for few.
 //
 // linear_f32_tile_kernel: 64 x 128 outputs per CTA of 128 threads, 8 x 8 per thread: 64 multiply-adds for every four 16-byte reads
 // of shared memory, so the pipe and not the reads is what is busy.  Steps of 16 input features through two buffers; the next
-// step's global reads are in flight (in registers) under the products of this one.  A product whose tiles leave SMs idle has its
-// input features cut into up to eight ranges, one per CTA of a cluster; the partial sums meet in distributed shared memory, where
-// every CTA adds up its share of the tile's rows in the order of the ranges (results do not depend on timing).
+// step's global reads are in flight (in registers) under the products of this one.  2000 rows of 16 experts, 768 x 1536: 292 us with
+// linear_simt_kernel (one read of shared memory per two multiply-adds, nothing ahead of its use), 150 here.
 //
 // linear_f32_rows_kernel: up to 16 rows (a decode step, the wanted logits).  A thread keeps four neighbouring columns of every row;
-// the warps of a CTA and the CTAs of a cluster share the input features, so w is read once, 512 bytes per warp at a time.
+// the warps of a CTA and the CTAs of a cluster share the input features, so w is read once, 512 bytes per warp at a time; the clusters'
+// partial sums meet in distributed shared memory, in the order of the ranges (results do not depend on timing).  6 rows, 768 x 4096: 128 us
+// with linear_simt_kernel, 14 here.
 #include <algorithm>
 
 #include "linear.cuh"
@@ -57,7 +58,7 @@ __device__ __forceinline__ Operands operands(const b2kv_linear_args& a, int g) {
     return o;
 }
 
-__global__ void __launch_bounds__(kThreads, 3) linear_f32_tile_kernel(const __grid_constant__ b2kv_linear_args a, int splits) {
+__global__ void __launch_bounds__(kThreads, 3) linear_f32_tile_kernel(const __grid_constant__ b2kv_linear_args a) {
     struct Ring {
         float x[2][kStep][kLdX], w[2][kStep][kBN];
     };
@@ -68,12 +69,8 @@ __global__ void __launch_bounds__(kThreads, 3) linear_f32_tile_kernel(const __gr
     grid_dependency_wait();
     const int g = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const Operands op = operands(a, g);
-    const int split = splits > 1 ? static_cast<int>(cluster_rank()) : 0;
-    const int row0 = blockIdx.y * kBM, col0 = static_cast<int>(blockIdx.x) / splits * kBN;
-    if (row0 >= op.n_rows) return;  // (all CTAs of a cluster)
-    const int steps = (a.K + kStep - 1) / kStep;
-    const int k_first = static_cast<int>(static_cast<long long>(steps) * split / splits) * kStep;
-    const int k_end = min(static_cast<int>(static_cast<long long>(steps) * (split + 1) / splits) * kStep, a.K);
+    const int row0 = blockIdx.y * kBM, col0 = blockIdx.x * kBN;
+    if (row0 >= op.n_rows) return;
 
     // x: a warp reads one 16-byte piece of 32 rows (the same pieces of the other rows next); w: whole rows of 128 columns
     float4 xr[2], wr[4];
@@ -81,13 +78,13 @@ __global__ void __launch_bounds__(kThreads, 3) linear_f32_tile_kernel(const __gr
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int r = row0 + lane + 32 * i, k = k0 + warp * 4;
-            xr[i] = r < op.n_rows && k < k_end ? *reinterpret_cast<const float4*>(op.x + static_cast<int64_t>(r) * a.ld_x + k)
+            xr[i] = r < op.n_rows && k < a.K ? *reinterpret_cast<const float4*>(op.x + static_cast<int64_t>(r) * a.ld_x + k)
                                                : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int k = k0 + warp + 4 * i, c = col0 + lane * 4;
-            wr[i] = k < k_end && c < a.N ? __ldg(reinterpret_cast<const float4*>(op.w + static_cast<int64_t>(k) * a.ld_w + c))
+            wr[i] = k < a.K && c < a.N ? __ldg(reinterpret_cast<const float4*>(op.w + static_cast<int64_t>(k) * a.ld_w + c))
                                          : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
@@ -103,12 +100,12 @@ __global__ void __launch_bounds__(kThreads, 3) linear_f32_tile_kernel(const __gr
     // a warp has 32 rows x 64 columns, a thread rows r, r + 16 .. + 3 and columns c, c + 32 .. + 3 of them
     const int tr = (warp & 1) * 32 + (lane >> 3) * 4, tc = (warp >> 1) * 64 + (lane & 7) * 4;
     float acc[8][8] = {};
-    read(k_first);
+    read(0);
     write(0);
     __syncthreads();
     int buf = 0;
-    for (int k0 = k_first; k0 < k_end; k0 += kStep, buf ^= 1) {
-        const bool more = k0 + kStep < k_end;
+    for (int k0 = 0; k0 < a.K; k0 += kStep, buf ^= 1) {
+        const bool more = k0 + kStep < a.K;
         if (more) read(k0 + kStep);
 #pragma unroll
         for (int k = 0; k < kStep; ++k) {
@@ -133,26 +130,11 @@ __global__ void __launch_bounds__(kThreads, 3) linear_f32_tile_kernel(const __gr
         for (int j = 0; j < 8; j += 4)
             *reinterpret_cast<float4*>(&sm.tile[tr + (i & 3) + (i >> 2) * 16][tc + j * 8]) =
                 make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
-    if (splits > 1) cluster_sync();
-    else __syncthreads();
-    const int c = (tid & 63) * 2, share = kBM / splits;
-    uint32_t peer[8];
-#pragma unroll
-    for (int s = 0; s < 8; ++s) peer[s] = s < splits ? peer_address(&sm.tile[0][c], s) : 0u;
-    const bool live = col0 + c < a.N;
-    for (int r = split * share + (tid >> 6); r < (split + 1) * share; r += 2) {
-        if (!live || row0 + r >= op.n_rows) break;
-        float2 v = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-            if (s >= splits) break;
-            const float2 p = peer_load2(peer[s] + r * kLdT * 4);
-            v.x += p.x, v.y += p.y;
-        }
-        lin::finish_pair<float>(a, g, op.first + row0 + r, col0 + c, v.x, v.y);
-    }
-    __syncwarp();
-    if (splits > 1) cluster_sync();  // the peers have read this CTA's part
+    __syncthreads();
+    const int c = (tid & 63) * 2;
+    if (col0 + c >= a.N) return;
+    for (int r = tid >> 6; r < min(kBM, op.n_rows - row0); r += 2)
+        lin::finish_pair<float>(a, g, op.first + row0 + r, col0 + c, sm.tile[r][c], sm.tile[r][c + 1]);
 }
 
 constexpr int kRowsThreads = 256, kRowsCols = 128, kChunkK = 128;
@@ -253,17 +235,12 @@ int linear_f32(const b2kv_linear_args& a, void* stream) {
         return B2KV_ERR_UNSUPPORTED;
     const int max_rows = a.group_rows ? a.max_group_rows : a.rows, sms = device_sm_count();
     const long long tiles_n = (a.N + kBN - 1) / kBN;
-    int splits = 1;
-    auto forced = [](int by_shape) {  // the knob of the tensor-core kernel for few rows
-        int s = 1;
-        while (s < 8 && s * 2 <= tune_get("matmul_splits")) s *= 2;
-        return tune_get("matmul_splits") > 0 ? s : by_shape;
-    };
     if (max_rows <= 16) {
         // ranges of at least one chunk, two CTAs per SM at most
         const long long tiles = tiles_n * a.groups;
-        while (splits < 8 && tiles * splits * 2 <= 2 * sms && splits * 2 * kChunkK <= a.K) splits *= 2;
-        splits = forced(splits);
+        int splits = 1;
+        const int forced = tune_get("matmul_splits");
+        while (splits < 8 && (forced > 0 ? splits * 2 <= forced : tiles * splits * 2 <= 2 * sms && splits * 2 * kChunkK <= a.K)) splits *= 2;
         if (tiles_n * splits > 0x7fffffffLL || a.groups > 65535) return B2KV_ERR_UNSUPPORTED;
         OverlapLaunch launch(dim3(static_cast<unsigned>(tiles_n * splits), 1, a.groups), kRowsThreads, 0, stream, splits);
         B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg,
@@ -272,19 +249,10 @@ int linear_f32(const b2kv_linear_args& a, void* stream) {
                                          a, splits));
         return B2KV_OK;
     }
-    const long long tiles_m = (max_rows + kBM - 1) / kBM, tiles = tiles_n * tiles_m * a.groups;
-    // The work of the fullest SM, in CTAs of whole input features; a range keeps eight steps at least.  (With rows grouped by
-    // expert most of the tiles that max_group_rows allows for are empty: no ranges.)
-    double best = 1e30;
-    for (int s = 1; s <= 8 && !(s > 1 && a.group_rows); s *= 2) {
-        if (s > 1 && a.K < 8 * kStep * s) break;
-        const double cost = static_cast<double>((tiles * s + sms - 1) / sms) / s + 0.02 * (s - 1);
-        if (cost < 0.95 * best) best = cost, splits = s;
-    }
-    splits = forced(splits);
-    if (tiles_m > 65535 || a.groups > 65535 || tiles_n * splits > 0x7fffffffLL) return B2KV_ERR_UNSUPPORTED;
-    OverlapLaunch launch(dim3(static_cast<unsigned>(tiles_n * splits), static_cast<unsigned>(tiles_m), a.groups), kThreads, 0, stream, splits);
-    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, linear_f32_tile_kernel, a, splits));
+    const long long tiles_m = (max_rows + kBM - 1) / kBM;
+    if (tiles_m > 65535 || a.groups > 65535 || tiles_n > 0x7fffffffLL) return B2KV_ERR_UNSUPPORTED;
+    OverlapLaunch launch(dim3(static_cast<unsigned>(tiles_n), static_cast<unsigned>(tiles_m), a.groups), kThreads, 0, stream);
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, linear_f32_tile_kernel, a));
     return B2KV_OK;
 }
 

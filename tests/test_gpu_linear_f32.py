@@ -1,5 +1,6 @@
-"""fp32 products on the CUDA cores (the choice left open) against float64: few rows and tiles, their edges, ranges of input features,
-every kind of segment, groups."""
+"""fp32 products (the choice left open) against float64: tiles and their edges, ranges of input features, every kind of segment,
+groups.  Up to 16 rows take the kernel for few rows, more with at least 128 input features the tensor cores, everything else (fewer input
+features, rows of experts) the tiles of the CUDA cores."""
 import numpy as np
 import pytest
 import torch
@@ -40,7 +41,8 @@ def test_store_and_residual(pkg, rows, K, cols):
 @pytest.mark.parametrize("splits", [1, 2, 4, 8])
 @pytest.mark.parametrize("rows,K", [(3, 2048), (16, 1000), (70, 1040), (64, 64)])
 def test_ranges_of_input_features(pkg, rows, K, splits):
-    """Any number of ranges, also more than there are steps."""
+    """Any number of ranges, also more than there are steps: of the kernel for few rows and, at 70 rows, of the tensor cores (64 rows of
+    64 input features go to a kernel without ranges, which leaves the knob alone)."""
     from llm_experiments_b200 import _native
     from llm_experiments_b200 import projection as proj
 
@@ -54,6 +56,13 @@ def test_ranges_of_input_features(pkg, rows, K, splits):
     finally:
         _native.tune("matmul_splits", 0)
     bounded(out, x, w, bias.double())
+
+
+@pytest.mark.parametrize("splits", [3, 5, 6, 7])
+@pytest.mark.parametrize("rows,K", [(17, 384), (70, 1040), (300, 452)])
+def test_any_number_of_ranges_on_the_tensor_cores(pkg, rows, K, splits):
+    """Clusters of any size share rows that they do not divide, with a step or two of input features each, or none."""
+    test_ranges_of_input_features(pkg, rows, K, splits)
 
 
 @pytest.mark.parametrize("rows", [6, 90])
@@ -74,11 +83,11 @@ def test_kinds(pkg, rows, kind):
     assert (out[rows] == 7).all() and (out[:, -1] == 7).all()
 
 
-@pytest.mark.parametrize("counts", [(3, 0, 16, 1), (0, 130, 64, 1, 0)])
-def test_rows_of_experts(pkg, counts):
+@pytest.mark.parametrize("counts,K", [((3, 0, 16, 1), 132), ((0, 130, 64, 1, 0), 132), ((0, 130, 64, 1, 0), 1044), ((65, 700), 16), ((17, 1), 516)])
+def test_rows_of_experts(pkg, counts, K):
     from llm_experiments_b200 import projection as proj
 
-    ctx, K, n = make_ctx(pkg), 132, 140
+    ctx, n = make_ctx(pkg), 140
     offs = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
     x, w = rnd((sum(counts), K), F32, 9), rnd((len(counts) * K, n), F32, 10, K ** -0.5)
     out = torch.empty((sum(counts), n), dtype=F32, device="cuda")
