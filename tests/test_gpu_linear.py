@@ -145,6 +145,36 @@ def test_rows_grouped_by_expert(pkg, path, dtype, counts, K, n, glu_kind):
     assert (out[R] == 7).all()
 
 
+@pytest.mark.parametrize("rows", [3, 40, 100])
+@pytest.mark.parametrize("K", [72, 1000])
+def test_few_rows_with_more_tiles_than_sms(pkg, rows, K):
+    """Two CTAs per SM where they fit, rings of as few stages as there are."""
+    from llm_experiments_b200 import projection as proj
+
+    ctx, n = make_ctx(pkg), 128 * (torch.cuda.get_device_properties(0).multi_processor_count + 2) + 24
+    x, w = rnd((rows, K), torch.bfloat16, 31), rnd((K, n), torch.bfloat16, 32, K ** -0.5)
+    out = torch.full((rows + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), K, [proj.OutputSegment(n, proj.SEG_STORE, wrap(pkg, out))], path=ROWS)
+    close(out[:rows], x.double() @ w.double(), torch.bfloat16)
+    assert (out[rows] == 7).all()
+
+
+@pytest.mark.parametrize("most,K", [(16, 1000), (128, 1000), (128, 200)])
+def test_experts_of_unequal_rows_with_more_tiles_than_sms(pkg, most, K):
+    """Every expert has as many stages as its own rows leave room for: none, one, around the sixteens, and the most there may be."""
+    from llm_experiments_b200 import projection as proj
+
+    ctx, n, counts = make_ctx(pkg), 520, [min(most, c) for c in (0, 1, 15, 16, 17, 33, 64, 96, 97, 128)] * 4
+    offs = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    x, w = rnd((sum(counts), K), torch.bfloat16, 33), rnd((len(counts) * K, n), torch.bfloat16, 34, K ** -0.5)
+    out = torch.full((sum(counts) + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), K, [proj.OutputSegment(n, proj.SEG_STORE, wrap(pkg, out))], groups=len(counts), group_w=K * n,
+        group_rows=torch.from_numpy(offs).cuda(), max_group_rows=most, path=ROWS)
+    for e in range(len(counts)):
+        close(out[offs[e]:offs[e + 1]], x[offs[e]:offs[e + 1]].double() @ w[e * K:(e + 1) * K].double(), torch.bfloat16)
+    assert (out[-1] == 7).all()
+
+
 def activated(kind, z, limit, proj):
     if kind == proj.SEG_RELU2:
         return z.clamp(min=0) ** 2
