@@ -285,16 +285,16 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
     const int c = (tid & 63) * 2, share = (kBM + splits - 1) / splits;
     bool complete = true;
     for (int s = 0; s < splits; ++s) complete = complete && peer_load1(peer_address(smem_u32(const_cast<int*>(&sm.abort_flag)), s)) == 0;
-    if (complete && col0 + c < a.N) {
-        for (int r = split * share + (tid >> 6); r < min((split + 1) * share, kBM) && row0 + r < a.rows; r += kThreads / 64) {
-            float2 v = make_float2(0.f, 0.f);
-            for (int s = 0; s < splits; ++s) {
-                const float2 p = peer_load2(peer_address(smem_u32(tile + r * kLdT + c), s));
-                v.x += p.x, v.y += p.y;
-            }
-            lin::finish_pair<float>(a, g, row0 + r, col0 + c, v.x, v.y);
-        }
-    }
+    if (complete && col0 + c < a.N)
+        lin::finish_rows<float>(a, g, col0 + c, row0, split * share + (tid >> 6), min(min((split + 1) * share, kBM), a.rows - row0), kThreads / 64,
+                                [&](int r) {
+                                    float2 v = make_float2(0.f, 0.f);
+                                    for (int s = 0; s < splits; ++s) {
+                                        const float2 p = peer_load2(peer_address(smem_u32(tile + r * kLdT + c), s));
+                                        v.x += p.x, v.y += p.y;
+                                    }
+                                    return v;
+                                });
     __syncwarp();
     if (splits > 1) cluster_sync();  // the peers have read this CTA's part
     if (warp == 0) {

@@ -1,5 +1,5 @@
 """fp32 products (the choice left open) against float64: tiles and their edges, ranges of input features, every kind of segment,
-groups.  Up to 16 rows take the kernel for few rows, more with at least 128 input features the tensor cores, everything else (fewer input
+groups.  Up to 16 rows take the kernel for few rows (one row from 16 input features on), more with at least 128 input features the tensor cores, everything else (fewer input
 features, rows of experts) the tiles of the CUDA cores."""
 import numpy as np
 import pytest
