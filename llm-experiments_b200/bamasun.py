@@ -318,9 +318,9 @@ def _attend(ctx, state: BamasunState, i: int, xs: GPUBuffer2D, step: Step) -> GP
     gqa.gqa_append(ctx, y, a, step.places, cache, lc.kv_from is None, w.q_norm, w.k_norm, state.cfg.eps)
     # (in fp32 prompt portions go row by row as well, but many rows of one sequence share what they read)
     few = step.n_few if state.dtype == torch.float32 else step.n_single
-    for r0, r1, path in ((0, few, 0), (few, step.n_single, gqa.RUNS)):
+    for r0, r1, runs in ((0, few, False), (few, step.n_single, True)):
         if r0 < r1:
-            gqa.gqa_decode(ctx, sub(y, r0, r1 - r0), a, w.slopes, step.single_places(r0, r1), cache, sub(out, r0, r1 - r0), step.span, path)
+            gqa.gqa_decode(ctx, sub(y, r0, r1 - r0), a, w.slopes, step.single_places(r0, r1), cache, sub(out, r0, r1 - r0), step.span, runs=runs)
     if step.plans:
         gqa.gqa_prefill(ctx, y, a, w.slopes, step.plans[0], cache, out)
     return out

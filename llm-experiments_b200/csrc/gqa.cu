@@ -468,25 +468,36 @@ extern "C" size_t b2kv_gqa_decode_workspace_bytes(int rows, int H, int G, int vd
     return gqa_decode_tc_workspace(rows, H, G, vdim, span);
 }
 
-extern "C" int b2kv_gqa_decode(const void* q, int64_t ld_q, const void* k_cache, const void* v_cache, void* out, int64_t ld_out,
-                               const float* slopes, const int32_t* row_slot, const int32_t* row_pos, int n_slots, int T_max,
-                               int rows, int H, int G, int dim, int vdim, int span, float scale, int dtype, int path,
-                               void* workspace, size_t workspace_bytes, int32_t* dev_status, void* stream) {
+static int gqa_decode(const GqaDecodeArgs& a, int dtype, int path, bool runs, void* workspace, size_t workspace_bytes, void* stream) {
     if (elt_bytes(dtype) == 0) return B2KV_ERR_UNSUPPORTED;
-    if (!q || !k_cache || !v_cache || !out || !row_pos) return B2KV_ERR_BAD_ARG;
-    if (n_slots <= 0 || T_max <= 0 || rows <= 0 || H <= 0 || G <= 0 || H % G != 0 || dim <= 0 || vdim <= 0 || span <= 0 ||
-        path < 0 || path > 3 || ld_q < static_cast<int64_t>(H) * dim || ld_out < static_cast<int64_t>(H) * vdim)
+    if (!a.q || !a.k_cache || !a.v_cache || !a.out || !a.row_pos) return B2KV_ERR_BAD_ARG;
+    if (a.n_slots <= 0 || a.T_max <= 0 || a.rows <= 0 || a.H <= 0 || a.G <= 0 || a.H % a.G != 0 || a.dim <= 0 || a.vdim <= 0 || a.span <= 0 ||
+        path < 0 || path > 2 || a.ld_q < static_cast<int64_t>(a.H) * a.dim || a.ld_out < static_cast<int64_t>(a.H) * a.vdim)
         return B2KV_ERR_BAD_ARG;
-    const GqaDecodeArgs a{q, k_cache, v_cache, out, slopes, row_slot, row_pos, dev_status, ld_q, ld_out,
-                          n_slots, T_max, rows, H, G, dim, vdim, span, scale};
     if (path == 2 && dtype != B2KV_DTYPE_BF16) return B2KV_ERR_UNSUPPORTED;
     if (dtype == B2KV_DTYPE_BF16 && path != 1) {
         const int rc = gqa_decode_tc(a, workspace, workspace_bytes, stream);
         if (rc != B2KV_ERR_UNSUPPORTED || path == 2) return rc;
     }
-    if (dtype == B2KV_DTYPE_F32 && path == 3) {
+    if (dtype == B2KV_DTYPE_F32 && path == 0 && runs) {
         const int rc = launch_runs_f32(a, stream);
         if (rc != B2KV_ERR_UNSUPPORTED) return rc;
     }
     return dtype == B2KV_DTYPE_F32 ? launch_simt<float>(a, stream) : launch_simt<__nv_bfloat16>(a, stream);
+}
+
+extern "C" int b2kv_gqa_decode(const void* q, int64_t ld_q, const void* k_cache, const void* v_cache, void* out, int64_t ld_out,
+                               const float* slopes, const int32_t* row_slot, const int32_t* row_pos, int n_slots, int T_max,
+                               int rows, int H, int G, int dim, int vdim, int span, float scale, int dtype, int path,
+                               void* workspace, size_t workspace_bytes, int32_t* dev_status, void* stream) {
+    return gqa_decode({q, k_cache, v_cache, out, slopes, row_slot, row_pos, dev_status, ld_q, ld_out, n_slots, T_max, rows, H, G, dim, vdim,
+                       span, scale}, dtype, path, false, workspace, workspace_bytes, stream);
+}
+
+extern "C" int b2kv_gqa_decode_runs(const void* q, int64_t ld_q, const void* k_cache, const void* v_cache, void* out, int64_t ld_out,
+                                    const float* slopes, const int32_t* row_slot, const int32_t* row_pos, int n_slots, int T_max,
+                                    int rows, int H, int G, int dim, int vdim, int span, float scale, int dtype, int path,
+                                    void* workspace, size_t workspace_bytes, int32_t* dev_status, void* stream) {
+    return gqa_decode({q, k_cache, v_cache, out, slopes, row_slot, row_pos, dev_status, ld_q, ld_out, n_slots, T_max, rows, H, G, dim, vdim,
+                       span, scale}, dtype, path, true, workspace, workspace_bytes, stream);
 }

@@ -10,7 +10,7 @@ from tests.kv_util import make_ctx
 pytestmark = pytest.mark.gpu
 
 F32, BF = torch.float32, torch.bfloat16
-SIMT, TC, RUNS = 1, 2, 3
+SIMT, TC = 1, 2
 
 
 def wrap(pkg, t):
@@ -151,8 +151,8 @@ def test_single_rows(pkg, path, dtype, heads, kv, dim, vdim, bias):
 
 @pytest.mark.parametrize("heads,kv,dim,vdim", [(3, 1, 4, 8), (4, 2, 64, 64), (2, 1, 72, 128), (2, 2, 128, 20)])
 @pytest.mark.parametrize("runs", [((0, 0, 65),), ((2, 0, 64), (0, 60, 7), (1, 199, 1), (2, 64, 31), (0, 0, 40)), ((1, 130, 96), (0, 3, 33))])
-@pytest.mark.parametrize("path", [0, RUNS])
-def test_runs_of_rows_in_fp32(pkg, heads, kv, dim, vdim, runs, path):
+@pytest.mark.parametrize("said", [False, True])
+def test_runs_of_rows_in_fp32(pkg, heads, kv, dim, vdim, runs, said):
     """Prompt portions of 16-row tiles and their parts, several sequences in a tile, one of them twice; nothing that a row must not
     see reaches it, not even what is no number."""
     from llm_experiments_b200 import gqa
@@ -171,7 +171,7 @@ def test_runs_of_rows_in_fp32(pkg, heads, kv, dim, vdim, runs, path):
     out = torch.full((len(pos) + 1, heads * vdim + 8), 7.0, dtype=F32, device="cuda")
     slopes = gqa.geometric_slopes(heads).cuda()
     places = RowPlaces(torch.tensor(slots, dtype=torch.int32, device="cuda"), torch.tensor(pos, dtype=torch.int32, device="cuda"))
-    in_batch(pkg, ctx, lambda: gqa.gqa_decode(ctx, wrap(pkg, y), shape, wrap1(pkg, slopes), places, cache, wrap(pkg, out[:len(pos)]), 240, path=path))
+    in_batch(pkg, ctx, lambda: gqa.gqa_decode(ctx, wrap(pkg, y), shape, wrap1(pkg, slopes), places, cache, wrap(pkg, out[:len(pos)]), 240, runs=said))
     k, v = (np64(t) for t in cache_views(cache, shape))
     want = reference(np64(y)[:, :heads * dim].reshape(len(pos), heads, dim), k, v, slots, pos, shape, bo.head_slopes(heads))
     got = np64(out)[:len(pos), :heads * vdim]
@@ -193,17 +193,17 @@ def test_the_kernel_for_runs_is_the_callers_choice(pkg):
         b[:2] = a
     y = rnd((rows, 4 * 64), F32, 7)
 
-    def attend(cache, slots, path):
+    def attend(cache, slots, path, runs=False):
         out = torch.empty_like(y)
         places = RowPlaces(torch.tensor(slots, dtype=torch.int32, device="cuda"), torch.arange(rows, dtype=torch.int32, device="cuda"))
-        in_batch(pkg, ctx, lambda: gqa.gqa_decode(ctx, wrap(pkg, y), shape, None, places, cache, wrap(pkg, out), 240, path=path))
+        in_batch(pkg, ctx, lambda: gqa.gqa_decode(ctx, wrap(pkg, y), shape, None, places, cache, wrap(pkg, out), 240, path=path, runs=runs))
         return out
 
     one, turns = [1] * rows, [i % 2 for i in range(rows)]
-    assert torch.equal(attend(large, one, gqa.RUNS), attend(small, one, gqa.RUNS))
+    assert torch.equal(attend(large, one, 0, True), attend(small, one, 0, True))
     assert torch.equal(attend(small, turns, 0), attend(small, turns, SIMT))
-    torch.testing.assert_close(attend(small, turns, gqa.RUNS), attend(small, turns, SIMT), rtol=2e-5, atol=2e-5)
-    assert not torch.equal(attend(small, one, gqa.RUNS), attend(small, one, SIMT))
+    torch.testing.assert_close(attend(small, turns, 0, True), attend(small, turns, SIMT), rtol=2e-5, atol=2e-5)
+    assert not torch.equal(attend(small, one, 0, True), attend(small, one, SIMT))
 
 
 @pytest.mark.parametrize("share", [1, 2, 3, 5, 16])
