@@ -401,9 +401,7 @@ int b2kv_layernorm_rows(const float* y, int64_t ld_y, const int32_t* row_index, 
  * x is [rows, K] with row pitch ld_x; w is [K, N] row-major with row pitch ld_w.  Group g (0 <= g < groups) reads
  * x + g * group_x and w + g * group_w and writes seg.out + g * seg.group: the heads of a per-head product.  With group_rows
  * (device, groups + 1 row offsets) group g instead owns rows group_rows[g] .. group_rows[g + 1] - 1 of x and of the outputs:
- * the experts of a mixture, whose rows are sorted by expert; no group has more than max_group_rows of them.  With group_x_rows
- * as well, the rows of x of group g start at group_x_rows[g] (runs of rows anywhere in a cache; x has x_rows rows), and
- * group_w = 0 gives all groups one w: tiled kernel only.
+ * the experts of a mixture, whose rows are sorted by expert; no group has more than max_group_rows of them.
  * Offsets and pitches are in elements.  Segment boundaries are even.  The product runs on the tensor cores for bf16 when
  * pitches, offsets and boundaries allow it (multiples of 8 elements; boundaries multiples of 32): at most 128 rows per
  * group stream the weights once, more go to the tiled kernel.  fp32 products of more than 16 rows and at least 128 input
@@ -436,10 +434,19 @@ typedef struct b2kv_linear_args {
     b2kv_segment seg[B2KV_MAX_SEGMENTS];
     int32_t rows, K, N, groups, max_group_rows, n_seg, dtype, path;
     float limit;
-    int32_t x_rows;              /* with group_x_rows: rows of x */
-    const int32_t* group_x_rows; /* with group_rows: first row of x of every group (device), or NULL: group_rows */
 } b2kv_linear_args;
 int b2kv_linear(const b2kv_linear_args* args, int32_t* dev_status, void* stream);
+
+/*
+ * b2kv_linear with more than its arguments say (NULL: nothing more).  With group_x_rows (device; group_rows too) the rows of x of group
+ * g start at group_x_rows[g] (runs of rows anywhere in a cache; x has x_rows rows), and group_w = 0 gives all groups one w: tiled
+ * kernel only.  flags: 0.
+ */
+typedef struct b2kv_linear_options {
+    const int32_t* group_x_rows;
+    int32_t x_rows, flags;
+} b2kv_linear_options;
+int b2kv_linear_opt(const b2kv_linear_args* args, const b2kv_linear_options* options, int32_t* dev_status, void* stream);
 
 /*
  * Latent attention (one latent row and one rotated key part per token, shared by all heads, are what the cache holds).

@@ -54,7 +54,13 @@ class LinearArgs(ctypes.Structure):
                 ("ld_w", _i64), ("group_w", _i64), ("ld_residual", _i64), ("seg", Segment * MAX_SEGMENTS),
                 ("rows", ctypes.c_int32), ("K", ctypes.c_int32), ("N", ctypes.c_int32), ("groups", ctypes.c_int32),
                 ("max_group_rows", ctypes.c_int32), ("n_seg", ctypes.c_int32), ("dtype", ctypes.c_int32),
-                ("path", ctypes.c_int32), ("limit", _f), ("x_rows", ctypes.c_int32), ("group_x_rows", _vp)]
+                ("path", ctypes.c_int32), ("limit", _f)]
+
+
+class LinearOptions(ctypes.Structure):
+    """``b2kv_linear_options``."""
+
+    _fields_ = [("group_x_rows", _vp), ("x_rows", ctypes.c_int32), ("flags", ctypes.c_int32)]
 
 
 class GlaArgs(ctypes.Structure):
@@ -112,6 +118,7 @@ SIGNATURES = {
     "b2kv_layernorm_rows": (_i, [_vp, _i64, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _i, _i, _f, _i, _vp]),
     "b2kv_rmsnorm": (_i, [_vp, _i64, _vp, _vp, _f, _vp, _i64, _i, _i, _f, _i, _vp]),
     "b2kv_linear": (_i, [ctypes.POINTER(LinearArgs), _vp, _vp]),
+    "b2kv_linear_opt": (_i, [ctypes.POINTER(LinearArgs), ctypes.POINTER(LinearOptions), _vp, _vp]),
     "b2kv_latent_append": (_i, [_vp, _i64, _i, _i, _i, _i, _vp, _i, _i, _vp, _f, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp]),
     "b2kv_latent_decode_workspace_bytes": (_sz, [_i, _i, _i, _i, _i]),
     "b2kv_latent_decode": (_i, [_vp, _vp, _i64, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp,

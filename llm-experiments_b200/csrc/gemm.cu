@@ -65,6 +65,7 @@ struct GemmParams {
 constexpr int kMaxGroups = 1024;
 struct SegParams {
     b2kv_linear_args a;
+    const int32_t* group_x_rows;  // first row of A of every group, or null: group_rows
     int M, N, K;
     int tiles_m, tiles_n, tile_cols;
     int32_t* dev_status;
@@ -166,7 +167,7 @@ __device__ __forceinline__ Tile find_tile(int t, const SegParams& p, const Group
     const int within = t - first * p.tiles_n;  // row tiles run fastest: they share the group's columns of W
     const int row0 = p.a.group_rows[lo], down = within % rows_here * tile_rows;
     return {row0 + down, p.a.group_rows[lo + 1], within / rows_here, p.a.group_w == 0 ? 0 : lo * p.K,
-            (p.a.group_x_rows != nullptr ? p.a.group_x_rows[lo] : row0) + down};
+            (p.group_x_rows != nullptr ? p.group_x_rows[lo] : row0) + down};
 }
 
 __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_addr, int grow, int row_end, int col_base, uint32_t* slab);
@@ -760,11 +761,12 @@ extern "C" int b2kv_matmul(const void* a, const void* w, const void* bias, const
 }
 
 // b2kv_linear with many rows: one product, or rows grouped by expert.
-int b2kv::linear_tiled_tc(const b2kv_linear_args& a, int32_t* dev_status, void* stream) {
+int b2kv::linear_tiled_tc(const b2kv_linear_args& a, const b2kv_linear_options& o, int32_t* dev_status, void* stream) {
     if (a.dtype != B2KV_DTYPE_BF16) return B2KV_ERR_UNSUPPORTED;
     const bool grouped = a.group_rows != nullptr;
     if (a.groups > 1 && !grouped) return B2KV_ERR_UNSUPPORTED;
-    if (grouped && (a.groups > gemm::kMaxGroups || (a.group_w != static_cast<int64_t>(a.K) * a.ld_w && !(a.group_w == 0 && a.group_x_rows)))) return B2KV_ERR_UNSUPPORTED;
+    const bool one_w = a.group_w == 0 && o.group_x_rows != nullptr;
+    if (grouped && (a.groups > gemm::kMaxGroups || (a.group_w != static_cast<int64_t>(a.K) * a.ld_w && !one_w))) return B2KV_ERR_UNSUPPORTED;
     if (!aligned16(a.x) || !aligned16(a.w) || a.ld_x % 8 || a.ld_w % 8 || a.ld_x < a.K || a.ld_w < a.N) return B2KV_ERR_UNSUPPORTED;
     int first = 0;
     for (int s = 0; s < a.n_seg; ++s) {  // 16-byte accesses in the epilogue; 32 columns lie in one segment
@@ -776,12 +778,12 @@ int b2kv::linear_tiled_tc(const b2kv_linear_args& a, int32_t* dev_status, void* 
     }
     if (a.bias && !aligned16(a.bias)) return B2KV_ERR_UNSUPPORTED;
     if (a.residual && (!aligned16(a.residual) || a.ld_residual % 4 != 0)) return B2KV_ERR_UNSUPPORTED;
-    gemm::SegParams p{a, a.rows, a.N, a.K, 0, 0, 0, dev_status};
+    gemm::SegParams p{a, o.group_x_rows, a.rows, a.N, a.K, 0, 0, 0, dev_status};
     // with groups the number of tiles is only known on the device: every group may end in a partly filled tile
     const long long part = grouped ? a.groups : 0;
     const long long tiles_m = (static_cast<long long>(a.rows) + gemm::kBM - 1) / gemm::kBM + part;
     const long long tiles_m_pair = (static_cast<long long>(a.rows) + 2 * gemm::kBM - 1) / (2 * gemm::kBM) + part;
     const bool tall = grouped ? a.rows / a.groups > 2 * gemm::kBM : a.rows > 2 * gemm::kBM;
-    return gemm::launch(p, a.x, a.group_x_rows ? a.x_rows : a.rows, a.ld_x, a.w, a.group_w ? static_cast<int64_t>(a.groups) * a.K : a.K, a.ld_w, tiles_m,
-                        tiles_m_pair, tall, grouped, stream);
+    return gemm::launch(p, a.x, o.group_x_rows ? o.x_rows : a.rows, a.ld_x, a.w, grouped && !one_w ? static_cast<int64_t>(a.groups) * a.K : a.K,
+                        a.ld_w, tiles_m, tiles_m_pair, tall, grouped, stream);
 }

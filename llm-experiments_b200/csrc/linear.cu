@@ -171,14 +171,20 @@ static int rows_in_slices(const b2kv_linear_args& all, int32_t* dev_status, void
 using namespace b2kv;
 
 extern "C" int b2kv_linear(const b2kv_linear_args* args, int32_t* dev_status, void* stream) {
+    return b2kv_linear_opt(args, nullptr, dev_status, stream);
+}
+
+extern "C" int b2kv_linear_opt(const b2kv_linear_args* args, const b2kv_linear_options* options, int32_t* dev_status, void* stream) {
     if (args == nullptr) return B2KV_ERR_BAD_ARG;
     const b2kv_linear_args& a = *args;
+    const b2kv_linear_options o = options != nullptr ? *options : b2kv_linear_options{};
+    if (o.flags != 0) return B2KV_ERR_BAD_ARG;
     if (elt_bytes(a.dtype) == 0) return B2KV_ERR_UNSUPPORTED;
     if (!a.x || !a.w || a.rows <= 0 || a.K <= 0 || a.N <= 0 || a.groups <= 0 || a.path < 0 || a.path > 4) return B2KV_ERR_BAD_ARG;
     if (a.n_seg < 1 || a.n_seg > B2KV_MAX_SEGMENTS || a.seg[a.n_seg - 1].end != a.N) return B2KV_ERR_BAD_ARG;
     if (a.bias && a.groups > 1) return B2KV_ERR_BAD_ARG;
     if (a.group_rows && (a.max_group_rows <= 0 || a.max_group_rows > a.rows)) return B2KV_ERR_BAD_ARG;
-    if (a.group_x_rows && (!a.group_rows || a.x_rows <= 0)) return B2KV_ERR_BAD_ARG;
+    if (o.group_x_rows && (!a.group_rows || o.x_rows <= 0)) return B2KV_ERR_BAD_ARG;
     int first = 0;
     for (int s = 0; s < a.n_seg; ++s) {
         const b2kv_segment& sg = a.seg[s];
@@ -187,9 +193,9 @@ extern "C" int b2kv_linear(const b2kv_linear_args* args, int32_t* dev_status, vo
         if ((sg.end & 1) && (s + 1 < a.n_seg || lin::is_pair(sg.kind))) return B2KV_ERR_BAD_ARG;
         first = sg.end;
     }
-    if (a.group_x_rows) return a.path == 0 || a.path == 3 ? linear_tiled_tc(a, dev_status, stream) : B2KV_ERR_UNSUPPORTED;
+    if (o.group_x_rows) return a.path == 0 || a.path == 3 ? linear_tiled_tc(a, o, dev_status, stream) : B2KV_ERR_UNSUPPORTED;
     if (a.path == 2) return linear_rows_tc(a, dev_status, stream);
-    if (a.path == 3) return linear_tiled_tc(a, dev_status, stream);
+    if (a.path == 3) return linear_tiled_tc(a, o, dev_status, stream);
     if (a.path == 4) return lin::launch_thin(a, stream);
     if (a.path == 0 && a.dtype == B2KV_DTYPE_BF16) {
         int rc = lin::launch_thin(a, stream);
@@ -199,7 +205,7 @@ extern "C" int b2kv_linear(const b2kv_linear_args* args, int32_t* dev_status, vo
         } else if (a.groups > 1 && a.group_rows == nullptr) {
             rc = lin::rows_in_slices(a, dev_status, stream);
         } else {
-            rc = linear_tiled_tc(a, dev_status, stream);
+            rc = linear_tiled_tc(a, o, dev_status, stream);
         }
         if (rc != B2KV_ERR_UNSUPPORTED) return rc;
     }

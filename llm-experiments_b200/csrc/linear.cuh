@@ -184,6 +184,6 @@ int linear_f32_tc(const b2kv_linear_args& a, int32_t* dev_status, void* stream);
 
 // bf16 kernels on the tensor cores; B2KV_ERR_UNSUPPORTED when the shape is not one they take.
 int linear_rows_tc(const b2kv_linear_args& a, int32_t* dev_status, void* stream);   // linear_rows.cu
-int linear_tiled_tc(const b2kv_linear_args& a, int32_t* dev_status, void* stream);  // gemm.cu
+int linear_tiled_tc(const b2kv_linear_args& a, const b2kv_linear_options& o, int32_t* dev_status, void* stream);  // gemm.cu
 
 }  // namespace b2kv

@@ -160,7 +160,8 @@ def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Se
         a.bias = bias.buffer.data_ptr()
     if group_rows is not None:
         a.group_rows = group_rows.data_ptr()
+    options = None
     if group_x_rows is not None:
-        a.group_x_rows, a.x_rows = group_x_rows.data_ptr(), x.shape[0]
+        options = ctypes.byref(_native.LinearOptions(group_x_rows=group_x_rows.data_ptr(), x_rows=x.shape[0]))
     stream = batch_op_begin(ctx)
-    _native.check(_native.lib.b2kv_linear(ctypes.byref(a), dev_status_ptr(ctx), stream))
+    _native.check(_native.lib.b2kv_linear_opt(ctypes.byref(a), options, dev_status_ptr(ctx), stream))

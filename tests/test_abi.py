@@ -100,3 +100,14 @@ def test_workspace_size_grows_with_the_problem(pkg):
     assert 0 < small < big
     assert lib.b2kv_decode_workspace_bytes(0, 4, 64, 256, 0) == 0
     assert lib.b2kv_decode_workspace_bytes(1, 4, 64, 256, 9) == 0
+
+
+def test_the_arguments_of_a_product_keep_their_size(pkg):
+    """A program built against an earlier header passes these bytes and no more; what came later has a struct of its own."""
+    native = pkg._native
+    assert ctypes.sizeof(native.LinearArgs) == 216 and native.LinearArgs.limit.offset == 208
+    lib, a = native.lib, native.LinearArgs(x=0x1000, w=0x1000, rows=4, K=8, N=8, groups=1, n_seg=1, dtype=1, ld_x=8, ld_w=8)
+    a.seg[0] = native.Segment(out=0x1000, ld=8, end=8)
+    for options in (native.LinearOptions(flags=1 << 30), native.LinearOptions(group_x_rows=0x1000, x_rows=4), native.LinearOptions(group_x_rows=0x1000)):
+        assert lib.b2kv_linear_opt(ctypes.byref(a), ctypes.byref(options), None, None) == -1
+    assert lib.b2kv_linear_opt(None, None, None, None) == -1
