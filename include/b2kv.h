@@ -26,13 +26,17 @@
  *   alignment    every pointer 16-byte aligned, D*sizeof(element) a multiple of 16,
  *                every stride*sizeof(element) a multiple of 16.
  *   stream       a cudaStream_t passed as void* (NULL = the legacy default stream).
- *   overlap      the kernels of a decode step (append, Q/K/V projection, decode, row products,
- *                layernorm, length advance) are launched with programmatic stream
- *                serialisation: each may be scheduled while the kernel before it in the
- *                stream is still running, sets itself up (and streams the first weight
- *                tiles, which no kernel writes), and waits for that kernel to complete
- *                before it reads anything else or writes at all.  Results are those of
- *                plain stream order; b2kv_tune("serial_launches", 1) switches it off.
+ *   overlap      most kernels (all of a decode step, products, recurrences, experts, fp32
+ *                prompts) are launched with programmatic stream serialisation: each may be
+ *                scheduled while the kernel before it in the stream is still running, sets
+ *                itself up, and waits for that kernel to complete before it reads what
+ *                kernels write or writes at all.  Results are those of plain stream order;
+ *                b2kv_tune("serial_launches", 1) switches it off.  The one thing that is read
+ *                before that wait are the first weight tiles of bf16 products of at most 128
+ *                rows, so their w must not be an output of a kernel that lets the next one
+ *                start early and may still run: of a bf16 product of at most 128 rows, or of
+ *                one with B2KV_LINEAR_AHEAD.  (A kernel that is not of those two kinds, any
+ *                other stream operation or a synchronisation in between is enough.)
  *   return       0 on success, a negative B2KV_ERR_* code otherwise; nothing is
  *                launched when an argument check fails.
  *   dev_status   optional int32 device word (NULL to skip).  A kernel that detects a
@@ -440,8 +444,10 @@ int b2kv_linear(const b2kv_linear_args* args, int32_t* dev_status, void* stream)
 /*
  * b2kv_linear with more than its arguments say (NULL: nothing more).  With group_x_rows (device; group_rows too) the rows of x of group
  * g start at group_x_rows[g] (runs of rows anywhere in a cache; x has x_rows rows), and group_w = 0 gives all groups one w: tiled
- * kernel only.  flags: 0.
+ * kernel only.  flags: B2KV_LINEAR_AHEAD lets the kernel behind this one in the stream start before the outputs are stored (see
+ * "overlap"): for outputs that no product takes for its w.
  */
+#define B2KV_LINEAR_AHEAD 1
 typedef struct b2kv_linear_options {
     const int32_t* group_x_rows;
     int32_t x_rows, flags;

@@ -39,6 +39,7 @@ _f = ctypes.c_float
 
 SEG_STORE, SEG_F32, SEG_GLU_SILU, SEG_GLU_CLAMP, SEG_RELU2, SEG_SOFTCAP, SEG_DECAY = 0, 1, 2, 3, 4, 5, 6
 MAX_SEGMENTS = 3
+LINEAR_AHEAD = 1
 
 
 class Segment(ctypes.Structure):

@@ -58,6 +58,7 @@ struct GemmParams {
     int M, N, K;
     int gelu;
     int tiles_m, tiles_n, tile_cols;
+    int ahead;            // the kernel behind may start before the outputs are stored (it may read its weights then)
     int32_t* dev_status;  // optional status word: receives B2KV_DEV_WAIT_TIMEOUT when a bounded wait ran out
 };
 
@@ -68,6 +69,7 @@ struct SegParams {
     const int32_t* group_x_rows;  // first row of A of every group, or null: group_rows
     int M, N, K;
     int tiles_m, tiles_n, tile_cols;
+    int ahead;
     int32_t* dev_status;
 };
 
@@ -224,7 +226,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                                     tl.k_row0 + kb * kBK);
                 }
             }
-            grid_launch_dependents();  // the next kernel sets up under the last products and outputs
+            if (p.ahead) grid_launch_dependents();  // the next kernel sets up under the last products and outputs
             if (!ok) sm.abort_flag = 1;
         }
         __syncwarp();
@@ -579,7 +581,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                                          tl.tn * p.tile_cols + r * (p.tile_cols / 2) + sp * 64, tl.k_row0 + kb * kBKP);
                 }
             }
-            grid_launch_dependents();  // the next kernel sets up under the last products and outputs
+            if (p.ahead) grid_launch_dependents();  // the next kernel sets up under the last products and outputs
             if (!ok) sm.abort_flag = 1;
         }
         __syncwarp();
@@ -756,7 +758,7 @@ extern "C" int b2kv_matmul(const void* a, const void* w, const void* bias, const
     if (!aligned16(a) || !aligned16(w) || !aligned16(out) || !aligned16(residual) || !aligned16(bias)) return B2KV_ERR_ALIGN;
     const long long tiles_m = (static_cast<long long>(M) + gemm::kBM - 1) / gemm::kBM;
     gemm::GemmParams p{static_cast<const __nv_bfloat16*>(bias), static_cast<const __nv_bfloat16*>(residual),
-                       static_cast<__nv_bfloat16*>(out), M, N, K, activation, 0, 0, 0, dev_status};
+                       static_cast<__nv_bfloat16*>(out), M, N, K, activation, 0, 0, 0, 0, dev_status};
     return gemm::launch(p, a, M, K, w, K, N, tiles_m, (tiles_m + 1) / 2, M > 2 * gemm::kBM, false, stream);
 }
 
@@ -778,7 +780,7 @@ int b2kv::linear_tiled_tc(const b2kv_linear_args& a, const b2kv_linear_options& 
     }
     if (a.bias && !aligned16(a.bias)) return B2KV_ERR_UNSUPPORTED;
     if (a.residual && (!aligned16(a.residual) || a.ld_residual % 4 != 0)) return B2KV_ERR_UNSUPPORTED;
-    gemm::SegParams p{a, o.group_x_rows, a.rows, a.N, a.K, 0, 0, 0, dev_status};
+    gemm::SegParams p{a, o.group_x_rows, a.rows, a.N, a.K, 0, 0, 0, o.flags & B2KV_LINEAR_AHEAD, dev_status};
     // with groups the number of tiles is only known on the device: every group may end in a partly filled tile
     const long long part = grouped ? a.groups : 0;
     const long long tiles_m = (static_cast<long long>(a.rows) + gemm::kBM - 1) / gemm::kBM + part;

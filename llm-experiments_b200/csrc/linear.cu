@@ -178,7 +178,7 @@ extern "C" int b2kv_linear_opt(const b2kv_linear_args* args, const b2kv_linear_o
     if (args == nullptr) return B2KV_ERR_BAD_ARG;
     const b2kv_linear_args& a = *args;
     const b2kv_linear_options o = options != nullptr ? *options : b2kv_linear_options{};
-    if (o.flags != 0) return B2KV_ERR_BAD_ARG;
+    if (o.flags & ~B2KV_LINEAR_AHEAD) return B2KV_ERR_BAD_ARG;
     if (elt_bytes(a.dtype) == 0) return B2KV_ERR_UNSUPPORTED;
     if (!a.x || !a.w || a.rows <= 0 || a.K <= 0 || a.N <= 0 || a.groups <= 0 || a.path < 0 || a.path > 4) return B2KV_ERR_BAD_ARG;
     if (a.n_seg < 1 || a.n_seg > B2KV_MAX_SEGMENTS || a.seg[a.n_seg - 1].end != a.N) return B2KV_ERR_BAD_ARG;

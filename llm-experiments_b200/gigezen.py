@@ -245,7 +245,7 @@ class GigezenState(SequenceState):
         hl = self.rows("h_out", step.n_out, cfg.width, self.dtype)
         rms_norm(ctx, x, w.final_norm, hl, cfg.eps, weight_offset=1.0, row_index=step.row_index)
         out = self.rows("logits", step.n_out, cfg.vocab_size, torch.float32)
-        linear(ctx, hl, w.head, cfg.width, [OutputSegment(cfg.vocab_size, SEG_F32, out)])
+        linear(ctx, hl, w.head, cfg.width, [OutputSegment(cfg.vocab_size, SEG_F32, out)], ahead=True)
         self.logits = out
 
 
@@ -274,10 +274,10 @@ def _attend_rows(ctx, state: GigezenState, i: int, y: GPUBuffer2D, z: GPUBuffer2
     ql = state.rows("q_latent", n, a.heads * a.kv_rank, state.dtype)
     ol = state.rows("o_latent", n, a.heads * a.kv_rank, state.dtype)
     linear(ctx, y, w.key_absorb, a.dim, [OutputSegment(a.kv_rank, SEG_STORE, ql, group=a.kv_rank)], groups=a.heads,
-           group_x=a.dim + a.rot, group_w=a.dim * a.kv_rank)
+           group_x=a.dim + a.rot, group_w=a.dim * a.kv_rank, ahead=True)
     latent.latent_decode(ctx, ql, y, a, places, state.cache_of(i), ol, span)
     linear(ctx, ol, _sub(w.expand, 0, a.kv_rank, w.k_cols), a.kv_rank, [OutputSegment(a.vdim, SEG_STORE, z, group=a.vdim)],
-           groups=a.heads, group_x=a.kv_rank, group_w=a.vdim)
+           groups=a.heads, group_x=a.kv_rank, group_w=a.vdim, ahead=True)
 
 
 def _layer(ctx, state: GigezenState, i: int, x: GPUBuffer2D, step: Step) -> None:
@@ -295,14 +295,14 @@ def _layer(ctx, state: GigezenState, i: int, x: GPUBuffer2D, step: Step) -> None
         segments.append(OutputSegment(w.y_cols + w.router_cols, SEG_F32, logits))
     if lc.dense_ff:
         segments.append(OutputSegment(w.y_cols + 2 * w.ff_cols, SEG_GLU_CLAMP, _sub(z, 0, T, w.a_cols)))
-    linear(ctx, h, w.w_in, cfg.width, segments, limit=lc.limit)
+    linear(ctx, h, w.w_in, cfg.width, segments, limit=lc.limit, ahead=True)
     latent.latent_append(ctx, y, a, w.inv_freq, step.places, cache, w.latent_norm, cfg.eps)
     n_single = step.n_single
     if n_single:
         _attend_rows(ctx, state, i, _sub(y, 0, n_single), _sub(z, 0, n_single, 0, a.heads * a.vdim), step.single_places(), step.span)
     if step.plans:
         _attend_prompts(ctx, state, i, y, _sub(z, 0, T, 0, a.heads * a.vdim), step.plans[a.window])
-    linear(ctx, z, w.w_out, w.a_cols + w.ff_cols, [OutputSegment(cfg.width, SEG_F32, x)], residual=x)
+    linear(ctx, z, w.w_out, w.a_cols + w.ff_cols, [OutputSegment(cfg.width, SEG_F32, x)], residual=x, ahead=True)
     if lc.router:
         moe.moe_feed_forward(ctx, h, logits, w.experts, lc.router, _moe_scratch(state, lc, w, T), x)
     if state.layer_tap is not None:
@@ -331,10 +331,10 @@ def _attend_prompts(ctx, state: GigezenState, i: int, y: GPUBuffer2D, z: GPUBuff
         # all portions in one launch: a thousand rows alone leave most of the chip idle
         linear(ctx, _b2(latents), w.expand, a.kv_rank, [OutputSegment(cols, SEG_STORE, _sub(kv, 0, plan.kv_rows))], groups=n, group_w=0,
                group_rows=plan.groups[:n + 1], max_group_rows=max(p[3] for p in plan.portions), group_x_rows=plan.groups[n + 1:],
-               rows=plan.kv_rows)
+               rows=plan.kv_rows, ahead=True)
     for _, _, cache_row, visible, kv_row in () if together else plan.portions:
         linear(ctx, _b2(latents[cache_row:cache_row + visible]), w.expand, a.kv_rank,
-               [OutputSegment(cols, SEG_STORE, _sub(kv, kv_row, visible))])
+               [OutputSegment(cols, SEG_STORE, _sub(kv, kv_row, visible))], ahead=True)
     latent.latent_prefill(ctx, y, _sub(kv, 0, plan.kv_rows, 0, a.heads * a.dim), _sub(kv, 0, plan.kv_rows, w.k_cols), a, plan,
                           cache, z)
 

@@ -86,7 +86,7 @@ def moe_feed_forward(ctx: GPUContext, h: GPUBuffer2D, logits: GPUBuffer2D, w: Ex
     n = rows * shape.top
     view = lambda b: GPUBuffer2D(buffer=b.buffer[:n], shape=(n, b.shape[1]), size=n * b.shape[1])  # noqa: E731
     linear(ctx, view(s.sorted_h), w.gate_up, width, [OutputSegment(2 * w.ff, SEG_GLU_SILU, s.m)],
-           group_w=width * w.gate_up.buffer.stride(0), **grouped)
+           group_w=width * w.gate_up.buffer.stride(0), **grouped, ahead=True)
     linear(ctx, view(s.m), w.down, w.ff, [OutputSegment(width, SEG_STORE, s.y)], group_w=w.ff * w.down.buffer.stride(0),
-           **grouped)
+           **grouped, ahead=True)
     combine(ctx, x, shape, s)

@@ -34,7 +34,8 @@ def matmul(ctx: GPUContext, A: GPUBuffer2D, B: GPUBuffer2D, C: GPUBuffer2D, resi
     dispatches which follow a matmul in the reference's block (src/wgpu_backend.py:857-930) into
     it: ``bias`` (a ``GPUBuffer1D`` of N values, ``bias_add``), ``activation="gelu"``
     (``x * sigmoid(1.702 x)``, ``gelu``) and ``residual`` (``residual_add``), applied in that order:
-    ``C = act(A @ B + bias) + residual``."""
+    ``C = act(A @ B + bias) + residual``.  ``B`` may be the ``C`` of a tiled GEMM before; the ``C`` of a product of at most 128 rows
+    may not be the ``B`` of another one right behind it, whose first tiles are read ahead of its end."""
     M, K = A.shape
     K2, N = B.shape
     # same checks and texts as validate_matmul_shapes (simple-llm/src/gpu/gpu_ops.py:84-99)
@@ -123,7 +124,8 @@ class OutputSegment:
 def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Sequence[OutputSegment],
            residual: Optional[GPUBuffer2D] = None, limit: float = 0.0, groups: int = 1, group_x: int = 0, group_w: int = 0,
            group_rows: Optional[torch.Tensor] = None, max_group_rows: int = 0, path: int = 0,
-           bias: Optional[GPUBuffer1D] = None, group_x_rows: Optional[torch.Tensor] = None, rows: Optional[int] = None) -> None:
+           bias: Optional[GPUBuffer1D] = None, group_x_rows: Optional[torch.Tensor] = None, rows: Optional[int] = None,
+           ahead: bool = False) -> None:
     """``x @ w`` (``+ bias``, fp32) with the output columns cut into segments, fp32 or bfloat16 storage, any sizes (``b2kv_linear``).
 
     ``x`` ``[rows, >= k]`` and ``w`` (rows of the weight matrix, ``[in, out]``) may be views with a row pitch.  With
@@ -132,7 +134,11 @@ def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Se
     group_rows[g + 1] - 1`` of ``x`` (the experts of a mixture; at most ``max_group_rows`` rows each).  With
     ``group_x_rows`` as well (int32 ``[groups]``), group g's rows of ``x`` start there, ``rows`` counts all groups' rows, and
     ``group_w`` 0 is one matrix for all (tiled kernel).  ``path`` forces a
-    kernel (1 CUDA cores, 2 weight streaming, 3 tiled, 4 few input features)."""
+    kernel (1 CUDA cores, 2 weight streaming, 3 tiled, 4 few input features).
+
+    Products of at most 128 bfloat16 rows read the first tiles of ``w`` before the kernel ahead of them has ended.  So ``w`` may be
+    the output of a product of more rows, but not of one whose caller said ``ahead``: that none of its outputs is a ``w`` and the
+    kernel behind it may start early; nor, right behind it, of a product of at most 128 rows."""
     rows, n = x.shape[0] if group_x_rows is None else rows, segments[-1].end
     if rows <= 0 or k <= 0 or n <= 0:
         raise ValueError(f"linear: Invalid dimensions x=({rows}, {k}), w=({k}, {n})")
@@ -161,7 +167,10 @@ def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Se
     if group_rows is not None:
         a.group_rows = group_rows.data_ptr()
     options = None
-    if group_x_rows is not None:
-        options = ctypes.byref(_native.LinearOptions(group_x_rows=group_x_rows.data_ptr(), x_rows=x.shape[0]))
+    if group_x_rows is not None or ahead:
+        options = _native.LinearOptions(flags=_native.LINEAR_AHEAD if ahead else 0)
+        if group_x_rows is not None:
+            options.group_x_rows, options.x_rows = group_x_rows.data_ptr(), x.shape[0]
+        options = ctypes.byref(options)
     stream = batch_op_begin(ctx)
     _native.check(_native.lib.b2kv_linear_opt(ctypes.byref(a), options, dev_status_ptr(ctx), stream))

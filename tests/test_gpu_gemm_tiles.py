@@ -100,3 +100,29 @@ def test_gelu_where_the_denominator_is_large(pkg):
     seen = want.abs() > 1.2e-38
     torch.testing.assert_close(out.double()[seen], want[seen], rtol=2.0 ** -8 + 2.0 ** -16, atol=0)  # bf16, and __expf of 90: 2^-16.5
     assert seen.sum() > 200 * n * 0.95
+
+
+@pytest.mark.parametrize("by_linear", [False, True])
+@pytest.mark.parametrize("rows", [256, 1024, 2048])
+def test_a_product_used_as_a_weight_right_away(pkg, rows, by_linear):
+    """The output of a tiled product is the second operand of the next one, of few rows, which reads its first tiles ahead of everything
+    else: it finds what was written, call after call, and not what lay there before."""
+    from llm_experiments_b200 import projection as proj
+
+    ctx, K, n = make_ctx(pkg), 2048, 1024
+    a, x = rnd((rows, K), BF, 21), rnd((8, rows), BF, 22)
+    weights = [rnd((K, n), BF, 23 + i, K ** -0.5) for i in range(6)]
+    c, out = torch.zeros((rows, n), dtype=BF, device="cuda"), [torch.empty((8, n), dtype=BF, device="cuda") for _ in weights]
+    pkg.gpu.batch_begin(ctx)
+    for w, o in zip(weights, out):
+        if by_linear:
+            proj.linear(ctx, wrap(pkg, a), wrap(pkg, w), K, [proj.OutputSegment(n, proj.SEG_STORE, wrap(pkg, c))])
+            proj.linear(ctx, wrap(pkg, x), wrap(pkg, c), rows, [proj.OutputSegment(n, proj.SEG_STORE, wrap(pkg, o))])
+        else:
+            proj.matmul(ctx, wrap(pkg, a), wrap(pkg, w), wrap(pkg, c))
+            proj.matmul(ctx, wrap(pkg, x), wrap(pkg, c), wrap(pkg, o))
+    pkg.gpu.batch_commit(ctx)
+    for w, o in zip(weights, out):
+        want = x.double() @ (a.double() @ w.double()).to(BF).double()
+        # c rounds once more or less at a tie: half a bf16 step of each of the terms at most, which are rows of order one
+        torch.testing.assert_close(o.double(), want, rtol=2.0 ** -7, atol=2.0 ** -8 * rows ** 0.5)
