@@ -59,32 +59,37 @@ struct SharedStorage {
     volatile int abort_flag;
 };
 
-// x -> (bf16(x), bf16(x - bf16(x))) of one row of Q, K or V (grid: rows, 3), and of K and V a copy in the cache.
+// x -> (bf16(x), bf16(x - bf16(x))) of a few rows of Q, K or V (grid: rows / per_cta, 3), and of K and V a copy in the cache.  As many rows per
+// CTA as give its threads a piece each: with one row of 128 elements per CTA the CTAs' launches were what bound it (16 x 129 rows of two
+// heads of 64, the whole call: 16.6 us so, 11.1 with eight).
 struct SplitArgs {
     const float* src[3];
     __nv_bfloat16 *hi[3], *lo[3];
     float* cache[3];  // null: none
     int64_t stride_b, stride_t, stride_h;
-    int N, E, D;
+    int64_t rows;
+    int N, E, D, per_cta;
 };
 __global__ void __launch_bounds__(256) split_kernel(const __grid_constant__ SplitArgs a) {
     grid_launch_dependents();
     grid_dependency_wait();
     const int which = blockIdx.y;
-    const int64_t row = blockIdx.x;
-    const float4* const x = reinterpret_cast<const float4*>(a.src[which] + row * a.E);
-    uint2* const hi = reinterpret_cast<uint2*>(a.hi[which] + row * a.E);
-    uint2* const lo = reinterpret_cast<uint2*>(a.lo[which] + row * a.E);
-    float* const cache = a.cache[which] == nullptr ? nullptr : a.cache[which] + row / a.N * a.stride_b + row % a.N * a.stride_t;
-    for (int i = threadIdx.x; i < a.E / 4; i += blockDim.x) {
+    const int64_t row0 = static_cast<int64_t>(blockIdx.x) * a.per_cta;
+    const int pieces = a.E / 4;  // of a row
+    const float4* const x = reinterpret_cast<const float4*>(a.src[which] + row0 * a.E);
+    uint2* const hi = reinterpret_cast<uint2*>(a.hi[which] + row0 * a.E);
+    uint2* const lo = reinterpret_cast<uint2*>(a.lo[which] + row0 * a.E);
+    const int all = static_cast<int>(min(static_cast<int64_t>(a.per_cta), a.rows - row0)) * pieces;
+    for (int i = threadIdx.x; i < all; i += blockDim.x) {
         const float4 v = x[i];
         const uint32_t h0 = pack_bf16(v.x, v.y), h1 = pack_bf16(v.z, v.w);
         hi[i] = make_uint2(h0, h1);
         lo[i] = make_uint2(pack_bf16(v.x - __uint_as_float(h0 << 16), v.y - __uint_as_float(h0 & 0xffff0000u)),
                            pack_bf16(v.z - __uint_as_float(h1 << 16), v.w - __uint_as_float(h1 & 0xffff0000u)));
-        if (cache != nullptr) {
-            const int h = i * 4 / a.D, d = i * 4 - h * a.D;
-            *reinterpret_cast<float4*>(cache + h * a.stride_h + d) = v;
+        if (a.cache[which] != nullptr) {
+            const int r = i / pieces, e = (i - r * pieces) * 4, h = e / a.D;
+            const int64_t row = row0 + r;
+            *reinterpret_cast<float4*>(a.cache[which] + row / a.N * a.stride_b + row % a.N * a.stride_t + h * a.stride_h + (e - h * a.D)) = v;
         }
     }
 }
@@ -417,18 +422,24 @@ static int launch_prefill_tc_f32(const PrefillParams& p_in, void* scratch, void*
         split.cache[i] = static_cast<float*>(cache[i]);
     }
     split.stride_b = p.stride_b, split.stride_t = p.stride_t, split.stride_h = p.stride_h;
-    split.N = p.N, split.E = E, split.D = kD;
-    constexpr size_t smem = sizeof(tcf::SharedStorage<kD>) + 1024;
+    constexpr int kSplitThreads = 256;
+    split.rows = rows, split.N = p.N, split.E = E, split.D = kD, split.per_cta = std::max(1, kSplitThreads / (E / 4));
+    // CTAs that could all have an SM of their own get one: launched while the halves are still written they take places in pairs, two on
+    // one SM and none on others (head_dim 64, N = 4096, 4 heads: 103.8 us, 93.1 so)
+    constexpr size_t kAlone = 116 * 1024;
+    const size_t smem = std::max(sizeof(tcf::SharedStorage<kD>) + 1024, ctas <= device_sm_count() ? kAlone : size_t{0});
     auto kernel = tcf::prefill_tc_f32_kernel<kD>;
     static bool configured[64] = {false};
     int dev = 0;
     B2KV_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return B2KV_ERR_UNSUPPORTED;
     if (!configured[dev]) {
-        B2KV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        const size_t most = std::max(sizeof(tcf::SharedStorage<kD>) + 1024, kAlone);
+        B2KV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)));
         configured[dev] = true;
     }
-    OverlapLaunch first(dim3(static_cast<unsigned>(rows), 3), std::min(256, (E / 4 + 31) / 32 * 32), 0, stream);
+    OverlapLaunch first(dim3(static_cast<unsigned>((rows + split.per_cta - 1) / split.per_cta), 3), std::min(kSplitThreads, (split.per_cta * (E / 4) + 31) / 32 * 32), 0,
+                        stream);
     B2KV_CUDA_TRY(cudaLaunchKernelEx(&first.cfg, tcf::split_kernel, split));
     OverlapLaunch launch(static_cast<unsigned>(ctas), tcf::kThreads, smem, stream);
     B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, kernel, tm[0], tm[1], tm[2], tm[3], tm[4], tm[5], p));

@@ -90,6 +90,22 @@ def test_prefill_writes_cache_rows_bit_exact_then_decode_continues(pkg, ctx, dty
                                atol=tol["atol"])
 
 
+@pytest.mark.parametrize("B,N,H,D", [(5, 131, 1, 64), (3, 128, 3, 128), (2, 257, 5, 64), (1, 129, 20, 128)])
+@pytest.mark.parametrize("layout", ["bthd", "bhtd"])
+def test_prefill_f32_halves_by_several_rows_per_cta(pkg, ctx, B, N, H, D, layout):
+    """Rows of one to many heads: several per CTA with a remainder, one per CTA, rows of more pieces than threads."""
+    Q, K, V = (U.randn((B, N, H * D), torch.float32, ctx.device, s) for s in (14, 15, 16))
+    cache = pkg.gpu.kv_cache_create(ctx, pkg.gpu.KVCacheConfig(batch_size=B, max_seq_len=N + 3, n_layers=1, n_heads=H, head_dim=D, layout=layout))
+    O, L, M = _run_flash(pkg, ctx, Q, K, V, B, N, H, D, torch.float32, cache=cache)
+    Ow, Lw, Mw = c_oracle.prefill(*(U.to_oracle(t.reshape(B * N, H * D)) for t in (Q, K, V)), B, N, H, D)
+    np.testing.assert_allclose(U.to_f32(O), Ow, rtol=1e-4, atol=3e-5)  # what b2kv.h states for operands of two halves
+    np.testing.assert_allclose(L.cpu().numpy(), Lw, rtol=1e-4, atol=3e-5)
+    np.testing.assert_allclose(M.cpu().numpy(), Mw, rtol=1e-4, atol=3e-5)
+    for which, rows in (("k", K), ("v", V)):
+        view = U.logical_view(cache, cache.layers[0], which)
+        assert torch.equal(view[:, :N].reshape(B, N, H * D), rows) and float(view[:, N:].abs().sum()) == 0.0
+
+
 @pytest.mark.parametrize("B,N,H,with_cache", [(1, 256, 1, False), (2, 512, 3, True), (1, 1280, 2, True), (2, 2048, 2, False)])
 def test_prefill_cta_pair_kernel_vs_oracle_and_one_cta_kernel(pkg, ctx, B, N, H, with_cache):
     """The CTA-pair kernel (opt-in through the "prefill_variant" knob) against the oracle and against
