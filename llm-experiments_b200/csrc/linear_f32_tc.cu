@@ -19,8 +19,12 @@
 //   * a product whose tiles leave SMs idle has its input features cut into ranges, one per CTA of a cluster, whose sums meet in
 //     distributed shared memory, in order.
 //
-// A number that is not finite (or rounds to none in bf16) makes no parts: it sets a flag and the CTA computes its sums again
-// with plain multiply-adds.  Every wait is bounded; after one ran out nothing is stored and the status word is set.
+// What the parts cannot carry is computed again with plain multiply-adds, in order, element by element: sums that are not finite (an
+// operand is not, or rounds to none in bf16, or finite operands' products overflow, where the sign of a partial product says nothing),
+// and rows of x and columns of w with a number whose three parts do not add up to it (some below 2^-109, where the last part
+// is below the smallest number of bf16).  The bits of every other row and column are what they are without it.  One such row among 693,
+// 3072 -> 768: 137 us instead of 39; with a whole tile again, one chain of global loads per thread, it took 9.3 ms.  Every wait is bounded; after one ran out nothing is stored and the
+// status word is set.
 #include <algorithm>
 
 #include "linear.cuh"
@@ -47,6 +51,7 @@ struct Shared {
     alignas(8) uint64_t full[kStages], empty[kStages], sum_full[2], sum_empty[2], done;
     uint32_t tmem_base;
     volatile int odd, abort_flag;
+    uint32_t odd_rows[kBM / 32], odd_cols[kBN / 32];
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -74,20 +79,89 @@ __device__ __forceinline__ int peer_load1(uint32_t addr) {
     return v;
 }
 
-// The three parts of four numbers, to `at` and one and two parts further on.  `check` becomes NaN where a number has no parts.
-__device__ __forceinline__ void split3(const float4& v, uint8_t* at, float2& check) {
+// The three parts of four numbers, to `at` and one and two parts further on.  What two parts leave of a number is the third if its
+// lower 16 bits are zero; they are collected in `check` (those of what is not finite are set: infinity less infinity).
+__device__ __forceinline__ void split3(const float4& v, uint8_t* at, uint32_t& check) {
     const float2 minus = make_float2(-1.f, -1.f);
     float2 r0 = make_float2(v.x, v.y), r1 = make_float2(v.z, v.w);
 #pragma unroll
     for (int part = 0; part < 3; ++part) {
         const uint32_t a = pack_bf16(r0.x, r0.y), b = pack_bf16(r1.x, r1.y);
         *reinterpret_cast<uint2*>(at + part * kPartBytes) = make_uint2(a, b);
-        if (part == 2) break;  // (what is not finite is not a number by now: infinity less infinity)
+        if (part == 2) break;
         r0 = __ffma2_rn(make_float2(__uint_as_float(a << 16), __uint_as_float(a & 0xffff0000u)), minus, r0);
         r1 = __ffma2_rn(make_float2(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u)), minus, r1);
     }
-    const float2 none = make_float2(0.f, 0.f);
-    check = __ffma2_rn(r0, none, __ffma2_rn(r1, none, check));
+    check |= (__float_as_uint(r0.x) | __float_as_uint(r0.y)) | (__float_as_uint(r1.x) | __float_as_uint(r1.y));
+}
+__device__ __forceinline__ bool has_no_parts(float v) {
+    const float r = v - __bfloat162float(__float2bfloat16_rn(v));
+    return (__float_as_uint(r - __bfloat162float(__float2bfloat16_rn(r))) & 0xffffu) != 0 || !(fabsf(v) < INFINITY);
+}
+
+// The sums of the input features [k_first, k_end) that need it, again: all threads, the tile of sums and the stages behind it.
+__device__ __noinline__ void sums_again(const b2kv_linear_args& a, Shared& sm, float* tile, const float* x, const float* w, int row0, int col0,
+                                        int k_first, int k_end) {
+    constexpr int kLdX = kBK + 4;
+    float* const xs = tile + kBM * kLdT;    // [row][input feature]
+    float* const ws = xs + kBM * kLdX;      // [input feature][column]
+    static_assert((kBM * kLdT + kBM * kLdX + kBK * kBN) * 4 <= kStages * kStageBytes, "both operands of a step fit behind the tile");
+    const int tid = threadIdx.x, n_rows = min(kBM, a.rows - row0), n_cols = min(kBN, a.N - col0);
+    if (tid < kBM / 32) sm.odd_rows[tid] = 0;
+    if (tid < kBN / 32) sm.odd_cols[tid] = 0;
+    // element i of a thread: a row of the tile per four i, so that a row is one element of 128 threads, and so is a column
+    auto row_of = [&](int i) { return (tid >> 7) + 4 * i; };
+    auto col_of = [&](int i) { return (tid + 37 * i) & (kBN - 1); };
+    uint32_t again = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+        for (int k0 = k_first; k0 < k_end; k0 += kBK) {
+            const int kn = min(kBK, k_end - k0);
+            __syncthreads();
+            for (int i = tid; i < kBM * (kBK / 4); i += kThreads) {
+                const int r = i / (kBK / 4), k = i % (kBK / 4) * 4;
+                const float4 v = r < n_rows && k < kn ? *reinterpret_cast<const float4*>(x + static_cast<int64_t>(row0 + r) * a.ld_x + k0 + k)
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+                *reinterpret_cast<float4*>(xs + r * kLdX + k) = v;
+                if (pass == 0 && (has_no_parts(v.x) || has_no_parts(v.y) || has_no_parts(v.z) || has_no_parts(v.w)))
+                    atomicOr(&sm.odd_rows[r >> 5], 1u << (r & 31));
+            }
+            for (int i = tid; i < kBK * (kBN / 4); i += kThreads) {
+                const int k = i / (kBN / 4), c = i % (kBN / 4) * 4;
+                const float4 v = k < kn && c < n_cols ? *reinterpret_cast<const float4*>(w + static_cast<int64_t>(k0 + k) * a.ld_w + col0 + c)
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+                *reinterpret_cast<float4*>(ws + k * kBN + c) = v;
+                if (pass == 0) {
+                    const uint32_t odd = (has_no_parts(v.x) ? 1u : 0u) | (has_no_parts(v.y) ? 2u : 0u) | (has_no_parts(v.z) ? 4u : 0u) |
+                                         (has_no_parts(v.w) ? 8u : 0u);
+                    if (odd != 0) atomicOr(&sm.odd_cols[c >> 5], odd << (c & 31));
+                }
+            }
+            __syncthreads();
+            for (uint32_t left = again; left != 0; left &= left - 1) {
+                const int i = __ffs(left) - 1, r = row_of(i), c = col_of(i);
+                float sum = tile[r * kLdT + c];
+#pragma unroll 8
+                for (int k = 0; k < kn; ++k) sum = fmaf(xs[r * kLdX + k], ws[k * kBN + c], sum);
+                tile[r * kLdT + c] = sum;
+            }
+        }
+        __syncthreads();
+        if (pass == 1) break;
+        for (int i = 0; i < kBM * kBN / kThreads; ++i) {
+            const int r = row_of(i), c = col_of(i);
+            float& sum = tile[r * kLdT + c];
+            if (r < n_rows && c < n_cols && ((sm.odd_rows[r >> 5] >> (r & 31) & 1) || (sm.odd_cols[c >> 5] >> (c & 31) & 1) || !(fabsf(sum) < INFINITY)))
+                again |= 1u << i, sum = 0.f;
+        }
+    }
+}
+
+// One sum over all input features, in order: where the ranges' sums are infinities that are no number together.
+__device__ __noinline__ float sum_in_order(const float* row, const float* col, int K, int64_t ld_w) {
+    float sum = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < K; ++k) sum = fmaf(row[k], col[static_cast<int64_t>(k) * ld_w], sum);
+    return sum;
 }
 
 __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid_constant__ b2kv_linear_args a, int splits, int32_t* dev_status) {
@@ -201,14 +275,12 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
         float4 xv[8], wv[8];
         // (whole tiles without a condition per piece: instructions are what the parts cost, 38 us for the first size above with one)
         const bool rows_in = row0 + kBM <= a.rows, cols_in = col0 + kBN <= a.N;
-        const float* const xp = x + static_cast<int64_t>(row0 + xr) * a.ld_x + xc;
-        const float* const wp = w + static_cast<int64_t>(wk) * a.ld_w + col0 + wc;
-        const int64_t x_step = 16 * a.ld_x, w_step = 8 * a.ld_w;
+
         auto read_x = [&](int k0) {
             if (rows_in && k0 + kBK <= k_end) {
-                const float* p = xp + k0;
+                const float* p = x + static_cast<int64_t>(row0 + xr) * a.ld_x + xc + k0;
 #pragma unroll
-                for (int i = 0; i < 8; ++i, p += x_step) xv[i] = *reinterpret_cast<const float4*>(p);
+                for (int i = 0; i < 8; ++i, p += 16 * a.ld_x) xv[i] = *reinterpret_cast<const float4*>(p);
                 return;
             }
 #pragma unroll
@@ -220,9 +292,9 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
         };
         auto read_w = [&](int k0) {
             if (cols_in && k0 + kBK <= k_end) {
-                const float* p = wp + static_cast<int64_t>(k0) * a.ld_w;
+                const float* p = w + static_cast<int64_t>(k0 + wk) * a.ld_w + col0 + wc;
 #pragma unroll
-                for (int i = 0; i < 8; ++i, p += w_step) wv[i] = *reinterpret_cast<const float4*>(p);
+                for (int i = 0; i < 8; ++i, p += 8 * a.ld_w) wv[i] = *reinterpret_cast<const float4*>(p);
                 return;
             }
 #pragma unroll
@@ -232,7 +304,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         };
-        float2 check = make_float2(0.f, 0.f);
+        uint32_t check = 0;
         if (steps > 0) read_x(k_first), read_w(k_first);
         bool ok = true;
         for (int s = 0; s < steps; ++s) {
@@ -257,7 +329,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.full[st]);
         }
-        if (check.x != 0.f || check.y != 0.f) sm.odd = 1;  // (NaN)
+        if (check & 0xffffu) sm.odd = 1;
         if (!ok) sm.abort_flag = 1;
     }
     grid_launch_dependents();
@@ -269,19 +341,14 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
         float* const mine = tile + r * kLdT + c0;
 #pragma unroll
         for (int j = 0; j < 64; j += 4) *reinterpret_cast<float4*>(mine + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-        if (sm.odd) {
-            const float* const row = x + static_cast<int64_t>(min(row0 + r, a.rows - 1)) * a.ld_x;
-            for (int j = 0; j < 64 && col0 + c0 + j < a.N; ++j) {
-                const float* const col = w + col0 + c0 + j;
-                float sum = 0.f;
-                for (int k = k_first; k < k_end; ++k) sum = fmaf(row[k], col[static_cast<int64_t>(k) * a.ld_w], sum);
-                mine[j] = sum;
-            }
-        }
+        float check[4] = {};  // become NaN
+#pragma unroll
+        for (int j = 0; j < 64; ++j) check[j & 3] = fmaf(acc[j], 0.f, check[j & 3]);
+        if ((check[0] + check[1]) + (check[2] + check[3]) != 0.f) sm.odd = 1;
     }
-    __syncwarp();
+    __syncthreads();
+    if (sm.odd) sums_again(a, sm, tile, x, w, row0, col0, k_first, k_end);
     if (splits > 1) cluster_sync();
-    else __syncthreads();
     const int c = (tid & 63) * 2, share = (kBM + splits - 1) / splits;
     bool complete = true;
     for (int s = 0; s < splits; ++s) complete = complete && peer_load1(peer_address(smem_u32(const_cast<int*>(&sm.abort_flag)), s)) == 0;
@@ -289,10 +356,15 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
         lin::finish_rows<float>(a, g, col0 + c, row0, split * share + (tid >> 6), min(min((split + 1) * share, kBM), a.rows - row0), kThreads / 64,
                                 [&](int r) {
                                     float2 v = make_float2(0.f, 0.f);
+                                    bool nan_x = false, nan_y = false;
                                     for (int s = 0; s < splits; ++s) {
                                         const float2 p = peer_load2(peer_address(smem_u32(tile + r * kLdT + c), s));
                                         v.x += p.x, v.y += p.y;
+                                        nan_x = nan_x || p.x != p.x, nan_y = nan_y || p.y != p.y;
                                     }
+                                    const float* const row = x + static_cast<int64_t>(row0 + r) * a.ld_x;
+                                    if (v.x != v.x && !nan_x) v.x = sum_in_order(row, w + col0 + c, a.K, a.ld_w);
+                                    if (v.y != v.y && !nan_y) v.y = sum_in_order(row, w + col0 + c + 1, a.K, a.ld_w);
                                     return v;
                                 });
     __syncwarp();

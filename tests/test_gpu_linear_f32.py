@@ -127,3 +127,64 @@ def test_numbers_that_have_no_parts(pkg, K):
     plain[[3, 140]] = False
     plain[:, [13, 190]] = False
     torch.testing.assert_close(got[0][plain].double(), (x.double() @ w.double())[plain], rtol=1e-4, atol=1e-3)
+
+
+def product(pkg, ctx, x, w, path=0):
+    from llm_experiments_b200 import projection as proj
+
+    out = torch.empty((x.shape[0], w.shape[1]), dtype=F32, device="cuda")
+    run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), x.shape[1], [proj.OutputSegment(w.shape[1], proj.SEG_STORE, wrap(pkg, out))], path=path)
+    return out
+
+
+@pytest.mark.parametrize("splits", [0, 3])
+@pytest.mark.parametrize("odd", [float("nan"), float("inf"), 3.4e38, 1e-37])
+def test_rows_beside_one_that_has_no_parts_keep_their_bits(pkg, odd, splits):
+    """A row of x and a column of w with a number that three bf16 parts do not hold: nothing else in their tile changes, and they are
+    what plain multiply-adds make of them."""
+    from llm_experiments_b200 import _native
+
+    ctx, rows, K, n = make_ctx(pkg), 200, 516, 260
+    x, w = rnd((rows, K), F32, 15), rnd((K, n), F32, 16)
+    _native.tune("matmul_splits", splits)
+    try:
+        plain = product(pkg, ctx, x, w)
+        x[77, K - 3], w[130, 201] = odd, odd
+        got = product(pkg, ctx, x, w)
+    finally:
+        _native.tune("matmul_splits", 0)
+    want = product(pkg, ctx, x, w, path=1)
+    mine = torch.zeros((rows, n), dtype=torch.bool, device="cuda")
+    mine[77], mine[:, 201] = True, True
+    assert torch.equal(got[~mine], plain[~mine])
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()], want[want.isinf()])
+    finite = mine & want.isfinite()
+    size = x.double().abs() @ w.double().abs()
+    assert ((got.double() - want.double()).abs() <= 2 * (K + 1) * 2.0 ** -24 * size)[finite].all()  # (both are off by their sums)
+
+
+@pytest.mark.parametrize("splits", [0, 3])
+@pytest.mark.parametrize("K", [128, 1028])
+def test_finite_operands_whose_products_overflow(pkg, K, splits):
+    """A sum beyond the range is infinite of the sign that the sums in order have, not a difference of infinities of parts or of ranges."""
+    from llm_experiments_b200 import _native
+
+    ctx, rows, n = make_ctx(pkg), 140, 132
+    x, w = rnd((rows, K), F32, 17), rnd((K, n), F32, 18)
+    x[3, 7], w[7, 5], x[9], w[:, 11] = 1e30, -1e30, rnd((K,), F32, 19, 1e20), rnd((K,), F32, 20, 1e19)
+    _native.tune("matmul_splits", splits)
+    try:
+        got = product(pkg, ctx, x, w)
+    finally:
+        _native.tune("matmul_splits", 0)
+    want = product(pkg, ctx, x, w, path=1)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()], want[want.isinf()])
+    assert got[3, 5] == -float("inf") and got.isinf().sum() >= 2
+
+
+@pytest.mark.parametrize("sx,sw", [(1e-33, 1e10), (1e-36, 1e10), (1e15, 1e-38), (1e-41, 1e25), (1e-30, 1e-3), (1e18, 1e18)])
+@pytest.mark.parametrize("rows,K", [(130, 256), (17, 1028)])
+def test_operands_of_any_size(pkg, rows, K, sx, sw):
+    """Down to subnormal numbers, whose parts bf16 does not hold: the bound of fp32 sums."""
+    x, w = rnd((rows, K), F32, 21, sx), rnd((K, 200), F32, 22, sw)
+    bounded(product(pkg, make_ctx(pkg), x, w), x, w)
