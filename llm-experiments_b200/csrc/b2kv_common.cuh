@@ -213,6 +213,43 @@ __device__ __forceinline__ void named_barrier_sync(int id) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kThreads) : "memory");
 }
 
+// ---------------------------------------------------------------------------------------
+// thread-block clusters
+// ---------------------------------------------------------------------------------------
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// The two halves of a cluster barrier; every thread of every CTA of the cluster executes both, in turn.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+    cluster_arrive();
+    cluster_wait();
+}
+// Address of the same shared-memory object (`local`: its address in this CTA's window) in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t peer_address(uint32_t local, uint32_t rank) {
+    uint32_t addr;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local), "r"(rank));
+    return addr;
+}
+__device__ __forceinline__ uint32_t peer_address(const void* local, uint32_t rank) { return peer_address(smem_u32(local), rank); }
+__device__ __forceinline__ void peer_store_u32(uint32_t local, uint32_t rank, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(peer_address(local, rank)), "r"(v) : "memory");
+}
+__device__ __forceinline__ float2 peer_load2(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ int peer_load1(uint32_t addr) {
+    int v;
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+
 // Programmatic dependent launch, device side (no-ops in a kernel launched in plain stream order).
 // wait: returns when every kernel before this one in the stream has completed and its writes are visible.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -323,21 +323,6 @@ struct PairStorage {
     volatile int abort_flag;
 };
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Address of the same shared-memory object in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t map_to_cta(const void* ptr, uint32_t rank) {
-    uint32_t out;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_u32(ptr)), "r"(rank));
-    return out;
-}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -530,7 +515,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     constexpr int kABytesP = Smem::kABytesP, kWSpanP = Smem::kWSpanP;
     Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = static_cast<int>(cluster_ctarank());  // 0 = leader
+    const int r = static_cast<int>(cluster_rank());  // 0 = leader
     const int cid = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
     const int n_k = (p.K + kBKP - 1) / kBKP;
 
@@ -553,7 +538,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     tc_fence_before();
     grid_dependency_wait();  // what comes before hides behind the kernel ahead
     __syncthreads();
-    cluster_sync_all();  // the peer's barriers are initialised before anything is sent to them
+    cluster_sync();  // the peer's barriers are initialised before anything is sent to them
     tc_fence_after();
     const uint32_t tmem = sm.tmem_base;
     const int n_tiles = setup_tiles(p, table, 2 * kBM);  // tiles of 256 rows x tile_cols columns
@@ -571,7 +556,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     ok = mbar_wait(&sm.empty[s], ((it / kStagesP) & 1) ^ 1);
                     if (!ok) break;
                     if (r == 0) mbar_arrive_expect_tx(&sm.full[s], 2 * (kABytesP + spans * kWSpanP));
-                    const uint32_t lead_full = map_to_cta(&sm.full[s], 0);
+                    const uint32_t lead_full = peer_address(&sm.full[s], 0);
 #pragma unroll
                     for (int ks = 0; ks < kBKP / 64; ++ks)  // 64 input features (one swizzle span) per box of A
                         tma_load_2d_pair(sm.stage[s] + ks * (kBM * 128), &tm_a, lead_full, kb * kBKP + ks * 64,
@@ -634,7 +619,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             epilogue_rows(p, tmem + lane_base + buf * kBN, tl.row0 + r * kBM + row, tl.row_end, tl.tn * p.tile_cols, slab_of(table, quarter));
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_cta(&sm.acc_empty[buf], 0));
+            if (lane == 0) mbar_arrive_cluster(peer_address(&sm.acc_empty[buf], 0));
         }
         if (!ok) sm.abort_flag = 1;
     }
@@ -643,7 +628,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     // tensor memory
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();
+    cluster_sync();
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem, kTmemCols);

@@ -21,26 +21,6 @@ namespace linf32 {
 constexpr int kBM = 64, kBN = 128, kStep = 16, kThreads = 128;
 constexpr int kLdX = kBM + 4, kLdT = kBN + 4;
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t peer_address(const void* local, uint32_t rank) {
-    uint32_t addr;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(local)), "r"(rank));
-    return addr;
-}
-__device__ __forceinline__ float2 peer_load2(uint32_t addr) {
-    float2 v;
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
-    return v;
-}
-
 // Rows of a CTA's group, and where its operands start.
 struct Operands {
     const float *x, *w;

@@ -54,31 +54,6 @@ struct Shared {
     uint32_t odd_rows[kBM / 32], odd_cols[kBN / 32];
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t peer_address(uint32_t local, uint32_t rank) {
-    uint32_t addr;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local), "r"(rank));
-    return addr;
-}
-__device__ __forceinline__ float2 peer_load2(uint32_t addr) {
-    float2 v;
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
-    return v;
-}
-__device__ __forceinline__ int peer_load1(uint32_t addr) {
-    int v;
-    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-    return v;
-}
-
 // The three parts of four numbers, to `at` and one and two parts further on.  What two parts leave of a number is the third if its
 // lower 16 bits are zero; they are collected in `check` (those of what is not finite are set: infinity less infinity).
 __device__ __forceinline__ void split3(const float4& v, uint8_t* at, uint32_t& check) {

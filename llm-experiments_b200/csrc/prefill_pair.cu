@@ -85,21 +85,6 @@ struct PairShared {
 
 // ---- cluster / pair forms of the PTX wrappers ---------------------------------------------
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Address of the same shared-memory object in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t map_to_cta(const void* p, uint32_t rank) {
-    uint32_t out;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_u32(p)), "r"(rank));
-    return out;
-}
 // Arrival on a barrier of the peer (or own) CTA.  The data it announces lives in tensor memory and is
 // ordered by tcgen05.wait::st + tcgen05.fence::before_thread_sync, so the arrival itself needs no
 // cluster-wide release of this thread's memory writes (which costs thousands of cycles per step).
@@ -269,7 +254,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     PairShared& sm = *reinterpret_cast<PairShared*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = static_cast<int>(cluster_ctarank());  // 0 = leader
+    const int r = static_cast<int>(cluster_rank());  // 0 = leader
     const int pair_idx = blockIdx.x >> 1;
     const int n_pb = p.N / (2 * kRows);
     // Launch order as in the one-CTA kernel: groups of `group` (sequence, head) pairs, inside a group the heaviest
@@ -315,7 +300,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     }
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();  // the peer's barriers are initialised before anything is sent to them
+    cluster_sync();  // the peer's barriers are initialised before anything is sent to them
     tc_fence_after();
     const uint32_t tmem = sm.tmem_base;
 
@@ -323,7 +308,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         // ------------------------------ TMA producer (both CTAs) ------------------------------
         if (lane == 0) {
             const int x0 = h * kD;
-            const uint32_t lead_q = map_to_cta(&sm.q_full, 0);
+            const uint32_t lead_q = peer_address(&sm.q_full, 0);
             if (r == 0) mbar_arrive_expect_tx(&sm.q_full, 2 * kQBytes);
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) tma_load_3d_pair(sm.q + hf * kQHalf, &tm_q, lead_q, x0 + hf * 64, q0 + r * kRows, b);
@@ -336,7 +321,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                     ok = mbar_wait_pair(&sm.k_empty[st], ((jj / kStages) & 1) ^ 1);
                     if (!ok) break;
                     if (r == 0) mbar_arrive_expect_tx(&sm.k_full[st], 2 * kKBytes);
-                    const uint32_t lead_k = map_to_cta(&sm.k_full[st], 0);
+                    const uint32_t lead_k = peer_address(&sm.k_full[st], 0);
 #pragma unroll
                     for (int hf = 0; hf < 2; ++hf)
                         tma_load_3d_pair(sm.k[st] + hf * kKHalf, &tm_k, lead_k, x0 + hf * 64, jj * kKeys + r * 64, b);
@@ -347,7 +332,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                     ok = mbar_wait_pair(&sm.v_empty[st], ((jv / kStages) & 1) ^ 1);
                     if (!ok) break;
                     if (r == 0) mbar_arrive_expect_tx(&sm.v_full[st], 2 * kVBytes);
-                    tma_load_3d_pair(sm.v[st], &tm_v, map_to_cta(&sm.v_full[st], 0), x0 + r * 64, jv * kKeys, b);
+                    tma_load_3d_pair(sm.v[st], &tm_v, peer_address(&sm.v_full[st], 0), x0 + r * 64, jv * kKeys, b);
                 }
             }
             // The pair's own K / V rows are the last two steps; they are still in the rings.  Once the
@@ -438,8 +423,8 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const uint32_t s_tmem = tmem + lane_base + kColS0 + g * 128;
         const uint32_t o_tmem = tmem + lane_base + kColOut;
         const uint32_t p_tmem = tmem + lane_base + kColP0 + g * 64;
-        const uint32_t lead_p = map_to_cta(&sm.p_ready[g], 0);
-        const uint32_t lead_free = map_to_cta(&sm.s_free[g], 0);
+        const uint32_t lead_p = peer_address(&sm.p_ready[g], 0);
+        const uint32_t lead_free = peer_address(&sm.s_free[g], 0);
         const float c = p.q_prescale;  // log2(e) / sqrt(D)
         // m_seen: the reference maximum this group's partial sum l is relative to;
         // m_true: the true maximum over this group's steps (for the M output).
@@ -552,7 +537,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     // the tensor memory of the pair
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();
+    cluster_sync();
     if (warp == 9) {
         tc_fence_after();
         tmem_dealloc_pair(tmem, kPairTmemCols);

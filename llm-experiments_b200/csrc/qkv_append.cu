@@ -95,21 +95,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
         : "memory");
 }
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// The two halves of a cluster barrier; every thread of every CTA of the cluster executes both, in turn.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// Stores a 32-bit word at shared-memory address `local` (an address of this CTA's window) of CTA `rank`.
-__device__ __forceinline__ void peer_store_u32(uint32_t local, uint32_t rank, uint32_t v) {
-    uint32_t addr;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local), "r"(rank));
-    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-
 constexpr int ring_stages(int Bn, int ring_bytes) {
     const int fit = ring_bytes / (kWBytes + 2 * Bn * 128);
     return fit < 2 ? 2 : (fit > kMaxStagesP ? kMaxStagesP : fit);
