@@ -120,6 +120,9 @@ class OutputSegment:
     group: int = 0
 
 
+_AHEAD = ctypes.byref(_native.LinearOptions(flags=_native.LINEAR_AHEAD))
+
+
 @reference_op("linear")
 def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Sequence[OutputSegment],
            residual: Optional[GPUBuffer2D] = None, limit: float = 0.0, groups: int = 1, group_x: int = 0, group_w: int = 0,
@@ -166,11 +169,9 @@ def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Se
         a.bias = bias.buffer.data_ptr()
     if group_rows is not None:
         a.group_rows = group_rows.data_ptr()
-    options = None
-    if group_x_rows is not None or ahead:
-        options = _native.LinearOptions(flags=_native.LINEAR_AHEAD if ahead else 0)
-        if group_x_rows is not None:
-            options.group_x_rows, options.x_rows = group_x_rows.data_ptr(), x.shape[0]
-        options = ctypes.byref(options)
+    options = _AHEAD if ahead else None
+    if group_x_rows is not None:
+        options = ctypes.byref(_native.LinearOptions(group_x_rows=group_x_rows.data_ptr(), x_rows=x.shape[0],
+                                                     flags=_native.LINEAR_AHEAD if ahead else 0))
     stream = batch_op_begin(ctx)
     _native.check(_native.lib.b2kv_linear_opt(ctypes.byref(a), options, dev_status_ptr(ctx), stream))
