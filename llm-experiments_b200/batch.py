@@ -32,7 +32,7 @@ def validate_buffer_shape_2d(buffer: GPUBuffer2D, expected_shape: Tuple[int, int
         raise ValueError(f"{name} shape mismatch: got {buffer.shape}, expected {expected_shape}")
 
 
-def _current_handle(device: torch.device) -> int:
+def current_handle(device: torch.device) -> int:
     """The raw handle of torch's current stream.  (A stream object for it costs 2 us, three times per step of a decoding loop
     whose kernels take less than ten.)"""
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
@@ -44,7 +44,7 @@ def batch_begin(ctx: GPUContext, enable_profiling: bool = False) -> None:
     reference function and bracketed by CUDA events; ``batch_commit`` then synchronises and adds
     the durations to ``ctx.perf_monitor`` (the reference stores the flag, gpu_ops.py:245-250, and
     leaves the recording to the caller, gpu_device.py:569-608)."""
-    stream, handle = ctx.stream, _current_handle(ctx.device)
+    stream, handle = ctx.stream, current_handle(ctx.device)
     if stream is None or stream.cuda_stream != handle:
         stream = ctx.stream = torch.cuda.current_stream(ctx.device)
     ctx.batch_state = BatchState(encoder=stream, retained_buffers=[], enable_profiling=enable_profiling,
@@ -61,7 +61,7 @@ def batch_op_begin(ctx: GPUContext) -> int:
         raise RuntimeError(f"Batch operation limit ({max_ops}) exceeded. Call batch_commit() to flush operations.")
     # The kernels go to the batch's stream; the few torch operations beside them (length counters) go to
     # torch's current stream.  They are ordered only when the two are the same stream.
-    if _current_handle(ctx.device) != state.stream_handle:
+    if current_handle(ctx.device) != state.stream_handle:
         raise RuntimeError("The current CUDA stream changed since batch_begin; commit the batch and begin a new one "
                            "on the new stream")
     state.operation_count += 1

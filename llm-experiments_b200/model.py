@@ -244,6 +244,8 @@ class GraphedDecodeStep:
         ctx, state = self.ctx, self.state
         if ctx.config.check_device_status:
             raise ValueError("check_device_status synchronises in batch_commit, which a graph capture cannot hold")
+        if hasattr(state, "wait_for_lengths"):
+            state.wait_for_lengths()
         caches = state.caches
         cap = caches[0].max_seq_len
         keep_len = [c.current_len for c in caches]
@@ -286,6 +288,8 @@ class GraphedDecodeStep:
         caches = self.state.caches
         if caches[0].current_len >= caches[0].max_seq_len:
             raise ValueError(f"Cache is full: current_len={caches[0].current_len}, max_seq_len={caches[0].max_seq_len}")
+        if hasattr(self.state, "wait_for_lengths"):
+            self.state.wait_for_lengths()
         self.graph.replay()
         if hasattr(self.state, "advance_host"):
             self.state.advance_host()

@@ -17,7 +17,7 @@ import torch
 
 from ._native import check as _check
 from ._native import lib as _lib
-from .batch import batch_begin, batch_commit, batch_op_begin
+from .batch import batch_begin, batch_commit, batch_op_begin, current_handle
 from .latent import PromptPlan, RowPlaces
 from .step_tail import argmax
 from .types import GPUBuffer1D, GPUBuffer2D, GPUContext, KVCache
@@ -95,6 +95,9 @@ class SequenceState:
 
     def __post_init__(self):
         # a model without any attention still has lengths and a capacity
+        self._lengths_event = None  # behind the last copy of lengths to the device, and the raw handle of its stream (None: it has ended)
+        self._lengths_stream = None
+        self.captured = False     # a graph holds one of the steps: they are replayed without a call of this module
         self._bare = None if self.owned else KVCache(layers=[], batch_size=self.batch_size, max_seq_len=self.max_seq_len,
                                                      current_len=0, n_heads=0, head_dim=0, seq_lens=self.seq_lens)
 
@@ -126,17 +129,36 @@ class SequenceState:
         self.lengths = [v + n for v in self.lengths]
         self._sync_upper_bound()
 
+    def wait_for_lengths(self) -> None:
+        """The current stream's work from here on sees the lengths of the last ``state_set_lengths``, also one on another stream."""
+        if self._lengths_stream is None or current_handle(self.seq_lens.device) == self._lengths_stream:
+            return
+        if not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream(self.seq_lens.device).wait_event(self._lengths_event)
+
     def _sync_upper_bound(self) -> None:
         for c in self.caches:
             c.current_len = max(self.lengths)
 
 
 def state_set_lengths(state: SequenceState, lens: Sequence[int]) -> None:
+    """Every sequence's length.  Takes effect in the order of torch's current stream, and steps on other streams (``decode_step``,
+    ``forward``, ``GraphedDecodeStep``) wait for it, the host does not: that would wait for every step still running.  It does where
+    a step is held by a graph, which may be replayed on any stream without a call of this module."""
     if len(lens) != state.batch_size or min(lens) < 0 or max(lens) > state.max_seq_len:
         raise ValueError(f"lengths must be {state.batch_size} values in [0, {state.max_seq_len}]")
     state.lengths = [int(v) for v in lens]
-    # in stream order, like the steps themselves: waiting for it here would wait for every step still running
-    state.seq_lens.copy_(torch.tensor(state.lengths, dtype=torch.int32), non_blocking=True)
+    host, device = torch.tensor(state.lengths, dtype=torch.int32), state.seq_lens.device
+    if device.type != "cuda" or state.captured or torch.cuda.is_current_stream_capturing():
+        state.seq_lens.copy_(host)  # (inside a capture that is an error)
+        state._lengths_stream = None
+    else:
+        state.wait_for_lengths()
+        state.seq_lens.copy_(host, non_blocking=True)
+        if state._lengths_event is None:
+            state._lengths_event = torch.cuda.Event()
+        state._lengths_event.record(torch.cuda.current_stream(device))
+        state._lengths_stream = current_handle(device)
     state._sync_upper_bound()
 
 
@@ -159,6 +181,8 @@ def decode_step(ctx: GPUContext, state: SequenceState, token_ids: GPUBuffer1D, n
     if upper >= state.max_seq_len:
         raise ValueError(f"Cache is full: current_len={upper}, max_seq_len={state.max_seq_len}")
     B = state.batch_size
+    state.captured = state.captured or (state.seq_lens.is_cuda and torch.cuda.is_current_stream_capturing())
+    state.wait_for_lengths()
     state.run(ctx, Step(ids=token_ids.buffer, places=RowPlaces(None, state.seq_lens), rows=B, n_single=B, n_few=B, span=upper + 1, plans={},
                         short=RowSegments(None, B, 1), long=None, row_index=None, n_out=B))
     if next_ids is not None:
@@ -217,6 +241,7 @@ def forward(ctx: GPUContext, state: SequenceState, entries: Sequence[Tuple[int, 
     segments = [RowSegments(table, len(r), max(n for _, n, _ in r)) if r else None
                 for table, r in ((pieces[5], runs[True]), (pieces[6], runs[False]))]
     batch_begin(ctx)
+    state.wait_for_lengths()
     state.run(ctx, Step(ids=pieces[0], places=RowPlaces(pieces[1], pieces[2]), rows=T, n_single=n_single, n_few=n_few, span=span, plans=plans,
                         short=segments[0], long=segments[1], row_index=pieces[3], n_out=n_out))
     batch_commit(ctx)

@@ -196,6 +196,61 @@ def test_long_decoding_with_the_graphed_step(pkg, name):
         U.check_rows(torch.cat(out[s]), oracle(name, seq)[-150:], BF, s)
 
 
+@pytest.mark.parametrize("how", ["eager", "forward", "graph", "captured_behind"])
+def test_lengths_set_on_one_stream_and_a_step_on_another(pkg, how):
+    """The stream that sets them is busy for a while; steps on another stream see them all the same, whatever form they have."""
+    from llm_experiments_b200 import serving
+    from llm_experiments_b200.model import GraphedDecodeStep
+
+    model, cfg = build(pkg, "TC", BF, batch=2, max_tokens=64)
+    ctx, state = model.ctx, model.state
+    ctx.config.check_device_status = False
+    model.forward([(0, U.tokens(cfg, 20, 50), []), (1, U.tokens(cfg, 24, 51), [])])
+    token = U.tokens(cfg, 1, 52)[0]
+    ids = serving.buffer1(torch.full((2,), token, dtype=torch.int32, device="cuda"))
+    kept = {i: t.clone() for i, t in state.recurrent.items()}
+    lens = ([20, 24], [7, 12], [3, 18], [0, 5])
+
+    def step(how):
+        for i, t in state.recurrent.items():
+            t.copy_(kept[i])
+        if how == "forward":
+            return model.forward([(0, [token], [0]), (1, [token], [0])]).clone()
+        if how == "eager":
+            pkg.gpu.batch_begin(ctx)
+            serving.decode_step(ctx, state, ids)
+            pkg.gpu.batch_commit(ctx)
+        else:
+            graphed.step()
+        return state.logits.buffer.clone()
+
+    def make_graph():
+        graphed = GraphedDecodeStep(ctx, state, step_fn=serving.decode_step)
+        graphed.token_ids.buffer.copy_(ids.buffer)
+        return graphed
+
+    if how == "graph":
+        graphed = make_graph()
+        graphed.capture()  # (it runs a step, which writes rows as well)
+    plain, want = "forward" if how == "forward" else "eager", []
+    for again in range(6):  # (a step writes the rows at its lengths, which longer sequences read: once more for each of them, they stay)
+        for n in lens:
+            serving.state_set_lengths(state, n)
+            want.append(step(plain))
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    for n, expected in zip(lens, want[-len(lens):]):
+        torch.cuda.synchronize()
+        with torch.cuda.stream(a):
+            torch.cuda._sleep(20_000_000)
+            serving.state_set_lengths(state, n)
+        with torch.cuda.stream(b):
+            if how == "captured_behind":
+                graphed = make_graph()
+            got = step("graph" if how == "captured_behind" else how)
+        torch.cuda.synchronize()
+        assert torch.equal(got, expected) and state.seq_lens.tolist() == [v + 1 for v in n] == state.lengths
+
+
 @pytest.mark.parametrize("name", ["ODD", "TC", "ONLY_GLA"])
 def test_greedy_generation_matches_the_oracle(pkg, name):
     """generate_text over the registry's model, fp32: the oracle's greedy tokens."""
