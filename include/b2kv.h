@@ -410,7 +410,7 @@ int b2kv_layernorm_rows(const float* y, int64_t ld_y, const int32_t* row_index, 
  * pitches, offsets and boundaries allow it (multiples of 8 elements; boundaries multiples of 32): at most 128 rows per
  * group stream the weights once, more go to the tiled kernel.  fp32 products of more than 16 rows and at least 128 input
  * features, not grouped by rows and made of 16-byte pieces, run there as well, their operands in three bf16 parts; everything
- * else runs on CUDA-core kernels.
+ * else runs on CUDA-core kernels.  So the order of a row's sums, not their error, follows from the number of rows.
  * A bf16 product of one segment with at most 32 input features runs on a CUDA-core kernel of its own.
  * path: 0 = choose, 1 = CUDA cores, 2 = weight streaming, 3 = tiled, 4 = few input features (refused when the shape is not one
  * it takes).

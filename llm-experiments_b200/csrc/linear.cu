@@ -1,5 +1,5 @@
-// b2kv_linear: argument checks, the choice of the kernel, the CUDA-core kernel for shapes and alignments that the others do not take, and the one for few input features (64 x 64 output tiles, 16 input features per step, 4 x 4 outputs per thread, fp32
-// accumulation).
+// b2kv_linear: argument checks, the choice of the kernel, and two CUDA-core kernels: one for shapes and alignments that no other kernel
+// takes (64 x 64 output tiles, 16 input features per step, 4 x 4 outputs per thread, fp32 accumulation) and one for few input features.
 #include "linear.cuh"
 
 namespace b2kv {
