@@ -4,6 +4,8 @@
 // const __restrict__: the compiler would take it for data that nothing writes and could load it before the wait.
 #include <math.h>
 
+#include <algorithm>
+
 #include "b2kv_common.cuh"
 
 namespace b2kv {
@@ -93,7 +95,7 @@ route_kernel(const float* logits, int64_t ld, int rows, int experts, int groups,
     }
 }
 
-// A CTA per row: the places of its choices among the sorted rows, and the copies of the row there (128-bit when aligned).  The row is
+// A CTA per row, or per `per` of its choices: their places among the sorted rows, and the copies of the row there (128-bit when aligned).  The row is
 // read once and its first pieces stay in registers; what bounds it is the copies' bytes (a CTA per choice, with the whole chain of
 // loads before its first copy, took 38 us for 2975 rows of 4 KB and six choices, this one 25).
 constexpr int kPlanThreads = 128;
@@ -102,9 +104,10 @@ template <bool kTable>  // the experts' first rows fit shared memory
 __global__ void __launch_bounds__(kPlanThreads)
 moe_plan_kernel(const int32_t* idx, int32_t* counts, int experts, int top, int32_t* offsets,
                 int32_t* slot, const uint8_t* h, int64_t pitch_h, uint8_t* sorted,
-                int64_t pitch_sorted, int row_bytes, bool vec) {
+                int64_t pitch_sorted, int row_bytes, bool vec, int per) {
     extern __shared__ int sm_plan[];  // [experts + 1]: row behind the last one of the experts before; then the places of the row's choices
-    const int row = blockIdx.x, lane = threadIdx.x & 31;
+    const int row = blockIdx.x, lane = threadIdx.x & 31, k_first = blockIdx.y * per, k_end = min(top, k_first + per);
+    const bool writes = row == 0 && k_first == 0;  // the offsets
     int* const first = kTable ? sm_plan : offsets;  // (without a table one CTA writes them where they belong)
     int* const place = kTable ? sm_plan + experts + 1 : slot + static_cast<int64_t>(row) * top;
     constexpr int kKeep = 4;
@@ -120,7 +123,7 @@ moe_plan_kernel(const int32_t* idx, int32_t* counts, int experts, int top, int32
     }
     if (threadIdx.x < 32) {
         int base = 0;
-        for (int e0 = 0; e0 < experts && (kTable || row == 0); e0 += 32) {
+        for (int e0 = 0; e0 < experts && (kTable || writes); e0 += 32) {
             const int n = e0 + lane < experts ? counts[e0 + lane] : 0;
             int end = n;
 #pragma unroll
@@ -131,9 +134,9 @@ moe_plan_kernel(const int32_t* idx, int32_t* counts, int experts, int top, int32
             if (e0 + lane < experts) first[e0 + lane] = base + end - n;
             base += __shfl_sync(0xffffffffu, end, 31);
         }
-        if (lane == 0 && (kTable || row == 0)) first[experts] = base;
+        if (lane == 0 && (kTable || writes)) first[experts] = base;
         __syncwarp();
-        for (int k = 0; k < top && !kTable; ++k) {
+        for (int k = k_first; k < k_end && !kTable; ++k) {
             const int e = idx[static_cast<int64_t>(row) * top + k];
             int before = 0;
             for (int i = lane; i < e; i += 32) before += counts[i];
@@ -141,22 +144,22 @@ moe_plan_kernel(const int32_t* idx, int32_t* counts, int experts, int top, int32
             for (int off = 16; off > 0; off >>= 1) before += __shfl_xor_sync(0xffffffffu, before, off);
             if (lane == 0) place[k] = before + atomicAdd(&counts[experts + e], 1);
         }
-        for (int k = lane; k < top && kTable; k += 32) {
+        for (int k = k_first + lane; k < k_end && kTable; k += 32) {
             const int e = idx[static_cast<int64_t>(row) * top + k];
             place[k] = first[e] + atomicAdd(&counts[experts + e], 1);
             slot[static_cast<int64_t>(row) * top + k] = place[k];
         }
     }
     __syncthreads();
-    if (row == 0 && kTable)
+    if (writes && kTable)
         for (int i = threadIdx.x; i <= experts; i += kPlanThreads) offsets[i] = first[i];
     if (!vec) {
-        for (int k = 0; k < top; ++k)
+        for (int k = k_first; k < k_end; ++k)
             for (int i = threadIdx.x; i < row_bytes / 2; i += kPlanThreads)
                 reinterpret_cast<uint16_t*>(sorted + place[k] * pitch_sorted)[i] = reinterpret_cast<const uint16_t*>(src)[i];
         return;
     }
-    for (int k = 0; k < top; ++k) {
+    for (int k = k_first; k < k_end; ++k) {
         uint4* const dst = reinterpret_cast<uint4*>(sorted + place[k] * pitch_sorted);
 #pragma unroll
         for (int u = 0; u < kKeep; ++u) {
@@ -251,10 +254,18 @@ extern "C" int b2kv_moe_plan(const int32_t* idx, int32_t* counts, int rows, int 
     const bool vec = (dim * es) % 16 == 0 && (ld_h * es) % 16 == 0 && (ld_sorted * es) % 16 == 0 && aligned16(h) && aligned16(sorted);
     const size_t bytes = (static_cast<size_t>(experts) + 1 + top) * sizeof(int);
     const bool table = bytes <= 48 * 1024;
-    OverlapLaunch launch(rows, kPlanThreads, table ? bytes : 0, stream);
+    // Few rows: several CTAs for the choices of one, up to three per SM and of at least 32 KB of copies (by 16 bits they count eight times): one
+    // after the other in one CTA they take longer than the row read again (8 rows of 32 KB, 64 choices: 84 us with a CTA per row, 34 so; with 300 rows of
+    // 2 KB two CTAs per row take longer than one, 54 us and 45).
+    const long long copied = static_cast<long long>(dim) * es * (vec ? 1 : 8) * top;
+    const long long wanted = std::max<long long>(1, std::min<long long>(3LL * device_sm_count() / rows, copied / (32 * 1024)));
+    const int most = static_cast<int>(std::min<long long>(wanted, top)), per = (top + most - 1) / most;
+    const long long parts = (top + per - 1) / per;
+    if (parts > 65535) return B2KV_ERR_UNSUPPORTED;
+    OverlapLaunch launch(dim3(rows, static_cast<unsigned>(parts)), kPlanThreads, table ? bytes : 0, stream);
     B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, table ? moe_plan_kernel<true> : moe_plan_kernel<false>, idx, counts, experts, top, offsets, slot,
                                      static_cast<const uint8_t*>(h), ld_h * es, static_cast<uint8_t*>(sorted), ld_sorted * es,
-                                     dim * es, vec));
+                                     dim * es, vec, per));
     return B2KV_OK;
 }
 

@@ -217,16 +217,18 @@ def test_folder_trace_runner_and_command_line(pkg, tmp_path):
     assert res.stdout.split() == [",".join(map(str, generate.generate_text(model, [3, 5, 8], 4, temperature=0.0)))]
 
 
-@pytest.mark.parametrize("experts,width", [(13, 24), (1024, 2056), (13000, 24), (13000, 9)])
-def test_rows_sorted_by_any_number_of_experts(pkg, experts, width):
-    """Also by more than a table in shared memory holds: the places of an expert's rows begin where the expert before ends."""
+@pytest.mark.parametrize("rows,experts,width", [(37, 13, 24), (37, 1024, 2056), (37, 13000, 24), (37, 13000, 9), (3, 16, 8200), (5, 13000, 16384),
+                                                (1300, 16, 40)])
+def test_rows_sorted_by_any_number_of_experts(pkg, rows, experts, width):
+    """Also by more than a table in shared memory holds, by one CTA per row or several: the places of an expert's rows begin where the
+    expert before ends."""
     from llm_experiments_b200 import moe
     from llm_experiments_b200.serving import buffer2
 
-    ctx, rows, top = make_ctx(pkg), 37, 5
+    ctx, top = make_ctx(pkg), 5
     gen = torch.Generator(device="cuda").manual_seed(experts)
     idx = torch.stack([torch.randperm(experts, generator=gen, device="cuda")[:top] for _ in range(rows)]).to(torch.int32)
-    idx[3, 0], idx[4, 1] = experts - 1, 0
+    idx[1, 0], idx[2, 1] = experts - 1, 0
     h = torch.randn((rows, width), generator=gen, device="cuda").to(BF)
     count = torch.bincount(idx.flatten().long(), minlength=experts).to(torch.int32)
     i32 = lambda *shape: torch.full(shape, -1, dtype=torch.int32, device="cuda")  # noqa: E731
