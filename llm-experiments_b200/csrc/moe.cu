@@ -170,7 +170,7 @@ moe_plan_kernel(const int32_t* idx, int32_t* counts, int experts, int top, int32
     }
 }
 
-template <typename T>
+template <typename T, int kAhead>  // kAhead: choices whose pieces are on their way together, with the row's own (1: as few registers as it goes)
 __global__ void __launch_bounds__(256) moe_combine_kernel(float* x, int64_t ld_x, const T* y,
                                                           int64_t ld_y, const int32_t* slot,
                                                           const float* score, int top, int dim, bool vec) {
@@ -189,8 +189,22 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(float* x, int64_t ld_x
     if (vec) {
         constexpr int kC = Elt<T>::kPerChunk;
         for (int i = threadIdx.x; i < dim / kC; i += blockDim.x) {
-            constexpr int kAhead = 6;  // choices whose pieces are on their way together, with the row's own
             float acc[kC] = {};
+            if constexpr (kAhead == 1) {
+                for (int k = 0; k < top; ++k) {
+                    float v[kC];
+                    Elt<T>::widen(reinterpret_cast<const uint4*>(y + sl[k] * ld_y)[i], v);
+#pragma unroll
+                    for (int j = 0; j < kC; ++j) acc[j] = fmaf(sc[k], v[j], acc[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < kC / 4; ++j) {
+                    float4* const p = reinterpret_cast<float4*>(xr + i * kC) + j;
+                    const float4 o = *p;
+                    *p = make_float4(o.x + acc[4 * j], o.y + acc[4 * j + 1], o.z + acc[4 * j + 2], o.w + acc[4 * j + 3]);
+                }
+                continue;
+            }
             float4 o[kC / 4];
 #pragma unroll
             for (int j = 0; j < kC / 4; ++j) o[j] = reinterpret_cast<const float4*>(xr + i * kC)[j];
@@ -276,12 +290,16 @@ extern "C" int b2kv_moe_combine(float* x, int64_t ld_x, const void* y, int64_t l
     if (!x || !y || !slot || !score || rows <= 0 || top <= 0 || dim <= 0 || ld_x < dim || ld_y < dim) return B2KV_ERR_BAD_ARG;
     if (top > kMaxTop) return B2KV_ERR_UNSUPPORTED;
     const bool vec = (dim * es) % 16 == 0 && (ld_y * es) % 16 == 0 && ld_x % 4 == 0 && dim % 4 == 0 && aligned16(x) && aligned16(y);
+    // Pieces on their way together pay unless registers then keep rows off the SM: two choices, rows by 16 bits, and many rows narrower
+    // than a CTA (3000 rows, two choices: 4096 columns 24.0 us with six, 19.4 one by one; six choices: 41.1 and 42.8, 1024 columns 8.8 and 8.2;
+    // 64 rows of 4096: 3.5 and 4.3).
+    const bool ahead = vec && top > 2 && (top > 6 || dim * es / 16 >= 256 || rows <= 1024);
     OverlapLaunch launch(rows, 256, 0, stream);
     if (dtype == B2KV_DTYPE_F32)
-        B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, moe_combine_kernel<float>, x, ld_x, static_cast<const float*>(y), ld_y, slot,
-                                         score, top, dim, vec));
+        B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, ahead ? moe_combine_kernel<float, 6> : moe_combine_kernel<float, 1>, x, ld_x,
+                                         static_cast<const float*>(y), ld_y, slot, score, top, dim, vec));
     else
-        B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, moe_combine_kernel<__nv_bfloat16>, x, ld_x,
+        B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, ahead ? moe_combine_kernel<__nv_bfloat16, 6> : moe_combine_kernel<__nv_bfloat16, 1>, x, ld_x,
                                          static_cast<const __nv_bfloat16*>(y), ld_y, slot, score, top, dim, vec));
     return B2KV_OK;
 }

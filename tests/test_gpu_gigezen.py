@@ -243,3 +243,23 @@ def test_rows_sorted_by_any_number_of_experts(pkg, rows, experts, width):
     e = idx.long()
     assert ((s.slot >= ends[e]) & (s.slot < ends[e + 1])).all()
     assert torch.equal(s.sorted_h.buffer[s.slot.long()], h[:, None].expand(rows, top, width)) and (s.sorted_h.buffer[-1] == 7).all()
+
+
+@pytest.mark.parametrize("rows,top,width", [(3, 1, 1024), (3, 2, 2056), (9, 6, 520), (1100, 6, 64), (1100, 7, 64), (5, 13, 2048), (5, 3, 33)])
+@pytest.mark.parametrize("dtype", [F32, BF])
+def test_weighted_sums_of_the_experts_rows(pkg, rows, top, width, dtype):
+    """Both forms of the sum, by 16-byte pieces and by elements, with a remainder of choices."""
+    from llm_experiments_b200 import moe
+    from llm_experiments_b200.serving import buffer2
+
+    ctx = make_ctx(pkg)
+    gen = torch.Generator(device="cuda").manual_seed(rows * top)
+    x, y = torch.randn((rows, width), generator=gen, device="cuda"), torch.randn((rows * top, width), generator=gen, device="cuda").to(dtype)
+    score, slot = torch.rand((rows, top), generator=gen, device="cuda"), torch.randperm(rows * top, generator=gen, device="cuda").to(torch.int32).view(rows, top)
+    want = x.double() + (score.double()[:, :, None] * y.double()[slot.long()]).sum(dim=1)
+    s = moe.MoeScratch(idx=None, score=score, slot=slot, counts=None, offsets=None, sorted_h=None, m=None, y=buffer2(y))
+    pkg.gpu.batch_begin(ctx)
+    moe.combine(ctx, buffer2(x), moe.RouterShape(experts=64, top=top), s)
+    pkg.gpu.batch_commit(ctx)
+    size = want.abs() + (score.double()[:, :, None] * y.double()[slot.long()].abs()).sum(dim=1)
+    assert ((x.double() - want).abs() <= (top + 1) * 2.0 ** -24 * size).all()
