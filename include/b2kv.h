@@ -525,8 +525,9 @@ int b2kv_gqa_append(void* y, int64_t ld_y, int H, int G, int dim, int vdim, cons
  * slopes (fp32 [H], NULL: no bias).  span is an upper bound of the tokens a row sees; the rows' own tokens are in the cache
  * already.  bf16 with dim and vdim multiples of 8 up to 128 runs on the tensor cores (the window of a row is cut into shares whose
  * partial results go to a workspace of b2kv_gqa_decode_workspace_bytes bytes), everything else on CUDA cores (dim and vdim
- * up to 512).  path: 0 = choose, 1 = CUDA cores, 2 = tensor cores.  b2kv_gqa_decode_runs is the same for rows that come in
- * runs of neighbouring rows of one sequence (prompt portions): in fp32, with path 0, sixteen rows read their keys and values together.
+ * up to 512).  path: 0 = choose, 1 = CUDA cores, 2 = tensor cores.  b2kv_gqa_decode_runs is the same where the rows behind
+ * the first `singles` come in runs of neighbouring rows of one sequence (prompt portions): in fp32, with path 0 and row_slot, sixteen
+ * of those read their keys and values together where there are enough of them.
  */
 size_t b2kv_gqa_decode_workspace_bytes(int rows, int H, int G, int vdim, int span, int dtype);
 int b2kv_gqa_decode(const void* q, int64_t ld_q, const void* k_cache, const void* v_cache, void* out, int64_t ld_out,
@@ -535,7 +536,7 @@ int b2kv_gqa_decode(const void* q, int64_t ld_q, const void* k_cache, const void
                     size_t workspace_bytes, int32_t* dev_status, void* stream);
 int b2kv_gqa_decode_runs(const void* q, int64_t ld_q, const void* k_cache, const void* v_cache, void* out, int64_t ld_out,
                          const float* slopes, const int32_t* row_slot, const int32_t* row_pos, int n_slots, int T_max, int rows, int H,
-                         int G, int dim, int vdim, int span, float scale, int dtype, int path, void* workspace,
+                         int G, int dim, int vdim, int span, float scale, int dtype, int path, int singles, void* workspace,
                          size_t workspace_bytes, int32_t* dev_status, void* stream);
 
 /*

@@ -131,7 +131,7 @@ SIGNATURES = {
     "b2kv_gqa_decode_workspace_bytes": (_sz, [_i, _i, _i, _i, _i, _i]),
     "b2kv_gqa_decode": (_i, [_vp, _i64, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp, _sz,
                              _vp, _vp]),
-    "b2kv_gqa_decode_runs": (_i, [_vp, _i64, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp, _sz,
+    "b2kv_gqa_decode_runs": (_i, [_vp, _i64, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _i, _vp, _sz,
                              _vp, _vp]),
     "b2kv_gqa_prefill_supported": (_i, [_i, _i, _i]),
     "b2kv_gqa_prefill": (_i, [_vp, _i64, _vp, _vp, _i64, _vp, _i64, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp, _vp]),

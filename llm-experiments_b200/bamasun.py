@@ -316,11 +316,9 @@ def _attend(ctx, state: BamasunState, i: int, xs: GPUBuffer2D, step: Step) -> GP
     out = state.rows(f"mixed{w.w_o.shape[0]}", T, w.w_o.shape[0], state.dtype)
     linear(ctx, xs, w.w_in, width, [OutputSegment(y.shape[1], SEG_STORE, y)], bias=w.bias, ahead=True)
     gqa.gqa_append(ctx, y, a, step.places, cache, lc.kv_from is None, w.q_norm, w.k_norm, state.cfg.eps)
-    # (in fp32 prompt portions go row by row as well, but many rows of one sequence share what they read)
-    few = step.n_few if state.dtype == torch.float32 else step.n_single
-    for r0, r1, runs in ((0, few, False), (few, step.n_single, True)):
-        if r0 < r1:
-            gqa.gqa_decode(ctx, sub(y, r0, r1 - r0), a, w.slopes, step.single_places(r0, r1), cache, sub(out, r0, r1 - r0), step.span, runs=runs)
+    if step.n_single:  # (prompt portions as well where they have no form of their own, in fp32 with many rows that share what they read)
+        gqa.gqa_decode(ctx, sub(y, 0, step.n_single), a, w.slopes, step.single_places(), cache, sub(out, 0, step.n_single), step.span,
+                       singles=step.n_few)
     if step.plans:
         gqa.gqa_prefill(ctx, y, a, w.slopes, step.plans[0], cache, out)
     return out

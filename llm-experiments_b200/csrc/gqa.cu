@@ -404,10 +404,15 @@ int launch_runs(const GqaDecodeArgs& a, void* stream) {
     return B2KV_OK;
 }
 
-// For rows that the caller says come in runs (a CTA takes the sequences of its 16 rows one after the other, so that single rows of
-// many sequences would be in line: 16 of them take as long as the one that sees most, times 16), and enough of them to fill CTAs.
+// For rows that the caller says come in runs, and enough of them (a CTA takes the sequences of its 16 rows one after the other, so that single rows of
+// many sequences would be in line: 16 of them take as long as the one that sees most, times 16).
 int launch_runs_f32(const GqaDecodeArgs& a, void* stream) {
-    if (a.rows < 64 || (a.rows + kRunRows - 1) / kRunRows > 65535) return B2KV_ERR_UNSUPPORTED;
+    // Enough CTAs that the SMs are busy with 64 threads each: below, a CTA's chain of token tiles takes longer than rows one by
+    // one over as many SMs (8 heads of 64: 100 rows behind 500 others 59 us and 52, 400 rows 78 and 179; of 128, with half as many CTAs per SM: 100
+    // rows 116 and 64, 400 rows 153 and 233).
+    const long long ctas = static_cast<long long>(a.H) * ((a.rows + kRunRows - 1) / kRunRows), sms = device_sm_count();
+    const bool few = a.rows < 64 || (std::max(a.dim, a.vdim) <= 64 ? 4 * ctas < 3 * sms : 2 * ctas < 3 * sms);
+    if ((few && tune_get("gqa_runs") == 0) || (a.rows + kRunRows - 1) / kRunRows > 65535) return B2KV_ERR_UNSUPPORTED;
     const int widest = std::max(a.dim, a.vdim);
     if (widest > 128 || a.dim % 4 || a.vdim % 4 || a.ld_q % 4 || !aligned16(a.q) || !aligned16(a.k_cache) || !aligned16(a.v_cache))
         return B2KV_ERR_UNSUPPORTED;
@@ -468,20 +473,25 @@ extern "C" size_t b2kv_gqa_decode_workspace_bytes(int rows, int H, int G, int vd
     return gqa_decode_tc_workspace(rows, H, G, vdim, span);
 }
 
-static int gqa_decode(const GqaDecodeArgs& a, int dtype, int path, bool runs, void* workspace, size_t workspace_bytes, void* stream) {
+// singles: rows in front of those that come in runs (all rows: none do).
+static int gqa_decode(const GqaDecodeArgs& a, int dtype, int path, int singles, void* workspace, size_t workspace_bytes, void* stream) {
     if (elt_bytes(dtype) == 0) return B2KV_ERR_UNSUPPORTED;
     if (!a.q || !a.k_cache || !a.v_cache || !a.out || !a.row_pos) return B2KV_ERR_BAD_ARG;
     if (a.n_slots <= 0 || a.T_max <= 0 || a.rows <= 0 || a.H <= 0 || a.G <= 0 || a.H % a.G != 0 || a.dim <= 0 || a.vdim <= 0 || a.span <= 0 ||
-        path < 0 || path > 2 || a.ld_q < static_cast<int64_t>(a.H) * a.dim || a.ld_out < static_cast<int64_t>(a.H) * a.vdim)
+        path < 0 || path > 2 || singles < 0 || a.ld_q < static_cast<int64_t>(a.H) * a.dim || a.ld_out < static_cast<int64_t>(a.H) * a.vdim)
         return B2KV_ERR_BAD_ARG;
     if (path == 2 && dtype != B2KV_DTYPE_BF16) return B2KV_ERR_UNSUPPORTED;
     if (dtype == B2KV_DTYPE_BF16 && path != 1) {
         const int rc = gqa_decode_tc(a, workspace, workspace_bytes, stream);
         if (rc != B2KV_ERR_UNSUPPORTED || path == 2) return rc;
     }
-    if (dtype == B2KV_DTYPE_F32 && path == 0 && runs) {
-        const int rc = launch_runs_f32(a, stream);
-        if (rc != B2KV_ERR_UNSUPPORTED) return rc;
+    if (dtype == B2KV_DTYPE_F32 && path == 0 && singles < a.rows && a.row_slot != nullptr) {
+        GqaDecodeArgs front = a, runs = a;
+        front.rows = singles, runs.rows = a.rows - singles;
+        runs.q = static_cast<const float*>(a.q) + singles * a.ld_q, runs.out = static_cast<float*>(a.out) + singles * a.ld_out;
+        runs.row_slot = a.row_slot + singles, runs.row_pos = a.row_pos + singles;
+        const int rc = launch_runs_f32(runs, stream);
+        if (rc != B2KV_ERR_UNSUPPORTED) return rc != B2KV_OK || singles == 0 ? rc : launch_simt<float>(front, stream);
     }
     return dtype == B2KV_DTYPE_F32 ? launch_simt<float>(a, stream) : launch_simt<__nv_bfloat16>(a, stream);
 }
@@ -491,13 +501,13 @@ extern "C" int b2kv_gqa_decode(const void* q, int64_t ld_q, const void* k_cache,
                                int rows, int H, int G, int dim, int vdim, int span, float scale, int dtype, int path,
                                void* workspace, size_t workspace_bytes, int32_t* dev_status, void* stream) {
     return gqa_decode({q, k_cache, v_cache, out, slopes, row_slot, row_pos, dev_status, ld_q, ld_out, n_slots, T_max, rows, H, G, dim, vdim,
-                       span, scale}, dtype, path, false, workspace, workspace_bytes, stream);
+                       span, scale}, dtype, path, rows, workspace, workspace_bytes, stream);
 }
 
 extern "C" int b2kv_gqa_decode_runs(const void* q, int64_t ld_q, const void* k_cache, const void* v_cache, void* out, int64_t ld_out,
                                     const float* slopes, const int32_t* row_slot, const int32_t* row_pos, int n_slots, int T_max,
-                                    int rows, int H, int G, int dim, int vdim, int span, float scale, int dtype, int path,
+                                    int rows, int H, int G, int dim, int vdim, int span, float scale, int dtype, int path, int singles,
                                     void* workspace, size_t workspace_bytes, int32_t* dev_status, void* stream) {
     return gqa_decode({q, k_cache, v_cache, out, slopes, row_slot, row_pos, dev_status, ld_q, ld_out, n_slots, T_max, rows, H, G, dim, vdim,
-                       span, scale}, dtype, path, true, workspace, workspace_bytes, stream);
+                       span, scale}, dtype, path, singles, workspace, workspace_bytes, stream);
 }

@@ -61,10 +61,10 @@ def gqa_append(ctx: GPUContext, y: GPUBuffer2D, shape: GqaShape, places: RowPlac
 
 @reference_op("gqa_decode")
 def gqa_decode(ctx: GPUContext, q: GPUBuffer2D, shape: GqaShape, slopes: Optional[GPUBuffer1D], places: RowPlaces, cache: KVCache,
-               out: GPUBuffer2D, span: int, path: int = 0, runs: bool = False) -> None:
+               out: GPUBuffer2D, span: int, path: int = 0, singles: Optional[int] = None) -> None:
     """Attention of single rows: ``q`` as ``gqa_append`` leaves it, ``out`` ``[rows, >= heads * vdim]``.  ``span`` bounds the tokens
-    any row sees.  ``path`` forces a kernel (1 CUDA cores, 2 tensor cores).  ``runs``: the rows are runs of neighbouring rows of one
-    sequence, as prompt portions are."""
+    any row sees.  ``path`` forces a kernel (1 CUDA cores, 2 tensor cores).  Behind the first ``singles`` rows
+    (``None``: all) they are runs of neighbouring rows of one sequence, as prompt portions are."""
     k, v = _caches(cache, shape)
     rows, dt = q.shape[0], dtype_code(q.buffer.dtype)
     nbytes = _native.lib.b2kv_gqa_decode_workspace_bytes(rows, shape.heads, shape.kv_heads, shape.vdim, span, dt) if path != 1 else 0
@@ -72,12 +72,11 @@ def gqa_decode(ctx: GPUContext, q: GPUBuffer2D, shape: GqaShape, slopes: Optiona
         cache.workspace = torch.empty(nbytes, dtype=torch.uint8, device=ctx.device)
     ws = cache.workspace if nbytes else None
     stream = batch_op_begin(ctx)
-    decode = _native.lib.b2kv_gqa_decode_runs if runs else _native.lib.b2kv_gqa_decode
-    _native.check(decode(
+    _native.check(_native.lib.b2kv_gqa_decode_runs(
         q.buffer.data_ptr(), q.buffer.stride(0), k, v, out.buffer.data_ptr(), out.buffer.stride(0),
         None if slopes is None else slopes.buffer.data_ptr(), places.slot_ptr(), places.pos.data_ptr(), cache.batch_size,
         cache.max_seq_len, rows, shape.heads, shape.kv_heads, shape.dim, shape.vdim, span, shape.scale, dt, path,
-        None if ws is None else ws.data_ptr(), 0 if ws is None else ws.numel(), dev_status_ptr(ctx), stream))
+        rows if singles is None else singles, None if ws is None else ws.data_ptr(), 0 if ws is None else ws.numel(), dev_status_ptr(ctx), stream))
 
 
 def prefill_supported(shape: GqaShape, dtype: torch.dtype) -> bool:

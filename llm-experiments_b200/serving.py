@@ -71,10 +71,9 @@ class Step:
     row_index: Optional[torch.Tensor]  # rows whose logits are wanted (None: all)
     n_out: int
 
-    def single_places(self, r0: int = 0, r1: Optional[int] = None) -> RowPlaces:
-        """Of the rows ``r0 .. r1 - 1`` (default: all) that go row by row.  (Without a table of sequences all rows are asked for.)"""
-        p, r1 = self.places, self.n_single if r1 is None else r1
-        return RowPlaces(None if p.slot is None else p.slot[r0:r1], p.pos[r0:r1])
+    def single_places(self) -> RowPlaces:
+        p = self.places
+        return RowPlaces(None if p.slot is None else p.slot[:self.n_single], p.pos[:self.n_single])
 
 
 @dataclass

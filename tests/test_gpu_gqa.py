@@ -66,7 +66,7 @@ def in_batch(pkg, ctx, fn):
     torch.cuda.synchronize()
 
 
-@pytest.mark.parametrize("dtype,heads,kv,dim,vdim,own", [(F32, 3, 1, 5, 7, True), (BF, 3, 3, 5, 7, True), (F32, 8, 2, 24, 40, True),
+@pytest.mark.parametrize("dtype,heads,kv,dim,vdim,own", [(F32, 3, 1, 5, 7, True), (BF, 3, 3, 5, 7, True), (F32, 8, 2, 24, 40, 0),
                                                         (BF, 6, 3, 40, 24, True), (BF, 32, 8, 128, 128, True), (BF, 4, 2, 72, 64, False)])
 @pytest.mark.parametrize("every,coef", [(0, 0.0), (1, 0.7), (37, 0.25)])
 def test_append_norms_scales_and_stores(pkg, dtype, heads, kv, dim, vdim, own, every, coef):
@@ -151,8 +151,8 @@ def test_single_rows(pkg, path, dtype, heads, kv, dim, vdim, bias):
 
 @pytest.mark.parametrize("heads,kv,dim,vdim", [(3, 1, 4, 8), (4, 2, 64, 64), (2, 1, 72, 128), (2, 2, 128, 20)])
 @pytest.mark.parametrize("runs", [((0, 0, 65),), ((2, 0, 64), (0, 60, 7), (1, 199, 1), (2, 64, 31), (0, 0, 40)), ((1, 130, 96), (0, 3, 33))])
-@pytest.mark.parametrize("said", [False, True])
-def test_runs_of_rows_in_fp32(pkg, heads, kv, dim, vdim, runs, said):
+@pytest.mark.parametrize("singles", [None, 0, 5])
+def test_runs_of_rows_in_fp32(pkg, heads, kv, dim, vdim, runs, singles):
     """Prompt portions of 16-row tiles and their parts, several sequences in a tile, one of them twice; nothing that a row must not
     see reaches it, not even what is no number."""
     from llm_experiments_b200 import gqa
@@ -171,7 +171,11 @@ def test_runs_of_rows_in_fp32(pkg, heads, kv, dim, vdim, runs, said):
     out = torch.full((len(pos) + 1, heads * vdim + 8), 7.0, dtype=F32, device="cuda")
     slopes = gqa.geometric_slopes(heads).cuda()
     places = RowPlaces(torch.tensor(slots, dtype=torch.int32, device="cuda"), torch.tensor(pos, dtype=torch.int32, device="cuda"))
-    in_batch(pkg, ctx, lambda: gqa.gqa_decode(ctx, wrap(pkg, y), shape, wrap1(pkg, slopes), places, cache, wrap(pkg, out[:len(pos)]), 240, runs=said))
+    pkg._native.tune("gqa_runs", 1)  # (however few they are)
+    try:
+        in_batch(pkg, ctx, lambda: gqa.gqa_decode(ctx, wrap(pkg, y), shape, wrap1(pkg, slopes), places, cache, wrap(pkg, out[:len(pos)]), 240, singles=singles))
+    finally:
+        pkg._native.tune("gqa_runs", 0)
     k, v = (np64(t) for t in cache_views(cache, shape))
     want = reference(np64(y)[:, :heads * dim].reshape(len(pos), heads, dim), k, v, slots, pos, shape, bo.head_slopes(heads))
     got = np64(out)[:len(pos), :heads * vdim]
@@ -187,23 +191,23 @@ def test_the_kernel_for_runs_is_the_callers_choice(pkg):
     from llm_experiments_b200 import gqa
     from llm_experiments_b200.latent import RowPlaces
 
-    ctx, shape, rows = make_ctx(pkg), gqa.GqaShape(4, 2, 64, 64, 0.125), 200
+    ctx, shape, rows = make_ctx(pkg), gqa.GqaShape(16, 4, 64, 64, 0.125), 200
     small, large = (make_cache(pkg, ctx, shape, n, 240, F32) for n in (2, 70))
     for a, b in zip(cache_views(small, shape), cache_views(large, shape)):
         b[:2] = a
-    y = rnd((rows, 4 * 64), F32, 7)
+    y = rnd((rows, 16 * 64), F32, 7)
 
-    def attend(cache, slots, path, runs=False):
+    def attend(cache, slots, path, singles=None):
         out = torch.empty_like(y)
         places = RowPlaces(torch.tensor(slots, dtype=torch.int32, device="cuda"), torch.arange(rows, dtype=torch.int32, device="cuda"))
-        in_batch(pkg, ctx, lambda: gqa.gqa_decode(ctx, wrap(pkg, y), shape, None, places, cache, wrap(pkg, out), 240, path=path, runs=runs))
+        in_batch(pkg, ctx, lambda: gqa.gqa_decode(ctx, wrap(pkg, y), shape, None, places, cache, wrap(pkg, out), 240, path=path, singles=singles))
         return out
 
     one, turns = [1] * rows, [i % 2 for i in range(rows)]
-    assert torch.equal(attend(large, one, 0, True), attend(small, one, 0, True))
+    assert torch.equal(attend(large, one, 0, 0), attend(small, one, 0, 0))
     assert torch.equal(attend(small, turns, 0), attend(small, turns, SIMT))
-    torch.testing.assert_close(attend(small, turns, 0, True), attend(small, turns, SIMT), rtol=2e-5, atol=2e-5)
-    assert not torch.equal(attend(small, one, 0, True), attend(small, one, SIMT))
+    torch.testing.assert_close(attend(small, turns, 0, 0), attend(small, turns, SIMT), rtol=2e-5, atol=2e-5)
+    assert not torch.equal(attend(small, one, 0, 0), attend(small, one, SIMT))
 
 
 @pytest.mark.parametrize("share", [1, 2, 3, 5, 16])
