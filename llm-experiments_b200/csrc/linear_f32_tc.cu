@@ -5,7 +5,7 @@
 // Therefore the leading products h h' are accumulated over the 64 input features of a step only; the partial sums are taken out of tensor memory
 // and added up in registers, rounded to nearest.  The other five products, 2^-8 of the first and less, stay in an accumulator of
 // their own until the end.  Measured against 64 bits, 2-norm of the error over that of the result: 8e-8 at 128 input features, 9e-8 at
-// 768, 1.1e-7 at 3072, where sums of fp32 multiply-adds in order are off by 2.0e-7, 5.0e-7 and 9.9e-7.  693 rows, 768 -> 3072: 35 us
+// 768, 1.1e-7 at 3072, where sums of fp32 multiply-adds in order are off by 2.0e-7, 5.0e-7 and 9.9e-7.  693 rows, 768 -> 3072: 31 us
 // against 127 of linear_f32_tile_kernel; 3072 -> 768: 39 and 130; 60 rows, 768 -> 3072: 15 and 25.
 //
 //   * a CTA has 128 x 128 outputs; steps of 64 input features through two stages of 96 KB;
@@ -23,8 +23,8 @@
 // operand is not, or rounds to none in bf16, or finite operands' products overflow, where the sign of a partial product says nothing),
 // and rows of x and columns of w with a number whose three parts do not add up to it (some below 2^-109, where the last part
 // is below the smallest number of bf16).  The bits of every other row and column are what they are without it.  One such row among 693,
-// 3072 -> 768: 137 us instead of 39; with a whole tile again, one chain of global loads per thread, it took 9.3 ms.  Every wait is bounded; after one ran out nothing is stored and the
-// status word is set.
+// 3072 -> 768: 137 us instead of 39; with a whole tile again, one chain of global loads per thread, it took 9.3 ms.
+// Every wait is bounded; after one ran out nothing is stored and the status word is set.
 #include <algorithm>
 
 #include "linear.cuh"

@@ -438,8 +438,8 @@ static int launch_prefill_tc_f32(const PrefillParams& p_in, void* scratch, void*
         B2KV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)));
         configured[dev] = true;
     }
-    OverlapLaunch first(dim3(static_cast<unsigned>((rows + split.per_cta - 1) / split.per_cta), 3), std::min(kSplitThreads, (split.per_cta * (E / 4) + 31) / 32 * 32), 0,
-                        stream);
+    const unsigned split_ctas = static_cast<unsigned>((rows + split.per_cta - 1) / split.per_cta);
+    OverlapLaunch first(dim3(split_ctas, 3), std::min(kSplitThreads, (split.per_cta * (E / 4) + 31) / 32 * 32), 0, stream);
     B2KV_CUDA_TRY(cudaLaunchKernelEx(&first.cfg, tcf::split_kernel, split));
     OverlapLaunch launch(static_cast<unsigned>(ctas), tcf::kThreads, smem, stream);
     B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, kernel, tm[0], tm[1], tm[2], tm[3], tm[4], tm[5], p));
