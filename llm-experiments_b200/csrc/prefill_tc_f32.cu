@@ -11,19 +11,22 @@
 //   * a first kernel writes the hi and lo halves of Q, K and V into a scratch buffer ([B*N, H*D] bfloat16 each) and, when the
 //     prompt goes to a contiguous cache, the K / V rows to their places there: they pass through its registers anyway (B = 2,
 //     N = 1000, H = 12, D = 64: three launches of it and the copy kernel behind the attention were 20 of 53 us);
-//   * one CTA per (sequence, head, 128 query rows), two CTAs per SM at head_dim 64.  Warp 8 loads the Q tile and, step by step, a
+//   * one CTA per (sequence, head, 128 query rows), at head_dim 64 in two forms: two CTAs per SM that fill each other's gaps, or one with
+//     two score buffers and rings of two tiles, whose QK^T of the next step runs under the softmax of this one (the rule and both
+//     times at prefill_tensor_core_f32).  What bounds the second is its products: 12 MMAs of QK^T and 24 of PV, 2900 clocks per step of
+//     128 keys.  Warp 8 loads the Q tile and, step by step, a
 //     128-key K tile and V tile (hi and lo: 64 KB each at head_dim 128, so the rings hold one step) with TMA tiled loads into
 //     128-byte-swizzled shared memory; warp 9 issues S = Q K^T (3 x head_dim/16 tcgen05.mma, both operands in
 //     shared memory) and O += P V (3 x 8, P read from tensor memory, V an MN-major shared-memory operand);
-//   * warps 0 - 7: two threads per query row = TMEM lane, one for each half of a step's keys.  QK^T, softmax and PV of the one
-//     query tile follow one another, and only another CTA fills the gaps: with half a row per thread two CTAs fit the registers
+//   * warps 0 - 7: two threads per query row = TMEM lane, one for each half of a step's keys.  With one score buffer QK^T, softmax and PV
+//     of the query tile follow one another, and only another CTA fills the gaps: with half a row per thread two CTAs fit the registers
 //     (B = 8, N = 2048, H = 12, D = 64: 443 us with four warps and one CTA per SM, 250 so; N = 4096, H = 8, B = 4: 408 and 286;
 //     one CTA per SM at D = 128, B = 2, N = 4096, H = 16: 506 and 454).  Scores in registers, the row's maximum exchanged through shared memory, running maximum
 //     and sum in the log2 domain in fp32, O rescaled only when the maximum has grown by more than 2^8, P written back as hi and
 //     lo halves (packed bfloat16) over the score buffer: hi in columns 0 - 63, lo in columns 64 - 127;
 //   * epilogue O / max(l, 1e-8) as fp32, L and M as the reference writes them (:762-768).
 //
-// Tensor memory: S / P columns 0 - 127, O columns 128 - 255.  Every mbarrier wait is bounded.
+// Tensor memory: S / P columns 0 - 127 (and 128 - 255), O behind.  Every mbarrier wait is bounded.
 #include <math.h>
 
 #include <algorithm>
@@ -43,17 +46,19 @@ constexpr int kBlockN = 128;
 constexpr int kHalfTileBytes = 128 * 128;  // 128 rows x 64 bf16
 constexpr int kSoftmaxWarps = 8, kCopyWarp = 8, kMmaWarp = 9;
 constexpr int kThreads = 320;
-constexpr int kTmemCols = 256;
-constexpr int kColS = 0, kColO = 128;
+constexpr int kColS = 0;  // score buffers of 128 columns, then O
 constexpr float kRescaleThreshold = 8.0f;
 
-template <int kD>
+// kBuf: score buffers (2: QK^T of the next step runs under this step's softmax).  Step j uses the barriers and buffers j % kBuf: the next but
+// one cannot begin before PV of this one has been issued, so that no wait by parity can be taken for an older phase.
+template <int kD, int kBuf>
 struct SharedStorage {
     static constexpr int kTileBytes = (kD / 64) * kHalfTileBytes;  // 128 rows x kD bf16
+    static constexpr int kRing = kD == 64 ? kBuf : 1;              // tiles of K and of V that fit
     alignas(1024) uint8_t q[2][kTileBytes];  // [hi / lo]
-    alignas(1024) uint8_t k[2][kTileBytes];
-    alignas(1024) uint8_t v[2][kTileBytes];
-    alignas(8) uint64_t q_full, k_full, k_empty, v_full, v_empty, s_full, p_ready, o_done;
+    alignas(1024) uint8_t k[kRing][2][kTileBytes];
+    alignas(1024) uint8_t v[kRing][2][kTileBytes];
+    alignas(8) uint64_t q_full, k_full[kRing], k_empty[kRing], v_full[kRing], v_empty[kRing], s_full[kBuf], p_ready[kBuf], o_done[kBuf];
     float exchange[2][2][kTileM];  // [parity of the step][half of the keys][row]: maxima; sums at the end
     uint32_t tmem_base;
     volatile int abort_flag;
@@ -94,14 +99,15 @@ __global__ void __launch_bounds__(256) split_kernel(const __grid_constant__ Spli
     }
 }
 
-template <int kD>
-__global__ void __launch_bounds__(kThreads, kD == 64 ? 2 : 1)
+template <int kD, int kBuf>
+__global__ void __launch_bounds__(kThreads, kD == 64 && kBuf == 1 ? 2 : 1)
 prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_constant__ CUtensorMap tm_ql,
                       const __grid_constant__ CUtensorMap tm_kh, const __grid_constant__ CUtensorMap tm_kl,
                       const __grid_constant__ CUtensorMap tm_vh, const __grid_constant__ CUtensorMap tm_vl,
                       const PrefillParams p) {
     extern __shared__ uint8_t smem_raw[];
-    using Smem = SharedStorage<kD>;
+    using Smem = SharedStorage<kD, kBuf>;
+    constexpr int kRing = Smem::kRing, kColO = kBuf * 128, kTmemCols = kBuf == 1 ? 256 : 512;
     constexpr int kHalves = kD / 64;
     constexpr int kTileBytes = Smem::kTileBytes;
     Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -126,13 +132,17 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
 
     if (threadIdx.x == 0) {
         mbar_init(&sm.q_full, 1);
-        mbar_init(&sm.k_full, 1);
-        mbar_init(&sm.k_empty, 1);
-        mbar_init(&sm.v_full, 1);
-        mbar_init(&sm.v_empty, 1);
-        mbar_init(&sm.s_full, 1);
-        mbar_init(&sm.p_ready, kSoftmaxWarps);
-        mbar_init(&sm.o_done, 1);
+        for (int i = 0; i < kRing; ++i) {
+            mbar_init(&sm.k_full[i], 1);
+            mbar_init(&sm.k_empty[i], 1);
+            mbar_init(&sm.v_full[i], 1);
+            mbar_init(&sm.v_empty[i], 1);
+        }
+        for (int i = 0; i < kBuf; ++i) {
+            mbar_init(&sm.s_full[i], 1);
+            mbar_init(&sm.p_ready[i], kSoftmaxWarps);
+            mbar_init(&sm.o_done[i], 1);
+        }
         sm.abort_flag = 0;
         fence_mbar_init();
     }
@@ -158,22 +168,23 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
             }
             bool ok = true;
             for (int j = 0; j < n && ok; ++j) {
-                const uint32_t par = (j & 1) ^ 1;
-                ok = mbar_wait(&sm.k_empty, par);
+                const int st = j % kRing;
+                const uint32_t par = ((j / kRing) & 1) ^ 1;
+                ok = mbar_wait(&sm.k_empty[st], par);
                 if (!ok) break;
-                mbar_arrive_expect_tx(&sm.k_full, 2 * kTileBytes);
+                mbar_arrive_expect_tx(&sm.k_full[st], 2 * kTileBytes);
 #pragma unroll
                 for (int hf = 0; hf < kHalves; ++hf) {
-                    tma_load_3d(sm.k[0] + hf * kHalfTileBytes, &tm_kh, &sm.k_full, x0 + hf * 64, j * kBlockN, b);
-                    tma_load_3d(sm.k[1] + hf * kHalfTileBytes, &tm_kl, &sm.k_full, x0 + hf * 64, j * kBlockN, b);
+                    tma_load_3d(sm.k[st][0] + hf * kHalfTileBytes, &tm_kh, &sm.k_full[st], x0 + hf * 64, j * kBlockN, b);
+                    tma_load_3d(sm.k[st][1] + hf * kHalfTileBytes, &tm_kl, &sm.k_full[st], x0 + hf * 64, j * kBlockN, b);
                 }
-                ok = mbar_wait(&sm.v_empty, par);
+                ok = mbar_wait(&sm.v_empty[st], par);
                 if (!ok) break;
-                mbar_arrive_expect_tx(&sm.v_full, 2 * kTileBytes);
+                mbar_arrive_expect_tx(&sm.v_full[st], 2 * kTileBytes);
 #pragma unroll
                 for (int hf = 0; hf < kHalves; ++hf) {
-                    tma_load_3d(sm.v[0] + hf * kHalfTileBytes, &tm_vh, &sm.v_full, x0 + hf * 64, j * kBlockN, b);
-                    tma_load_3d(sm.v[1] + hf * kHalfTileBytes, &tm_vl, &sm.v_full, x0 + hf * 64, j * kBlockN, b);
+                    tma_load_3d(sm.v[st][0] + hf * kHalfTileBytes, &tm_vh, &sm.v_full[st], x0 + hf * 64, j * kBlockN, b);
+                    tma_load_3d(sm.v[st][1] + hf * kHalfTileBytes, &tm_vl, &sm.v_full[st], x0 + hf * 64, j * kBlockN, b);
                 }
             }
             if (!ok) sm.abort_flag = 1;
@@ -185,15 +196,15 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
             constexpr uint32_t idesc_qk = instr_desc(0, 0, kBlockN);  // S[128 x 128 keys]
             constexpr uint32_t idesc_pv = instr_desc(0, 1, kD);       // O[128 x kD]
             const uint64_t dq[2] = {smem_desc(smem_u32(sm.q[0]), 16, 1024), smem_desc(smem_u32(sm.q[1]), 16, 1024)};
-            const uint64_t dk[2] = {smem_desc(smem_u32(sm.k[0]), 16, 1024), smem_desc(smem_u32(sm.k[1]), 16, 1024)};
-            const uint64_t dv[2] = {smem_desc(smem_u32(sm.v[0]), kHalfTileBytes, 1024),
-                                    smem_desc(smem_u32(sm.v[1]), kHalfTileBytes, 1024)};
-            const uint32_t s_tmem = tmem + kColS, o_tmem = tmem + kColO;
+            const uint64_t dk0 = smem_desc(smem_u32(sm.k[0][0]), 16, 1024), dv0 = smem_desc(smem_u32(sm.v[0][0]), kHalfTileBytes, 1024);
+            constexpr uint64_t kTile16 = kTileBytes >> 4;
+            const uint32_t o_tmem = tmem + kColO;
             // the three partial products of a split product: (hi, hi), (hi, lo), (lo, hi)
-            auto issue_qk = [&]() {
+            auto issue_qk = [&](int j) {
+                const uint32_t s_tmem = tmem + kColS + (j % kBuf) * 128;
 #pragma unroll
                 for (int t = 0; t < 3; ++t) {
-                    const uint64_t da = dq[t == 2 ? 1 : 0], db = dk[t == 1 ? 1 : 0];
+                    const uint64_t da = dq[t == 2 ? 1 : 0], db = dk0 + (2 * (j % kRing) + (t == 1 ? 1 : 0)) * kTile16;
 #pragma unroll
                     for (int kb = 0; kb < kHalves; ++kb) {
 #pragma unroll
@@ -203,37 +214,41 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
                         }
                     }
                 }
-                mma_commit(&sm.s_full);
-                mma_commit(&sm.k_empty);
+                mma_commit(&sm.s_full[j % kBuf]);
+                mma_commit(&sm.k_empty[j % kRing]);
             };
             auto issue_pv = [&](int j) {
+                const uint32_t s_tmem = tmem + kColS + (j % kBuf) * 128;
 #pragma unroll
                 for (int t = 0; t < 3; ++t) {
                     const uint32_t pa = s_tmem + (t == 2 ? 64 : 0);  // P hi in columns 0 - 63, P lo in 64 - 127
-                    const uint64_t db = dv[t == 1 ? 1 : 0];
+                    const uint64_t db = dv0 + (2 * (j % kRing) + (t == 1 ? 1 : 0)) * kTile16;
 #pragma unroll
                     for (int kk = 0; kk < 8; ++kk)
                         mma_ts(o_tmem, pa + kk * 8, db + static_cast<uint64_t>((kk * 2048) >> 4), idesc_pv,
                                (j | t | kk) ? 1u : 0u);
                 }
-                mma_commit(&sm.o_done);
-                mma_commit(&sm.v_empty);
+                mma_commit(&sm.o_done[j % kBuf]);
+                mma_commit(&sm.v_empty[j % kRing]);
             };
-            bool ok = mbar_wait(&sm.q_full, 0) && mbar_wait(&sm.k_full, 0);
-            if (ok) {
+            bool ok = mbar_wait(&sm.q_full, 0);
+            for (int j = 0; j < kBuf && j < n && ok; ++j) {
+                ok = mbar_wait(&sm.k_full[j % kRing], (j / kRing) & 1);
+                if (!ok) break;
                 tc_fence_after();
-                issue_qk();
+                issue_qk(j);
             }
             for (int j = 0; j < n && ok; ++j) {
-                ok = mbar_wait(&sm.p_ready, j & 1) && mbar_wait(&sm.v_full, j & 1);
+                ok = mbar_wait(&sm.p_ready[j % kBuf], (j / kBuf) & 1) && mbar_wait(&sm.v_full[j % kRing], (j / kRing) & 1);
                 if (!ok) break;
                 tc_fence_after();
                 issue_pv(j);
-                if (j + 1 < n) {
-                    ok = mbar_wait(&sm.k_full, (j + 1) & 1);
+                const int jn = j + kBuf;
+                if (jn < n) {
+                    ok = mbar_wait(&sm.k_full[jn % kRing], (jn / kRing) & 1);
                     if (!ok) break;
                     tc_fence_after();
-                    issue_qk();  // overwrites P(j): the tensor pipe runs its MMAs in order, PV(j) has read it by then
+                    issue_qk(jn);  // overwrites P(j): the tensor pipe runs its MMAs in order, PV(j) has read it by then
                 }
             }
             if (!ok) sm.abort_flag = 1;
@@ -243,13 +258,13 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
         // ------------------------------ softmax: two threads per query row ------------------------------
         const int row = threadIdx.x & (kTileM - 1), half = warp >> 2;  // row inside the tile = TMEM lane; half of the keys
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        const uint32_t s_tmem = tmem + lane_base + kColS;
         const uint32_t o_tmem = tmem + lane_base + kColO + half * (kD / 2);
         const float c = p.q_prescale;  // log2(e) / sqrt(D)
         float m_used = -INFINITY, m_run = -INFINITY, l = 0.f;
         bool ok = true;  // (a thread whose wait ran out goes on without waiting: its partners wait for it at the named barrier)
         for (int j = 0; j < n; ++j) {
-            ok = ok && mbar_wait(&sm.s_full, j & 1);
+            ok = ok && mbar_wait(&sm.s_full[j % kBuf], (j / kBuf) & 1);
+            const uint32_t s_tmem = tmem + lane_base + kColS + (j % kBuf) * 128;
             __syncwarp();
             tc_fence_after();
             uint32_t r[64];
@@ -306,7 +321,7 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
             }
             l = l * factor + ((sums[0] + sums[1]) + (sums[2] + sums[3]));
             if (__any_sync(0xffffffffu, need)) {
-                ok = ok && mbar_wait(&sm.o_done, (j - 1) & 1);
+                ok = ok && mbar_wait(&sm.o_done[(j - 1) % kBuf], ((j - 1) / kBuf) & 1);
                 __syncwarp();
                 tc_fence_after();
 #pragma unroll 1
@@ -322,11 +337,11 @@ prefill_tc_f32_kernel(const __grid_constant__ CUtensorMap tm_qh, const __grid_co
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.p_ready);
+            if (lane == 0) mbar_arrive(&sm.p_ready[j % kBuf]);
         }
         sm.exchange[n & 1][half][row] = l;
-        // every PV is waited for in order here or by nobody, so the parity names the last one
-        ok = ok && mbar_wait(&sm.o_done, (n - 1) & 1);
+        // (the scores of the last step were complete behind PV of the step kBuf before: the parity names the last one)
+        ok = ok && mbar_wait(&sm.o_done[(n - 1) % kBuf], ((n - 1) / kBuf) & 1);
         named_barrier_sync<64>(1 + (warp & 3));
         l += sm.exchange[n & 1][half ^ 1][row];
         if (__all_sync(0xffffffffu, ok)) {
@@ -395,7 +410,7 @@ size_t prefill_f32_scratch_bytes(int B, int N, int H, int D) {
     return 6ull * static_cast<size_t>(B) * N * H * D * sizeof(__nv_bfloat16);
 }
 
-template <int kD>
+template <int kD, int kBuf>
 static int launch_prefill_tc_f32(const PrefillParams& p_in, void* scratch, void* stream) {
     PrefillParams p = p_in;
     if (p.group == 0) {
@@ -427,14 +442,14 @@ static int launch_prefill_tc_f32(const PrefillParams& p_in, void* scratch, void*
     // CTAs that could all have an SM of their own get one: launched while the halves are still written they take places in pairs, two on
     // one SM and none on others (head_dim 64, N = 4096, 4 heads: 103.8 us, 93.1 so)
     constexpr size_t kAlone = 116 * 1024;
-    const size_t smem = std::max(sizeof(tcf::SharedStorage<kD>) + 1024, ctas <= device_sm_count() ? kAlone : size_t{0});
-    auto kernel = tcf::prefill_tc_f32_kernel<kD>;
+    const size_t smem = std::max(sizeof(tcf::SharedStorage<kD, kBuf>) + 1024, ctas <= device_sm_count() ? kAlone : size_t{0});
+    auto kernel = tcf::prefill_tc_f32_kernel<kD, kBuf>;
     static bool configured[64] = {false};
     int dev = 0;
     B2KV_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return B2KV_ERR_UNSUPPORTED;
     if (!configured[dev]) {
-        const size_t most = std::max(sizeof(tcf::SharedStorage<kD>) + 1024, kAlone);
+        const size_t most = std::max(sizeof(tcf::SharedStorage<kD, kBuf>) + 1024, kAlone);
         B2KV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)));
         configured[dev] = true;
     }
@@ -451,9 +466,15 @@ int prefill_tensor_core_f32(const PrefillParams& p, int D, void* scratch, size_t
         return B2KV_ERR_UNSUPPORTED;
     if ((static_cast<size_t>(p.B) * p.N * p.H * D) % 8 != 0) return B2KV_ERR_UNSUPPORTED;  // halves stay 16-byte aligned
     if (tensor_map_encoder() == nullptr) return B2KV_ERR_UNSUPPORTED;
-    if (D == 128) return launch_prefill_tc_f32<128>(p, scratch, stream);
-    if (D == 64) return launch_prefill_tc_f32<64>(p, scratch, stream);
-    return B2KV_ERR_UNSUPPORTED;
+    if (D == 128) return launch_prefill_tc_f32<128, 1>(p, scratch, stream);
+    if (D != 64) return B2KV_ERR_UNSUPPORTED;
+    // Two score buffers where a CTA is alone on its SM anyway, or nearly so and walks through several steps; else two CTAs share an SM and
+    // fill each other's gaps.  One buffer and two, us: 64 CTAs of 2 steps 10.1, 8.6; 128 of 32 94.5, 63.6; 192 of 8 36.4, 26.4; 256 of
+    // 16 59.2, 42.8; but 192 of 2 20.7, 22.8; 384 of 4 41.9, 42.8; 1536 of 16 250, 266.  (At head_dim 128, with one tile of K and V in
+    // shared memory: 144 of 6 30.5, 31.2; 1024 of 32 457, 480.)
+    const long long steps = (p.N + tcf::kTileM - 1) / tcf::kTileM, ctas = steps * p.H * p.B, sms = device_sm_count();
+    if (ctas <= sms || (ctas <= 2 * sms && steps > 4)) return launch_prefill_tc_f32<64, 2>(p, scratch, stream);
+    return launch_prefill_tc_f32<64, 1>(p, scratch, stream);
 }
 
 }  // namespace b2kv

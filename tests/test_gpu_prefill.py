@@ -287,3 +287,20 @@ def test_fp32_tensor_core_prefill_fills_the_cache_bit_exact(pkg, ctx, layout):
     flat = lambda a: U.to_oracle(a.reshape(B * N, E))  # noqa: E731
     Ow, _, _ = c_oracle.prefill(flat(Q), flat(K), flat(V), B, N, H, D, want_stats=False)
     np.testing.assert_allclose(U.to_f32(O), Ow, **SPLIT_TOL)
+
+
+@pytest.mark.parametrize("B,N,H", [(1, 1100, 4), (3, 128, 40), (2, 600, 14), (1, 513, 59), (1, 512, 60), (3, 129, 75), (37, 500, 2)])
+def test_fp32_prompts_with_one_score_buffer_and_two(pkg, ctx, B, N, H):
+    """Few CTAs of many steps and of one, up to two per SM of more than four steps, and just beyond: against 64 bits at the tolerance of split
+    operands, a last step that is not whole, L and M among the outputs."""
+    D = 64
+    Q, K, V = (U.randn((B, N, H * D), torch.float32, ctx.device, s) for s in (61, 62, 63))
+    O, L, M = _run_flash(pkg, ctx, Q, K, V, B, N, H, D, torch.float32)
+    q, k, v = (t.view(B, N, H, D).transpose(1, 2).double() for t in (Q, K, V))
+    s = (q @ k.transpose(2, 3)) * D ** -0.5
+    s.masked_fill_(torch.ones(N, N, dtype=torch.bool, device=s.device).triu(1), float("-inf"))
+    m = s.amax(dim=-1)
+    e = torch.exp(s - m[..., None])
+    np.testing.assert_allclose(O.view(B, N, H, D).cpu().numpy(), ((e / e.sum(-1, keepdim=True)) @ v).transpose(1, 2).cpu().numpy(), **SPLIT_TOL)
+    np.testing.assert_allclose(L.view(B, N, H).cpu().numpy(), e.sum(-1).transpose(1, 2).cpu().numpy(), rtol=1e-4)
+    np.testing.assert_allclose(M.view(B, N, H).cpu().numpy(), m.transpose(1, 2).cpu().numpy(), rtol=1e-4, atol=3e-5)
