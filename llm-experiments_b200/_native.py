@@ -6,10 +6,14 @@ this module fails with instructions to build it: there is no CPU or PyTorch fall
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import pathlib
+import struct
 
 _PKG = pathlib.Path(__file__).resolve().parent
 LIB_PATH = _PKG / "libb2kv.so"
+CALLS_PATH = _PKG / "b2kv_calls.so"  # calls without ctypes' conversions (csrc/calls.c); where it is not built ctypes makes them
 SERVE_LIB_PATH = _PKG / "libb2kv_serve.so"  # the part models are served with (build.py --serve), where that is all there is
 
 DTYPE_F32 = 0
@@ -159,7 +163,36 @@ def _not_built(name: str):
     return call
 
 
-def _load() -> ctypes.CDLL:
+_TYPES = {_vp: "p", _i: "i", _i64: "l", _sz: "l", _f: "f", ctypes.c_uint32: "i", ctypes.c_char_p: None}
+
+
+def _calls():
+    """The extension module of ``csrc/calls.c``, or None."""
+    if not CALLS_PATH.exists():
+        return None
+    loader = importlib.machinery.ExtensionFileLoader("b2kv_calls", str(CALLS_PATH))
+    try:
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("b2kv_calls", loader))
+        loader.exec_module(module)
+    except ImportError:  # built for another interpreter
+        return None
+    return module
+
+
+class Library:
+    """The entry points: what ``csrc/calls.c`` can call, and ctypes functions for the rest (texts)."""
+
+    def __init__(self, lib: ctypes.CDLL, calls):
+        self.cdll = lib
+        for name, (restype, argtypes) in SIGNATURES.items():
+            fn = getattr(lib, name)
+            kinds = ["p" if issubclass(t, ctypes._Pointer) else _TYPES[t] for t in argtypes]
+            if calls is not None and None not in kinds and restype in (_i, _sz) and hasattr(fn, "argtypes"):
+                fn = calls.bind(ctypes.cast(fn, _vp).value, "".join(kinds), "i" if restype is _i else "z", fn)
+            setattr(self, name, fn)
+
+
+def _load() -> Library:
     path = LIB_PATH if LIB_PATH.exists() or not SERVE_LIB_PATH.exists() else SERVE_LIB_PATH
     if not path.exists():
         raise ImportError(
@@ -175,10 +208,36 @@ def _load() -> ctypes.CDLL:
         fn = getattr(lib, name)  # AttributeError here means header and library disagree
         fn.restype = restype
         fn.argtypes = argtypes
-    return lib
+    return Library(lib, calls)
 
 
+calls = _calls()
 lib = _load()
+
+# The structures as bytes, which calls.c passes on as they are (a ctypes structure takes longer to fill than its call).
+_LINEAR_ARGS = struct.Struct("5P5q" + "P2q2i" * MAX_SEGMENTS + "8if4x")
+_LINEAR_OPTIONS = struct.Struct("P2i")
+assert _LINEAR_ARGS.size == ctypes.sizeof(LinearArgs) and _LINEAR_OPTIONS.size == ctypes.sizeof(LinearOptions)
+_NO_SEGMENT = (0, 0, 0, 0, 0)
+
+
+def _structure(cls, packed: bytes):
+    return packed if calls is not None else ctypes.byref(cls.from_buffer_copy(packed))
+
+
+def linear_args(x, w, residual, bias, group_rows, ld_x, group_x, ld_w, group_w, ld_residual, segments, rows, k, n, groups, max_group_rows, dtype,
+                path, limit):
+    """``b2kv_linear_args`` for ``lib``; ``segments``: (out, ld, group, end, kind) of each."""
+    if len(segments) > MAX_SEGMENTS:
+        raise IndexError(f"at most {MAX_SEGMENTS} segments")
+    flat = [v for s in segments for v in s] + [v for _ in range(MAX_SEGMENTS - len(segments)) for v in _NO_SEGMENT]
+    return _structure(LinearArgs, _LINEAR_ARGS.pack(x, w, residual, bias, group_rows, ld_x, group_x, ld_w, group_w, ld_residual, *flat, rows, k, n,
+                                                    groups, max_group_rows, len(segments), dtype, path, limit))
+
+
+def linear_options(group_x_rows: int, x_rows: int, flags: int):
+    """``b2kv_linear_options`` for ``lib``."""
+    return _structure(LinearOptions, _LINEAR_OPTIONS.pack(group_x_rows, x_rows, flags))
 
 
 def check(status: int) -> None:

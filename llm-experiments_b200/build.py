@@ -15,11 +15,13 @@ import os
 import pathlib
 import subprocess
 import sys
+import sysconfig
 
 PKG = pathlib.Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 OUT = PKG / "libb2kv.so"
+CALLS = PKG / "b2kv_calls.so"  # the C ABI's calls from Python, an extension module of this interpreter
 SERVE_OUT = PKG / "libb2kv_serve.so"
 OBJ_DIR = PKG / "build"
 SERVE_SOURCES = ("api", "append", "gemm", "gla", "gla_chunked", "gla_run", "gqa", "gqa_decode_tc", "latent", "latent_decode_tc", "latent_prefill", "linear", "linear_f32", "linear_f32_tc", "linear_rows", "moe", "rows",
@@ -51,7 +53,16 @@ def up_to_date(out: pathlib.Path = OUT) -> bool:
     return out.exists() and out.stat().st_mtime >= _newest_input()
 
 
+def build_calls(force: bool = False) -> None:
+    """``b2kv_calls.so`` with the C compiler; nothing where there are no headers of this interpreter (ctypes makes the calls then)."""
+    src, include = CSRC / "calls.c", pathlib.Path(sysconfig.get_paths()["include"])
+    if (not force and CALLS.exists() and CALLS.stat().st_mtime >= src.stat().st_mtime) or not (include / "Python.h").exists():
+        return
+    subprocess.run([os.environ.get("CC", "gcc"), "-O2", "-Wall", "-shared", "-fPIC", "-I", str(include), str(src), "-o", str(CALLS)], check=True)
+
+
 def build(force: bool = False, verbose: bool = False, serve: bool = False) -> pathlib.Path:
+    build_calls(force)
     out = SERVE_OUT if serve else OUT
     if not force and up_to_date(out):
         return out

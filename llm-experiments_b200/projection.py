@@ -10,7 +10,6 @@ the cache.  Checks and texts follow ``kv_cache_update``; bf16 caches with a cont
 """
 from __future__ import annotations
 
-import ctypes
 from dataclasses import dataclass
 from typing import Optional, Sequence
 
@@ -120,7 +119,7 @@ class OutputSegment:
     group: int = 0
 
 
-_AHEAD = ctypes.byref(_native.LinearOptions(flags=_native.LINEAR_AHEAD))
+_AHEAD = _native.linear_options(0, 0, _native.LINEAR_AHEAD)
 
 
 @reference_op("linear")
@@ -149,29 +148,23 @@ def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Se
         raise ValueError("linear: x and w must share one dtype and have contiguous rows")
     if w.shape[1] < n or (group_x == 0 and x.shape[1] < k):
         raise ValueError(f"linear: Dimension mismatch x {tuple(x.shape)}, w {tuple(w.shape)}, k={k}, n={n}")
-    a = _native.LinearArgs(x=x.buffer.data_ptr(), w=w.buffer.data_ptr(), ld_x=x.buffer.stride(0), group_x=group_x,
-                           ld_w=w.buffer.stride(0), group_w=group_w, rows=rows, K=k, N=n, groups=groups,
-                           max_group_rows=max_group_rows, n_seg=len(segments), dtype=dtype_code(x.buffer.dtype), path=path,
-                           limit=limit)
+    outs = []
     for i, s in enumerate(segments):
+        out = s.out.buffer
         want = torch.float32 if s.kind in (SEG_F32, SEG_SOFTCAP, SEG_DECAY) else x.buffer.dtype
-        if s.out.buffer.dtype != want or s.out.buffer.stride(1) != 1 or s.out.shape[0] < rows:
+        if out.dtype != want or out.stride(1) != 1 or s.out.shape[0] < rows:
             raise ValueError(f"linear: output of segment {i} must be {want} with at least {rows} rows of contiguous elements")
-        a.seg[i] = _native.Segment(out=s.out.buffer.data_ptr(), ld=s.out.buffer.stride(0), group=s.group, end=s.end,
-                                   kind=s.kind)
-    if residual is not None:
-        if residual.buffer.dtype != torch.float32:
-            raise ValueError("linear: the residual must be float32")
-        a.residual, a.ld_residual = residual.buffer.data_ptr(), residual.buffer.stride(0)
-    if bias is not None:
-        if bias.buffer.dtype != torch.float32 or bias.size < n:
-            raise ValueError(f"linear: the bias must be {n} float32 values")
-        a.bias = bias.buffer.data_ptr()
-    if group_rows is not None:
-        a.group_rows = group_rows.data_ptr()
+        outs.append((out.data_ptr(), out.stride(0), s.group, s.end, s.kind))
+    if residual is not None and residual.buffer.dtype != torch.float32:
+        raise ValueError("linear: the residual must be float32")
+    if bias is not None and (bias.buffer.dtype != torch.float32 or bias.size < n):
+        raise ValueError(f"linear: the bias must be {n} float32 values")
+    a = _native.linear_args(x.buffer.data_ptr(), w.buffer.data_ptr(), 0 if residual is None else residual.buffer.data_ptr(),
+                            0 if bias is None else bias.buffer.data_ptr(), 0 if group_rows is None else group_rows.data_ptr(), x.buffer.stride(0),
+                            group_x, w.buffer.stride(0), group_w, 0 if residual is None else residual.buffer.stride(0), outs, rows, k, n, groups,
+                            max_group_rows, dtype_code(x.buffer.dtype), path, limit)
     options = _AHEAD if ahead else None
     if group_x_rows is not None:
-        options = ctypes.byref(_native.LinearOptions(group_x_rows=group_x_rows.data_ptr(), x_rows=x.shape[0],
-                                                     flags=_native.LINEAR_AHEAD if ahead else 0))
+        options = _native.linear_options(group_x_rows.data_ptr(), x.shape[0], _native.LINEAR_AHEAD if ahead else 0)
     stream = batch_op_begin(ctx)
-    _native.check(_native.lib.b2kv_linear_opt(ctypes.byref(a), options, dev_status_ptr(ctx), stream))
+    _native.check(_native.lib.b2kv_linear_opt(a, options, dev_status_ptr(ctx), stream))
