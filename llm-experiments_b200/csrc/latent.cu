@@ -108,6 +108,98 @@ latent_append_kernel(T* y, int64_t ld_y, int H, int dim, int rot, int rot_dims, 
     for (int j = rot_dims + threadIdx.x; j < rot; j += kAppendThreads) key[j] = kr[j];
 }
 
+// The same with a warp per row, for many rows whose parts are all made of 16-byte pieces: nothing waits for a barrier, and every lane has
+// pieces of the queries and of the latent to move, where a CTA's threads are mostly idle (2975 rows, 16 heads of 64 rotated elements, latents of 512,
+// behind a product: 14 us, 27 with a CTA per row; without latents of its own 7 and 11).
+constexpr int kWarpHalf = 64, kWarpRows = kAppendThreads / 32;  // rotated pairs at most; rows per CTA
+
+template <typename T>
+__global__ void __launch_bounds__(kAppendThreads)
+latent_append_warps_kernel(T* y, int64_t ld_y, int H, int dim, int rot, int rot_dims, const float* inv_freq, int down_col, int kv_rank,
+                           const float* w_norm, float eps, T* key_cache, T* latent_cache, const int32_t* row_slot, const int32_t* row_pos,
+                           int n_slots, int T_max, int rows, int32_t* dev_status) {
+    constexpr int kC = Elt<T>::kPerChunk, kKeep = 4, kTogether = 4;
+    __shared__ float angle[kWarpRows][2][kWarpHalf];
+    grid_launch_dependents();
+    if (threadIdx.x == 0) grid_dependency_wait();
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = blockIdx.x * kWarpRows + warp;
+    if (r >= rows) return;
+    int slot, pos;
+    if (!row_place(row_slot, row_pos, r, n_slots, T_max, slot, pos)) {
+        if (lane == 0) report_status(dev_status, B2KV_DEV_BAD_POSITION);
+        return;
+    }
+    T* const row = y + static_cast<int64_t>(r) * ld_y;
+    const bool own = latent_cache != nullptr;
+    const int lat_pieces = own ? kv_rank / kC : 0, half = rot_dims / 2, pieces = half / kC;
+    const uint4* const lat = reinterpret_cast<const uint4*>(row + down_col);
+    uint4 keep[kKeep];
+#pragma unroll
+    for (int u = 0; u < kKeep; ++u)
+        if (lane + 32 * u < lat_pieces) keep[u] = lat[lane + 32 * u];
+    float* const cs = angle[warp][0];
+    float* const sn = angle[warp][1];
+    for (int j = lane; j < half; j += 32) sincosf(static_cast<float>(pos) * inv_freq[j], &sn[j], &cs[j]);
+    __syncwarp();
+    const int n = H * pieces;
+    for (int i0 = 0; i0 < n; i0 += 32 * kTogether) {
+        uint4 u4[kTogether], v4[kTogether];
+#pragma unroll
+        for (int t = 0; t < kTogether; ++t) {
+            const int i = i0 + 32 * t + lane;
+            if (i >= n) break;
+            const uint4* q = reinterpret_cast<const uint4*>(row + i / pieces * (dim + rot) + dim) + i % pieces;
+            u4[t] = q[0], v4[t] = q[pieces];
+        }
+#pragma unroll
+        for (int t = 0; t < kTogether; ++t) {
+            const int i = i0 + 32 * t + lane;
+            if (i >= n) break;
+            const int j = i % pieces;
+            uint4* q = reinterpret_cast<uint4*>(row + i / pieces * (dim + rot) + dim) + j;
+            rotate_pieces<T>(&u4[t], &v4[t], cs + j * kC, sn + j * kC);
+            q[0] = u4[t], q[pieces] = v4[t];
+        }
+    }
+    if (!own) return;
+    float sum = 0.f;
+    auto squares = [&](const uint4& p) {
+        float f[kC];
+        Elt<T>::widen(p, f);
+#pragma unroll
+        for (int e = 0; e < kC; ++e) sum = fmaf(f[e], f[e], sum);
+    };
+#pragma unroll
+    for (int u = 0; u < kKeep; ++u)
+        if (lane + 32 * u < lat_pieces) squares(keep[u]);
+    for (int i = lane + 32 * kKeep; i < lat_pieces; i += 32) squares(lat[i]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    const float scale = 1.0f / sqrtf(sum / static_cast<float>(kv_rank) + eps);
+    const int64_t place = static_cast<int64_t>(slot) * T_max + pos;
+    uint4* const latent = reinterpret_cast<uint4*>(latent_cache + place * kv_rank);
+    auto store = [&](int i, const uint4& p) {
+        float f[kC];
+        Elt<T>::widen(p, f);
+#pragma unroll
+        for (int e = 0; e < kC; ++e) f[e] = f[e] * scale * w_norm[i * kC + e];
+        latent[i] = narrow(f);
+    };
+#pragma unroll
+    for (int u = 0; u < kKeep; ++u)
+        if (lane + 32 * u < lat_pieces) store(lane + 32 * u, keep[u]);
+    for (int i = lane + 32 * kKeep; i < lat_pieces; i += 32) store(i, lat[i]);
+    const uint4* const kr = reinterpret_cast<const uint4*>(row + down_col + kv_rank);
+    uint4* const key = reinterpret_cast<uint4*>(key_cache + place * rot);
+    if (lane < pieces) {
+        uint4 u4 = kr[lane], v4 = kr[lane + pieces];
+        rotate_pieces<T>(&u4, &v4, cs + lane * kC, sn + lane * kC);
+        key[lane] = u4, key[lane + pieces] = v4;
+    }
+    for (int i = 2 * pieces + lane; i < rot / kC; i += 32) key[i] = kr[i];
+}
+
 // One CTA per (head, query row); its warps take the visible tokens in turn, each with an online softmax of its own, and
 // are merged at the end.  A lane holds kPer elements of the latent space.
 constexpr int kWarps = 4;
@@ -211,6 +303,20 @@ extern "C" int b2kv_latent_append(void* y, int64_t ld_y, int H, int dim, int rot
     if (latent_cache && (!w_norm || kv_rank <= 0 || down_col < 0 || ld_y < down_col + kv_rank + rot)) return B2KV_ERR_BAD_ARG;
     const int per = 16 / elt_bytes(dtype);
     const bool vec = aligned16(y) && ld_y % per == 0 && dim % per == 0 && rot % per == 0 && (rot_dims / 2) % per == 0;
+    // a warp per row where that gives every SM several rows (few rows: a CTA each is quicker, its threads share the row's pieces)
+    if (vec && rows >= 512 && rot_dims / 2 <= kWarpHalf && (rot_dims / 2) / per <= 32 &&
+        (latent_cache == nullptr || (kv_rank % per == 0 && down_col % per == 0 && aligned16(latent_cache) && aligned16(key_cache)))) {
+        OverlapLaunch warps((rows + kWarpRows - 1) / kWarpRows, kAppendThreads, 0, stream);
+        if (dtype == B2KV_DTYPE_F32)
+            B2KV_CUDA_TRY(cudaLaunchKernelEx(&warps.cfg, latent_append_warps_kernel<float>, static_cast<float*>(y), ld_y, H, dim, rot, rot_dims, inv_freq,
+                                             down_col, kv_rank, w_norm, eps, static_cast<float*>(key_cache), static_cast<float*>(latent_cache),
+                                             row_slot, row_pos, n_slots, T_max, rows, dev_status));
+        else
+            B2KV_CUDA_TRY(cudaLaunchKernelEx(&warps.cfg, latent_append_warps_kernel<__nv_bfloat16>, static_cast<__nv_bfloat16*>(y), ld_y, H, dim, rot,
+                                             rot_dims, inv_freq, down_col, kv_rank, w_norm, eps, static_cast<__nv_bfloat16*>(key_cache),
+                                             static_cast<__nv_bfloat16*>(latent_cache), row_slot, row_pos, n_slots, T_max, rows, dev_status));
+        return B2KV_OK;
+    }
     OverlapLaunch launch(rows, kAppendThreads, 0, stream);
     if (dtype == B2KV_DTYPE_F32)
         B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, latent_append_kernel<float>, static_cast<float*>(y), ld_y, H, dim, rot,

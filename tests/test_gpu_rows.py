@@ -1,0 +1,104 @@
+"""Row operations around the 32-bit residual stream against float64: one row, as many as fit the device together and more, widths around
+what a thread keeps in registers, odd ones and views with a pitch; the rotations and norms of latent rows by a CTA each and by a warp each."""
+import pytest
+import torch
+
+from tests.kv_util import make_ctx
+from tests.test_gpu_linear import rnd, wrap
+
+pytestmark = pytest.mark.gpu
+
+F32, BF = torch.float32, torch.bfloat16
+
+
+def b1(pkg, t):
+    return pkg.gpu.GPUBuffer1D(buffer=t, shape=tuple(t.shape), size=t.numel())
+
+
+def norm_close(got, want, dtype):
+    """fp32 sums of at most 8200 squares in any order, one rounding of the result."""
+    tol = dict(rtol=1e-5, atol=1e-5) if dtype == F32 else dict(rtol=2.0 ** -8, atol=2.0 ** -8)
+    torch.testing.assert_close(got.double(), want, **tol)
+
+
+@pytest.mark.parametrize("dtype", [F32, BF])
+@pytest.mark.parametrize("rows,size", [(1, 4), (7, 30), (64, 1024), (5, 1028), (3001, 36), (2500, 1023), (1700, 2048), (2, 4096), (700, 4100), (3, 8196)])
+def test_norms_of_any_number_of_rows(pkg, dtype, rows, size):
+    ctx = make_ctx(pkg)
+    x, w, b = rnd((rows + 3, size + 4), F32, 1)[:, :size] * 3 + 1, rnd((size,), F32, 2), rnd((size,), F32, 3)
+    index = torch.randperm(rows + 3, device="cuda")[:rows].to(torch.int32)
+    rms, ln, res = (torch.full((rows + 1, size + 4), 7.0, dtype=d, device="cuda") for d in (dtype, dtype, F32))
+    before = res[:rows, :size].normal_().double()
+    pkg.gpu.batch_begin(ctx)
+    pkg.gpu.rms_norm(ctx, wrap(pkg, x), b1(pkg, w), wrap(pkg, rms[:rows, :size]), 1e-5, weight_offset=1.0, row_index=index)
+    pkg.gpu.layernorm_rows(ctx, wrap(pkg, x), b1(pkg, w), b1(pkg, b), 1e-5, x=wrap(pkg, res[:rows, :size]), output=wrap(pkg, ln[:rows, :size]), row_index=index)
+    pkg.gpu.batch_commit(ctx)
+    y = x[index.long()].double()
+    norm_close(rms[:rows, :size], y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5) * (w.double() + 1), dtype)
+    want = before + torch.nn.functional.layer_norm(y, (size,), w.double(), b.double(), 1e-5)
+    norm_close(res[:rows, :size], want, F32)
+    norm_close(ln[:rows, :size], want, dtype)
+    assert all((t[rows] == 7).all() and (t[:, size:] == 7).all() for t in (rms, ln, res))
+
+
+@pytest.mark.parametrize("dtype", [F32, BF])
+@pytest.mark.parametrize("rows,dim", [(1, 4), (9, 36), (300, 2048), (3, 30), (1500, 1028)])
+def test_embedding_rows_of_any_width(pkg, dtype, rows, dim):
+    ctx = make_ctx(pkg)
+    table, ids = rnd((50, dim), dtype, 4), torch.randint(0, 50, (rows,), device="cuda", dtype=torch.int32)
+    out, copy = torch.empty((rows, dim), device="cuda"), torch.empty((rows, dim), dtype=dtype, device="cuda")
+    pkg.gpu.batch_begin(ctx)
+    pkg.gpu.embedding_rows(ctx, wrap(pkg, table), ids, wrap(pkg, out), scale=1.5, copy=wrap(pkg, copy))
+    pkg.gpu.batch_commit(ctx)
+    want = table[ids.long()].float() * 1.5
+    assert torch.equal(out, want) and torch.equal(copy, want.to(dtype))
+
+
+@pytest.mark.parametrize("dtype", [F32, BF])
+@pytest.mark.parametrize("H,rot,dims,rank,own", [(3, 64, 64, 512, True), (16, 32, 16, 72, True), (5, 128, 128, 1096, True), (2, 64, 48, 64, False)])
+def test_latent_rows_by_warps_and_by_ctas(pkg, dtype, H, rot, dims, rank, own):
+    """As many rows as take a warp each against the same ones in portions that take a CTA each: rotations and copies bit for bit."""
+    from llm_experiments_b200 import latent
+
+    ctx, rows, dim = make_ctx(pkg), 517, 24
+    ctx.config.check_device_status = True
+    shape = latent.LatentShape(H, dim, rot, dims, 8, rank, 0, 1.0)
+    y = rnd((rows, H * (dim + rot) + rank + rot + 8), dtype, 5)
+    w, inv = rnd((rank,), F32, 6) + 1, b1(pkg, 10000.0 ** (-torch.arange(dims // 2, device="cuda") / (dims // 2)))
+    pos, got = torch.randperm(600, device="cuda")[:rows].to(torch.int32), []
+    for step in (rows, 200):
+        cache = pkg.gpu.kv_cache_create(ctx, pkg.gpu.KVCacheConfig(batch_size=1, max_seq_len=600, n_layers=1, n_heads=1, head_dim=rot, v_head_dim=rank,
+                                                                   dtype=dtype, ragged=True))
+        mine = y.clone()
+        for r in range(0, rows, step):
+            part = mine[r:r + step]
+            pkg.gpu.batch_begin(ctx)
+            pkg.gpu.latent_append(ctx, wrap(pkg, part), shape, inv, latent.RowPlaces(torch.zeros(len(part), dtype=torch.int32, device="cuda"), pos[r:r + step]), cache,
+                                  b1(pkg, w) if own else None, 1e-5)
+            pkg.gpu.batch_commit(ctx)
+        got.append((mine, cache.layers[0].k_cache.buffer, cache.layers[0].v_cache.buffer))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    if own:
+        lat = y[:, H * (dim + rot):][:, :rank].double()
+        want = lat / torch.sqrt((lat * lat).mean(-1, keepdim=True) + 1e-5) * w.double()
+        for _, _, v in got:
+            norm_close(v.view(600, rank)[pos.long()], want, dtype)
+    else:
+        assert not got[0][2].any()
+
+
+def test_a_position_outside_the_cache_is_reported_among_many_rows(pkg):
+    from llm_experiments_b200 import latent
+
+    ctx, rows = make_ctx(pkg), 600
+    ctx.config.check_device_status = True
+    cache = pkg.gpu.kv_cache_create(ctx, pkg.gpu.KVCacheConfig(batch_size=1, max_seq_len=rows, n_layers=1, n_heads=1, head_dim=16, v_head_dim=64, dtype=BF, ragged=True))
+    y, pos = rnd((rows, 40 + 80), BF, 7), torch.arange(rows, dtype=torch.int32, device="cuda")
+    pos[300] = rows
+    pkg.gpu.batch_begin(ctx)
+    pkg.gpu.latent_append(ctx, wrap(pkg, y), latent.LatentShape(1, 24, 16, 16, 8, 64, 0, 1.0), b1(pkg, torch.ones(8, device="cuda")),
+                          latent.RowPlaces(torch.zeros(rows, dtype=torch.int32, device="cuda"), pos), cache, b1(pkg, torch.ones(64, device="cuda")), 1e-5)
+    with pytest.raises(RuntimeError, match="position"):
+        pkg.gpu.batch_commit(ctx)
+    filled = cache.layers[0].v_cache.buffer.view(rows, 64).any(dim=1)
+    assert not filled[300] and filled.sum() == rows - 1
