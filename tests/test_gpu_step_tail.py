@@ -174,3 +174,37 @@ def test_embedding_reports_ids_outside_the_table(pkg, ctx):
     finally:
         ctx.config.check_device_status = False
     assert torch.equal(out.buffer.cpu(), torch.ones((2, 8)))  # the bad id was clamped to row 0, nothing faulted
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,size", [(1, 2048), (8, 4096), (148, 2052), (149, 2052), (3, 8188), (2, 8196), (5, 6000)])
+def test_layernorm_of_few_wide_rows(pkg, ctx, dtype, n, size):
+    """A row per CTA of 512 threads, its edges in rows and in width, a guard behind."""
+    x = U.randn((n, size), dtype, ctx.device, 31) * 2 + 1
+    g, b = (U.randn((size,), dtype, ctx.device, s) for s in (32, 33))
+    out = torch.full((n + 1, size), 7.0, dtype=dtype, device=ctx.device)
+    one = lambda t: pkg.gpu.GPUBuffer1D(buffer=t, shape=tuple(t.shape), size=t.numel())  # noqa: E731
+    pkg.gpu.batch_begin(ctx)
+    pkg.gpu.layernorm(ctx, U.buf2d(pkg, ctx, x), one(g), one(b), U.buf2d(pkg, ctx, out[:n]))
+    pkg.gpu.batch_commit(ctx)
+    want = torch.nn.functional.layer_norm(x.double(), (size,), g.double(), b.double(), ctx.config.layernorm_epsilon)
+    tol = dict(rtol=1e-5, atol=1e-5) if dtype == torch.float32 else dict(rtol=2.0 ** -8, atol=2.0 ** -8)
+    torch.testing.assert_close(out[:n].double(), want, **tol)
+    assert (out[n] == 7).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("size", [1, 7, 1000, 1024, 4104, 32768, 40001])
+def test_argmax_of_any_width(pkg, ctx, dtype, size):
+    """Whole pieces and odd widths; equals anywhere, rows without a number, one number at the end."""
+    x = U.randn((5, size), dtype, ctx.device, 34)
+    x[1, size // 2:] = 9.0
+    x[2] = float("nan")
+    x[3] = float("-inf")
+    x[4, : size - 1] = float("nan")
+    out = torch.full((6,), -7, dtype=torch.int32, device=ctx.device)
+    pkg.gpu.batch_begin(ctx)
+    pkg.gpu.argmax(ctx, U.buf2d(pkg, ctx, x), pkg.gpu.GPUBuffer1D(buffer=out[:5], shape=(5,), size=5))
+    pkg.gpu.batch_commit(ctx)
+    first = int((x[0] == x[0].max()).nonzero()[0])
+    assert out.tolist() == [first, size // 2, 0, 0, size - 1, -7]
