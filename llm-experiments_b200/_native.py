@@ -124,6 +124,8 @@ SIGNATURES = {
     "b2kv_rmsnorm": (_i, [_vp, _i64, _vp, _vp, _f, _vp, _i64, _i, _i, _f, _i, _vp]),
     "b2kv_linear": (_i, [ctypes.POINTER(LinearArgs), _vp, _vp]),
     "b2kv_linear_opt": (_i, [ctypes.POINTER(LinearArgs), ctypes.POINTER(LinearOptions), _vp, _vp]),
+    "b2kv_linear_ws": (_i, [ctypes.POINTER(LinearArgs), ctypes.POINTER(LinearOptions), _vp, _sz, _vp, _vp]),
+    "b2kv_linear_workspace_bytes": (_sz, [ctypes.POINTER(LinearArgs)]),
     "b2kv_latent_append": (_i, [_vp, _i64, _i, _i, _i, _i, _vp, _i, _i, _vp, _f, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp]),
     "b2kv_latent_decode_workspace_bytes": (_sz, [_i, _i, _i, _i, _i]),
     "b2kv_latent_decode": (_i, [_vp, _vp, _i64, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp,

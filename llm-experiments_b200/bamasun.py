@@ -267,13 +267,13 @@ class BamasunState(SequenceState):
         for i, (lc, lw) in enumerate(zip(cfg.layers, w.layers)):
             mixed = _attend(ctx, self, i, xs, step) if lc.attention is not None else _recur(ctx, self, i, xs, step)
             y = self.rows("y", T, lw.w_o.shape[1], torch.float32)
-            linear(ctx, mixed, lw.w_o, mixed.shape[1], [OutputSegment(cfg.width, SEG_F32, y)], ahead=True)
+            linear(ctx, mixed, lw.w_o, mixed.shape[1], [OutputSegment(cfg.width, SEG_F32, y)], ahead=True, scratch=self.scratch)
             _add_normed(ctx, y, cfg, lw.norm1, x, copy)
             if lc.ff:
                 ff = lw.w_up.shape[1]
                 hidden = self.rows(f"hidden{ff}", T, ff, self.dtype)
-                linear(ctx, xs, lw.w_up, cfg.width, [OutputSegment(ff, SEG_RELU2, hidden)], ahead=True)
-                linear(ctx, hidden, lw.w_down, ff, [OutputSegment(cfg.width, SEG_F32, y)], ahead=True)
+                linear(ctx, xs, lw.w_up, cfg.width, [OutputSegment(ff, SEG_RELU2, hidden)], ahead=True, scratch=self.scratch)
+                linear(ctx, hidden, lw.w_down, ff, [OutputSegment(cfg.width, SEG_F32, y)], ahead=True, scratch=self.scratch)
                 _add_normed(ctx, y, cfg, lw.norm2, x, copy)
             if self.layer_tap is not None:
                 self.layer_tap.append(x.buffer.clone())
@@ -282,7 +282,7 @@ class BamasunState(SequenceState):
         hl = self.rows("h_out", step.n_out, cfg.width, self.dtype)
         layernorm_rows(ctx, x, w.final_norm.w, w.final_norm.b, cfg.eps, output=hl, row_index=step.row_index)
         out = self.rows("logits", step.n_out, cfg.vocab_size, torch.float32)
-        linear(ctx, hl, w.head, cfg.width, [OutputSegment(cfg.vocab_size, SEG_SOFTCAP, out)], limit=cfg.softcap, ahead=True)
+        linear(ctx, hl, w.head, cfg.width, [OutputSegment(cfg.vocab_size, SEG_SOFTCAP, out)], limit=cfg.softcap, ahead=True, scratch=self.scratch)
         self.logits = out
 
 
@@ -314,7 +314,7 @@ def _attend(ctx, state: BamasunState, i: int, xs: GPUBuffer2D, step: Step) -> GP
     a, cache = lc.attention, state.cache_of(i)
     y = state.rows(f"in{w.w_in.shape[1]}", T, w.w_in.shape[1], state.dtype)
     out = state.rows(f"mixed{w.w_o.shape[0]}", T, w.w_o.shape[0], state.dtype)
-    linear(ctx, xs, w.w_in, width, [OutputSegment(y.shape[1], SEG_STORE, y)], bias=w.bias, ahead=True)
+    linear(ctx, xs, w.w_in, width, [OutputSegment(y.shape[1], SEG_STORE, y)], bias=w.bias, ahead=True, scratch=state.scratch)
     gqa.gqa_append(ctx, y, a, step.places, cache, lc.kv_from is None, w.q_norm, w.k_norm, state.cfg.eps)
     if step.n_single:  # (prompt portions as well where they have no form of their own, in fp32 with many rows that share what they read)
         gqa.gqa_decode(ctx, sub(y, 0, step.n_single), a, w.slopes, step.single_places(), cache, sub(out, 0, step.n_single), step.span,
@@ -329,7 +329,7 @@ def _recur(ctx, state: BamasunState, i: int, xs: GPUBuffer2D, step: Step) -> GPU
     y = state.rows(f"in{w.w_in.shape[1]}", T, w.w_in.shape[1], state.dtype)
     alpha = state.rows(f"decay{w.w_a2.shape[1]}", T, w.w_a2.shape[1], torch.float32)
     out = state.rows(f"mixed{w.w_o.shape[0]}", T, w.w_o.shape[0], state.dtype)
-    linear(ctx, xs, w.w_in, width, [OutputSegment(y.shape[1], SEG_STORE, y)], ahead=True)
+    linear(ctx, xs, w.w_in, width, [OutputSegment(y.shape[1], SEG_STORE, y)], ahead=True, scratch=state.scratch)
     linear(ctx, sub(y, 0, T, w.cols[4]), w.w_a2, w.w_a2.shape[0], [OutputSegment(alpha.shape[1], SEG_DECAY, alpha)],
            limit=g.tau, bias=w.a2_bias, ahead=True)
     for segments in (step.short, step.long):

@@ -174,7 +174,19 @@ extern "C" int b2kv_linear(const b2kv_linear_args* args, int32_t* dev_status, vo
     return b2kv_linear_opt(args, nullptr, dev_status, stream);
 }
 
+// More than 16 rows of fp32: the tensor cores, unless there are too few input features to be worth the parts.
+static bool f32_on_tensor_cores(const b2kv_linear_args& a) { return a.path == 0 && a.dtype == B2KV_DTYPE_F32 && a.rows > 16 && a.K >= 128; }
+
 extern "C" int b2kv_linear_opt(const b2kv_linear_args* args, const b2kv_linear_options* options, int32_t* dev_status, void* stream) {
+    return b2kv_linear_ws(args, options, nullptr, 0, dev_status, stream);
+}
+
+extern "C" size_t b2kv_linear_workspace_bytes(const b2kv_linear_args* args) {
+    return args != nullptr && args->rows > 0 && args->N > 0 && f32_on_tensor_cores(*args) ? linear_f32_tc_workspace(*args) : 0;
+}
+
+extern "C" int b2kv_linear_ws(const b2kv_linear_args* args, const b2kv_linear_options* options, void* workspace,
+                              size_t workspace_bytes, int32_t* dev_status, void* stream) {
     if (args == nullptr) return B2KV_ERR_BAD_ARG;
     const b2kv_linear_args& a = *args;
     const b2kv_linear_options o = options != nullptr ? *options : b2kv_linear_options{};
@@ -210,8 +222,7 @@ extern "C" int b2kv_linear_opt(const b2kv_linear_args* args, const b2kv_linear_o
         if (rc != B2KV_ERR_UNSUPPORTED) return rc;
     }
     if (a.path == 0 && a.dtype == B2KV_DTYPE_F32) {
-        // many rows: the tensor cores, unless there are too few input features to be worth the parts
-        int rc = a.rows > 16 && a.K >= 128 ? linear_f32_tc(a, dev_status, stream) : B2KV_ERR_UNSUPPORTED;
+        int rc = f32_on_tensor_cores(a) ? linear_f32_tc(a, workspace, workspace_bytes, dev_status, stream) : B2KV_ERR_UNSUPPORTED;
         if (rc == B2KV_ERR_UNSUPPORTED) rc = linear_f32(a, stream);
         if (rc != B2KV_ERR_UNSUPPORTED) return rc;
     }

@@ -179,8 +179,9 @@ __device__ __forceinline__ void finish_pair(const b2kv_linear_args& a, int g, in
 
 // fp32 on the CUDA cores; B2KV_ERR_UNSUPPORTED where rows are not made of 16-byte pieces.
 int linear_f32(const b2kv_linear_args& a, void* stream);  // linear_f32.cu
-// fp32 on the tensor cores, operands in three bf16 parts; same contract.
-int linear_f32_tc(const b2kv_linear_args& a, int32_t* dev_status, void* stream);  // linear_f32_tc.cu
+// fp32 on the tensor cores, operands in three bf16 parts; same contract.  The parts are made ahead where there is scratch for them.
+int linear_f32_tc(const b2kv_linear_args& a, void* workspace, size_t workspace_bytes, int32_t* dev_status, void* stream);  // linear_f32_tc.cu
+size_t linear_f32_tc_workspace(const b2kv_linear_args& a);
 
 // bf16 kernels on the tensor cores; B2KV_ERR_UNSUPPORTED when the shape is not one they take.
 int linear_rows_tc(const b2kv_linear_args& a, int32_t* dev_status, void* stream);   // linear_rows.cu

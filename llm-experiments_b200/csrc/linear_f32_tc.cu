@@ -9,9 +9,12 @@
 // against 127 of linear_f32_tile_kernel; 3072 -> 768: 39 and 130; 60 rows, 768 -> 3072: 15 and 25.
 //
 //   * a CTA has 128 x 128 outputs; steps of 64 input features through two stages of 96 KB;
-//   * warps 8-15 read fp32 rows of x and w, a step ahead in registers, and write the parts as the operands the MMAs want: x K-major,
-//     w as it lies (MN-major), 128-byte swizzle;
-//   * a thread of warp 0 issues 24 tcgen05.mma per step: 6 x 64 clocks per 16 input features, a sixth of the tensor peak, which is
+//   * more than 128 rows, and scratch: the parts are made by a kernel ahead, once for all tiles (b2kv_linear_ws), and warp 8 copies them with
+//     TMA, warp 9 issues the products.  In the same kernel every row of tiles makes the parts of w and every column of tiles those of x
+//     again, which takes longer than the products (693 rows, 3072 -> 768: 36.8 us, 32.5 with the kernel ahead; 3000 rows, 1024 -> 4096: 205 and 157);
+//   * otherwise warps 8-15 read fp32 rows of x and w, a step ahead in registers, and write the parts as the operands the MMAs want: x K-major,
+//     w as it lies (MN-major), 128-byte swizzle; a thread of warp 0 issues the products;
+//   * 24 tcgen05.mma per step: 6 x 64 clocks per 16 input features, a sixth of the tensor peak, which is
 //     four times what the CUDA cores have.  Issuing takes as long as the products do, so it is not for the warps that make the parts
 //     (48 us with one of them), and a seventeenth warp would leave all others 96 registers (41 us, and spills);
 //   * warps 0-7 take the leading sums out (two accumulators in turn), thread = row and half of the columns, warp 0 always one step
@@ -29,6 +32,7 @@
 
 #include "linear.cuh"
 #include "tc_ptx.cuh"
+#include "tma_map.cuh"
 
 namespace b2kv {
 namespace linf32tc {
@@ -41,11 +45,21 @@ constexpr int kStageBytes = 6 * kPartBytes;         // x: h, m, l; w: h, m, l
 constexpr int kSumWarps = 8, kSplitWarps = 8;
 constexpr int kThreads = 32 * (kSumWarps + kSplitWarps);  // 128 registers each
 constexpr int kLdT = kBN + 4;                       // words per row of the tile of sums (over the stages, once they are free)
+constexpr int kMinTileSteps = 900;                  // tiles x steps from which a kernel ahead makes the parts
 constexpr int kMaxSplits = 8;                       // ranges of input features
 constexpr int kTmemCols = 512;                      // leading sums 2 x 128, the others 128
 constexpr int kColRest = 2 * kBN;
 constexpr size_t kSmem = kStages * kStageBytes + 1024;
 static_assert(kBM * kLdT * 4 <= kStages * kStageBytes, "the tile of sums fits the stages");
+
+// The parts of x and w in scratch memory, [3][rows][ldx] and [3][K][ldw] bf16, and per 128 x 64 piece of x and 64 x 128 piece of w whether it has
+// a number that three parts do not add up to.
+struct Parts {
+    uint16_t *x, *w;
+    int32_t *odd_x, *odd_w;  // [tiles_m][steps], [tiles_n][steps]
+    int ldx, ldw;
+};
+constexpr int pad8(int n) { return (n + 7) / 8 * 8; }
 
 struct Shared {
     alignas(8) uint64_t full[kStages], empty[kStages], sum_full[2], sum_empty[2], done;
@@ -56,13 +70,14 @@ struct Shared {
 
 // The three parts of four numbers, to `at` and one and two parts further on.  What two parts leave of a number is the third if its
 // lower 16 bits are zero; they are collected in `check` (those of what is not finite are set: infinity less infinity).
-__device__ __forceinline__ void split3(const float4& v, uint8_t* at, uint32_t& check) {
+template <typename Step = int>
+__device__ __forceinline__ void split3(const float4& v, uint8_t* at, uint32_t& check, Step part_bytes = kPartBytes) {
     const float2 minus = make_float2(-1.f, -1.f);
     float2 r0 = make_float2(v.x, v.y), r1 = make_float2(v.z, v.w);
 #pragma unroll
     for (int part = 0; part < 3; ++part) {
         const uint32_t a = pack_bf16(r0.x, r0.y), b = pack_bf16(r1.x, r1.y);
-        *reinterpret_cast<uint2*>(at + part * kPartBytes) = make_uint2(a, b);
+        *reinterpret_cast<uint2*>(at + part * part_bytes) = make_uint2(a, b);
         if (part == 2) break;
         r0 = __ffma2_rn(make_float2(__uint_as_float(a << 16), __uint_as_float(a & 0xffff0000u)), minus, r0);
         r1 = __ffma2_rn(make_float2(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u)), minus, r1);
@@ -72,6 +87,38 @@ __device__ __forceinline__ void split3(const float4& v, uint8_t* at, uint32_t& c
 __device__ __forceinline__ bool has_no_parts(float v) {
     const float r = v - __bfloat162float(__float2bfloat16_rn(v));
     return (__float_as_uint(r - __bfloat162float(__float2bfloat16_rn(r))) & 0xffffu) != 0 || !(fabsf(v) < INFINITY);
+}
+
+// One CTA per piece of x (the first tiles_m * steps CTAs) or of w.
+constexpr int kMakeThreads = 256;
+__global__ void __launch_bounds__(kMakeThreads) make_parts_kernel(const __grid_constant__ b2kv_linear_args a, const __grid_constant__ Parts p, int pieces_x) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int steps = (a.K + kBK - 1) / kBK;
+    const bool of_x = static_cast<int>(blockIdx.x) < pieces_x;
+    const int piece = of_x ? blockIdx.x : blockIdx.x - pieces_x, step = piece % steps, tile = piece / steps;
+    const float* const src = static_cast<const float*>(of_x ? a.x : a.w);
+    const int64_t ld = of_x ? a.ld_x : a.ld_w;
+    const int row0 = of_x ? tile * kBM : step * kBK, col0 = of_x ? step * kBK : tile * kBN;
+    const int n_rows = of_x ? min(kBM, a.rows - row0) : min(kBK, a.K - row0), n_cols = of_x ? min(kBK, a.K - col0) : min(kBN, a.N - col0);
+    uint16_t* const out = of_x ? p.x : p.w;
+    const int out_ld = of_x ? p.ldx : p.ldw, shift = of_x ? 4 : 5;  // 16-byte pieces per row of the piece: 64 / 4, 128 / 4
+    const int64_t part_bytes = static_cast<int64_t>(of_x ? a.rows : a.K) * out_ld * 2;
+    float4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int e = i * kMakeThreads + threadIdx.x, r = e >> shift, c = (e & ((1 << shift) - 1)) * 4;
+        v[i] = r < n_rows && c < n_cols ? *reinterpret_cast<const float4*>(src + (row0 + r) * ld + col0 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    uint32_t check = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int e = i * kMakeThreads + threadIdx.x, r = e >> shift, c = (e & ((1 << shift) - 1)) * 4;
+        if (r < n_rows && c < n_cols)
+            split3(v[i], reinterpret_cast<uint8_t*>(out + static_cast<int64_t>(row0 + r) * out_ld + col0 + c), check, part_bytes);
+    }
+    const int odd = __syncthreads_or((check & 0xffffu) != 0);
+    if (threadIdx.x == 0) (of_x ? p.odd_x : p.odd_w)[piece] = odd;
 }
 
 // The sums of the input features [k_first, k_end) that need it, again: all threads, the tile of sums and the stages behind it.
@@ -139,14 +186,18 @@ __device__ __noinline__ float sum_in_order(const float* row, const float* col, i
     return sum;
 }
 
-__global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid_constant__ b2kv_linear_args a, int splits, int32_t* dev_status) {
+// kMade: the parts are in scratch memory.
+template <bool kMade>
+__global__ void __launch_bounds__(kThreads, 1)
+linear_f32_tc_kernel(const __grid_constant__ b2kv_linear_args a, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
+                     const __grid_constant__ Parts p, int splits, int32_t* dev_status) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ Shared sm;
     uint8_t* const ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = blockIdx.z;
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
-            mbar_init(&sm.full[s], kSplitWarps);
+            mbar_init(&sm.full[s], kMade ? 1 : kSplitWarps);
             mbar_init(&sm.empty[s], 1);
         }
         for (int s = 0; s < 2; ++s) {
@@ -176,6 +227,32 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
     const int steps = static_cast<int>(static_cast<long long>(all_steps) * (split + 1) / splits) - step0;
     const int k_first = step0 * kBK, k_end = min(a.K, (step0 + steps) * kBK);
 
+    // the products of step s, once all parts are there and the sums of the step before last are taken out
+    auto issue = [&](int s) {
+        constexpr uint32_t idesc = instr_desc(0, 1, kBN);
+        constexpr uint64_t kPart = kPartBytes >> 4;
+        const int st = s % kStages;
+        if (!mbar_wait(&sm.full[st], (s / kStages) & 1) || !mbar_wait(&sm.sum_empty[s & 1], ((s >> 1) & 1) ^ 1)) return false;
+        tc_fence_after();
+        const uint64_t dx = smem_desc(smem_u32(ring + st * kStageBytes), 16, 1024);
+        const uint64_t dw = smem_desc(smem_u32(ring + st * kStageBytes + 3 * kPartBytes), kBK * 128, 1024);
+#pragma unroll
+        for (int kk = 0; kk < kBK / 16; ++kk)  // 16 input features: 32 bytes of x's rows, 16 rows of w
+            mma_ss(tmem + (s & 1) * kBN, dx + 2 * kk, dw + 128 * kk, idesc, kk ? 1u : 0u);
+        mma_commit(&sm.sum_full[s & 1]);
+#pragma unroll
+        for (int kk = 0; kk < kBK / 16; ++kk) {
+            const uint64_t ax = dx + 2 * kk, bw = dw + 128 * kk;
+            mma_ss(tmem + kColRest, ax, bw + 2 * kPart, idesc, (s | kk) ? 1u : 0u);
+            mma_ss(tmem + kColRest, ax + 2 * kPart, bw, idesc, 1u);
+            mma_ss(tmem + kColRest, ax + kPart, bw + kPart, idesc, 1u);
+            mma_ss(tmem + kColRest, ax, bw + kPart, idesc, 1u);
+            mma_ss(tmem + kColRest, ax + kPart, bw, idesc, 1u);
+        }
+        mma_commit(&sm.empty[st]);
+        if (s + 1 == steps) mma_commit(&sm.done);
+        return true;
+    };
     float acc[64];
     if (warp < kSumWarps) {
         // ------------------------------ sums: thread = row, half of the columns ------------------------------
@@ -192,34 +269,8 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
                 for (int j = 0; j < 32; ++j) acc[half * 32 + j] += __uint_as_float(r[j]);
             }
         };
-        // the products of step s, once all parts are written and the sums of the step before last are taken out
-        auto issue = [&](int s) {
-            constexpr uint32_t idesc = instr_desc(0, 1, kBN);
-            constexpr uint64_t kPart = kPartBytes >> 4;
-            const int st = s % kStages;
-            if (!mbar_wait(&sm.full[st], (s / kStages) & 1) || !mbar_wait(&sm.sum_empty[s & 1], ((s >> 1) & 1) ^ 1)) return false;
-            tc_fence_after();
-            const uint64_t dx = smem_desc(smem_u32(ring + st * kStageBytes), 16, 1024);
-            const uint64_t dw = smem_desc(smem_u32(ring + st * kStageBytes + 3 * kPartBytes), kBK * 128, 1024);
-#pragma unroll
-            for (int kk = 0; kk < kBK / 16; ++kk)  // 16 input features: 32 bytes of x's rows, 16 rows of w
-                mma_ss(tmem + (s & 1) * kBN, dx + 2 * kk, dw + 128 * kk, idesc, kk ? 1u : 0u);
-            mma_commit(&sm.sum_full[s & 1]);
-#pragma unroll
-            for (int kk = 0; kk < kBK / 16; ++kk) {
-                const uint64_t ax = dx + 2 * kk, bw = dw + 128 * kk;
-                mma_ss(tmem + kColRest, ax, bw + 2 * kPart, idesc, (s | kk) ? 1u : 0u);
-                mma_ss(tmem + kColRest, ax + 2 * kPart, bw, idesc, 1u);
-                mma_ss(tmem + kColRest, ax + kPart, bw + kPart, idesc, 1u);
-                mma_ss(tmem + kColRest, ax, bw + kPart, idesc, 1u);
-                mma_ss(tmem + kColRest, ax + kPart, bw, idesc, 1u);
-            }
-            mma_commit(&sm.empty[st]);
-            if (s + 1 == steps) mma_commit(&sm.done);
-            return true;
-        };
         auto issue_by_warp0 = [&](int s) {
-            if (warp != 0 || s >= steps) return true;
+            if (kMade || warp != 0 || s >= steps) return true;
             bool good = true;
             if (lane == 0) good = issue(s);
             return __all_sync(0xffffffffu, good) != 0;
@@ -240,6 +291,35 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
             ok = __all_sync(0xffffffffu, mbar_wait(&sm.done, 0));
             tc_fence_after();
             if (ok) add(t_lane + kColRest);
+        }
+        if (!ok) sm.abort_flag = 1;
+    } else if (kMade) {
+        bool ok = true;
+        if (warp == kSumWarps) {
+            // ------------------------------ copies of the parts ------------------------------
+            if (lane == 0) {
+                for (int s = 0; s < steps && ok; ++s) {
+                    const int st = s % kStages, k = k_first + s * kBK;
+                    ok = mbar_wait(&sm.empty[st], ((s / kStages) & 1) ^ 1);
+                    if (!ok) break;
+                    mbar_arrive_expect_tx(&sm.full[st], kStageBytes);
+                    uint8_t* const to = ring + st * kStageBytes;
+#pragma unroll
+                    for (int part = 0; part < 3; ++part) {
+                        tma_load_3d(to + part * kPartBytes, &tm_x, &sm.full[st], k, row0, part);
+                        tma_load_3d(to + (3 + part) * kPartBytes, &tm_w, &sm.full[st], col0, k, part);
+                        tma_load_3d(to + (3 + part) * kPartBytes + kBK * 128, &tm_w, &sm.full[st], col0 + 64, k, part);
+                    }
+                }
+            }
+            __syncwarp();
+        } else if (warp == kSumWarps + 1) {
+            if (lane == 0)
+                for (int s = 0; s < steps && ok; ++s) ok = issue(s);
+            __syncwarp();
+        } else if (warp == kSumWarps + 2) {
+            for (int s = lane; s < steps; s += 32)
+                if (p.odd_x[blockIdx.y * all_steps + step0 + s] | p.odd_w[col0 / kBN * all_steps + step0 + s]) sm.odd = 1;
         }
         if (!ok) sm.abort_flag = 1;
     } else {
@@ -353,11 +433,45 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_tc_kernel(const __grid
 
 }  // namespace linf32tc
 
-int linear_f32_tc(const b2kv_linear_args& a, int32_t* dev_status, void* stream) {
+// Scratch of the parts: none where they are made in the products' kernel.
+static size_t parts_bytes(const b2kv_linear_args& a, linf32tc::Parts* p, void* at) {
     using namespace linf32tc;
-    if (a.dtype != B2KV_DTYPE_F32 || a.group_rows != nullptr) return B2KV_ERR_UNSUPPORTED;
-    if (!aligned16(a.x) || !aligned16(a.w) || a.K % 4 || a.N % 4 || a.ld_x % 4 || a.ld_w % 4 || a.group_x % 4 || a.group_w % 4)
-        return B2KV_ERR_UNSUPPORTED;
+    // The tiles make more of the same parts the more of them there are: 36 tiles of 12 steps 16.2 us and 18.6 with the kernel ahead, 60 of 12
+    // 19.9 and 21.3, 78 of 12 29.5 and 26.0, 144 of 12 30.4 and 27.6, 36 of 48 36.8 and 32.5, 96 of 16 37.2 and 31.4, 768 of 16 205 and 157.
+    const long long tiles = static_cast<long long>((a.rows + kBM - 1) / kBM) * ((a.N + kBN - 1) / kBN);
+    if (a.rows <= kBM || a.groups > 1 || tiles * ((a.K + kBK - 1) / kBK) < kMinTileSteps) return 0;
+    const size_t steps = (a.K + kBK - 1) / kBK, tiles_m = (a.rows + kBM - 1) / kBM, tiles_n = (a.N + kBN - 1) / kBN;
+    const size_t ldx = pad8(a.K), ldw = pad8(a.N), x = 3 * static_cast<size_t>(a.rows) * ldx, w = 3 * static_cast<size_t>(a.K) * ldw;
+    if (p != nullptr) {
+        p->x = static_cast<uint16_t*>(at), p->w = p->x + x;
+        p->odd_x = reinterpret_cast<int32_t*>(p->w + w), p->odd_w = p->odd_x + tiles_m * steps;
+        p->ldx = static_cast<int>(ldx), p->ldw = static_cast<int>(ldw);
+    }
+    return (x + w) * 2 + (tiles_m + tiles_n) * steps * sizeof(int32_t);
+}
+
+// Three matrices of rows x cols bf16, boxes of box_rows x 64 of one of them, 128-byte swizzle; zero outside.
+static bool make_parts_map(CUtensorMap* map, const uint16_t* base, int rows, int cols, int ld, int box_rows) {
+    EncodeTiledFn fn = tensor_map_encoder();
+    if (fn == nullptr) return false;
+    const cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows), 3};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * 2, static_cast<cuuint64_t>(ld) * 2 * static_cast<cuuint64_t>(rows)};
+    const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<uint16_t*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+static bool f32_tc_takes(const b2kv_linear_args& a) {
+    return a.dtype == B2KV_DTYPE_F32 && a.group_rows == nullptr && aligned16(a.x) && aligned16(a.w) && a.K % 4 == 0 && a.N % 4 == 0 && a.ld_x % 4 == 0 &&
+           a.ld_w % 4 == 0 && a.group_x % 4 == 0 && a.group_w % 4 == 0;
+}
+
+size_t linear_f32_tc_workspace(const b2kv_linear_args& a) { return f32_tc_takes(a) ? parts_bytes(a, nullptr, nullptr) : 0; }
+
+int linear_f32_tc(const b2kv_linear_args& a, void* workspace, size_t workspace_bytes, int32_t* dev_status, void* stream) {
+    using namespace linf32tc;
+    if (!f32_tc_takes(a)) return B2KV_ERR_UNSUPPORTED;
     const long long tiles_m = (a.rows + kBM - 1) / kBM, tiles_n = (a.N + kBN - 1) / kBN, tiles = tiles_m * tiles_n * a.groups;
     const int steps = (a.K + kBK - 1) / kBK;
     static bool configured[64] = {false};
@@ -366,12 +480,13 @@ int linear_f32_tc(const b2kv_linear_args& a, int32_t* dev_status, void* stream) 
     B2KV_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return B2KV_ERR_UNSUPPORTED;
     if (!configured[dev]) {
-        B2KV_CUDA_TRY(cudaFuncSetAttribute(linear_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem)));
+        B2KV_CUDA_TRY(cudaFuncSetAttribute(linear_f32_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem)));
+        B2KV_CUDA_TRY(cudaFuncSetAttribute(linear_f32_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem)));
         clusters[dev][1] = device_sm_count();
         for (int s = 2; s <= kMaxSplits; ++s) {
             OverlapLaunch most(static_cast<unsigned>(s * device_sm_count()), kThreads, kSmem, stream, s);
             most.cfg.numAttrs = 1;  // the cluster
-            if (cudaOccupancyMaxActiveClusters(&clusters[dev][s], linear_f32_tc_kernel, &most.cfg) != cudaSuccess) {
+            if (cudaOccupancyMaxActiveClusters(&clusters[dev][s], linear_f32_tc_kernel<false>, &most.cfg) != cudaSuccess) {
                 (void)cudaGetLastError();
                 clusters[dev][s] = 0;
             }
@@ -390,7 +505,19 @@ int linear_f32_tc(const b2kv_linear_args& a, int32_t* dev_status, void* stream) 
     if (tune_get("matmul_splits") > 0) splits = std::min(tune_get("matmul_splits"), kMaxSplits);
     if (tiles_m > 65535 || a.groups > 65535 || tiles_n * splits > 0x7fffffffLL) return B2KV_ERR_UNSUPPORTED;
     OverlapLaunch launch(dim3(static_cast<unsigned>(tiles_n * splits), static_cast<unsigned>(tiles_m), a.groups), kThreads, kSmem, stream, splits);
-    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, linear_f32_tc_kernel, a, splits, dev_status));
+    Parts parts{};
+    CUtensorMap tx{}, tw{};
+    const size_t need = workspace != nullptr && aligned16(workspace) ? parts_bytes(a, &parts, workspace) : 0;
+    if (need > 0 && workspace_bytes >= need && make_parts_map(&tx, parts.x, a.rows, a.K, parts.ldx, kBM) &&
+        make_parts_map(&tw, parts.w, a.K, a.N, parts.ldw, kBK)) {
+        const long long pieces_x = tiles_m * steps, pieces = pieces_x + tiles_n * steps;
+        if (pieces > 0x7fffffffLL) return B2KV_ERR_UNSUPPORTED;
+        OverlapLaunch make(static_cast<unsigned>(pieces), kMakeThreads, 0, stream);
+        B2KV_CUDA_TRY(cudaLaunchKernelEx(&make.cfg, make_parts_kernel, a, parts, static_cast<int>(pieces_x)));
+        B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, linear_f32_tc_kernel<true>, a, tx, tw, parts, splits, dev_status));
+        return B2KV_OK;
+    }
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, linear_f32_tc_kernel<false>, a, tx, tw, parts, splits, dev_status));
     return B2KV_OK;
 }
 

@@ -245,7 +245,7 @@ class GigezenState(SequenceState):
         hl = self.rows("h_out", step.n_out, cfg.width, self.dtype)
         rms_norm(ctx, x, w.final_norm, hl, cfg.eps, weight_offset=1.0, row_index=step.row_index)
         out = self.rows("logits", step.n_out, cfg.vocab_size, torch.float32)
-        linear(ctx, hl, w.head, cfg.width, [OutputSegment(cfg.vocab_size, SEG_F32, out)], ahead=True)
+        linear(ctx, hl, w.head, cfg.width, [OutputSegment(cfg.vocab_size, SEG_F32, out)], ahead=True, scratch=self.scratch)
         self.logits = out
 
 
@@ -295,14 +295,14 @@ def _layer(ctx, state: GigezenState, i: int, x: GPUBuffer2D, step: Step) -> None
         segments.append(OutputSegment(w.y_cols + w.router_cols, SEG_F32, logits))
     if lc.dense_ff:
         segments.append(OutputSegment(w.y_cols + 2 * w.ff_cols, SEG_GLU_CLAMP, _sub(z, 0, T, w.a_cols)))
-    linear(ctx, h, w.w_in, cfg.width, segments, limit=lc.limit, ahead=True)
+    linear(ctx, h, w.w_in, cfg.width, segments, limit=lc.limit, ahead=True, scratch=state.scratch)
     latent.latent_append(ctx, y, a, w.inv_freq, step.places, cache, w.latent_norm, cfg.eps)
     n_single = step.n_single
     if n_single:
         _attend_rows(ctx, state, i, _sub(y, 0, n_single), _sub(z, 0, n_single, 0, a.heads * a.vdim), step.single_places(), step.span)
     if step.plans:
         _attend_prompts(ctx, state, i, y, _sub(z, 0, T, 0, a.heads * a.vdim), step.plans[a.window])
-    linear(ctx, z, w.w_out, w.a_cols + w.ff_cols, [OutputSegment(cfg.width, SEG_F32, x)], residual=x, ahead=True)
+    linear(ctx, z, w.w_out, w.a_cols + w.ff_cols, [OutputSegment(cfg.width, SEG_F32, x)], residual=x, ahead=True, scratch=state.scratch)
     if lc.router:
         moe.moe_feed_forward(ctx, h, logits, w.experts, lc.router, _moe_scratch(state, lc, w, T), x)
     if state.layer_tap is not None:

@@ -11,7 +11,7 @@ the cache.  Checks and texts follow ``kv_cache_update``; bf16 caches with a cont
 from __future__ import annotations
 
 from dataclasses import dataclass
-from typing import Optional, Sequence
+from typing import Dict, Optional, Sequence
 
 import torch
 
@@ -127,7 +127,7 @@ def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Se
            residual: Optional[GPUBuffer2D] = None, limit: float = 0.0, groups: int = 1, group_x: int = 0, group_w: int = 0,
            group_rows: Optional[torch.Tensor] = None, max_group_rows: int = 0, path: int = 0,
            bias: Optional[GPUBuffer1D] = None, group_x_rows: Optional[torch.Tensor] = None, rows: Optional[int] = None,
-           ahead: bool = False) -> None:
+           ahead: bool = False, scratch: Optional[Dict[str, torch.Tensor]] = None) -> None:
     """``x @ w`` (``+ bias``, fp32) with the output columns cut into segments, fp32 or bfloat16 storage, any sizes (``b2kv_linear``).
 
     ``x`` ``[rows, >= k]`` and ``w`` (rows of the weight matrix, ``[in, out]``) may be views with a row pitch.  With
@@ -140,7 +140,10 @@ def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Se
 
     Products of at most 128 bfloat16 rows read the first tiles of ``w`` before the kernel ahead of them has ended.  So ``w`` may be
     the output of a product of more rows, but not of one whose caller said ``ahead``: that none of its outputs is a ``w`` and the
-    kernel behind it may start early; nor, right behind it, of a product of at most 128 rows."""
+    kernel behind it may start early; nor, right behind it, of a product of at most 128 rows.
+
+    ``scratch`` (of one model's steps, one after the other) keeps the memory in which float32 products of more than 128 rows lay
+    their operands out once; without it they do so tile by tile."""
     rows, n = x.shape[0] if group_x_rows is None else rows, segments[-1].end
     if rows <= 0 or k <= 0 or n <= 0:
         raise ValueError(f"linear: Invalid dimensions x=({rows}, {k}), w=({k}, {n})")
@@ -166,5 +169,13 @@ def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Se
     options = _AHEAD if ahead else None
     if group_x_rows is not None:
         options = _native.linear_options(group_x_rows.data_ptr(), x.shape[0], _native.LINEAR_AHEAD if ahead else 0)
+    ws = None
+    if scratch is not None and rows > 128 and x.buffer.dtype == torch.float32:
+        nbytes = _native.lib.b2kv_linear_workspace_bytes(a)
+        if nbytes:
+            ws = scratch.get("linear")
+            if ws is None or ws.numel() < nbytes:
+                ws = scratch["linear"] = torch.empty(nbytes, dtype=torch.uint8, device=x.buffer.device)
     stream = batch_op_begin(ctx)
-    _native.check(_native.lib.b2kv_linear_opt(a, options, dev_status_ptr(ctx), stream))
+    _native.check(_native.lib.b2kv_linear_ws(a, options, None if ws is None else ws.data_ptr(), 0 if ws is None else ws.numel(),
+                                             dev_status_ptr(ctx), stream))

@@ -188,3 +188,37 @@ def test_operands_of_any_size(pkg, rows, K, sx, sw):
     """Down to subnormal numbers, whose parts bf16 does not hold: the bound of fp32 sums."""
     x, w = rnd((rows, K), F32, 21, sx), rnd((K, 200), F32, 22, sw)
     bounded(product(pkg, make_ctx(pkg), x, w), x, w)
+
+
+@pytest.mark.parametrize("rows,K,n", [(693, 768, 3072), (1300, 1040, 644), (130, 16388, 388), (2100, 132, 2500)])
+def test_parts_made_ahead_have_the_same_bits(pkg, rows, K, n):
+    """With scratch memory the operands of large products are laid out by a kernel ahead: the same numbers, also where some have no parts,
+    and in a scratch that another product left full of its own."""
+    from llm_experiments_b200 import projection as proj
+
+    ctx = make_ctx(pkg)
+    x, w, bias = rnd((rows, K + 4), F32, 21)[:, :K], rnd((K, n + 4), F32, 22, K ** -0.5)[:, :n], rnd((n,), F32, 23)
+    scratch = {"linear": torch.full((1 << 27,), 0x7f, dtype=torch.uint8, device="cuda")}
+    for odd in (False, True):
+        if odd:
+            x[5, 7], x[rows - 1, K - 1], w[3, n - 1], w[K - 1, 0], x[9, 11] = float("inf"), 1e-39, float("nan"), 3.4e38, -2e-36
+        out = [torch.full((rows + 1, n + 1), 7.0, dtype=F32, device="cuda") for _ in range(2)]
+        for o, s in zip(out, (None, scratch)):
+            run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), K, [proj.OutputSegment(n, proj.SEG_STORE, wrap(pkg, o[:, :n]))], scratch=s,
+                bias=pkg.gpu.GPUBuffer1D(buffer=bias, shape=(n,), size=n))
+        assert torch.equal(out[0].view(torch.int32), out[1].view(torch.int32))
+        if not odd:
+            bounded(out[1][:rows, :n], x, w, bias.double())
+
+
+def test_scratch_grows_and_is_left_alone_where_it_is_of_no_use(pkg):
+    from llm_experiments_b200 import projection as proj
+
+    ctx, scratch, sizes = make_ctx(pkg), {}, []
+    for rows, K, n in ((100, 1024, 1024), (300, 256, 64), (1200, 1024, 1024), (1100, 1024, 1024), (2000, 1024, 1024)):
+        x, w = rnd((rows, K), F32, 24), rnd((K, n), F32, 25, K ** -0.5)
+        out = torch.empty((rows, n), dtype=F32, device="cuda")
+        run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), K, [proj.OutputSegment(n, proj.SEG_STORE, wrap(pkg, out))], scratch=scratch)
+        bounded(out, x, w)
+        sizes.append(scratch["linear"].numel() if scratch else 0)
+    assert sizes[0] == sizes[1] == 0 and 0 < sizes[2] == sizes[3] < sizes[4]
