@@ -245,3 +245,47 @@ def test_segments_outside_the_buffers_are_refused(pkg):
         for seg in ((0, 21, 0), (5, 16, 0), (0, 20, 1), (-1, 4, 0)):
             with pytest.raises(RuntimeError, match="position"):
                 layer.run(y, al, [seg], range(20), layer.states(1), path)
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 24, 40), (3, 128, 256), (2, 64, 72)])
+def test_spans_of_chunks(pkg, heads, dim, vdim):
+    """Lengths around one span and two (a span is 256 tokens), in the company of each other and of short ones, then each continued by a portion
+    of another length: the outputs and states of the equations, and alone the same bits."""
+    layer = Layer(pkg, heads, dim, vdim, 16.0, BF, z_mean=2.0, z_std=1.0, seed=17)
+    first, then = (255, 256, 257, 511, 513, 30, 770), (300, 17, 256, 1, 273, 520, 16)
+    state, alone, last = layer.states(len(first)), [layer.states(1) for _ in first], [None] * len(first)
+    for lens, start in ((first, [0] * len(first)), (then, first)):
+        y, al = layer.rows(sum(lens))
+        segments = [(sum(lens[:i]), n, i) for i, n in enumerate(lens)]
+        got = layer.run(y, al, segments, np.concatenate([s + np.arange(n) for s, n in zip(start, lens)]), state, CHUNK)
+        for (r0, n, i), s in zip(segments, start):
+            part = slice(r0, r0 + n)
+            assert np.array_equal(layer.run(y[part], al[part], [(0, n, 0)], s + np.arange(n), alone[i], CHUNK), got[part]), (n, s)
+            assert torch.equal(alone[i][0], state[i]), (n, s)
+            want, last[i] = layer.want(y[part], al[part], last[i])
+            close(got[part], want, BF, (n, s))
+            state_close(state[i], last[i])
+
+
+def test_spans_over_slices_of_a_bounded_workspace(pkg):
+    """Many sequences of several spans, which one slice of the workspace does not hold: the bits of each alone."""
+    layer = Layer(pkg, 8, 128, 256, 16.0, BF, z_mean=2.0, z_std=1.0, seed=19)
+    lens = (700, 513, 300) * 8
+    y, al = layer.rows(sum(lens))
+    segments, pos = [(sum(lens[:i]), n, i) for i, n in enumerate(lens)], np.concatenate([np.arange(n) for n in lens])
+    state = layer.states(len(lens))
+    got = layer.run(y, al, segments, pos, state, CHUNK)
+    for r0, n, slot in segments[:3] + segments[-3:]:
+        alone = layer.states(1)
+        assert np.array_equal(layer.run(y[r0:r0 + n], al[r0:r0 + n], [(0, n, 0)], range(n), alone, CHUNK), got[r0:r0 + n]), n
+        assert torch.equal(alone[0], state[slot]), n
+
+
+def test_an_infinite_state_is_not_turned_into_nan_by_a_span(pkg):
+    """Decays whose product over a span is below the smallest number: what is infinite stays so."""
+    layer = Layer(pkg, 1, 16, 32, 1.0, BF, z_mean=-0.7, z_std=0.0, seed=23)
+    y, al = layer.rows(600)
+    state = torch.ones((1, 1, 16, 32), device="cuda")
+    state[0, 0, 3, 5] = float("inf")
+    layer.run(y, al, [(0, 600, 0)], 10 + np.arange(600), state, CHUNK)
+    assert torch.isinf(state[0, 0, 3, 5]) and torch.isfinite(state).sum() == 16 * 32 - 1
