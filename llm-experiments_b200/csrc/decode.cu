@@ -25,6 +25,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 
@@ -163,20 +164,7 @@ constexpr int kMaxPiecesPerPair = 16;          // ... and so is a batch whose lo
 // rounding adds, a small chunk at least a thirty-second of an equal share).
 __host__ __device__ constexpr int max_chunks(int n_ctas) { return n_ctas * (2 + kChunksPerShare * (kStaticDen - kStaticNum) / kStaticDen) + 2; }
 
-// Every thread of the calling warp takes part (the lengths are summed across the lanes).
-__device__ __forceinline__ Geometry geometry_of(const DecodeParams& p, int n_ctas, int tile, int lane) {
-    long long sum = 0;
-    int longest = 0;
-    for (int b = lane; b < p.B; b += 32) {
-        const int n = seq_len_of(p, b);
-        sum += n;
-        longest = max(longest, n);
-    }
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
-        sum += __shfl_xor_sync(0xffffffffu, sum, off);
-        longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, off));
-    }
+__device__ __forceinline__ Geometry cut(const DecodeParams& p, long long sum, int longest, int n_ctas, int tile) {
     Geometry ge;
     ge.total = sum * p.H;
     const long long per = (ge.total + n_ctas - 1) / n_ctas;  // an equal share
@@ -194,6 +182,23 @@ __device__ __forceinline__ Geometry geometry_of(const DecodeParams& p, int n_cta
     ge.a_end = min(static_cast<long long>(n_ctas) * ge.sa, ge.total);
     ge.n_chunks = n_ctas + static_cast<int>((ge.total - ge.a_end + ge.sb - 1) / ge.sb);
     return ge;
+}
+
+// Every thread of the calling warp takes part (the lengths are summed across the lanes).
+__device__ __forceinline__ Geometry geometry_of(const DecodeParams& p, int n_ctas, int tile, int lane) {
+    long long sum = 0;
+    int longest = 0;
+    for (int b = lane; b < p.B; b += 32) {
+        const int n = seq_len_of(p, b);
+        sum += n;
+        longest = max(longest, n);
+    }
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, off));
+    }
+    return cut(p, sum, longest, n_ctas, tile);
 }
 
 __device__ __forceinline__ void chunk_range(const Geometry& ge, long long g, long long& start, long long& end) {
@@ -290,7 +295,14 @@ __device__ __forceinline__ long long claim_chunk(const DecodeParams& p, const Ge
 // producer warp
 // --------------------------------------------------------------------------------------
 
-template <typename Cfg, typename T, int D, int TILE_T, int STAGES>
+// What a launch knows of its work.
+enum Plan {
+    kGeneral,  // nothing: any cache, any lengths
+    kFew,      // no block table, up to 32 sequences of lengths whose sum fits 32 bits
+    kWhole,    // a CTA per (sequence, head), none is cut
+};
+
+template <typename Cfg, typename T, int D, int TILE_T, int STAGES, int kPlan>
 __device__ __forceinline__ void decode_producer(const DecodeParams& p, const CUtensorMap* tm_k,
                                                 const CUtensorMap* tm_v, uint8_t* stages, uint64_t* full,
                                                 uint64_t* empty, StageMeta* meta, Geometry* geo, int lane) {
@@ -303,7 +315,22 @@ __device__ __forceinline__ void decode_producer(const DecodeParams& p, const CUt
     bool ok = true;
 
     const uint64_t l2_policy = l2_policy_evict_first();
-    const Geometry ge = geometry_of(p, gridDim.x, TILE_T, lane);
+    // kFew: a lane per sequence, summed up once.  The first copy of a short launch waits for all of this, and no longer for the count of a
+    // pair's pieces: 8 sequences of 32 heads and 128 to 1024 tokens 24.2 us, 25.0 with 64-bit sums taken twice and the pieces counted
+    // ahead.  (Through a block table, where a tile is many copies, it is the other way round: 51.2 and 50.5.)
+    constexpr bool few = kPlan == kFew;
+    const int own_len = few && lane < p.B ? seq_len_of(p, lane) : 0;
+    unsigned own_incl = static_cast<unsigned>(own_len);
+    if (few) {
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const unsigned up = __shfl_up_sync(0xffffffffu, own_incl, off);
+            if (lane >= off) own_incl += up;
+        }
+    }
+    const Geometry ge = kPlan == kWhole ? Geometry{0, 0, 0, 1, static_cast<int>(gridDim.x), static_cast<int>(gridDim.x)}
+                        : few ? cut(p, __shfl_sync(0xffffffffu, own_incl, 31), __reduce_max_sync(0xffffffffu, own_len), gridDim.x, TILE_T)
+                              : geometry_of(p, gridDim.x, TILE_T, lane);
     if (lane == 0) *geo = ge;  // (published to the other warps with the first stage's barrier)
     const bool on_demand = ge.n_chunks > ge.n_static;
 
@@ -315,11 +342,28 @@ __device__ __forceinline__ void decode_producer(const DecodeParams& p, const CUt
     };
     auto chunk_start = [&](long long g) {
         ChunkStart cs;
+        if (kPlan == kWhole) {  // (positions relative to the sequence's first: nothing else is looked at)
+            cs.b = static_cast<int>(g) / p.H;
+            cs.h = static_cast<int>(g) - cs.b * p.H;
+            cs.tok_before = 0;
+            cs.len_b = seq_len_of(p, cs.b);
+            cs.c_start = static_cast<long long>(cs.h) * cs.len_b;
+            cs.c_end = cs.c_start + cs.len_b;
+            if (cs.len_b == 0) cs.b = p.B;
+            return cs;
+        }
         chunk_range(ge, g, cs.c_start, cs.c_end);
         cs.b = p.B;
         cs.tok_before = 0;
         cs.len_b = 0;
-        if (cs.c_start < cs.c_end) locate_sequence(p, cs.c_start, lane, cs.b, cs.tok_before, cs.len_b);
+        if (cs.c_start < cs.c_end && few) {
+            const unsigned hit = __ballot_sync(0xffffffffu, static_cast<long long>(own_incl) * p.H > cs.c_start);
+            cs.b = __ffs(hit) - 1;  // (a position of the token space lies in some sequence)
+            cs.tok_before = __shfl_sync(0xffffffffu, own_incl - static_cast<unsigned>(own_len), cs.b);
+            cs.len_b = __shfl_sync(0xffffffffu, own_len, cs.b);
+        } else if (cs.c_start < cs.c_end) {
+            locate_sequence(p, cs.c_start, lane, cs.b, cs.tok_before, cs.len_b);
+        }
         cs.h = (cs.b < p.B) ? static_cast<int>((cs.c_start - cs.tok_before * p.H) / cs.len_b) : 0;
         return cs;
     };
@@ -352,23 +396,27 @@ __device__ __forceinline__ void decode_producer(const DecodeParams& p, const CUt
             int t_begin, t_end;
             piece_of(c_start, c_end, pair_off, len_b, TILE_T, t_begin, t_end);
             // how many chunks hold a piece with tokens of this pair (the merge counts them in)
-            int pieces = 0;
-            {
+            auto count_pieces = [&]() {
+                if (kPlan == kWhole) return 1;
+                int n = 0;
                 const long long g_first = chunk_of(ge, pair_off), g_last = chunk_of(ge, pair_off + len_b - 1);
                 for (long long g = g_first + lane; g <= g_last; g += 32) {
                     long long s0, s1;
                     chunk_range(ge, g, s0, s1);
                     int t0, t1;
                     piece_of(s0, s1, pair_off, len_b, TILE_T, t0, t1);
-                    pieces += (t0 < t1) ? 1 : 0;
+                    n += (t0 < t1) ? 1 : 0;
                 }
-    #pragma unroll
-                for (int off = 16; off >= 1; off >>= 1) pieces += __shfl_xor_sync(0xffffffffu, pieces, off);
-            }
+#pragma unroll
+                for (int off = 16; off >= 1; off >>= 1) n += __shfl_xor_sync(0xffffffffu, n, off);
+                return n;
+            };
+            int pieces = kPlan == kFew ? 0 : count_pieces();
             // a pair in one piece has a slot of its own (used when a merge kernel follows), a piece of several is one
             // of its chunk's two
             const int bh = b * p.H + h;
-            int slot = pieces == 1 ? p.n_slots - p.B * p.H + bh : piece_slot(chunk, c_start, pair_off);
+            auto slot_of = [&]() { return pieces == 1 ? p.n_slots - p.B * p.H + bh : piece_slot(chunk, c_start, pair_off); };
+            int slot = slot_of();
             if (t_begin < t_end && (slot < 0 || slot >= p.n_slots)) {
                 report_status(p.dev_status, B2KV_DEV_BAD_POSITION);  // cannot happen: sized on the host
                 t_end = t_begin;
@@ -391,23 +439,41 @@ __device__ __forceinline__ void decode_producer(const DecodeParams& p, const CUt
                 }
                 uint8_t* sbase = stages + static_cast<size_t>(stage) * Cfg::kStageBytes;
                 const bool first = (t0 == t_begin);
-                if (lane == 0) {
-                    StageMeta mt;
-                    mt.slot = slot;
-                    mt.ntok = ntok;
-                    mt.flags = (first ? kFlagFirst : 0) | (t0 + TILE_T >= t_end ? kFlagLast : 0) | (pieces == 1 ? kFlagWhole : 0);
-                    mt.pieces = pieces;
-                    mt.pair_off = pair_off;
-                    mt.len = len_b;
-                    mt.bh = bh;
-                    meta[stage] = mt;
-                    // a tiled load always delivers the whole box (rows past the end arrive as zeros or as
-                    // the next rows of the cache; the consumers use the first ntok only)
-                    const uint32_t rows = p.use_tensor_map ? static_cast<uint32_t>(TILE_T) : static_cast<uint32_t>(ntok);
-                    const uint32_t bytes = 2u * rows * Cfg::kRowBytes + (first ? Cfg::kRowBytes : 0);
-                    mbar_arrive_expect_tx(&full[stage], bytes);
-                }
-                __syncwarp();
+                // The stage's description and its arrival.  Of a pair's first tile of kFew they come behind its copies, whose bytes may be
+                // counted ahead of the arrival that the barrier's phase waits for.
+                auto describe = [&]() {
+                    if (lane == 0) {
+                        StageMeta mt;
+                        mt.slot = slot;
+                        mt.ntok = ntok;
+                        mt.flags = (first ? kFlagFirst : 0) | (t0 + TILE_T >= t_end ? kFlagLast : 0) | (pieces == 1 ? kFlagWhole : 0);
+                        mt.pieces = pieces;
+                        mt.pair_off = pair_off;
+                        mt.len = len_b;
+                        mt.bh = bh;
+                        meta[stage] = mt;
+                        // a tiled load always delivers the whole box (rows past the end arrive as zeros or as
+                        // the next rows of the cache; the consumers use the first ntok only)
+                        const uint32_t rows = p.use_tensor_map ? static_cast<uint32_t>(TILE_T) : static_cast<uint32_t>(ntok);
+                        const uint32_t bytes = 2u * rows * Cfg::kRowBytes + (first ? Cfg::kRowBytes : 0);
+                        mbar_arrive_expect_tx(&full[stage], bytes);
+                    }
+                    __syncwarp();
+                };
+                auto issued = [&]() {
+                    if (kPlan == kFew && first) {
+                        __syncwarp();
+                        pieces = count_pieces();
+                        slot = slot_of();
+                        describe();
+                    }
+                    ++fills;
+                    if (++stage == STAGES) {
+                        stage = 0;
+                        phase ^= 1u;
+                    }
+                };
+                if (kPlan != kFew || !first) describe();
                 if (first && lane == 31) {
                     bulk_g2s(sbase + 2 * Cfg::kTileBytes,
                              qbase + (static_cast<size_t>(b) * p.H + h) * Cfg::kRowBytes, Cfg::kRowBytes, &full[stage]);
@@ -415,11 +481,7 @@ __device__ __forceinline__ void decode_producer(const DecodeParams& p, const CUt
                 if (p.use_tensor_map) {
                     if (lane == 0) tma_load_4d(sbase, tm_k, &full[stage], 0, t0, h, b);
                     if (lane == 1) tma_load_4d(sbase + Cfg::kTileBytes, tm_v, &full[stage], 0, t0, h, b);
-                    ++fills;
-                    if (++stage == STAGES) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
+                    issued();
                     continue;
                 }
                 const int nruns = (ntok + p.run_len - 1) / p.run_len;
@@ -449,11 +511,7 @@ __device__ __forceinline__ void decode_producer(const DecodeParams& p, const CUt
                         bulk_g2s(sbase + Cfg::kTileBytes + dst, vbase + off, bytes, &full[stage]);
                     }
                 }
-                ++fills;
-                if (++stage == STAGES) {
-                    stage = 0;
-                    phase ^= 1u;
-                }
+                issued();
             }
             // next (sequence, head); empty sequences own no tokens and are skipped
             if (++h == p.H) {
@@ -872,7 +930,7 @@ __device__ __forceinline__ void decode_merger(const DecodeParams& p, uint64_t* h
 // kernel
 // --------------------------------------------------------------------------------------
 
-template <typename T, int D, int TILE_T, int STAGES, int NCW>
+template <typename T, int D, int TILE_T, int STAGES, int NCW, int kPlan>
 __global__ void __launch_bounds__((NCW + 2) * 32, DecodeCfg<T, D, TILE_T, STAGES, NCW>::kCtasPerSm)
 decode_split_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v) {
@@ -907,7 +965,7 @@ decode_split_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap tm
     }
     __syncthreads();
     if (warp == NCW) {
-        decode_producer<Cfg, T, D, TILE_T, STAGES>(p, &tm_k, &tm_v, stages, full, empty, meta, geo, lane);
+        decode_producer<Cfg, T, D, TILE_T, STAGES, kPlan>(p, &tm_k, &tm_v, stages, full, empty, meta, geo, lane);
     } else if (warp == NCW + 1) {
         decode_merger<Cfg, T, D, TILE_T, NCW>(p, hand_full, hand_empty, hand_meta, merge, geo, lane);
     } else {
@@ -1020,6 +1078,9 @@ constexpr int default_tile(int row_bytes) {
 // Most CTAs per SM that a launch uses: the grid is persistent, more would only add partials.
 constexpr int kMaxCtasPerSm = 4;
 
+// Tiles of a (sequence, head) that are not worth being cut.
+constexpr int kWholeTiles = 4;
+
 // Partial-result slots for a grid of `n_ctas`: two per chunk (a chunk shares at most its first and its last
 // (sequence, head) with other chunks) and one per (sequence, head) for pairs in one piece.
 static size_t partial_slots(int n_ctas, int B, int H) {
@@ -1037,32 +1098,45 @@ static unsigned long long next_call_id() {
     return id == 0 ? 1 : id;
 }
 
-template <typename T, int D, int TILE_T, int STAGES, int NCW>
-static int launch_decode(DecodeParams p, void* out, void* workspace, size_t workspace_bytes, void* stream) {
-    using Cfg = DecodeCfg<T, D, TILE_T, STAGES, NCW>;
-    auto kernel = decode_split_kernel<T, D, TILE_T, STAGES, NCW>;
-    static bool configured[64] = {false};
-    static int ctas_per_sm[64] = {0};
+// CTAs per SM of a kernel, at most kMaxCtasPerSm, or what the caller asked for.  `occupancy`: per device, 0 before the first call.
+template <typename Cfg, typename K>
+static int ctas_per_sm(K kernel, int (&occupancy)[64], int* per_sm) {
     int dev = 0;
     B2KV_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return B2KV_ERR_UNSUPPORTED;
-    if (!configured[dev]) {
-        B2KV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(Cfg::kSmemBytes)));
+    if (occupancy[dev] == 0) {
+        B2KV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::kSmemBytes)));
         int occ = 0;
-        B2KV_CUDA_TRY(
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, Cfg::kThreads, Cfg::kSmemBytes));
+        B2KV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, Cfg::kThreads, Cfg::kSmemBytes));
         if (occ < 1) return B2KV_ERR_UNSUPPORTED;
-        ctas_per_sm[dev] = occ;
-        configured[dev] = true;
+        occupancy[dev] = occ;
     }
-    int per_sm = tune_get("decode_grid_per_sm");
-    if (per_sm <= 0 || per_sm > ctas_per_sm[dev]) per_sm = ctas_per_sm[dev];
-    if (per_sm > kMaxCtasPerSm) per_sm = kMaxCtasPerSm;
+    *per_sm = tune_get("decode_grid_per_sm");
+    if (*per_sm <= 0 || *per_sm > occupancy[dev]) *per_sm = occupancy[dev];
+    if (*per_sm > kMaxCtasPerSm) *per_sm = kMaxCtasPerSm;
+    return B2KV_OK;
+}
+
+// kShort: few tiles per (sequence, head) go to kWhole.
+template <typename T, int D, int TILE_T, int STAGES, int NCW, int kPlan = kGeneral, bool kShort = false>
+static int launch_decode(DecodeParams p, void* out, void* workspace, size_t workspace_bytes, void* stream) {
+    using Cfg = DecodeCfg<T, D, TILE_T, STAGES, NCW>;
+    auto kernel = decode_split_kernel<T, D, TILE_T, STAGES, NCW, kPlan>;
+    static int occupancy[64] = {0};
+    int per_sm = 0;
+    const int rc = ctas_per_sm<Cfg>(kernel, occupancy, &per_sm);
+    if (rc != B2KV_OK) return rc;
     const int grid_full = device_sm_count() * per_sm;
     // no more CTAs than tiles of work (upper bound from T_upper)
-    const long long tiles_upper = static_cast<long long>(p.B) * p.H * ((p.T_upper + TILE_T - 1) / TILE_T);
-    int grid = static_cast<int>(tiles_upper < grid_full ? tiles_upper : grid_full);
+    const long long tiles_each = (p.T_upper + TILE_T - 1) / TILE_T, pairs = static_cast<long long>(p.B) * p.H;
+    // A few tiles per (sequence, head), and a CTA for each: streaming them one after the other takes less than finding out how they are
+    // cut and putting pieces together (4 heads of 161 fp32 rows of 64: 10.2 us, 14.4 with a CTA per tile; 3 sequences of 12 heads, 100 to
+    // 220 bf16 rows of 128: 12.2 and 18.5).
+    if constexpr (kShort) {
+        if (tiles_each <= kWholeTiles && pairs <= grid_full && p.partial_out == nullptr && p.gather.peer_out == nullptr && !tune_get("decode_merge_kernel"))
+            return launch_decode<T, D, TILE_T, STAGES, NCW, kWhole>(p, out, workspace, workspace_bytes, stream);
+    }
+    int grid = static_cast<int>(kPlan == kWhole ? pairs : std::min<long long>(pairs * tiles_each, grid_full));
     if (grid < 1) grid = 1;
     const size_t slots = partial_slots(grid, p.B, p.H);
     if (slots > 0x7fffffffull) return B2KV_ERR_UNSUPPORTED;
@@ -1129,6 +1203,7 @@ static int launch_decode(DecodeParams p, void* out, void* workspace, size_t work
 template <typename T, int D>
 static int dispatch_variant(const DecodeParams& p, void* out, void* ws, size_t ws_bytes, void* stream) {
     constexpr int kRow = D * static_cast<int>(sizeof(T));
+    const bool few = p.block_table == nullptr && p.B <= 32 && p.T_upper < (1 << 26);
     // Variants of the ring for the headline row size (256 bytes: bf16 head_dim 128, fp32 head_dim 64);
     // other row sizes use the default (8 KB tiles, 4 stages, 4 consumer warps).
     if constexpr (kRow == 256) {
@@ -1155,11 +1230,13 @@ static int dispatch_variant(const DecodeParams& p, void* out, void* ws, size_t w
             // shape) or, through a block table, as three CTAs of two (three copy warps per SM for the many short
             // copies: 683 against 706 us with 16-token blocks).
             default:
-                if (p.block_table != nullptr) return launch_decode<T, D, 64, 2, 8>(p, out, ws, ws_bytes, stream);
-                return launch_decode<T, D, 64, 3, 8>(p, out, ws, ws_bytes, stream);
+                if (p.block_table != nullptr) return launch_decode<T, D, 64, 2, 8, kGeneral, true>(p, out, ws, ws_bytes, stream);
+                return few ? launch_decode<T, D, 64, 3, 8, kFew, true>(p, out, ws, ws_bytes, stream)
+                           : launch_decode<T, D, 64, 3, 8, kGeneral, true>(p, out, ws, ws_bytes, stream);
         }
     } else {
-        return launch_decode<T, D, default_tile(kRow), 4, 4>(p, out, ws, ws_bytes, stream);
+        return few ? launch_decode<T, D, default_tile(kRow), 4, 4, kFew, true>(p, out, ws, ws_bytes, stream)
+                   : launch_decode<T, D, default_tile(kRow), 4, 4, kGeneral, true>(p, out, ws, ws_bytes, stream);
     }
 }
 
