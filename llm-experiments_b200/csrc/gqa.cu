@@ -137,9 +137,11 @@ __global__ void __launch_bounds__(kAppendThreads) gqa_append_kernel(T* y, T* k_c
     rv.scaled(v_cache + place * nv, v, nullptr, 1.f, nv);
 }
 
-// One CTA per (head, query row); its warps take the visible tokens in turn, each with an online softmax of its own, and are
-// merged at the end.  A lane holds kPer elements of the query and of the output.
-constexpr int kWarps = 4;
+// One CTA per (head, query row); its warps take the visible tokens in turn, a few at a time, each with an online softmax of its own, and are
+// merged at the end.  A lane holds kPer elements of the query and of the output.  Few rows are a chain of loads, sums over the warp and
+// exponentials, so tokens that are on their way together share it: three rows of 200 to 600 tokens (12 heads of 64, fp32) 12 us, 25 with four warps
+// and token after token.
+constexpr int kWarps = 8;
 
 template <typename T, int kPer>
 __global__ void __launch_bounds__(kWarps * 32) gqa_decode_kernel(const GqaDecodeArgs a) {
@@ -164,24 +166,43 @@ __global__ void __launch_bounds__(kWarps * 32) gqa_decode_kernel(const GqaDecode
         acc[c] = 0.f;
     }
     float m = -INFINITY, l = 0.f;
-    for (int t = warp; t <= pos; t += kWarps) {
-        const T* key = keys + static_cast<int64_t>(t) * a.G * a.dim;
-        const T* value = values + static_cast<int64_t>(t) * a.G * a.vdim;
-        float v[kPer], s = 0.f;
+    constexpr int kTogether = kPer <= 4 ? 4 : 2;
+    for (int t0 = warp * kTogether; t0 <= pos; t0 += kWarps * kTogether) {
+        float v[kTogether][kPer], s[kTogether];
 #pragma unroll
-        for (int c = 0; c < kPer; ++c) {
-            const int d = c * 32 + lane;
-            v[c] = d < a.vdim ? Elt<T>::to_float(value[d]) : 0.f;
-            s = fmaf(q[c], d < a.dim ? Elt<T>::to_float(key[d]) : 0.f, s);
+        for (int u = 0; u < kTogether; ++u) {
+            const T* key = keys + static_cast<int64_t>(t0 + u) * a.G * a.dim;
+            const T* value = values + static_cast<int64_t>(t0 + u) * a.G * a.vdim;
+            const bool in = t0 + u <= pos;
+            s[u] = 0.f;
+#pragma unroll
+            for (int c = 0; c < kPer; ++c) {
+                const int d = c * 32 + lane;
+                v[u][c] = in && d < a.vdim ? Elt<T>::to_float(value[d]) : 0.f;
+                s[u] = fmaf(q[c], in && d < a.dim ? Elt<T>::to_float(key[d]) : 0.f, s[u]);
+            }
         }
+        float mn = m;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-        s = s * a.scale - slope * static_cast<float>(pos - t);
-        const float mn = fmaxf(m, s), f = expf(m - mn), p = expf(s - mn);
-        l = l * f + p;
+        for (int u = 0; u < kTogether; ++u) {
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], off);
+            s[u] = s[u] * a.scale - slope * static_cast<float>(pos - t0 - u);
+            if (t0 + u <= pos) mn = fmaxf(mn, s[u]);
+        }
+        const float f = expf(m - mn);
+        l *= f;
         m = mn;
 #pragma unroll
-        for (int c = 0; c < kPer; ++c) acc[c] = fmaf(acc[c], f, p * v[c]);
+        for (int c = 0; c < kPer; ++c) acc[c] *= f;
+#pragma unroll
+        for (int u = 0; u < kTogether; ++u) {
+            if (t0 + u > pos) break;
+            const float p = expf(s[u] - mn);
+            l += p;
+#pragma unroll
+            for (int c = 0; c < kPer; ++c) acc[c] = fmaf(p, v[u][c], acc[c]);
+        }
     }
 #pragma unroll
     for (int c = 0; c < kPer; ++c)
@@ -408,10 +429,10 @@ int launch_runs(const GqaDecodeArgs& a, void* stream) {
 // many sequences would be in line: 16 of them take as long as the one that sees most, times 16).
 int launch_runs_f32(const GqaDecodeArgs& a, void* stream) {
     // Enough CTAs that the SMs are busy with 64 threads each: below, a CTA's chain of token tiles takes longer than rows one by
-    // one over as many SMs (8 heads of 64: 100 rows behind 500 others 59 us and 52, 400 rows 78 and 179; of 128, with half as many CTAs per SM: 100
-    // rows 116 and 64, 400 rows 153 and 233).
+    // one over as many SMs (8 heads of 64 behind 500 tokens: 100 rows 58 us and 47, 160 rows 57 and 69; of 128, with half as many CTAs per SM: 100
+    // rows 116 and 54, 400 rows 153 and 219).
     const long long ctas = static_cast<long long>(a.H) * ((a.rows + kRunRows - 1) / kRunRows), sms = device_sm_count();
-    const bool few = a.rows < 64 || (std::max(a.dim, a.vdim) <= 64 ? 4 * ctas < 3 * sms : 2 * ctas < 3 * sms);
+    const bool few = a.rows < 64 || (std::max(a.dim, a.vdim) <= 64 ? 2 * ctas < sms : 2 * ctas < 3 * sms);
     if ((few && tune_get("gqa_runs") == 0) || (a.rows + kRunRows - 1) / kRunRows > 65535) return B2KV_ERR_UNSUPPORTED;
     const int widest = std::max(a.dim, a.vdim);
     if (widest > 128 || a.dim % 4 || a.vdim % 4 || a.ld_q % 4 || !aligned16(a.q) || !aligned16(a.k_cache) || !aligned16(a.v_cache))
