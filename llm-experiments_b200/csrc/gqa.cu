@@ -234,18 +234,23 @@ __global__ void __launch_bounds__(kWarps * 32) gqa_decode_kernel(const GqaDecode
 // over the warp for every token: 174 us for 693 rows of three prompts (12 heads of 64, 4 of them for keys), against 90
 // (100 with 32 rows: half as many warps to hide one another's waits).
 // Rows of other sequences in the same 16 are taken in turn; a weight of zero is never multiplied with what a row must not see.
+__device__ __forceinline__ void copy16_or_zero(void* dst, const void* src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
 constexpr int kRunRows = 16, kRunTokens = 64, kRunThreads = 64;
 
-template <int kD>  // dim and vdim, rounded up
+// kD: dim and vdim, rounded up; kLate: the last rows first.
+template <int kD, bool kLate>
 __global__ void __launch_bounds__(kRunThreads) gqa_run_f32_kernel(const __grid_constant__ GqaDecodeArgs a) {
     constexpr int kLd = kD + 4, kLdP = kRunTokens + 4, kCols = kD / 64;
+    constexpr bool kAhead = kD > 64;
     extern __shared__ float4 sm_run[];
     float* const s_q = reinterpret_cast<float*>(sm_run);  // [rows][kLd]
     float* const s_k = s_q + kRunRows * kLd;              // [tokens][kLd]
     float* const s_v = s_k + kRunTokens * kLd;            // [tokens][kLd]
     float* const s_p = s_v + kRunTokens * kLd;            // [rows][kLdP]
     __shared__ int s_slot[kRunRows], s_pos[kRunRows];
-    const int h = blockIdx.x, i0 = static_cast<int>(blockIdx.y) * kRunRows, n_rows = min(kRunRows, a.rows - i0);
+    const int h = blockIdx.x, i0 = static_cast<int>(kLate ? gridDim.y - 1 - blockIdx.y : blockIdx.y) * kRunRows, n_rows = min(kRunRows, a.rows - i0);
     const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16, g = h / (a.H / a.G);
     grid_launch_dependents();
     grid_dependency_wait();
@@ -288,20 +293,42 @@ __global__ void __launch_bounds__(kRunThreads) gqa_run_f32_kernel(const __grid_c
         const int64_t base = static_cast<int64_t>(here) * a.T_max * a.G + g;
         const float* const keys = static_cast<const float*>(a.k_cache) + base * a.dim;
         const float* const values = static_cast<const float*>(a.v_cache) + base * a.vdim;
-        for (int t0 = 0; t0 <= last; t0 += kRunTokens) {
-            __syncthreads();
+        // Rows of 128: keys and values come with copies of their own, the next tile's keys under this one's softmax and output, the next values
+        // under the next scores (two prompts of 300 and 400 tokens, 8 heads: 62 us, 84 with the copies where they are waited for).  Of rows of 64 an SM
+        // holds twice as many CTAs, which hide each other's loads (48 us so, 51 with copies ahead).
+        auto request = [&](float* to, const float* from, int width, int t0) {
+            if (t0 <= last) {
 #pragma unroll 4
-            for (int i = tid; i < kRunTokens * (kD / 4); i += kRunThreads) {
-                const int t = i / (kD / 4), c = i % (kD / 4) * 4;
-                const bool in = t0 + t <= last;
-                *reinterpret_cast<float4*>(s_k + t * kLd + c) =
-                    in && c < a.dim ? *reinterpret_cast<const float4*>(keys + static_cast<int64_t>(t0 + t) * a.G * a.dim + c)
-                                    : make_float4(0.f, 0.f, 0.f, 0.f);
-                *reinterpret_cast<float4*>(s_v + t * kLd + c) =
-                    in && c < a.vdim ? *reinterpret_cast<const float4*>(values + static_cast<int64_t>(t0 + t) * a.G * a.vdim + c)
-                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int i = tid; i < kRunTokens * (kD / 4); i += kRunThreads) {
+                    const int t = i / (kD / 4), c = i % (kD / 4) * 4;
+                    const bool in = t0 + t <= last && c < width;
+                    copy16_or_zero(to + t * kLd + c, in ? from + static_cast<int64_t>(t0 + t) * a.G * width + c : from, in);
+                }
             }
-            __syncthreads();
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        if (kAhead) {
+            request(s_k, keys, a.dim, 0);
+            request(s_v, values, a.vdim, 0);
+        }
+        for (int t0 = 0; t0 <= last; t0 += kRunTokens) {
+            if (kAhead) {
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                __syncthreads();
+#pragma unroll 4
+                for (int i = tid; i < kRunTokens * (kD / 4); i += kRunThreads) {
+                    const int t = i / (kD / 4), c = i % (kD / 4) * 4;
+                    const bool in = t0 + t <= last;
+                    *reinterpret_cast<float4*>(s_k + t * kLd + c) =
+                        in && c < a.dim ? *reinterpret_cast<const float4*>(keys + static_cast<int64_t>(t0 + t) * a.G * a.dim + c)
+                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+                    *reinterpret_cast<float4*>(s_v + t * kLd + c) =
+                        in && c < a.vdim ? *reinterpret_cast<const float4*>(values + static_cast<int64_t>(t0 + t) * a.G * a.vdim + c)
+                                         : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            }
+            __syncthreads();  // the keys are here
             float s[4][4] = {};
 #pragma unroll 4
             for (int c = 0; c < a.dim; c += 4) {
@@ -316,6 +343,10 @@ __global__ void __launch_bounds__(kRunThreads) gqa_run_f32_kernel(const __grid_c
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                         s[i][j] = fmaf(qv[i].w, kv[j].w, fmaf(qv[i].z, kv[j].z, fmaf(qv[i].y, kv[j].y, fmaf(qv[i].x, kv[j].x, s[i][j]))));
+            }
+            if (kAhead) {
+                __syncthreads();  // everybody has read them
+                request(s_k, keys, a.dim, t0 + kRunTokens);
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -341,7 +372,12 @@ __global__ void __launch_bounds__(kRunThreads) gqa_run_f32_kernel(const __grid_c
                     s_p[(ty * 4 + i) * kLdP + t] = p;
                 }
             }
-            __syncwarp();  // a row's weights are written and read by the same 16 lanes
+            if (kAhead) {
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+                __syncthreads();  // the values are here
+            } else {
+                __syncwarp();  // a row's weights are written and read by the same 16 lanes
+            }
             if (alone && t0 + kRunTokens - 1 <= all) {
                 for (int t = 0; t < kRunTokens; t += 4) {
                     float4 p[4];
@@ -386,6 +422,10 @@ __global__ void __launch_bounds__(kRunThreads) gqa_run_f32_kernel(const __grid_c
                     }
                 }
             }
+            if (kAhead) {
+                __syncthreads();  // everybody has read them
+                request(s_v, values, a.vdim, t0 + kRunTokens);
+            }
         }
     }
     float* const out = static_cast<float*>(a.out) + i0 * a.ld_out + h * a.vdim;
@@ -409,19 +449,27 @@ __global__ void __launch_bounds__(kRunThreads) gqa_run_f32_kernel(const __grid_c
     }
 }
 
-template <int kD>
+template <int kD, bool kLate>
 int launch_runs(const GqaDecodeArgs& a, void* stream) {
     constexpr size_t smem = ((kRunRows + 2 * kRunTokens) * (kD + 4) + kRunRows * (kRunTokens + 4)) * sizeof(float);
-    static bool configured[64] = {false};
+    static int resident[64] = {0};  // CTAs that the device holds
     int dev = 0;
     B2KV_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return B2KV_ERR_UNSUPPORTED;
-    if (!configured[dev]) {
-        B2KV_CUDA_TRY(cudaFuncSetAttribute(gqa_run_f32_kernel<kD>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        configured[dev] = true;
+    if (resident[dev] == 0) {
+        B2KV_CUDA_TRY(cudaFuncSetAttribute(gqa_run_f32_kernel<kD, kLate>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        int n = 0;
+        B2KV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gqa_run_f32_kernel<kD, kLate>, kRunThreads, smem));
+        resident[dev] = n * device_sm_count();
     }
     OverlapLaunch launch(dim3(a.H, (a.rows + kRunRows - 1) / kRunRows), kRunThreads, smem, stream);
-    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, gqa_run_f32_kernel<kD>, a));
+    // A prompt's late rows see the most tokens and must not be what is left at the end (352 CTAs of which 296 fit, rows of 128: 77 us, 62 with the
+    // late rows first).  Of rows of 64, two and a half times as many fit, and the order that mixes late and early rows is better (57 us, 61 with
+    // the late rows first, of 792 CTAs of which 740 fit; 48 and 54 of 528).
+    if constexpr (kD > 64 && !kLate) {
+        if (static_cast<long long>(launch.cfg.gridDim.x) * launch.cfg.gridDim.y > resident[dev]) return launch_runs<kD, true>(a, stream);
+    }
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, gqa_run_f32_kernel<kD, kLate>, a));
     return B2KV_OK;
 }
 
@@ -429,15 +477,15 @@ int launch_runs(const GqaDecodeArgs& a, void* stream) {
 // many sequences would be in line: 16 of them take as long as the one that sees most, times 16).
 int launch_runs_f32(const GqaDecodeArgs& a, void* stream) {
     // Enough CTAs that the SMs are busy with 64 threads each: below, a CTA's chain of token tiles takes longer than rows one by
-    // one over as many SMs (8 heads of 64 behind 500 tokens: 100 rows 58 us and 47, 160 rows 57 and 69; of 128, with half as many CTAs per SM: 100
-    // rows 116 and 54, 400 rows 153 and 219).
+    // one over as many SMs (8 heads of 64 behind 500 tokens: 100 rows 58 us and 47, 160 rows 57 and 69; of 128, with half as many CTAs per SM: 200
+    // rows 111 and 100, 300 rows 132 and 159).
     const long long ctas = static_cast<long long>(a.H) * ((a.rows + kRunRows - 1) / kRunRows), sms = device_sm_count();
-    const bool few = a.rows < 64 || (std::max(a.dim, a.vdim) <= 64 ? 2 * ctas < sms : 2 * ctas < 3 * sms);
+    const bool few = a.rows < 64 || (std::max(a.dim, a.vdim) <= 64 ? 2 * ctas < sms : 4 * ctas < 3 * sms);
     if ((few && tune_get("gqa_runs") == 0) || (a.rows + kRunRows - 1) / kRunRows > 65535) return B2KV_ERR_UNSUPPORTED;
     const int widest = std::max(a.dim, a.vdim);
     if (widest > 128 || a.dim % 4 || a.vdim % 4 || a.ld_q % 4 || !aligned16(a.q) || !aligned16(a.k_cache) || !aligned16(a.v_cache))
         return B2KV_ERR_UNSUPPORTED;
-    return widest <= 64 ? launch_runs<64>(a, stream) : launch_runs<128>(a, stream);
+    return widest <= 64 ? launch_runs<64, false>(a, stream) : launch_runs<128, false>(a, stream);
 }
 
 template <typename T>
