@@ -148,7 +148,9 @@ using namespace b2kv;
 static bool takes_chunks(int path, int dtype, int max_n) { return path == 2 || (path == 0 && dtype == B2KV_DTYPE_BF16 && max_n > 16); }
 
 extern "C" size_t b2kv_gla_workspace_bytes(int H, int dim, int vdim, int n_segments, int max_n, int dtype, int path) {
-    if (H <= 0 || dim <= 0 || vdim <= 0 || n_segments <= 0 || max_n <= 0 || !takes_chunks(path, dtype, max_n)) return 0;
+    if (H <= 0 || dim <= 0 || vdim <= 0 || n_segments <= 0 || max_n <= 0) return 0;
+    if (dtype == B2KV_DTYPE_F32 && path == 0) return gla_run_f32_workspace(H, dim, vdim, n_segments, max_n);
+    if (!takes_chunks(path, dtype, max_n)) return 0;
     return gla_chunked_workspace(H, dim, vdim, n_segments, max_n, dtype);
 }
 

@@ -13,6 +13,7 @@ size_t gla_chunked_workspace(int H, int dim, int vdim, int n_segments, int max_n
 
 // fp32 runs with the state in registers; B2KV_ERR_UNSUPPORTED where rows are not made of 16-byte pieces.
 int gla_run_f32(const b2kv_gla_args& a, int32_t* dev_status, void* stream);  // gla_run.cu
+size_t gla_run_f32_workspace(int H, int dim, int vdim, int n_segments, int max_n);  // 0: of no use
 
 namespace gla {
 

@@ -289,3 +289,46 @@ def test_an_infinite_state_is_not_turned_into_nan_by_a_span(pkg):
     state[0, 0, 3, 5] = float("inf")
     layer.run(y, al, [(0, 600, 0)], 10 + np.arange(600), state, CHUNK)
     assert torch.isinf(state[0, 0, 3, 5]) and torch.isfinite(state).sum() == 16 * 32 - 1
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 20, 40), (3, 128, 256), (2, 64, 72), (1, 4, 4)])
+def test_spans_of_tokens_in_fp32(pkg, heads, dim, vdim):
+    """As for chunks, with spans of 64 tokens in launches with a segment of more than 192; the decays of half of the channels multiply up to
+    nothing over a span.  Alone, a segment has the same bits where it is cut the same way."""
+    layer = Layer(pkg, heads, dim, vdim, 4.0, F32, z_mean=2.0, z_std=4.0, seed=29)
+    first, then = (63, 64, 65, 193, 129, 5, 400), (256, 17, 64, 2, 128, 320, 16)
+    state, last = layer.states(len(first)), [None] * len(first)
+    for lens, start in ((first, [0] * len(first)), (then, first)):
+        y, al = layer.rows(sum(lens))
+        segments, was = [(sum(lens[:i]), n, i) for i, n in enumerate(lens)], state.clone()
+        got = layer.run(y, al, segments, np.concatenate([s + np.arange(n) for s, n in zip(start, lens)]), state, 0)
+        for (r0, n, i), s in zip(segments, start):
+            part = slice(r0, r0 + n)
+            if n <= 64 or n > 192:
+                assert np.array_equal(layer.run(y[part], al[part], [(0, n, 0)], s + np.arange(n), was[i:i + 1], 0), got[part]), (n, s)
+                assert torch.equal(was[i], state[i]), (n, s)
+            want, last[i] = layer.want(y[part], al[part], last[i])
+            close(got[part], want, F32, (n, s))
+            state_close(state[i], last[i])
+
+
+def test_spans_of_tokens_over_slices_of_a_bounded_workspace(pkg):
+    layer = Layer(pkg, 8, 128, 256, 16.0, F32, z_mean=2.0, z_std=1.0, seed=31)
+    lens = (4300, 64, 200, 4288)  # 68 spans of four segments, 63 at a time
+    y, al = layer.rows(sum(lens))
+    segments, pos = [(sum(lens[:i]), n, i) for i, n in enumerate(lens)], np.concatenate([np.arange(n) for n in lens])
+    state = layer.states(len(lens))
+    got = layer.run(y, al, segments, pos, state, 0)
+    for r0, n, slot in segments:
+        alone = layer.states(1)
+        assert np.array_equal(layer.run(y[r0:r0 + n], al[r0:r0 + n], [(0, n, 0)], range(n), alone, 0), got[r0:r0 + n]), n
+        assert torch.equal(alone[0], state[slot]), n
+
+
+def test_an_infinite_state_is_not_turned_into_nan_by_a_span_of_tokens(pkg):
+    layer = Layer(pkg, 1, 16, 32, 1.0, F32, z_mean=-1.5, z_std=0.0, seed=37)  # 0.18 ** 64 is below the smallest number
+    y, al = layer.rows(300)
+    state = torch.ones((1, 1, 16, 32), device="cuda")
+    state[0, 0, 3, 5] = float("inf")
+    layer.run(y, al, [(0, 300, 0)], 10 + np.arange(300), state, 0)
+    assert torch.isinf(state[0, 0, 3, 5]) and torch.isfinite(state).sum() == 16 * 32 - 1
