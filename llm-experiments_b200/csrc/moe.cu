@@ -12,7 +12,7 @@ namespace b2kv {
 namespace {
 
 constexpr int kMaxExperts = 1024, kMaxTop = 64;
-constexpr int kRouteWarps = 4;
+constexpr int kRouteWarps = 4, kRouteWarpsMany = 32;
 
 // Largest value over a warp and, among equals, the lowest index.
 __device__ __forceinline__ void warp_best(float& v, int& i) {
@@ -31,8 +31,11 @@ __global__ void zero_counts_kernel(int32_t* counts, int n) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) counts[i] = 0;
 }
 
-// A warp per row.  A score that is taken, or whose group is not kept, is replaced by -1 (scores are positive).
-__global__ void __launch_bounds__(kRouteWarps * 32)
+// A warp per row.  A score that is taken, or whose group is not kept, is replaced by -1 (scores are positive).  Many rows: what bounds it is the
+// counting, two choices per nanosecond wherever they fall, so a CTA of 32 rows counts its own and adds them up expert by expert (3548
+// rows, 6 of 64 experts: 9.7 us, 16.2 with every choice counted in memory; 8000 rows 10.1 and 32.8).
+template <int kWarps>
+__global__ void __launch_bounds__(kWarps * 32)
 route_kernel(const float* logits, int64_t ld, int rows, int experts, int groups, int keep, int top,
              int32_t* idx, float* score, int32_t* counts) {
     extern __shared__ float sm_route[];
@@ -40,11 +43,17 @@ route_kernel(const float* logits, int64_t ld, int rows, int experts, int groups,
     if (threadIdx.x == 0) grid_dependency_wait();
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = blockIdx.x * kRouteWarps + warp;
-    if (row >= rows) return;
+    const int row = blockIdx.x * kWarps + warp;
+    constexpr bool kOwnCounts = kWarps > kRouteWarps;
+    int* const own = reinterpret_cast<int*>(sm_route + kWarps * 2 * experts);  // [experts]
+    if (kOwnCounts) {
+        for (int e = threadIdx.x; e < experts; e += kWarps * 32) own[e] = 0;
+        __syncthreads();
+    }
+    if (!kOwnCounts && row >= rows) return;
     float* s = sm_route + warp * 2 * experts;  // scores
     float* best = s + experts;                 // largest score of every group (-1: taken)
-    const float* z = logits + row * ld;
+    const float* z = logits + min(row, rows - 1) * ld;  // (a warp without a row stays for the barrier)
     float mx = -INFINITY;
     for (int e = lane; e < experts; e += 32) mx = fmaxf(mx, s[e] = z[e]);
 #pragma unroll
@@ -78,7 +87,7 @@ route_kernel(const float* logits, int64_t ld, int rows, int experts, int groups,
             if (best[e / per] >= 0.f) s[e] = -1.f;
         __syncwarp();
     }
-    for (int k = 0; k < top; ++k) {
+    for (int k = 0; k < top && row < rows; ++k) {
         float v = -2.f;
         int i = 0x7fffffff;
         for (int e = lane; e < experts; e += 32)
@@ -88,10 +97,15 @@ route_kernel(const float* logits, int64_t ld, int rows, int experts, int groups,
         if (lane == 0) {
             idx[static_cast<int64_t>(row) * top + k] = i;
             score[static_cast<int64_t>(row) * top + k] = v;
-            atomicAdd(&counts[i], 1);
+            atomicAdd(kOwnCounts ? &own[i] : &counts[i], 1);
             s[i] = -1.f;
         }
         __syncwarp();
+    }
+    if (kOwnCounts) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < experts; e += kWarps * 32)
+            if (own[e] != 0) atomicAdd(&counts[e], own[e]);
     }
 }
 
@@ -250,9 +264,14 @@ extern "C" int b2kv_route(const float* logits, int64_t ld, int rows, int experts
     if (experts > kMaxExperts || top > kMaxTop) return B2KV_ERR_UNSUPPORTED;
     OverlapLaunch zero(1, 256, 0, stream);
     B2KV_CUDA_TRY(cudaLaunchKernelEx(&zero.cfg, zero_counts_kernel, counts, 2 * experts));
-    OverlapLaunch launch((rows + kRouteWarps - 1) / kRouteWarps, kRouteWarps * 32,
-                         static_cast<size_t>(kRouteWarps) * 2 * experts * sizeof(float), stream);
-    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, route_kernel, logits, ld, rows, experts, groups, keep, top, idx, score, counts));
+    const size_t many_bytes = (static_cast<size_t>(kRouteWarpsMany) * 2 + 1) * experts * sizeof(float);
+    // (1500 rows: 6.9 us and 8.2, but the kernel behind begins later, 20.4 and 18.8 together; 3001 rows, 6 of 160 experts, of whose 192 choices few meet:
+    // 14.8 and 12.0)
+    const bool many = rows >= 2048 && kRouteWarpsMany * top >= 3 * experts && many_bytes <= 48 * 1024;
+    const int warps = many ? kRouteWarpsMany : kRouteWarps;
+    OverlapLaunch launch((rows + warps - 1) / warps, warps * 32, many ? many_bytes : static_cast<size_t>(kRouteWarps) * 2 * experts * sizeof(float), stream);
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, many ? route_kernel<kRouteWarpsMany> : route_kernel<kRouteWarps>, logits, ld, rows, experts, groups, keep,
+                                     top, idx, score, counts));
     return B2KV_OK;
 }
 

@@ -102,3 +102,26 @@ def test_a_position_outside_the_cache_is_reported_among_many_rows(pkg):
         pkg.gpu.batch_commit(ctx)
     filled = cache.layers[0].v_cache.buffer.view(rows, 64).any(dim=1)
     assert not filled[300] and filled.sum() == rows - 1
+
+
+@pytest.mark.parametrize("rows", [2047, 2048, 2049, 2079, 3000])
+@pytest.mark.parametrize("experts,groups,keep,top", [(64, 1, 1, 6), (64, 8, 3, 6), (8, 1, 1, 2), (96, 1, 1, 9), (60, 1, 1, 6)])
+def test_choices_of_many_rows_are_counted(pkg, rows, experts, groups, keep, top):
+    """A CTA of 32 rows counts for itself: the choices and scores of the same rows a few at a time, and every expert's count."""
+    native = pkg._native
+    g = torch.Generator(device="cuda").manual_seed(rows + experts)
+    logits = torch.randn(rows, experts + 4, generator=g, device="cuda")
+    logits[5] = float("nan")
+
+    def route(first, n):
+        idx, score = torch.full((n, top), -7, dtype=torch.int32, device="cuda"), torch.full((n, top), -7.0, device="cuda")
+        counts = torch.full((2 * experts,), 9, dtype=torch.int32, device="cuda")
+        native.check(native.lib.b2kv_route(logits[first:].data_ptr(), experts + 4, n, experts, groups, keep, top, idx.data_ptr(), score.data_ptr(),
+                                           counts.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        assert torch.equal(counts[:experts].long(), torch.bincount(idx.view(-1).long(), minlength=experts)) and not counts[experts:].any()
+        return idx, score
+
+    idx, score = route(0, rows)
+    few = [route(i, min(300, rows - i)) for i in range(0, rows, 300)]
+    assert torch.equal(idx, torch.cat([i for i, _ in few])) and torch.equal(score, torch.cat([s for _, s in few]))
