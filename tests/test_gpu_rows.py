@@ -125,3 +125,35 @@ def test_choices_of_many_rows_are_counted(pkg, rows, experts, groups, keep, top)
     idx, score = route(0, rows)
     few = [route(i, min(300, rows - i)) for i in range(0, rows, 300)]
     assert torch.equal(idx, torch.cat([i for i, _ in few])) and torch.equal(score, torch.cat([s for _, s in few]))
+
+
+@pytest.mark.parametrize("rank", [8, 264, 512])
+@pytest.mark.parametrize("span", [300, 700, 3000])
+def test_shares_of_latent_rows_at_any_place(pkg, rank, span):
+    """Rows in 2 to 12 shares, some of them empty, merged from and to memory by pairs of elements and, one element off, by elements."""
+    native = pkg._native
+    g = torch.Generator(device="cuda").manual_seed(rank + span)
+    H, dim, rot, n = 20, 16, 8, 4
+    bf = lambda *s: torch.randn(s, generator=g, device="cuda").bfloat16()  # noqa: E731
+    ql, q, key, lat = bf(n, H, rank), bf(n, H * (dim + rot)), bf(n, span, rot), bf(n, span, rank)
+    pos = torch.tensor([span - 1, 0, span // 2, 65], dtype=torch.int32, device="cuda")
+    nbytes = native.lib.b2kv_latent_decode_workspace_bytes(n, H, rank, span, native.DTYPE_BF16)
+    assert nbytes > 0
+    scale = (dim + rot) ** -0.5
+    ws, outs = torch.empty(nbytes + 16, dtype=torch.uint8, device="cuda"), []
+    for off_ws, off_out in ((0, 0), (4, 0), (0, 1)):
+        out = torch.full((n * H * rank + 8,), 7.0, dtype=torch.bfloat16, device="cuda")
+        native.check(native.lib.b2kv_latent_decode(ql.data_ptr(), q.data_ptr(), H * (dim + rot), dim, key.data_ptr(), lat.data_ptr(),
+                                                   out[off_out:].data_ptr(), None, pos.data_ptr(), n, span, n, H, rank, rot, 0, span, scale,
+                                                   native.DTYPE_BF16, 2, ws[off_ws:].data_ptr(), nbytes, None,
+                                                   torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        assert (out[:off_out] == 7).all() and (out[off_out + n * H * rank:] == 7).all()
+        outs.append(out[off_out:off_out + n * H * rank].view(n, H, rank))
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    for i, p in enumerate(pos.tolist()):
+        l, k = lat[i, :p + 1].double(), key[i, :p + 1].double()
+        s = ql[i].double() @ l.T + q[i].double().view(H, dim + rot)[:, dim:] @ k.T
+        want = torch.softmax(s * scale, 1) @ l
+        # weights and outputs are rounded to bf16: 2^-9 of the output, and of every weight's share of it
+        assert ((outs[0][i].double() - want).abs() <= 2.0**-8 * want.abs() + 2.0**-8 * l.abs().amax(0)).all()
