@@ -7,11 +7,12 @@
 // for every token, took 939 us for runs of up to 400 tokens (6 heads, 64 x 128), this one 80 (100 with
 // the tokens one after the other: eight at a time, their sums over the lanes run side by side).
 //
-// 400 tokens one after the other are a chain, on half of the SMs with a warp per scheduler, so long runs are cut into spans of 64 tokens
-// where there is scratch memory.  A first pass makes every span's own part of the state from zero, and the product of its decays
+// 400 tokens one after the other are a chain, on half of the SMs with a warp per scheduler, so runs of more than 192 tokens are cut into spans
+// of 64 where there is scratch memory.  A first pass makes every span's own part of the state from zero, and the product of its decays
 // (all but the last one's); gla_spans_kernel carries the state through, S <- diag(D) S + L, and leaves what each span begins with;
 // the second pass walks all spans side by side.  Two thirds more work: three prompts of 62 to 400 tokens, 6 heads of 64 x 128, 59 us in all, 124 as
-// chains.  Spans begin at multiples of 64 tokens from the segment's first token.
+// chains.  Spans begin at multiples of 64 tokens
+// from the segment's first token, and the sums are in one order whatever else is in the step.
 // o goes to the output rows as it is (they are fp32); gla_norm_kernel applies the head's norm and the gate there.
 #include <algorithm>
 
@@ -24,10 +25,11 @@ namespace {
 constexpr int kWarps = 4, kCols = 8 * kWarps;  // value columns of a CTA
 constexpr int kTok = 8, kRing = 3;
 constexpr int kSpanTokens = 64;
-constexpr int kMinSpanned = 193;  // tokens of the longest segment
+constexpr int kMinSpanned = 193;  // tokens of a segment that is cut
+constexpr int kMaxSpannedCtas = 32;  // value columns of a state / 32
 constexpr size_t kMaxSpanBytes = size_t{256} << 20;  // spans at a time, more only where a state per segment takes more
 
-__host__ __device__ constexpr int spans_of(int n) { return (n + kSpanTokens - 1) / kSpanTokens; }
+__host__ __device__ constexpr int spans_of(int n) { return n < kMinSpanned ? 1 : (n + kSpanTokens - 1) / kSpanTokens; }
 
 // The spans [first, first + count) of every segment: states [segment][span][H][dim][vdim], products of decays [segment][span][H][dim].
 struct Spans {
@@ -65,8 +67,7 @@ gla_run_kernel(const __grid_constant__ b2kv_gla_args a, int parts, const Spans s
     const int span = spans.first + static_cast<int>(blockIdx.z), all_spans = kPass == kWholeRun ? 1 : spans_of(sg.n);
     if (kPass != kWholeRun) {
         if (span >= all_spans || (kPass == kOwnPart && span + 1 == all_spans)) return;
-        sg.row0 += span * kSpanTokens;
-        sg.n = min(kSpanTokens, sg.n - span * kSpanTokens);
+        if (all_spans > 1) sg.row0 += span * kSpanTokens, sg.n = min(kSpanTokens, sg.n - span * kSpanTokens);
     }
     const int h = static_cast<int>(blockIdx.x) / parts, c0 = static_cast<int>(blockIdx.x) % parts * kCols;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, dg = lane >> 2, c = c0 + warp * 8 + (lane & 3) * 2;
@@ -285,10 +286,7 @@ template <int kD, bool kPadded>
 int launch_runs(const b2kv_gla_args& a, int parts, int32_t* dev_status, void* stream) {
     const dim3 grid(static_cast<unsigned>(a.H * parts), a.n_segments);
     const size_t need = gla_run_f32_workspace(a.H, a.dim, a.vdim, a.n_segments, a.max_n);
-    // Two passes pay where the chain is long and what they add runs on SMs that would be idle (CTAs of 32 value columns; us as one chain and
-    // in spans): 72 CTAs, 400 tokens 124 and 59; 192, 400 168 and 99; 64, 700 238 and 79; but 24, 128 31 and 36; 512, 300 187 and 266.
-    const bool idle = static_cast<long long>(grid.x) * grid.y <= 2LL * device_sm_count();
-    if (need == 0 || !idle || a.workspace == nullptr || !aligned16(a.workspace) || a.workspace_bytes < need) {
+    if (need == 0 || a.workspace == nullptr || !aligned16(a.workspace) || a.workspace_bytes < need) {
         OverlapLaunch run(grid, 32 * kWarps, 0, stream);
         B2KV_CUDA_TRY(cudaLaunchKernelEx(&run.cfg, gla_run_kernel<kD, kPadded, kWholeRun>, a, parts, Spans{}, dev_status));
         return B2KV_OK;
@@ -315,7 +313,10 @@ int launch_runs(const b2kv_gla_args& a, int parts, int32_t* dev_status, void* st
 
 size_t gla_run_f32_workspace(int H, int dim, int vdim, int n_segments, int max_n) {
     using namespace gla;
-    if (dim > 128 || dim % 4 || vdim % 4 || max_n < kMinSpanned || H > 65535) return 0;
+    // Two passes pay where the chain is long and what they add runs on SMs that would be idle (CTAs of 32 value columns; us as one chain and
+    // in spans): 72 CTAs, 400 tokens 124 and 59; 192, 400 168 and 99; 64, 700 238 and 79; but 24, 128 31 and 36; 512, 300 187 and 266.  So it is
+    // states that few CTAs hold; not by the number of segments, on which a sequence's sums must not depend.
+    if (dim > 128 || dim % 4 || vdim % 4 || max_n < kMinSpanned || H * ((vdim + kCols - 1) / kCols) > kMaxSpannedCtas) return 0;
     const size_t each = span_floats(H, dim, vdim) * sizeof(float), segments = static_cast<size_t>(n_segments);
     return std::min(each * segments * spans_of(max_n), std::max(kMaxSpanBytes, each * segments));  // (grows with segments and tokens)
 }
