@@ -11,6 +11,11 @@
 // the warps of a CTA and the CTAs of a cluster share the input features, so w is read once, 512 bytes per warp at a time; the clusters'
 // partial sums meet in distributed shared memory, in the order of the ranges (results do not depend on timing).  6 rows, 768 x 4096: 128 us
 // with linear_simt_kernel, 14 here.
+//
+// linear_f32_thin_kernel: up to 32 input features and more than 16 rows (a low-rank bottleneck).  What they cost is the outputs and what happens to
+// them, of which a tile of 64 x 128 has 64 per thread on a few SMs: a thread keeps two columns of w and goes through a few rows.  The sums
+// are in the order of the tiles, to the bit.  1056 rows, 16 -> 384 decays: 6.8 us, 12.7 in tiles; 4000 rows,
+// 32 -> 4096 as they are: 36.1 and 39.7.
 #include <algorithm>
 
 #include "linear.cuh"
@@ -205,6 +210,35 @@ __global__ void __launch_bounds__(kRowsThreads) linear_f32_rows_kernel(const __g
     if (splits > 1) cluster_sync();
 }
 
+constexpr int kThinThreads = 128, kThinK = 32, kThinRows = 32;
+
+template <int kK>
+__global__ void __launch_bounds__(kThinThreads) linear_f32_thin_kernel(const __grid_constant__ b2kv_linear_args a, int row_tile) {
+    __shared__ float xs[kThinRows][kK];
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int row0 = static_cast<int>(blockIdx.y) * row_tile, n = min(row_tile, a.rows - row0);
+    const int c = (static_cast<int>(blockIdx.x) * kThinThreads + threadIdx.x) * 2;
+    const float* const x = static_cast<const float*>(a.x) + static_cast<int64_t>(row0) * a.ld_x;
+    for (int i = threadIdx.x; i < n * kK; i += kThinThreads) {
+        const int r = i / kK, k = i % kK;
+        xs[r][k] = k < a.K ? x[static_cast<int64_t>(r) * a.ld_x + k] : 0.f;
+    }
+    float2 w[kK];  // (N is a multiple of 4)
+#pragma unroll
+    for (int k = 0; k < kK; ++k)
+        w[k] = c < a.N && k < a.K ? *reinterpret_cast<const float2*>(static_cast<const float*>(a.w) + static_cast<int64_t>(k) * a.ld_w + c)
+                                  : make_float2(0.f, 0.f);
+    __syncthreads();
+    if (c >= a.N) return;
+    lin::finish_rows<float>(a, 0, c, row0, 0, n, 1, [&](int r) {
+        float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < kK; ++k) v = __ffma2_rn(make_float2(xs[r][k], xs[r][k]), w[k], v);
+        return v;
+    });
+}
+
 }  // namespace linf32
 
 int linear_f32(const b2kv_linear_args& a, void* stream) {
@@ -230,6 +264,18 @@ int linear_f32(const b2kv_linear_args& a, void* stream) {
                                                        : (max_rows <= 8 ? linear_f32_rows_kernel<8> : linear_f32_rows_kernel<16>),
                                          a, splits));
         return B2KV_OK;
+    }
+    if (a.K <= kThinK && a.groups == 1 && a.group_rows == nullptr) {
+        // rows per CTA: few, unless the columns of w are then read for nothing (more than four CTAs per SM)
+        const long long cols = (a.N / 2 + kThinThreads - 1) / kThinThreads;
+        int row_tile = kThinRows;
+        while (row_tile > 8 && cols * ((a.rows + row_tile - 1) / row_tile) < 4LL * sms) row_tile /= 2;
+        const dim3 grid(static_cast<unsigned>(cols), static_cast<unsigned>((a.rows + row_tile - 1) / row_tile));
+        if (grid.y <= 65535u) {
+            OverlapLaunch launch(grid, kThinThreads, 0, stream);
+            B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, a.K <= 16 ? linear_f32_thin_kernel<16> : linear_f32_thin_kernel<32>, a, row_tile));
+            return B2KV_OK;
+        }
     }
     const long long tiles_m = (max_rows + kBM - 1) / kBM;
     if (tiles_m > 65535 || a.groups > 65535 || tiles_n > 0x7fffffffLL) return B2KV_ERR_UNSUPPORTED;

@@ -222,3 +222,25 @@ def test_scratch_grows_and_is_left_alone_where_it_is_of_no_use(pkg):
         bounded(out, x, w)
         sizes.append(scratch["linear"].numel() if scratch else 0)
     assert sizes[0] == sizes[1] == 0 and 0 < sizes[2] == sizes[3] < sizes[4]
+
+
+@pytest.mark.parametrize("rows", [17, 31, 33, 200, 1100, 9000])
+@pytest.mark.parametrize("K,n", [(4, 4), (16, 384), (20, 260), (32, 100)])
+@pytest.mark.parametrize("kind", ["SEG_STORE", "SEG_F32", "SEG_DECAY", "SEG_SOFTCAP", "SEG_GLU_SILU"])
+def test_few_input_features_have_the_bits_of_the_tiles(pkg, rows, K, n, kind):
+    """Input features that are zero change no bit of a sum in order, and 36 of them take the tiles."""
+    from llm_experiments_b200 import projection as proj
+
+    ctx, kind = make_ctx(pkg), getattr(proj, kind)
+    x, w, bias, res = torch.zeros((rows, 36), dtype=F32, device="cuda"), torch.zeros((36, n), dtype=F32, device="cuda"), rnd((n,), F32, 6), rnd((rows, n), F32, 7)
+    x[:, :K], w[:K] = rnd((rows, K), F32, 8), rnd((K, n), F32, 9)
+    outs, cols = [], n // 2 if kind == proj.SEG_GLU_SILU else n
+    for k in (K, 36):
+        out = res.clone() if kind == proj.SEG_F32 else torch.full((rows, n), 7.0, dtype=F32, device="cuda")
+        run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), k, [proj.OutputSegment(n, kind, wrap(pkg, out[:, :cols]))], limit=3.0,
+            bias=pkg.gpu.GPUBuffer1D(buffer=bias, shape=(n,), size=n), residual=wrap(pkg, out) if kind == proj.SEG_F32 else None)
+        assert (out[:, cols:] == 7).all()
+        outs.append(out)
+    if kind == proj.SEG_STORE:
+        bounded(outs[0], x[:, :K], w[:K], bias.double())
+    assert torch.equal(outs[0], outs[1])
