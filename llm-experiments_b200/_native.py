@@ -10,10 +10,12 @@ import importlib.machinery
 import importlib.util
 import pathlib
 import struct
+import sysconfig
 
 _PKG = pathlib.Path(__file__).resolve().parent
 LIB_PATH = _PKG / "libb2kv.so"
-CALLS_PATH = _PKG / "b2kv_calls.so"  # calls without ctypes' conversions (csrc/calls.c); where it is not built ctypes makes them
+# Calls without ctypes' conversions (csrc/calls.c), for this interpreter; where it is not built ctypes makes them.
+CALLS_PATH = _PKG / ("b2kv_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
 SERVE_LIB_PATH = _PKG / "libb2kv_serve.so"  # the part models are served with (build.py --serve), where that is all there is
 
 DTYPE_F32 = 0
@@ -176,7 +178,7 @@ def _calls():
     try:
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("b2kv_calls", loader))
         loader.exec_module(module)
-    except ImportError:  # built for another interpreter
+    except ImportError:  # of another machine
         return None
     return module
 
@@ -192,6 +194,9 @@ class Library:
             if calls is not None and None not in kinds and restype in (_i, _sz) and hasattr(fn, "argtypes"):
                 fn = calls.bind(ctypes.cast(fn, _vp).value, "".join(kinds), "i" if restype is _i else "z", fn)
             setattr(self, name, fn)
+
+    def __getattr__(self, name: str):  # what SIGNATURES does not list
+        return getattr(self.cdll, name)
 
 
 def _load() -> Library:

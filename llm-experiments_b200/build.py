@@ -13,6 +13,7 @@ from __future__ import annotations
 import concurrent.futures
 import os
 import pathlib
+import platform
 import subprocess
 import sys
 import sysconfig
@@ -21,7 +22,7 @@ PKG = pathlib.Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 OUT = PKG / "libb2kv.so"
-CALLS = PKG / "b2kv_calls.so"  # the C ABI's calls from Python, an extension module of this interpreter
+CALLS = PKG / ("b2kv_calls" + sysconfig.get_config_var("EXT_SUFFIX"))  # the C ABI's calls from Python, for this interpreter alone
 SERVE_OUT = PKG / "libb2kv_serve.so"
 OBJ_DIR = PKG / "build"
 SERVE_SOURCES = ("api", "append", "gemm", "gla", "gla_chunked", "gla_run", "gqa", "gqa_decode_tc", "latent", "latent_decode_tc", "latent_prefill", "linear", "linear_f32", "linear_f32_tc", "linear_rows", "moe", "rows",
@@ -54,11 +55,27 @@ def up_to_date(out: pathlib.Path = OUT) -> bool:
 
 
 def build_calls(force: bool = False) -> None:
-    """``b2kv_calls.so`` with the C compiler; nothing where there are no headers of this interpreter (ctypes makes the calls then)."""
+    """The extension module of ``csrc/calls.c`` with the C compiler.  The library does without it (ctypes makes the calls then), so
+    where it cannot be built there is a note and no error."""
     src, include = CSRC / "calls.c", pathlib.Path(sysconfig.get_paths()["include"])
-    if (not force and CALLS.exists() and CALLS.stat().st_mtime >= src.stat().st_mtime) or not (include / "Python.h").exists():
+    if not force and CALLS.exists() and CALLS.stat().st_mtime >= src.stat().st_mtime:
         return
-    subprocess.run([os.environ.get("CC", "gcc"), "-O2", "-Wall", "-shared", "-fPIC", "-I", str(include), str(src), "-o", str(CALLS)], check=True)
+    why = None
+    if sys.platform != "linux" or platform.machine() != "x86_64":
+        why = "its calls are those of x86-64 Linux"
+    elif not (include / "Python.h").exists():
+        why = "there are no headers of this interpreter"
+    else:
+        cmd = [os.environ.get("CC", "gcc"), "-O2", "-Wall", "-shared", "-fPIC", "-I", str(include), str(src), "-o", str(CALLS)]
+        try:
+            res = subprocess.run(cmd, capture_output=True, text=True)
+            if res.returncode != 0:
+                why = f"{cmd[0]} failed: {res.stderr.strip()}"
+        except OSError as e:
+            why = str(e)
+    if why is not None:
+        CALLS.unlink(missing_ok=True)  # (one of an older source)
+        sys.stderr.write(f"{CALLS.name} is not built, calls go through ctypes: {why}\n")
 
 
 def build(force: bool = False, verbose: bool = False, serve: bool = False) -> pathlib.Path:

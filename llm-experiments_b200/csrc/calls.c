@@ -5,7 +5,7 @@
 // Types: p pointer, i 32-bit and l 64-bit integer, f float; the result i, z (size_t).  Integers are cut to their width without a
 // check, as ctypes does.  Only for the x86-64 System V calling convention: integers and floats are counted there separately, so the
 // order between the two does not matter, and an integer narrower than a register may come with anything above it.
-// A call with 20 arguments takes 0.6 us, 3.5 through ctypes.
+// Passing on the 19 arguments of a decode takes 0.2 us, 2.2 through ctypes.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <stddef.h>

@@ -1,6 +1,11 @@
 """Calls of the C ABI through the extension module: every argument arrives, whatever the order of integers and floats and however many there
 are, results keep their sign and width, and what it cannot pass on goes to the ctypes function."""
 import ctypes
+import importlib.machinery
+import importlib.util
+import pathlib
+import platform
+import sysconfig
 
 import pytest
 
@@ -63,3 +68,55 @@ def test_structures_are_those_of_the_header(pkg):
         assert [tuple(getattr(s, n) for n, _ in native.Segment._fields_) for s in a.seg] == segments + [(None, 0, 0, 0, 0)]
         o = native.LinearOptions.from_buffer_copy(native.linear_options(1, 2, 3))
         assert [getattr(o, n) for n, _ in native.LinearOptions._fields_] == [1, 2, 3]
+
+
+@pytest.fixture
+def builder(pkg, tmp_path, monkeypatch):
+    """``build.py`` with the module's place in a folder of the test."""
+    spec = importlib.util.spec_from_file_location("b2kv_build_for_test", pathlib.Path(pkg.__file__).parent / "build.py")
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    monkeypatch.setattr(module, "CALLS", tmp_path / module.CALLS.name)
+    return module
+
+
+def test_the_module_is_of_one_interpreter(pkg, builder):
+    assert builder.CALLS.name == pkg._native.CALLS_PATH.name == "b2kv_calls" + sysconfig.get_config_var("EXT_SUFFIX")
+
+
+@pytest.mark.parametrize("what", ["no compiler", "a compiler that fails", "another machine", "no headers"])
+def test_the_library_is_built_where_the_module_cannot_be(builder, tmp_path, monkeypatch, capfd, what):
+    if what == "another machine":
+        monkeypatch.setattr(platform, "machine", lambda: "aarch64")
+    if what == "no headers":
+        monkeypatch.setattr(sysconfig, "get_paths", lambda: {"include": str(tmp_path)})
+    monkeypatch.setenv("CC", str(tmp_path / "cc") if what == "no compiler" else "false")
+    monkeypatch.setattr(builder, "up_to_date", lambda out: True)
+    builder.CALLS.write_bytes(b"of an older source")
+    assert builder.build_calls(force=True) is None and not builder.CALLS.exists()
+    assert "ctypes" in capfd.readouterr().err
+    assert builder.build() == builder.OUT
+
+
+def test_calls_without_the_module(pkg, monkeypatch):
+    """The same entry points, structures and refusals through ctypes alone."""
+    native = pkg._native
+
+    def refused(self, module):
+        raise ImportError("of another machine")
+
+    monkeypatch.setattr(importlib.machinery.ExtensionFileLoader, "exec_module", refused)
+    monkeypatch.setattr(importlib.machinery.ExtensionFileLoader, "create_module", lambda self, spec: None)
+    spec = importlib.util.spec_from_file_location("b2kv_native_for_test", native.__file__)
+    other = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(other)
+    assert other.calls is None and other.lib.b2kv_version() == native.lib.b2kv_version()
+    args = [1 << 8, 2 << 8, 0, 0, 0, 1024, 0, 4096, 0, 0, [(3 << 8, 4096, 0, 4096, 0)], 700, 1024, 4096, 1, 0, 0, 0, 0.0]
+    sizes = [n.lib.b2kv_linear_workspace_bytes(n.linear_args(*args)) for n in (native, other)]
+    assert sizes[0] == sizes[1] > 0
+    args[0] = 0  # no input: refused before anything is launched
+    for n in (native, other):
+        assert n.lib.b2kv_linear_ws(n.linear_args(*args), n.linear_options(0, 0, 0), None, 0, None, None) == -1
+        with pytest.raises(IndexError):
+            n.linear_args(*args[:10], args[10] * (n.MAX_SEGMENTS + 1), *args[11:])
+    assert native.lib.b2kv_strerror(-1) == other.lib.b2kv_strerror(-1)
