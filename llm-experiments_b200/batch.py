@@ -10,7 +10,7 @@ commit raises (:352-353).
 from __future__ import annotations
 
 import functools
-from typing import Tuple
+from typing import Optional, Tuple
 
 import torch
 
@@ -36,6 +36,21 @@ def current_handle(device: torch.device) -> int:
     """The raw handle of torch's current stream.  (A stream object for it costs 2 us, three times per step of a decoding loop
     whose kernels take less than ten.)"""
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
+
+
+def scratch(kept: Optional[torch.Tensor], nbytes: int, device: torch.device) -> torch.Tensor:
+    """``kept``, or new memory where there is none or it is smaller than ``nbytes``."""
+    if kept is not None and kept.numel() >= nbytes:
+        return kept
+    give_up(kept)
+    return torch.empty(nbytes, dtype=torch.uint8, device=device)
+
+
+def give_up(t: Optional[torch.Tensor]) -> None:
+    """Before the last reference to scratch memory goes: work on the current stream, which need not be the one it was allocated on, may
+    still use it."""
+    if t is not None and t.is_cuda:
+        t.record_stream(torch.cuda.current_stream(t.device))
 
 
 def batch_begin(ctx: GPUContext, enable_profiling: bool = False) -> None:

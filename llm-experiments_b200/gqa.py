@@ -14,7 +14,7 @@ from typing import Optional
 import torch
 
 from . import _native
-from .batch import batch_op_begin, dev_status_ptr, reference_op
+from .batch import batch_op_begin, dev_status_ptr, reference_op, scratch
 from .kv_cache import dtype_code
 from .latent import PromptPlan, RowPlaces
 from .types import GPUBuffer1D, GPUBuffer2D, GPUContext, KVCache
@@ -68,8 +68,8 @@ def gqa_decode(ctx: GPUContext, q: GPUBuffer2D, shape: GqaShape, slopes: Optiona
     k, v = _caches(cache, shape)
     rows, dt = q.shape[0], dtype_code(q.buffer.dtype)
     nbytes = _native.lib.b2kv_gqa_decode_workspace_bytes(rows, shape.heads, shape.kv_heads, shape.vdim, span, dt) if path != 1 else 0
-    if nbytes and (cache.workspace is None or cache.workspace.numel() < nbytes):
-        cache.workspace = torch.empty(nbytes, dtype=torch.uint8, device=ctx.device)
+    if nbytes:
+        cache.workspace = scratch(cache.workspace, nbytes, ctx.device)
     ws = cache.workspace if nbytes else None
     stream = batch_op_begin(ctx)
     _native.check(_native.lib.b2kv_gqa_decode_runs(

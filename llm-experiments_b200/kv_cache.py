@@ -23,7 +23,7 @@ from typing import List, Optional, Tuple
 import torch
 
 from . import _native
-from .batch import batch_op_begin, dev_status_ptr, validate_buffer_shape_2d, reference_op
+from .batch import batch_op_begin, dev_status_ptr, reference_op, scratch, validate_buffer_shape_2d
 from .buffers import gpu_buffer_2d_create, gpu_buffer_zerofy
 from .types import GPUBuffer2D, GPUContext, KVCache, KVCacheConfig, KVCacheLayer
 
@@ -165,8 +165,7 @@ def decode_workspace(cache: KVCache) -> torch.Tensor:
     allocated on first use and grown if a tuning knob later asks for a finer split."""
     nbytes = _native.lib.b2kv_decode_workspace_bytes(cache.batch_size, cache.n_heads, cache.head_dim,
                                                      cache.max_seq_len, dtype_code(cache.dtype))
-    if cache.workspace is None or cache.workspace.numel() < nbytes:
-        cache.workspace = torch.empty(nbytes, dtype=torch.uint8, device=cache.layers[0].k_cache.buffer.device)
+    cache.workspace = scratch(cache.workspace, nbytes, cache.layers[0].k_cache.buffer.device)
     return cache.workspace
 
 

@@ -19,7 +19,7 @@ from typing import Optional
 import torch
 
 from . import _native
-from .batch import batch_op_begin, dev_status_ptr, reference_op
+from .batch import batch_op_begin, dev_status_ptr, reference_op, scratch
 from .kv_cache import dtype_code
 from .types import GPUBuffer1D, GPUBuffer2D, GPUContext, KVCache
 
@@ -80,8 +80,8 @@ def latent_decode(ctx: GPUContext, q_latent: GPUBuffer2D, y: GPUBuffer2D, shape:
     rows, dt = q_latent.shape[0], dtype_code(q_latent.buffer.dtype)
     span = min(span, shape.window) if shape.window > 0 else span
     nbytes = _native.lib.b2kv_latent_decode_workspace_bytes(rows, shape.heads, shape.kv_rank, span, dt) if path != 1 else 0
-    if nbytes and (cache.workspace is None or cache.workspace.numel() < nbytes):
-        cache.workspace = torch.empty(nbytes, dtype=torch.uint8, device=ctx.device)
+    if nbytes:
+        cache.workspace = scratch(cache.workspace, nbytes, ctx.device)
     ws = cache.workspace if nbytes else None
     stream = batch_op_begin(ctx)
     _native.check(_native.lib.b2kv_latent_decode(

@@ -17,7 +17,7 @@ import torch
 
 from . import _native
 from ._native import SEG_DECAY, SEG_F32, SEG_GLU_CLAMP, SEG_GLU_SILU, SEG_RELU2, SEG_SOFTCAP, SEG_STORE  # noqa: F401
-from .batch import batch_op_begin, dev_status_ptr, reference_op, validate_buffer_shape_2d
+from .batch import batch_op_begin, dev_status_ptr, reference_op, scratch as memory, validate_buffer_shape_2d
 from .kv_cache import _ptr, cache_strides, dtype_code
 from .types import GPUBuffer1D, GPUBuffer2D, GPUContext, KVCache
 
@@ -173,9 +173,7 @@ def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Se
     if scratch is not None and rows > 128 and x.buffer.dtype == torch.float32:
         nbytes = _native.lib.b2kv_linear_workspace_bytes(a)
         if nbytes:
-            ws = scratch.get("linear")
-            if ws is None or ws.numel() < nbytes:
-                ws = scratch["linear"] = torch.empty(nbytes, dtype=torch.uint8, device=x.buffer.device)
+            ws = scratch["linear"] = memory(scratch.get("linear"), nbytes, x.buffer.device)
     stream = batch_op_begin(ctx)
     _native.check(_native.lib.b2kv_linear_ws(a, options, None if ws is None else ws.data_ptr(), 0 if ws is None else ws.numel(),
                                              dev_status_ptr(ctx), stream))

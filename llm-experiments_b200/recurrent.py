@@ -14,7 +14,7 @@ from typing import Tuple
 import torch
 
 from . import _native
-from .batch import batch_op_begin, dev_status_ptr, reference_op
+from .batch import batch_op_begin, dev_status_ptr, reference_op, scratch
 from .kv_cache import dtype_code
 from .serving import RowSegments
 from .types import GPUBuffer1D, GPUBuffer2D, GPUContext
@@ -47,8 +47,8 @@ def gated_linear_attention(ctx: GPUContext, y: GPUBuffer2D, cols: Tuple[int, int
         raise ValueError("gated_linear_attention: alpha and norm are float32, out has the type of y")
     dt = dtype_code(y.buffer.dtype)
     nbytes = _native.lib.b2kv_gla_workspace_bytes(shape.heads, shape.dim, shape.vdim, segments.count, segments.max_n, dt, path)
-    if nbytes and (ctx.recurrent_workspace is None or ctx.recurrent_workspace.numel() < nbytes):
-        ctx.recurrent_workspace = torch.empty(nbytes, dtype=torch.uint8, device=ctx.device)
+    if nbytes:
+        ctx.recurrent_workspace = scratch(ctx.recurrent_workspace, nbytes, ctx.device)
     a = _native.GlaArgs(
         y=y.buffer.data_ptr(), alpha=alpha.buffer.data_ptr(), norm=norm.buffer.data_ptr(), state=state.data_ptr(), out=out.buffer.data_ptr(),
         segments=None if segments.table is None else segments.table.data_ptr(), row_pos=pos.data_ptr(),

@@ -17,7 +17,7 @@ import torch
 
 from ._native import check as _check
 from ._native import lib as _lib
-from .batch import batch_begin, batch_commit, batch_op_begin, current_handle
+from .batch import batch_begin, batch_commit, batch_op_begin, current_handle, give_up
 from .latent import PromptPlan, RowPlaces
 from .step_tail import argmax
 from .types import GPUBuffer1D, GPUBuffer2D, GPUContext, KVCache
@@ -97,6 +97,7 @@ class SequenceState:
         self._lengths_event = None  # behind the last copy of lengths to the device, and the raw handle of its stream (None: it has ended)
         self._lengths_stream = None
         self.captured = False     # a graph holds one of the steps: they are replayed without a call of this module
+        self._held = {}           # the memory that captured steps work in, by its address
         self._bare = None if self.owned else KVCache(layers=[], batch_size=self.batch_size, max_seq_len=self.max_seq_len,
                                                      current_len=0, n_heads=0, head_dim=0, seq_lens=self.seq_lens)
 
@@ -119,9 +120,17 @@ class SequenceState:
         writes are multiplied with zero weights and must be numbers."""
         t = self.scratch.get(name)
         if t is None or t.shape[0] < rows or t.shape[1] != cols:
+            give_up(t)
             t = torch.zeros((rows, cols), dtype=dtype, device=self.seq_lens.device)
             self.scratch[name] = t
         return GPUBuffer2D(buffer=t[:rows], shape=(rows, cols), size=rows * cols)
+
+    def hold(self) -> None:
+        """Behind a captured step: the memory it works in stays with the state.  A graph knows it by its address alone, and a larger step
+        replaces what has become too small."""
+        for t in (*self.scratch.values(), *(c.workspace for c in self.caches)):
+            if t is not None:
+                self._held[t.data_ptr()] = t
 
     def advance_host(self, n: int = 1) -> None:
         """Host-side part of advancing every sequence by ``n`` tokens."""
@@ -180,13 +189,16 @@ def decode_step(ctx: GPUContext, state: SequenceState, token_ids: GPUBuffer1D, n
     if upper >= state.max_seq_len:
         raise ValueError(f"Cache is full: current_len={upper}, max_seq_len={state.max_seq_len}")
     B = state.batch_size
-    state.captured = state.captured or (state.seq_lens.is_cuda and torch.cuda.is_current_stream_capturing())
+    capturing = state.seq_lens.is_cuda and torch.cuda.is_current_stream_capturing()
+    state.captured = state.captured or capturing
     state.wait_for_lengths()
     state.run(ctx, Step(ids=token_ids.buffer, places=RowPlaces(None, state.seq_lens), rows=B, n_single=B, n_few=B, span=upper + 1, plans={},
                         short=RowSegments(None, B, 1), long=None, row_index=None, n_out=B))
     if next_ids is not None:
         argmax(ctx, state.logits, next_ids)
     _check(_lib.b2kv_advance_lengths(state.seq_lens.data_ptr(), B, 1, batch_op_begin(ctx)))
+    if capturing:
+        state.hold()
     state.lengths = [v + 1 for v in state.lengths]
     for c in state.caches:
         c.current_len += 1

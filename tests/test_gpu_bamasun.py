@@ -251,6 +251,43 @@ def test_lengths_set_on_one_stream_and_a_step_on_another(pkg, how):
         assert torch.equal(got, expected) and state.seq_lens.tolist() == [v + 1 for v in n] == state.lengths
 
 
+def test_a_captured_step_keeps_its_memory(pkg):
+    """A captured step of many fp32 sequences, whose products lay their operands out in scratch memory; then a larger step, which needs more of
+    everything; then other tensors wherever the memory was.  The graph's step is the same as before, and so are the tensors."""
+    from llm_experiments_b200 import serving
+    from llm_experiments_b200.model import GraphedDecodeStep
+
+    pair = U.config([U.attention(4, 2, 64, 64, ff=4096), U.gla(2, 64, 64, 4.0, 8, 4096)], vocab=64, width=1024)
+    model, cfg = build_from(pkg, pair[0], U.weights(pair), F32, 264, 340), pair[0]
+    ctx, state = model.ctx, model.state
+    ctx.config.check_device_status = False
+    model.forward([(i, U.tokens(cfg, 3 + i % 4, i), []) for i in range(264)])
+    state.scratch.clear()  # (as a program that decodes first)
+    lens, kept = list(state.lengths), {i: t.clone() for i, t in state.recurrent.items()}
+    graphed = GraphedDecodeStep(ctx, state, step_fn=serving.decode_step)
+    graphed.token_ids.buffer.fill_(5)
+    graphed.capture()
+    logits = state.logits
+
+    def step():
+        serving.state_set_lengths(state, lens)
+        for i, t in state.recurrent.items():
+            t.copy_(kept[i])
+        graphed.step()
+        torch.cuda.synchronize()
+        return logits.buffer.clone()
+
+    want, old = step(), {t.data_ptr(): t.numel() * t.element_size() for t in state.scratch.values()}
+    assert "linear" in state.scratch
+    serving.state_set_lengths(state, lens)
+    model.forward([(0, U.tokens(cfg, 320, 7), [0])] + [(i, U.tokens(cfg, 2, i), [0, 1]) for i in range(1, 264)])
+    torch.cuda.synchronize()
+    assert state.scratch["linear"].data_ptr() not in old
+    fill = [torch.full((n,), 3, dtype=torch.uint8, device="cuda") for n in old.values() for _ in range(2)]
+    got = step()
+    assert torch.equal(got, want) and all(bool((t == 3).all()) for t in fill)
+
+
 @pytest.mark.parametrize("name", ["ODD", "TC", "ONLY_GLA"])
 def test_greedy_generation_matches_the_oracle(pkg, name):
     """generate_text over the registry's model, fp32: the oracle's greedy tokens."""

@@ -210,3 +210,46 @@ def test_a_recurrence_workspace_is_enough_for_fewer_segments(pkg, heads, dim, vd
     size = lambda n, t: pkg._native.lib.b2kv_gla_workspace_bytes(heads, dim, vdim, n, t, pkg._native.DTYPE_BF16, 0)  # noqa: E731
     sizes = [size(n, max_n) for n in range(1, 65)]
     assert sizes == sorted(sizes) and 0 < size(7, max_n // 2) <= size(7, max_n)
+
+
+def test_memory_of_a_captured_step_stays_when_it_is_replaced(pkg, ctx, monkeypatch):
+    """A graph knows a step's scratch memory by its address: what later steps replace is not given back, and nothing else is kept."""
+    import types
+    import weakref
+
+    from llm_experiments_b200 import batch, serving
+
+    class State(serving.SequenceState):
+        def run(self, ctx, step):
+            self.rows("x", step.rows, 4, torch.float32)
+            self.scratch["linear"] = batch.scratch(self.scratch.get("linear"), 100 * step.rows, torch.device("cpu"))
+            for c in self.caches:
+                c.workspace = batch.scratch(c.workspace, 10 * step.rows, torch.device("cpu"))
+
+    cache = pkg.gpu.kv_cache_create(ctx, _cfg(pkg.gpu, n_layers=1, ragged=True))
+    lens = types.SimpleNamespace(is_cuda=True, device=torch.device("cpu"), data_ptr=lambda: 0)
+    state = State(batch_size=2, max_seq_len=8, dtype=torch.float32, owned={0: cache}, seq_lens=lens, lengths=[0, 0])
+    monkeypatch.setattr(serving, "_lib", types.SimpleNamespace(b2kv_advance_lengths=lambda *a: 0))
+    monkeypatch.setattr(serving, "batch_op_begin", lambda ctx: 0)
+    capturing = [False]
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
+    alive = []
+
+    def step(rows):
+        state.run(ctx, types.SimpleNamespace(rows=rows))
+        alive.append([weakref.ref(t) for t in (state.scratch["x"], state.scratch["linear"], cache.workspace)])
+
+    token = types.SimpleNamespace(buffer=None)
+    serving.decode_step(ctx, state, token)
+    step(2)
+    step(5)
+    assert [r() is None for r in alive[0]] == [True] * 3  # (no graph yet)
+    capturing[0] = True
+    serving.decode_step(ctx, state, token)
+    capturing[0] = False
+    assert state.captured
+    for rows in (9, 17):
+        step(rows)
+    assert [r() is None for r in alive[1]] == [False] * 3  # the captured step's
+    assert [r() is None for r in alive[2]] == [True] * 3  # what came behind it and was too small in its turn
+    assert state.scratch["linear"].numel() == 1700 and state.scratch["x"].shape == (17, 4)
