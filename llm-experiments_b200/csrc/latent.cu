@@ -163,19 +163,38 @@ latent_append_warps_kernel(T* y, int64_t ld_y, int H, int dim, int rot, int rot_
         }
     }
     if (!own) return;
-    float sum = 0.f;
-    auto squares = [&](const uint4& p) {
+    // The squares in the order of latent_append_kernel, so that a token's latents do not depend on how many rows are in the step: element i is
+    // thread i % 256's there, and its warps' sums follow one another.  A piece's elements belong to threads side by side, those of a lane's
+    // pieces to the same ones again every kSets pieces.
+    constexpr int kSets = kAppendThreads / (32 * kC), kLanes = 32 / kC;  // kLanes: lanes that hold the threads of one warp there
+    float squares[kSets][kC] = {};
+    auto add = [&](int u, const uint4& p) {
         float f[kC];
         Elt<T>::widen(p, f);
 #pragma unroll
-        for (int e = 0; e < kC; ++e) sum = fmaf(f[e], f[e], sum);
+        for (int set = 0; set < kSets; ++set)
+#pragma unroll
+            for (int e = 0; e < kC; ++e)
+                if (u % kSets == set) squares[set][e] = fmaf(f[e], f[e], squares[set][e]);
     };
 #pragma unroll
     for (int u = 0; u < kKeep; ++u)
-        if (lane + 32 * u < lat_pieces) squares(keep[u]);
-    for (int i = lane + 32 * kKeep; i < lat_pieces; i += 32) squares(lat[i]);
+        if (lane + 32 * u < lat_pieces) add(u, keep[u]);
+    for (int u = kKeep; lane + 32 * u < lat_pieces; ++u) add(u, lat[lane + 32 * u]);
+    float sum = 0.f;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    for (int set = 0; set < kSets; ++set) {
+#pragma unroll
+        for (int off = kLanes / 2; off > 0; off >>= 1)
+#pragma unroll
+            for (int e = 0; e < kC; ++e) squares[set][e] += __shfl_xor_sync(0xffffffffu, squares[set][e], off);
+#pragma unroll
+        for (int off = kC / 2; off > 0; off >>= 1)
+#pragma unroll
+            for (int e = 0; e < off; ++e) squares[set][e] += squares[set][e + off];
+#pragma unroll
+        for (int w = 0; w < 32 / kLanes; ++w) sum += __shfl_sync(0xffffffffu, squares[set][0], w * kLanes);
+    }
     const float scale = 1.0f / sqrtf(sum / static_cast<float>(kv_rank) + eps);
     const int64_t place = static_cast<int64_t>(slot) * T_max + pos;
     uint4* const latent = reinterpret_cast<uint4*>(latent_cache + place * kv_rank);
@@ -303,8 +322,9 @@ extern "C" int b2kv_latent_append(void* y, int64_t ld_y, int H, int dim, int rot
     if (latent_cache && (!w_norm || kv_rank <= 0 || down_col < 0 || ld_y < down_col + kv_rank + rot)) return B2KV_ERR_BAD_ARG;
     const int per = 16 / elt_bytes(dtype);
     const bool vec = aligned16(y) && ld_y % per == 0 && dim % per == 0 && rot % per == 0 && (rot_dims / 2) % per == 0;
-    // a warp per row where that gives every SM several rows (few rows: a CTA each is quicker, its threads share the row's pieces)
-    if (vec && rows >= 512 && rot_dims / 2 <= kWarpHalf && (rot_dims / 2) / per <= 32 &&
+    // A warp per row where a CTA per row does not fit the device at once (six per SM), which then takes two turns: us with a CTA and
+    // with a warp each, 16 heads, bf16: 512 rows 4.3, 4.7; 888 4.5, 5.1; 896 6.2, 5.1; 2000 9.3, 5.3.  32 heads: 888 4.7, 6.1; 896 6.3, 6.1; 2000 9.5, 6.3.
+    if (vec && rows > 6 * device_sm_count() && rot_dims / 2 <= kWarpHalf && (rot_dims / 2) / per <= 32 &&
         (latent_cache == nullptr || (kv_rank % per == 0 && down_col % per == 0 && aligned16(latent_cache) && aligned16(key_cache)))) {
         OverlapLaunch warps((rows + kWarpRows - 1) / kWarpRows, kAppendThreads, 0, stream);
         if (dtype == B2KV_DTYPE_F32)

@@ -60,14 +60,14 @@ def test_latent_rows_by_warps_and_by_ctas(pkg, dtype, H, rot, dims, rank, own):
     """As many rows as take a warp each against the same ones in portions that take a CTA each: rotations and copies bit for bit."""
     from llm_experiments_b200 import latent
 
-    ctx, rows, dim = make_ctx(pkg), 517, 24
+    ctx, rows, dim = make_ctx(pkg), 917, 24
     ctx.config.check_device_status = True
     shape = latent.LatentShape(H, dim, rot, dims, 8, rank, 0, 1.0)
     y = rnd((rows, H * (dim + rot) + rank + rot + 8), dtype, 5)
     w, inv = rnd((rank,), F32, 6) + 1, b1(pkg, 10000.0 ** (-torch.arange(dims // 2, device="cuda") / (dims // 2)))
-    pos, got = torch.randperm(600, device="cuda")[:rows].to(torch.int32), []
+    pos, got = torch.randperm(1000, device="cuda")[:rows].to(torch.int32), []
     for step in (rows, 200):
-        cache = pkg.gpu.kv_cache_create(ctx, pkg.gpu.KVCacheConfig(batch_size=1, max_seq_len=600, n_layers=1, n_heads=1, head_dim=rot, v_head_dim=rank,
+        cache = pkg.gpu.kv_cache_create(ctx, pkg.gpu.KVCacheConfig(batch_size=1, max_seq_len=1000, n_layers=1, n_heads=1, head_dim=rot, v_head_dim=rank,
                                                                    dtype=dtype, ragged=True))
         mine = y.clone()
         for r in range(0, rows, step):
@@ -82,15 +82,38 @@ def test_latent_rows_by_warps_and_by_ctas(pkg, dtype, H, rot, dims, rank, own):
         lat = y[:, H * (dim + rot):][:, :rank].double()
         want = lat / torch.sqrt((lat * lat).mean(-1, keepdim=True) + 1e-5) * w.double()
         for _, _, v in got:
-            norm_close(v.view(600, rank)[pos.long()], want, dtype)
+            norm_close(v.view(1000, rank)[pos.long()], want, dtype)
     else:
         assert not got[0][2].any()
+
+
+@pytest.mark.parametrize("dtype", [F32, BF])
+@pytest.mark.parametrize("rank", [8, 72, 264, 512, 1096])
+def test_latents_do_not_depend_on_the_rows_of_a_step(pkg, dtype, rank):
+    """A token's latent has the same bits in a step of 1200 rows, of 200, and alone."""
+    from llm_experiments_b200 import latent
+
+    ctx, rows, rot = make_ctx(pkg), 1200, 16
+    y, w, inv = rnd((rows, 24 + rot + rank + rot), dtype, 8), rnd((rank,), F32, 9) + 1, b1(pkg, torch.ones(rot // 2, device="cuda"))
+    got = []
+    for step in (rows, 200, 1):
+        cache = pkg.gpu.kv_cache_create(ctx, pkg.gpu.KVCacheConfig(batch_size=1, max_seq_len=rows, n_layers=1, n_heads=1, head_dim=rot, v_head_dim=rank,
+                                                                   dtype=dtype, ragged=True))
+        mine = y.clone()
+        for r in range(0, rows, step)[:20]:
+            pos = torch.arange(r, r + step, dtype=torch.int32, device="cuda")
+            pkg.gpu.batch_begin(ctx)
+            pkg.gpu.latent_append(ctx, wrap(pkg, mine[r:r + step]), latent.LatentShape(1, 24, rot, rot, 8, rank, 0, 1.0), inv,
+                                  latent.RowPlaces(torch.zeros_like(pos), pos), cache, b1(pkg, w), 1e-5)
+            pkg.gpu.batch_commit(ctx)
+        got.append(cache.layers[0].v_cache.buffer.view(rows, rank))
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0][:20], got[2][:20])
 
 
 def test_a_position_outside_the_cache_is_reported_among_many_rows(pkg):
     from llm_experiments_b200 import latent
 
-    ctx, rows = make_ctx(pkg), 600
+    ctx, rows = make_ctx(pkg), 900
     ctx.config.check_device_status = True
     cache = pkg.gpu.kv_cache_create(ctx, pkg.gpu.KVCacheConfig(batch_size=1, max_seq_len=rows, n_layers=1, n_heads=1, head_dim=16, v_head_dim=64, dtype=BF, ragged=True))
     y, pos = rnd((rows, 40 + 80), BF, 7), torch.arange(rows, dtype=torch.int32, device="cuda")
