@@ -161,15 +161,17 @@ __global__ void __launch_bounds__(kCtaThreads) row_kernel(const T* __restrict__ 
 
 // Layer norm of the few rows of a decode step: latency, and nothing else.  A row has a CTA of 512 threads, and everything that is read is on
 // its way together (8 rows of 4096 bf16 between two products of a step: it ends 2.8 us behind the one ahead; by 128 threads, with gamma and
-// beta read behind the sums, 7.9 us).
-constexpr int kFewThreads = 512, kFewChunks = 4;  // rows of up to 8192 elements
-template <typename T, int kChunks>
+// beta read behind the sums, 7.9 us).  The sums are row_kernel's to the bit, so that a row does not depend on how many there are: its kTpr
+// threads' chunks are spread over the CTA, and their sums added up in its order.
+constexpr int kFewThreads = 512;
+template <typename T, int kTpr>
 __global__ void __launch_bounds__(kFewThreads) layernorm_few_kernel(const T* x, const T* ga, const T* be, T* y, int size, float eps) {
-    __shared__ float scratch[kFewThreads / 32];
+    constexpr int kShares = kFewThreads / kTpr, kChunks = kMaxRegChunks / kShares;
+    __shared__ float scratch[kFewThreads / 32], part[kMaxRegChunks][kTpr];
     grid_launch_dependents();
     if (threadIdx.x == 0) grid_dependency_wait();
     __syncthreads();
-    const int chunks = size / 4;
+    const int chunks = size / 4, t = threadIdx.x % kTpr;
     const T* const xr = x + static_cast<int64_t>(blockIdx.x) * size;
     float4 keep[kChunks], g[kChunks], b[kChunks];
 #pragma unroll
@@ -178,35 +180,48 @@ __global__ void __launch_bounds__(kFewThreads) layernorm_few_kernel(const T* x, 
         keep[c] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i < chunks) keep[c] = load4(xr, i), g[c] = load4(ga, i), b[c] = load4(be, i);
     }
-    float acc = 0.f;
+    auto sum = [&](const float (&of)[kChunks]) {
 #pragma unroll
-    for (int c = 0; c < kChunks; ++c) acc += (keep[c].x + keep[c].y) + (keep[c].z + keep[c].w);
-    const float mean = row_reduce<SumOp, kFewThreads>(acc, scratch) / static_cast<float>(size);
-    acc = 0.f;
+        for (int c = 0; c < kChunks; ++c) part[c * kShares + threadIdx.x / kTpr][t] = of[c];
+        __syncthreads();
+        float acc = 0.f;
+#pragma unroll
+        for (int c = 0; c < kMaxRegChunks; ++c) acc += part[c][t];
+        return row_reduce<SumOp, kTpr>(acc, scratch);  // (its barriers are between two uses of `part`)
+    };
+    float of[kChunks];
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c) of[c] = (keep[c].x + keep[c].y) + (keep[c].z + keep[c].w);
+    const float mean = sum(of) / static_cast<float>(size);
 #pragma unroll
     for (int c = 0; c < kChunks; ++c) {
         float4& v = keep[c];
         v.x -= mean, v.y -= mean, v.z -= mean, v.w -= mean;
-        if (static_cast<int>(threadIdx.x) + c * kFewThreads < chunks) acc += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+        of[c] = static_cast<int>(threadIdx.x) + c * kFewThreads < chunks ? (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w) : 0.f;
     }
-    const float scale = 1.0f / sqrtf(row_reduce<SumOp, kFewThreads>(acc, scratch) / static_cast<float>(size) + eps);
+    const float scale = 1.0f / sqrtf(sum(of) / static_cast<float>(size) + eps);
     T* const yr = y + static_cast<int64_t>(blockIdx.x) * size;
 #pragma unroll
     for (int c = 0; c < kChunks; ++c) {
         const int i = threadIdx.x + c * kFewThreads;
         if (i < chunks) {
-            const float4 v = keep[c];
-            store4(yr, i, make_float4(v.x * scale * g[c].x + b[c].x, v.y * scale * g[c].y + b[c].y, v.z * scale * g[c].z + b[c].z,
-                                      v.w * scale * g[c].w + b[c].w));
+            float4 v = keep[c];
+            v.x = v.x * scale * g[c].x + b[c].x, v.y = v.y * scale * g[c].y + b[c].y;
+            v.z = v.z * scale * g[c].z + b[c].z, v.w = v.w * scale * g[c].w + b[c].w;
+            store4(yr, i, v);
         }
     }
 }
 
+// Threads per row by row length (in 16-byte chunks when the row can be vectorised).
+int threads_per_row(int size) {
+    const int work = size % 4 == 0 ? size / 4 : size;
+    return work <= 64 ? 32 : (work <= 256 ? 64 : (work <= 1024 ? 128 : 256));
+}
+
 template <int kMode, typename T>
 int launch_rows(const T* x, const T* ga, const T* be, T* y, int64_t rows, int size, float eps, cudaStream_t stream) {
-    // threads per row by row length (in 16-byte chunks when the row can be vectorised)
-    const int work = size % 4 == 0 ? size / 4 : size;
-    const int tpr = work <= 64 ? 32 : (work <= 256 ? 64 : (work <= 1024 ? 128 : 256));
+    const int tpr = threads_per_row(size);
     const int64_t ctas = (rows + kCtaThreads / tpr - 1) / (kCtaThreads / tpr);
     if (ctas > 0x7fffffffLL) return B2KV_ERR_UNSUPPORTED;
     const unsigned grid = static_cast<unsigned>(ctas);
@@ -222,10 +237,11 @@ int launch_rows(const T* x, const T* ga, const T* be, T* y, int64_t rows, int si
 
 template <typename T>
 int launch_layernorm(const T* x, const T* ga, const T* be, T* y, int64_t rows, int size, float eps, cudaStream_t stream) {
-    if (rows > device_sm_count() || size < 2048 || size % 4 != 0 || size > 4 * kFewThreads * kFewChunks)
+    const int tpr = threads_per_row(size);
+    if (rows > device_sm_count() || size < 2048 || size % 4 != 0 || size > 4 * tpr * kMaxRegChunks)
         return launch_rows<0, T>(x, ga, be, y, rows, size, eps, stream);
     OverlapLaunch launch(static_cast<unsigned>(rows), kFewThreads, 0, stream);
-    auto kernel = size <= 4 * kFewThreads ? layernorm_few_kernel<T, 1> : (size <= 8 * kFewThreads ? layernorm_few_kernel<T, 2> : layernorm_few_kernel<T, 4>);
+    auto kernel = tpr == 128 ? layernorm_few_kernel<T, 128> : layernorm_few_kernel<T, 256>;
     B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, kernel, x, ga, be, y, size, eps));
     return B2KV_OK;
 }

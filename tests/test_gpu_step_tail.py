@@ -179,7 +179,7 @@ def test_embedding_reports_ids_outside_the_table(pkg, ctx):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("n,size", [(1, 2048), (8, 4096), (148, 2052), (149, 2052), (3, 8188), (2, 8196), (5, 6000)])
 def test_layernorm_of_few_wide_rows(pkg, ctx, dtype, n, size):
-    """A row per CTA of 512 threads, its edges in rows and in width, a guard behind."""
+    """A row per CTA, its edges in rows and in width, a guard behind."""
     x = U.randn((n, size), dtype, ctx.device, 31) * 2 + 1
     g, b = (U.randn((size,), dtype, ctx.device, s) for s in (32, 33))
     out = torch.full((n + 1, size), 7.0, dtype=dtype, device=ctx.device)
@@ -208,3 +208,20 @@ def test_argmax_of_any_width(pkg, ctx, dtype, size):
     pkg.gpu.batch_commit(ctx)
     first = int((x[0] == x[0].max()).nonzero()[0])
     assert out.tolist() == [first, size // 2, 0, 0, size - 1, -7]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("size", [2048, 2052, 4096, 6000, 8192])
+def test_layernorm_of_a_row_does_not_depend_on_the_others(pkg, ctx, dtype, size):
+    """The same bits whether a few rows take a CTA each or many rows share CTAs: one order of sums for a width."""
+    n = 400
+    x = U.randn((n, size), dtype, ctx.device, 35) * 2 + 1
+    g, b = (U.randn((size,), dtype, ctx.device, s) for s in (36, 37))
+    one = lambda t: pkg.gpu.GPUBuffer1D(buffer=t, shape=tuple(t.shape), size=t.numel())  # noqa: E731
+    out = [torch.empty_like(x) for _ in range(2)]
+    pkg.gpu.batch_begin(ctx)
+    for step, y in zip((n, 100), out):
+        for r in range(0, n, step):
+            pkg.gpu.layernorm(ctx, U.buf2d(pkg, ctx, x[r:r + step]), one(g), one(b), U.buf2d(pkg, ctx, y[r:r + step]))
+    pkg.gpu.batch_commit(ctx)
+    assert torch.equal(out[0], out[1])
