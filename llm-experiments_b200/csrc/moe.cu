@@ -265,9 +265,12 @@ extern "C" int b2kv_route(const float* logits, int64_t ld, int rows, int experts
     OverlapLaunch zero(1, 256, 0, stream);
     B2KV_CUDA_TRY(cudaLaunchKernelEx(&zero.cfg, zero_counts_kernel, counts, 2 * experts));
     const size_t many_bytes = (static_cast<size_t>(kRouteWarpsMany) * 2 + 1) * experts * sizeof(float);
-    // (1500 rows: 6.9 us and 8.2, but the kernel behind begins later, 20.4 and 18.8 together; 3001 rows, 6 of 160 experts, of whose 192 choices few meet:
-    // 14.8 and 12.0)
-    const bool many = rows >= 2048 && kRouteWarpsMany * top >= 3 * experts && many_bytes <= 48 * 1024;
+    // CTAs of 32 rows where many of their choices meet and there are choices enough for counting to be what takes the time; us with four rows and
+    // with 32.  2048 rows: 4 of 32 experts 9.5, 8.4; 6 of 64 12.4, 11.9; 8 of 64 15.0, 12.8.  3001: 2 of 16 8.4, 8.6; 4 of 32 11.5, 10.8; 6 of 64
+    // 15.9, 13.8.  8000: 2 of 16 15.7, 10.0; 6 of 64 36, 15.  With fewer that meet, 3001 rows: 4 of 64 12.1, 12.0; 6 of 96 12.9, 14.8; 6 of
+    // 160 13.2, 16.0 (from some 4500 rows on it would pay there too: 4 of 64 16.1, 12.6; 8000 rows, 6 of 160 25, 18).  1500 rows, 6 of 64: 10.1 and 9.3, but
+    // the kernel behind begins later, 18.8 and 20.4 together.
+    const bool many = rows >= 2048 && static_cast<long long>(rows) * top >= 8192 && kRouteWarpsMany * top >= 3 * experts && many_bytes <= 48 * 1024;
     const int warps = many ? kRouteWarpsMany : kRouteWarps;
     OverlapLaunch launch((rows + warps - 1) / warps, warps * 32, many ? many_bytes : static_cast<size_t>(kRouteWarps) * 2 * experts * sizeof(float), stream);
     B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, many ? route_kernel<kRouteWarpsMany> : route_kernel<kRouteWarps>, logits, ld, rows, experts, groups, keep,
