@@ -6,20 +6,16 @@
 //   o_t  = S^T (q_t P_t) + sum_{s <= t} A_ts v_s,   A_ts = sum_d q_td k_sd prod_{s < r <= t} alpha_rd
 //   S   <- diag(P_last) S + sum_s (k_s R_s) v_s^T
 //
-// Three kernels, five for more than a span of chunks.  What does not depend on the state is made for many chunks at once (gla_prepare_kernel): one CTA per chunk and
+// Three kernels.  What does not depend on the state is made for many chunks at once (gla_prepare_kernel): one CTA per chunk and
 // head, thread = two key channels; A's products of decays are carried along exactly instead of being taken apart into factors that
 // could overflow, and its entries are summed over the channels 32 at a time.  The result is a record per chunk and head that is
 // byte for byte what the second kernel wants in shared memory.  Records are made a slice of the segments at a time, which bounds the
 // workspace.
 //
-// gla_state_kernel has one CTA per (64 value columns of a head, segment, span of 16 chunks) and walks the span's chunks in order.  Nothing in the
-// recurrence connects value columns, and a chunk is a chain of dependent products, so what counts is how few warps share an SM's tensor pipe:
-// one or two per scheduler here.  The chain over a whole segment is what took the time (two prompts of 1750 tokens, 8 heads of 128 x 256: 64 CTAs,
-// 109 chunks of 1.66 us one after the other), so it is cut.  A first pass of the kernel makes every span's own part of the state from zero
-// (all but the last one's), gla_combine_kernel carries them through, S <- diag(P_16) .. diag(P_1) S + L, decay after decay as a chain would, and leaves
-// what each span begins with, the second pass walks all spans side by side: half as many products again; from the
-// records to the outputs 117 us, 201 as one chain.
-// Spans begin at multiples of 16 chunks from the segment's first token, whatever else is in the step, and so the sums are in one order.
+// gla_state_kernel has one CTA per (64 value columns of a head, segment) and walks the chunks in order.  Nothing in the recurrence
+// connects value columns, and a chunk is a chain of dependent products, so what counts is how few warps share an SM's tensor pipe:
+// one per scheduler here (with a whole head's 256 columns on one SM a prompt of 2048 tokens kept 8 SMs busy: two prompts of 1750 tokens, 8 heads of
+// 128 x 256, took 366 us, 181 so).
 //   * every warp owns 16 value columns of the state, transposed, as accumulators of mma.m16n8k16: the state never
 //     leaves registers between the first and the last chunk.  As an A operand of the first product the accumulators need no
 //     shuffle.  A step of the recurrence is sixteen tokens deep, one k-step of this instruction; larger tiles would have to
@@ -52,9 +48,7 @@ constexpr int kBox = 32;                           // value columns per copy of 
 constexpr int kMaxRing = 6;
 constexpr int kSmemLimit = 109 * 1024;     // two CTAs per SM
 constexpr size_t kSliceBytes = 128u << 20;  // records and o of a slice, at most (but at least kMinSlice chunks per segment)
-constexpr int kSpan = 16;     // chunks per span
-constexpr int kMinSlice = kSpan;
-constexpr int kMaxSpans = 4096;  // of a slice
+constexpr int kMinSlice = 8;
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
     asm volatile(
@@ -96,7 +90,7 @@ struct alignas(128) Record {
     float decay[kD];  // P_last
 };
 
-// Chunks [first, first + count) of every segment (whole spans, but for the last slice); record (segment, head, chunk) at ((segment * H + head) * count + chunk - first).
+// Chunks [first, first + count) of every segment; record (segment, head, chunk) at ((segment * H + head) * count + chunk - first).
 struct Slice {
     int first, count;
 };
@@ -219,15 +213,6 @@ __host__ __device__ inline int64_t record_count(const b2kv_gla_args& a, const Sl
     return static_cast<int64_t>(a.n_segments) * a.H * slice.count;
 }
 
-// What the spans of a slice begin with (and before that their own part of the state): [segment][span][head][dim][vdim] behind o.
-__host__ __device__ inline int spans_of(int chunks) { return (chunks + kSpan - 1) / kSpan; }
-template <typename R>
-__device__ __forceinline__ float* span_state(const b2kv_gla_args& a, const Slice& slice, int segment, int span, int h) {
-    float* const o = reinterpret_cast<float*>(reinterpret_cast<R*>(a.workspace) + record_count(a, slice));
-    return o + static_cast<int64_t>(a.n_segments) * slice.count * kChunk * a.H * a.vdim +
-           ((static_cast<int64_t>(segment) * spans_of(slice.count) + span) * a.H + h) * a.dim * a.vdim;
-}
-
 // One place of the ring: the record, then the CTA's part of v in boxes of 32 columns (64-byte swizzle).
 constexpr int kBoxBytes = kChunk * kBox * 2;
 __host__ __device__ constexpr int v_offset(int record) { return (record + 1023) / 1024 * 1024; }
@@ -237,11 +222,10 @@ struct Shared {
     alignas(8) uint64_t full[kMaxRing], empty[kMaxRing];
 };
 
-// kOwn: only the span's own part of the state, from zero.  spans: states begin with what gla_combine_kernel left (otherwise with a.state).
-template <int kD16, bool kOwn>
+template <int kD16>
 __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_constant__ CUtensorMap tm_v,
                                                                   const __grid_constant__ b2kv_gla_args a, const Slice slice,
-                                                                  int parts, int n_ring, bool spans, int32_t* dev_status) {
+                                                                  int parts, int n_ring, int32_t* dev_status) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ Shared sm;
     using R = Record<kD16>;
@@ -256,11 +240,8 @@ __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_
     __syncthreads();
     b2kv_row_segment sg;
     if (!segment_place(a, blockIdx.y, sg)) return;  // (reported by the other kernel)
-    const int span = blockIdx.z, all_chunks = (sg.n + kChunk - 1) / kChunk, first = slice.first + span * kSpan;
-    const int chunks = spans ? min(min(all_chunks - first, kSpan), slice.count - span * kSpan) : min(all_chunks - first, slice.count);
+    const int chunks = min((sg.n + kChunk - 1) / kChunk - slice.first, slice.count);
     if (chunks <= 0) return;
-    const bool last = first + chunks == all_chunks;
-    if (kOwn && last) return;  // (nobody asks what it leaves: the second pass does)
     const int v0 = (part * kWarps + warp) * kSlab;  // this warp's first value column
     const int left = a.vdim - part * kWarps * kSlab;
     const int n_warps = min(kWarps, (left + kSlab - 1) / kSlab), boxes = (min(left, kWarps * kSlab) + kBox - 1) / kBox;
@@ -274,11 +255,11 @@ __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_
     __syncthreads();
     if (warp >= n_warps) return;  // (there are no barriers of the whole CTA from here on)
     bool ok = true;
-    const int row0 = sg.row0 + first * kChunk, rows_left = sg.n - first * kChunk;
+    const int row0 = sg.row0 + slice.first * kChunk, rows_left = sg.n - slice.first * kChunk;
 
-    const R* const records = reinterpret_cast<const R*>(a.workspace) + (static_cast<int64_t>(blockIdx.y) * a.H + h) * slice.count + span * kSpan;
+    const R* const records = reinterpret_cast<const R*>(a.workspace) + (static_cast<int64_t>(blockIdx.y) * a.H + h) * slice.count;
     float* const o_rows = reinterpret_cast<float*>(reinterpret_cast<R*>(a.workspace) + record_count(a, slice)) +
-                          ((static_cast<int64_t>(blockIdx.y) * slice.count + span * kSpan) * kChunk * a.H + h) * a.vdim;
+                          ((static_cast<int64_t>(blockIdx.y) * slice.count * kChunk) * a.H + h) * a.vdim;
     auto request = [&](int ci, int slot) {
         uint8_t* const dst = ring + slot * kStride;
         uint64_t* const bar = &sm.full[slot];
@@ -293,8 +274,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_
     // ------------------------------ state: 16 value columns per warp ------------------------------
     const int row = lane >> 2, col = (lane & 3) * 2;  // place of this thread's first accumulator in a tile
     float* const state = a.state + (static_cast<int64_t>(sg.slot) * a.H + h) * a.dim * a.vdim;
-    float* const span_at = span_state<R>(a, slice, blockIdx.y, span, h);
-    const bool fresh = kOwn || (!spans && slice.first == 0 && a.row_pos[sg.row0] == 0);
+    const bool fresh = slice.first == 0 && a.row_pos[sg.row0] == 0;
     float c[2 * kD16][4];  // [tile of 8 key channels]
     auto each_state = [&](auto&& fn) {
 #pragma unroll
@@ -305,8 +285,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_
                 fn(c[j][e], static_cast<int64_t>(d) * a.vdim + v, v < a.vdim && d < a.dim);
             }
     };
-    const float* const begin = spans ? span_at : state;
-    each_state([&](float& x, int64_t at, bool live) { x = live && !fresh ? begin[at] : 0.f; });
+    each_state([&](float& x, int64_t at, bool live) { x = live && !fresh ? state[at] : 0.f; });
 
     const int mat = lane >> 3, r8 = lane & 7;
     // ldmatrix row addresses: [token][channel] tiles as they lie (tokens 0-7 | 8-15 outermost), and transposed
@@ -326,15 +305,13 @@ __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_
         uint32_t vf[4], q_hi[2][4], q_lo[2][4], k_hi[2][4], k_lo[2][4];  // [step of 16 key channels, even or odd]
         float o[2][4] = {};
         auto load = [&](int kk) {
-            if (!kOwn) ldsm4(q_hi[kk & 1], q_addr + kk * 32);
-            if (!kOwn) ldsm4(q_lo[kk & 1], q_addr + kLo + kk * 32);
+            ldsm4(q_hi[kk & 1], q_addr + kk * 32);
+            ldsm4(q_lo[kk & 1], q_addr + kLo + kk * 32);
             ldsm4t(k_hi[kk & 1], k_addr + kk * 32);
             ldsm4t(k_lo[kk & 1], k_addr + kLo + kk * 32);
         };
         ldsm4t(vf, v_addr);
-        if (kOwn) {
-            load(0);
-        } else {
+        {
             uint32_t a_hi[4], a_lo[4];
             ldsm4(a_hi, smem_u32(&b.a_hi[plain_t][plain_c]));
             ldsm4(a_lo, smem_u32(&b.a_lo[plain_t][plain_c]));
@@ -349,7 +326,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_
             if (kk + 1 < kD16) load(kk + 1);  // the next step's operands are on their way during this one's products
             uint32_t s_hi[4], s_lo[4];
 #pragma unroll
-            for (int e = 0; e < 4 && !kOwn; ++e) {
+            for (int e = 0; e < 4; ++e) {
                 const float(&t)[4] = c[2 * kk + (e >> 1)];
                 split2(t[2 * (e & 1)], t[2 * (e & 1) + 1], s_hi[e], s_lo[e]);
             }
@@ -361,18 +338,18 @@ __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_
             }
             const uint32_t(&qh)[4] = q_hi[kk & 1], (&ql)[4] = q_lo[kk & 1], (&kh)[4] = k_hi[kk & 1], (&kl)[4] = k_lo[kk & 1];
 #pragma unroll
-            for (int n = 0; n < 2 && !kOwn; ++n) mma16816(o[n], s_hi, qh[2 * n], qh[2 * n + 1]);
+            for (int n = 0; n < 2; ++n) mma16816(o[n], s_hi, qh[2 * n], qh[2 * n + 1]);
 #pragma unroll
             for (int u = 0; u < 2; ++u) mma16816(c[2 * kk + u], vf, kh[2 * u], kh[2 * u + 1]);
 #pragma unroll
-            for (int n = 0; n < 2 && !kOwn; ++n) mma16816(o[n], s_hi, ql[2 * n], ql[2 * n + 1]);
+            for (int n = 0; n < 2; ++n) mma16816(o[n], s_hi, ql[2 * n], ql[2 * n + 1]);
 #pragma unroll
             for (int u = 0; u < 2; ++u) mma16816(c[2 * kk + u], vf, kl[2 * u], kl[2 * u + 1]);
 #pragma unroll
-            for (int n = 0; n < 2 && !kOwn; ++n) mma16816(o[n], s_lo, qh[2 * n], qh[2 * n + 1]);
+            for (int n = 0; n < 2; ++n) mma16816(o[n], s_lo, qh[2 * n], qh[2 * n + 1]);
         }
 #pragma unroll
-        for (int n = 0; n < 2 && !kOwn; ++n)
+        for (int n = 0; n < 2; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int t = ci * kChunk + n * 8 + col + (e & 1), v = v0 + row + (e >> 1) * 8;
@@ -389,74 +366,14 @@ __global__ void __launch_bounds__(32 * kWarps, 1) gla_state_kernel(const __grid_
         __syncwarp();
         if (++slot == n_ring) slot = 0, phase ^= 1;
     }
-    // (the state at the end of a slice that is not the segment's end has been left by gla_combine_kernel)
-    if (kOwn || last || !spans) {
-        float* const end = kOwn ? span_at : state;
-        each_state([&](float& x, int64_t at, bool live) {
-            if (live) end[at] = x;
-        });
-    }
+    each_state([&](float& x, int64_t at, bool live) {
+        if (live) state[at] = x;
+    });
     if (!ok) {
         // (whoever asked for copies sees to it that they have landed before this memory is given up)
         if (tid == 0)
             for (int i = max(0, chunks - n_ring); i < chunks; ++i) mbar_wait(&sm.full[i % n_ring], (i / n_ring) & 1);
         report_status(dev_status, B2KV_DEV_WAIT_TIMEOUT);
-    }
-}
-
-// What the spans of a slice begin with, from their own parts of the state and what the segment begins the slice with: one CTA per (eight key
-// channels of a head, segment), thread = value column.
-constexpr int kCombineRows = 8, kCombineThreads = 256;
-static_assert(kCombineThreads >= kMaxVdim, "a thread per value column");
-template <typename R>
-__global__ void __launch_bounds__(kCombineThreads) gla_combine_kernel(const __grid_constant__ b2kv_gla_args a, const Slice slice) {
-    __shared__ float decay[2][kSpan][kCombineRows];
-    static_assert(kSpan * kCombineRows <= kCombineThreads, "a thread per decay of a span");
-    const int h = blockIdx.y, d0 = blockIdx.x * kCombineRows, v = threadIdx.x;
-    grid_launch_dependents();
-    if (threadIdx.x == 0) grid_dependency_wait();
-    __syncthreads();
-    b2kv_row_segment sg;
-    if (!segment_place(a, blockIdx.z, sg)) return;
-    const int all_chunks = (sg.n + kChunk - 1) / kChunk, chunks = min(all_chunks - slice.first, slice.count);
-    if (chunks <= 0) return;
-    const int spans = spans_of(chunks);
-    const bool more = slice.first + chunks < all_chunks;  // the segment goes on in the next slice
-    const R* const records = reinterpret_cast<const R*>(a.workspace) + (static_cast<int64_t>(blockIdx.z) * a.H + h) * slice.count;
-    const int ci = threadIdx.x / kCombineRows, cr = threadIdx.x % kCombineRows;  // this thread's decay of every span
-    auto decay_of = [&](int s) { return ci < kSpan && s * kSpan + ci < chunks ? records[s * kSpan + ci].decay[d0 + cr] : 1.f; };
-    float next = decay_of(0);
-    const bool live = v < a.vdim;
-    const bool fresh = slice.first == 0 && a.row_pos[sg.row0] == 0;
-    float* const state = a.state + ((static_cast<int64_t>(sg.slot) * a.H + h) * a.dim + d0) * a.vdim + v;
-    const int rows = min(kCombineRows, a.dim - d0);
-    float x[kCombineRows];
-#pragma unroll
-    for (int r = 0; r < kCombineRows; ++r) x[r] = live && r < rows && !fresh ? state[static_cast<int64_t>(r) * a.vdim] : 0.f;
-    for (int s = 0; s < spans; ++s) {
-        float* const at = span_state<R>(a, slice, blockIdx.z, s, h) + static_cast<int64_t>(d0) * a.vdim + v;
-        const bool has_own = live && (s + 1 < spans || more);  // (the last span of a segment has left none)
-        float own[kCombineRows];
-#pragma unroll
-        for (int r = 0; r < kCombineRows; ++r) own[r] = r < rows && has_own ? at[static_cast<int64_t>(r) * a.vdim] : 0.f;
-        if (ci < kSpan) decay[s & 1][ci][cr] = next;
-        __syncthreads();  // (two spans on the same half have the barrier of the one between them)
-        if (s + 1 < spans) next = decay_of(s + 1);
-#pragma unroll
-        for (int r = 0; r < kCombineRows; ++r)
-            if (live && r < rows) at[static_cast<int64_t>(r) * a.vdim] = x[r];
-#pragma unroll 4
-        for (int c = 0; c < kSpan; ++c) {
-#pragma unroll
-            for (int r = 0; r < kCombineRows; ++r) x[r] *= decay[s & 1][c][r];
-        }
-#pragma unroll
-        for (int r = 0; r < kCombineRows; ++r) x[r] += own[r];
-    }
-    if (more && live) {
-#pragma unroll
-        for (int r = 0; r < kCombineRows; ++r)
-            if (r < rows) state[static_cast<int64_t>(r) * a.vdim] = x[r];
     }
 }
 
@@ -518,13 +435,11 @@ int record_bytes(int dim) {
 size_t chunk_bytes(int H, int dim, int vdim) {
     return (static_cast<size_t>(record_bytes(dim)) + kChunk * static_cast<size_t>(vdim) * sizeof(float)) * H;
 }
-size_t span_bytes(int H, int dim, int vdim) { return static_cast<size_t>(dim) * vdim * sizeof(float) * H; }
 
 int slice_chunks(int H, int dim, int vdim, int n_segments, int max_n) {
     const int chunks = (max_n + kChunk - 1) / kChunk;
-    const size_t span = chunk_bytes(H, dim, vdim) * kSpan + span_bytes(H, dim, vdim);
-    const int fit = static_cast<int>(std::min<size_t>(kSliceBytes / (span * n_segments), kMaxSpans));
-    return std::min(chunks, std::max(kMinSlice, fit * kSpan));
+    const int fit = static_cast<int>(std::min<size_t>(kSliceBytes / (chunk_bytes(H, dim, vdim) * n_segments), 1u << 20));
+    return std::min(chunks, std::max(kMinSlice, fit));
 }
 
 template <int kD16>
@@ -540,11 +455,9 @@ int launch_chunked(const b2kv_gla_args& a, int32_t* dev_status, void* stream) {
     int dev = 0;
     B2KV_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return B2KV_ERR_UNSUPPORTED;
-    auto walk_kernel = gla_state_kernel<kD16, false>;
-    auto own_kernel = gla_state_kernel<kD16, true>;
+    auto kernel = gla_state_kernel<kD16>;
     if (configured[dev] < static_cast<int>(smem)) {
-        B2KV_CUDA_TRY(cudaFuncSetAttribute(walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        B2KV_CUDA_TRY(cudaFuncSetAttribute(own_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        B2KV_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
         configured[dev] = static_cast<int>(smem);
     }
     const int chunks = (a.max_n + kChunk - 1) / kChunk;
@@ -553,16 +466,8 @@ int launch_chunked(const b2kv_gla_args& a, int32_t* dev_status, void* stream) {
         const unsigned here = static_cast<unsigned>(std::min(slice.count, chunks - slice.first));
         OverlapLaunch prep(dim3(here, a.H, a.n_segments), kD16 <= 4 ? 32 : 8 * kD16, 0, stream);
         B2KV_CUDA_TRY(cudaLaunchKernelEx(&prep.cfg, gla_prepare_kernel<kD16>, a, slice, dev_status));
-        const bool spans = chunks > kSpan;
-        const dim3 grid(a.H * parts, a.n_segments, spans ? spans_of(here) : 1);
-        if (spans) {
-            OverlapLaunch own(grid, 32 * kWarps, smem, stream);
-            B2KV_CUDA_TRY(cudaLaunchKernelEx(&own.cfg, own_kernel, tv, a, slice, parts, n_ring, true, dev_status));
-            OverlapLaunch combine(dim3((a.dim + kCombineRows - 1) / kCombineRows, a.H, a.n_segments), kCombineThreads, 0, stream);
-            B2KV_CUDA_TRY(cudaLaunchKernelEx(&combine.cfg, gla_combine_kernel<R>, a, slice));
-        }
-        OverlapLaunch walk(grid, 32 * kWarps, smem, stream);
-        B2KV_CUDA_TRY(cudaLaunchKernelEx(&walk.cfg, walk_kernel, tv, a, slice, parts, n_ring, spans, dev_status));
+        OverlapLaunch walk(dim3(a.H * parts, a.n_segments), 32 * kWarps, smem, stream);
+        B2KV_CUDA_TRY(cudaLaunchKernelEx(&walk.cfg, kernel, tv, a, slice, parts, n_ring, dev_status));
         const unsigned pairs = here * kChunk * static_cast<unsigned>(a.H);
         OverlapLaunch finish(dim3((pairs + kFinishWarps - 1) / kFinishWarps, a.n_segments), 32 * kFinishWarps, 0, stream);
         B2KV_CUDA_TRY(cudaLaunchKernelEx(&finish.cfg, gla_finish_kernel<R>, a, slice));
@@ -578,9 +483,7 @@ bool chunked_sizes(int dim, int vdim, int dtype) {
 }  // namespace gla
 
 static size_t workspace_for(int H, int dim, int vdim, int n_segments, int max_n) {
-    const int chunks = gla::slice_chunks(H, dim, vdim, n_segments, max_n);
-    const size_t spans = max_n > gla::kSpan * gla::kChunk ? gla::spans_of(chunks) * gla::span_bytes(H, dim, vdim) : 0;
-    return (static_cast<size_t>(chunks) * gla::chunk_bytes(H, dim, vdim) + spans) * n_segments;
+    return static_cast<size_t>(gla::slice_chunks(H, dim, vdim, n_segments, max_n)) * gla::chunk_bytes(H, dim, vdim) * n_segments;
 }
 
 // Enough for fewer segments as well: slices are of whole chunks of all segments, so that fewer segments may take a little more.

@@ -249,7 +249,7 @@ def test_segments_outside_the_buffers_are_refused(pkg):
 
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 24, 40), (3, 128, 256), (2, 64, 72)])
 def test_spans_of_chunks(pkg, heads, dim, vdim):
-    """Lengths around one span and two (a span is 256 tokens), in the company of each other and of short ones, then each continued by a portion
+    """Lengths around 256 tokens and 512, in the company of each other and of short ones, then each continued by a portion
     of another length: the outputs and states of the equations, and alone the same bits."""
     layer = Layer(pkg, heads, dim, vdim, 16.0, BF, z_mean=2.0, z_std=1.0, seed=17)
     first, then = (255, 256, 257, 511, 513, 30, 770), (300, 17, 256, 1, 273, 520, 16)
@@ -268,7 +268,7 @@ def test_spans_of_chunks(pkg, heads, dim, vdim):
 
 
 def test_spans_over_slices_of_a_bounded_workspace(pkg):
-    """Many sequences of several spans, which one slice of the workspace does not hold: the bits of each alone."""
+    """Many sequences of several hundred tokens, which one slice of the workspace does not hold: the bits of each alone."""
     layer = Layer(pkg, 8, 128, 256, 16.0, BF, z_mean=2.0, z_std=1.0, seed=19)
     lens = (700, 513, 300) * 8
     y, al = layer.rows(sum(lens))
@@ -281,8 +281,19 @@ def test_spans_over_slices_of_a_bounded_workspace(pkg):
         assert torch.equal(alone[0], state[slot]), n
 
 
+def test_portions_of_whole_chunks_change_no_bit(pkg):
+    """A sequence in one run, and cut at multiples of sixteen tokens: one chain of chunks either way."""
+    layer = Layer(pkg, 3, 128, 256, 16.0, BF, z_mean=2.0, z_std=1.0, seed=41)
+    y, al = layer.rows(1000)
+    whole, parts = layer.states(1), layer.states(1)
+    want = layer.run(y, al, [(0, 1000, 0)], range(1000), whole, CHUNK)
+    for a, b in ((0, 160), (160, 512), (512, 1000)):
+        assert np.array_equal(layer.run(y[a:b], al[a:b], [(0, b - a, 0)], range(a, b), parts, CHUNK), want[a:b]), a
+    assert torch.equal(whole, parts)
+
+
 def test_an_infinite_state_is_not_turned_into_nan_by_a_span(pkg):
-    """Decays whose product over a span is below the smallest number: what is infinite stays so."""
+    """Decays whose product over some hundred tokens is below the smallest number: what is infinite stays so."""
     layer = Layer(pkg, 1, 16, 32, 1.0, BF, z_mean=-0.7, z_std=0.0, seed=23)
     y, al = layer.rows(600)
     state = torch.ones((1, 1, 16, 32), device="cuda")
