@@ -618,7 +618,8 @@ int b2kv_moe_combine(float* x, int64_t ld_x, const void* y, int64_t ld_y, const 
  * split-bfloat16 tensor-core kernel, "prefill_unfused_paged": 1 = b2kv_prefill_paged always
  * fills the pool with the copy kernel, "prefill_test_expire": 1 = test hook, the softmax warps of the one-CTA tensor-core prefill
  * behave as if their first bounded wait had run out (the launch then ends after about two seconds with
- * B2KV_DEV_WAIT_TIMEOUT in dev_status), "matmul_splits": ranges of input features per tile in b2kv_matmul_rows,
+ * B2KV_DEV_WAIT_TIMEOUT in dev_status), "linear_test_expire": 1 = the same for the warps that take sums out in fp32 products of more
+ * than 16 rows, "matmul_splits": ranges of input features per tile in b2kv_matmul_rows,
  * "serial_launches": 1 = plain stream order for every launch (see "overlap" at the top),
  * "gemm_variant": 1 = one CTA per output tile, 2 / 3 = CTA pairs with 64 / 128 input features per
  * ring stage in b2kv_matmul);

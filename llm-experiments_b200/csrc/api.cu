@@ -32,6 +32,7 @@ static Knob g_knobs[] = {
     {"prefill_f32_simt", 0},  // 1 = fp32 prompts never take the split-bfloat16 tensor-core kernel
     {"prefill_unfused_paged", 0},  // 1 = a paged cache is always filled by the copy kernel behind the attention
     {"prefill_test_expire", 0},  // test hook: 1 = the softmax warps of the one-CTA tensor-core prefill give up at once
+    {"linear_test_expire", 0},  // test hook: 1 = the warps that take sums out in the fp32 tensor-core product give up at once
     {"prefill_group", 0},  // one-CTA tensor-core prefill: (sequence, head) pairs per launch group; 0 = by size, -1 = all
     {"matmul_splits", 0},  // ranges of input features per tile in b2kv_matmul_rows (0 = by shape)
     {"decode_dynamic_chunks", 0},  // small chunks of the decode's token space handed out on demand: 0 = by size, 1 = always, 2 = never

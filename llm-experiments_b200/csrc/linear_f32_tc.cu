@@ -186,11 +186,16 @@ __device__ __noinline__ float sum_in_order(const float* row, const float* col, i
     return sum;
 }
 
+// After a wait that ran out: the last of `n` uses of the stages, copies (bars: full) or products (empty), end before their memory is given up.
+__device__ __noinline__ void settle(uint64_t* bars, int n) {
+    for (int i = max(0, n - kStages); i < n; ++i) mbar_wait(&bars[i % kStages], (i / kStages) & 1);
+}
+
 // kMade: the parts are in scratch memory.
 template <bool kMade>
 __global__ void __launch_bounds__(kThreads, 1)
 linear_f32_tc_kernel(const __grid_constant__ b2kv_linear_args a, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
-                     const __grid_constant__ Parts p, int splits, int32_t* dev_status) {
+                     const __grid_constant__ Parts p, int splits, bool expire, int32_t* dev_status) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ Shared sm;
     uint8_t* const ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -275,7 +280,7 @@ linear_f32_tc_kernel(const __grid_constant__ b2kv_linear_args a, const __grid_co
             if (lane == 0) good = issue(s);
             return __all_sync(0xffffffffu, good) != 0;
         };
-        bool ok = issue_by_warp0(0);
+        bool ok = !expire && issue_by_warp0(0);  // (test hook: as if the first wait had run out)
         for (int s = 0; s < steps && ok; ++s) {
             ok = issue_by_warp0(s + 1);
             if (!ok) break;
@@ -298,7 +303,8 @@ linear_f32_tc_kernel(const __grid_constant__ b2kv_linear_args a, const __grid_co
         if (warp == kSumWarps) {
             // ------------------------------ copies of the parts ------------------------------
             if (lane == 0) {
-                for (int s = 0; s < steps && ok; ++s) {
+                int s = 0;
+                for (; s < steps; ++s) {
                     const int st = s % kStages, k = k_first + s * kBK;
                     ok = mbar_wait(&sm.empty[st], ((s / kStages) & 1) ^ 1);
                     if (!ok) break;
@@ -311,11 +317,16 @@ linear_f32_tc_kernel(const __grid_constant__ b2kv_linear_args a, const __grid_co
                         tma_load_3d(to + (3 + part) * kPartBytes + kBK * 128, &tm_w, &sm.full[st], col0 + 64, k, part);
                     }
                 }
+                if (!ok) settle(sm.full, s);
             }
             __syncwarp();
         } else if (warp == kSumWarps + 1) {
-            if (lane == 0)
-                for (int s = 0; s < steps && ok; ++s) ok = issue(s);
+            if (lane == 0) {
+                int s = 0;
+                while (s < steps && issue(s)) ++s;
+                ok = s == steps;
+                if (!ok) settle(sm.empty, s);
+            }
             __syncwarp();
         } else if (warp == kSumWarps + 2) {
             for (int s = lane; s < steps; s += 32)
@@ -505,6 +516,7 @@ int linear_f32_tc(const b2kv_linear_args& a, void* workspace, size_t workspace_b
     if (tune_get("matmul_splits") > 0) splits = std::min(tune_get("matmul_splits"), kMaxSplits);
     if (tiles_m > 65535 || a.groups > 65535 || tiles_n * splits > 0x7fffffffLL) return B2KV_ERR_UNSUPPORTED;
     OverlapLaunch launch(dim3(static_cast<unsigned>(tiles_n * splits), static_cast<unsigned>(tiles_m), a.groups), kThreads, kSmem, stream, splits);
+    const bool expire = tune_get("linear_test_expire") != 0;
     Parts parts{};
     CUtensorMap tx{}, tw{};
     const size_t need = workspace != nullptr && aligned16(workspace) ? parts_bytes(a, &parts, workspace) : 0;
@@ -514,10 +526,10 @@ int linear_f32_tc(const b2kv_linear_args& a, void* workspace, size_t workspace_b
         if (pieces > 0x7fffffffLL) return B2KV_ERR_UNSUPPORTED;
         OverlapLaunch make(static_cast<unsigned>(pieces), kMakeThreads, 0, stream);
         B2KV_CUDA_TRY(cudaLaunchKernelEx(&make.cfg, make_parts_kernel, a, parts, static_cast<int>(pieces_x)));
-        B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, linear_f32_tc_kernel<true>, a, tx, tw, parts, splits, dev_status));
+        B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, linear_f32_tc_kernel<true>, a, tx, tw, parts, splits, expire, dev_status));
         return B2KV_OK;
     }
-    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, linear_f32_tc_kernel<false>, a, tx, tw, parts, splits, dev_status));
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, linear_f32_tc_kernel<false>, a, tx, tw, parts, splits, expire, dev_status));
     return B2KV_OK;
 }
 

@@ -211,6 +211,31 @@ def test_parts_made_ahead_have_the_same_bits(pkg, rows, K, n):
             bounded(out[1][:rows, :n], x, w, bias.double())
 
 
+@pytest.mark.parametrize("ahead", [False, True])
+def test_a_wait_that_runs_out_is_reported(pkg, ahead):
+    """The warps that take sums out behave as if their first wait had run out.  The other warps run out of their own bounded waits (about two
+    seconds), what is under way ends first, the status says so, and the next product is right."""
+    from llm_experiments_b200 import projection as proj
+
+    ctx, native, (rows, K, n) = make_ctx(pkg), pkg._native, (700, 1024, 1300)
+    x, w, out = rnd((rows, K), F32, 31), rnd((K, n), F32, 32, K ** -0.5), torch.full((rows, n), 7.0, dtype=F32, device="cuda")
+    scratch = {} if ahead else None
+    ctx.config.check_device_status = True
+
+    def product():
+        run(pkg, ctx, wrap(pkg, x), wrap(pkg, w), K, [proj.OutputSegment(n, proj.SEG_STORE, wrap(pkg, out))], scratch=scratch)
+
+    native.tune("linear_test_expire", 1)
+    try:
+        with pytest.raises(RuntimeError, match="bounded wait"):
+            product()
+    finally:
+        native.tune("linear_test_expire", 0)
+    assert (out == 7).all() and bool(scratch) == ahead
+    product()
+    bounded(out, x, w)
+
+
 def test_scratch_grows_and_is_left_alone_where_it_is_of_no_use(pkg):
     from llm_experiments_b200 import projection as proj
 
