@@ -567,8 +567,8 @@ int b2kv_gqa_prefill(const void* q, int64_t ld_q, const void* k_cache, const voi
  * segment of its own, of sequence i.  max_n bounds the segments' lengths.  Everything is computed in 32-bit; path 2 (segments
  * of a prompt; bf16, dim a multiple of 8 up to 128, vdim a multiple of 8 up to 256) takes sixteen tokens at a time through the tensor
  * cores with operands split into two bf16 halves and the state in fp32 registers, and wants a workspace (128-byte aligned) of
- * b2kv_gla_workspace_bytes bytes (enough for fewer segments and tokens as well; long fp32 segments are walked in parallel
- * where they have such a workspace, and without it token after token); path 1 takes token after token on CUDA cores for any
+ * b2kv_gla_workspace_bytes bytes (enough for fewer segments and tokens as well; long fp32 segments of narrow heads are
+ * walked in parallel where they have such a workspace, and without it token after token); path 1 takes token after token on CUDA cores for any
  * sizes and both types; 0 = choose (path 2 for segments of more than 16 tokens where the sizes have that form).
  */
 typedef struct b2kv_row_segment {

@@ -7,8 +7,8 @@
 // for every token, took 939 us for runs of up to 400 tokens (6 heads, 64 x 128), this one 80 (100 with
 // the tokens one after the other: eight at a time, their sums over the lanes run side by side).
 //
-// 400 tokens one after the other are a chain, on half of the SMs with a warp per scheduler, so runs of more than 192 tokens are cut into spans
-// of 64 where there is scratch memory.  A first pass makes every span's own part of the state from zero, and the product of its decays
+// 400 tokens one after the other are a chain, on half of the SMs with a warp per scheduler, so runs of more than 192 tokens over heads of up
+// to 64 key channels are cut into spans of 64 where there is scratch memory.  A first pass makes every span's own part of the state from zero, and the product of its decays
 // (all but the last one's); gla_spans_kernel carries the state through, S <- diag(D) S + L, and leaves what each span begins with;
 // the second pass walks all spans side by side.  Two thirds more work: three prompts of 62 to 400 tokens, 6 heads of 64 x 128, 59 us in all, 124 as
 // chains.  Spans begin at multiples of 64 tokens
@@ -26,7 +26,7 @@ constexpr int kWarps = 4, kCols = 8 * kWarps;  // value columns of a CTA
 constexpr int kTok = 8, kRing = 3;
 constexpr int kSpanTokens = 64;
 constexpr int kMinSpanned = 193;  // tokens of a segment that is cut
-constexpr int kMaxSpannedCtas = 32;  // value columns of a state / 32
+constexpr int kMaxSpannedDim = 64, kMaxSpannedCtas = 32;  // CTAs: value columns of a state / 32
 constexpr size_t kMaxSpanBytes = size_t{256} << 20;  // spans at a time, more only where a state per segment takes more
 
 __host__ __device__ constexpr int spans_of(int n) { return n < kMinSpanned ? 1 : (n + kSpanTokens - 1) / kSpanTokens; }
@@ -285,26 +285,28 @@ int span_count(const b2kv_gla_args& a) {
 template <int kD, bool kPadded>
 int launch_runs(const b2kv_gla_args& a, int parts, int32_t* dev_status, void* stream) {
     const dim3 grid(static_cast<unsigned>(a.H * parts), a.n_segments);
-    const size_t need = gla_run_f32_workspace(a.H, a.dim, a.vdim, a.n_segments, a.max_n);
-    if (need == 0 || a.workspace == nullptr || !aligned16(a.workspace) || a.workspace_bytes < need) {
-        OverlapLaunch run(grid, 32 * kWarps, 0, stream);
-        B2KV_CUDA_TRY(cudaLaunchKernelEx(&run.cfg, gla_run_kernel<kD, kPadded, kWholeRun>, a, parts, Spans{}, dev_status));
-        return B2KV_OK;
+    if constexpr (kD <= kMaxSpannedDim) {
+        const size_t need = gla_run_f32_workspace(a.H, a.dim, a.vdim, a.n_segments, a.max_n);
+        if (need > 0 && a.workspace != nullptr && aligned16(a.workspace) && a.workspace_bytes >= need) {
+            Spans spans{};
+            spans.count = span_count(a);
+            spans.states = static_cast<float*>(a.workspace);
+            spans.decays = spans.states + static_cast<size_t>(a.n_segments) * spans.count * a.H * a.dim * a.vdim;
+            const int all = spans_of(a.max_n);
+            for (; spans.first < all; spans.first += spans.count) {
+                const unsigned here = std::min(spans.count, all - spans.first);
+                OverlapLaunch own(dim3(grid.x, grid.y, here), 32 * kWarps, 0, stream);
+                B2KV_CUDA_TRY(cudaLaunchKernelEx(&own.cfg, gla_run_kernel<kD, kPadded, kOwnPart>, a, parts, spans, dev_status));
+                OverlapLaunch through(dim3((a.dim + kSpanRows - 1) / kSpanRows, a.H, a.n_segments), kSpanThreads, 0, stream);
+                B2KV_CUDA_TRY(cudaLaunchKernelEx(&through.cfg, gla_spans_kernel, a, spans));
+                OverlapLaunch run(dim3(grid.x, grid.y, here), 32 * kWarps, 0, stream);
+                B2KV_CUDA_TRY(cudaLaunchKernelEx(&run.cfg, gla_run_kernel<kD, kPadded, kOutputs>, a, parts, spans, dev_status));
+            }
+            return B2KV_OK;
+        }
     }
-    Spans spans{};
-    spans.count = span_count(a);
-    spans.states = static_cast<float*>(a.workspace);
-    spans.decays = spans.states + static_cast<size_t>(a.n_segments) * spans.count * a.H * a.dim * a.vdim;
-    const int all = spans_of(a.max_n);
-    for (; spans.first < all; spans.first += spans.count) {
-        const unsigned here = std::min(spans.count, all - spans.first);
-        OverlapLaunch own(dim3(grid.x, grid.y, here), 32 * kWarps, 0, stream);
-        B2KV_CUDA_TRY(cudaLaunchKernelEx(&own.cfg, gla_run_kernel<kD, kPadded, kOwnPart>, a, parts, spans, dev_status));
-        OverlapLaunch through(dim3((a.dim + kSpanRows - 1) / kSpanRows, a.H, a.n_segments), kSpanThreads, 0, stream);
-        B2KV_CUDA_TRY(cudaLaunchKernelEx(&through.cfg, gla_spans_kernel, a, spans));
-        OverlapLaunch run(dim3(grid.x, grid.y, here), 32 * kWarps, 0, stream);
-        B2KV_CUDA_TRY(cudaLaunchKernelEx(&run.cfg, gla_run_kernel<kD, kPadded, kOutputs>, a, parts, spans, dev_status));
-    }
+    OverlapLaunch run(grid, 32 * kWarps, 0, stream);
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&run.cfg, gla_run_kernel<kD, kPadded, kWholeRun>, a, parts, Spans{}, dev_status));
     return B2KV_OK;
 }
 
@@ -313,10 +315,12 @@ int launch_runs(const b2kv_gla_args& a, int parts, int32_t* dev_status, void* st
 
 size_t gla_run_f32_workspace(int H, int dim, int vdim, int n_segments, int max_n) {
     using namespace gla;
-    // Two passes pay where the chain is long and what they add runs on SMs that would be idle (CTAs of 32 value columns; us as one chain and
-    // in spans): 72 CTAs, 400 tokens 124 and 59; 192, 400 168 and 99; 64, 700 238 and 79; but 24, 128 31 and 36; 512, 300 187 and 266.  So it is
-    // states that few CTAs hold; not by the number of segments, on which a sequence's sums must not depend.
-    if (dim > 128 || dim % 4 || vdim % 4 || max_n < kMinSpanned || H * ((vdim + kCols - 1) / kCols) > kMaxSpannedCtas) return 0;
+    // Two passes pay where the chain is long and what they add runs on SMs that would be idle.  That is for states that few CTAs hold (32 value
+    // columns each) and heads of up to 64 key channels, whose chains leave issue slots even where the segments fill the device; us as one chain
+    // and in spans, 6 heads of 64 x 128 (24 CTAs): 1 run of 400 tokens 111, 45; 4 132, 69; 16 201, 173; 24 236, 251; of 200 tokens 1 47, 36; 4 77,
+    // 46; 16 84, 92.  4 heads of 128 x 256 (32 CTAs): 1 run of 400 126, 58; 4 204, 110; 8 197, 189; but 16 243, 348: those stay one
+    // chain.  The number of segments must not choose, a sequence's sums do not depend on its company.
+    if (dim > kMaxSpannedDim || dim % 4 || vdim % 4 || max_n < kMinSpanned || H * ((vdim + kCols - 1) / kCols) > kMaxSpannedCtas) return 0;
     const size_t each = span_floats(H, dim, vdim) * sizeof(float), segments = static_cast<size_t>(n_segments);
     return std::min(each * segments * spans_of(max_n), std::max(kMaxSpanBytes, each * segments));  // (grows with segments and tokens)
 }

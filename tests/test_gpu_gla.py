@@ -304,8 +304,8 @@ def test_an_infinite_state_is_not_turned_into_nan_by_a_span(pkg):
 
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 20, 40), (3, 128, 256), (2, 64, 72), (1, 4, 4), (5, 64, 256)])
 def test_spans_of_tokens_in_fp32(pkg, heads, dim, vdim):
-    """As for chunks, with spans of 64 tokens of segments of more than 192; the decays of half of the channels multiply up to nothing over a
-    span."""
+    """As for chunks, with spans of 64 tokens of segments of more than 192 (heads of up to 64 key channels); the decays of half of the channels
+    multiply up to nothing over a span."""
     layer = Layer(pkg, heads, dim, vdim, 4.0, F32, z_mean=2.0, z_std=4.0, seed=29)
     first, then = (63, 64, 192, 193, 129, 5, 400), (256, 17, 64, 2, 200, 320, 16)
     state, last = layer.states(len(first)), [None] * len(first)
@@ -323,8 +323,8 @@ def test_spans_of_tokens_in_fp32(pkg, heads, dim, vdim):
 
 
 def test_spans_of_tokens_over_slices_of_a_bounded_workspace(pkg):
-    layer = Layer(pkg, 4, 128, 256, 16.0, F32, z_mean=2.0, z_std=1.0, seed=31)
-    lens = (8300, 64, 200, 8256)  # 130 spans of four segments, 127 at a time
+    layer = Layer(pkg, 8, 64, 128, 16.0, F32, z_mean=2.0, z_std=1.0, seed=31)
+    lens = (16300, 64, 200, 16256)  # 255 spans of four segments, 254 at a time
     y, al = layer.rows(sum(lens))
     segments, pos = [(sum(lens[:i]), n, i) for i, n in enumerate(lens)], np.concatenate([np.arange(n) for n in lens])
     state = layer.states(len(lens))
