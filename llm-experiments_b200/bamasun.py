@@ -335,7 +335,7 @@ def _recur(ctx, state: BamasunState, i: int, xs: GPUBuffer2D, step: Step) -> GPU
     for segments in (step.short, step.long):
         if segments is not None:
             recurrent.gated_linear_attention(ctx, y, w.cols[:4], alpha, g, w.head_norm, state.cfg.eps, segments, step.places.pos,
-                                             state.recurrent[i], out)
+                                             state.recurrent[i], out, scratch=state.scratch)
     return out
 
 

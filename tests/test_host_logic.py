@@ -253,3 +253,30 @@ def test_memory_of_a_captured_step_stays_when_it_is_replaced(pkg, ctx, monkeypat
     assert [r() is None for r in alive[1]] == [False] * 3  # the captured step's
     assert [r() is None for r in alive[2]] == [True] * 3  # what came behind it and was too small in its turn
     assert state.scratch["linear"].numel() == 1700 and state.scratch["x"].shape == (17, 4)
+
+
+def test_memory_of_recurrent_layers_is_not_shared_by_two_models(pkg, ctx, monkeypatch):
+    """Two states of one context may have steps under way on two streams: each brings its own memory, and a call that brings none does not
+    write to what another fp32 call may still use."""
+    import types
+
+    from llm_experiments_b200 import recurrent
+    from llm_experiments_b200.serving import RowSegments
+
+    seen = []
+    lib = types.SimpleNamespace(b2kv_gla_workspace_bytes=lambda *a: 1000, b2kv_gla=lambda a, status, stream: seen.append(a._obj.workspace) or 0)
+    monkeypatch.setattr(recurrent, "_native", types.SimpleNamespace(lib=lib, check=lambda rc: None, GlaArgs=pkg._native.GlaArgs))
+    monkeypatch.setattr(recurrent, "batch_op_begin", lambda ctx: 0)
+    monkeypatch.setattr(recurrent, "dev_status_ptr", lambda ctx: 0)
+    two = lambda t: pkg.gpu.GPUBuffer2D(buffer=t, shape=tuple(t.shape), size=t.numel())  # noqa: E731
+    kept = [{}, {}, None, None]
+    alive = []  # (so that no address comes twice)
+    real = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **kw: alive.append(real(*a, **kw)) or alive[-1])
+    for again in range(2):
+        for scratch in kept:
+            y = two(torch.zeros((300, 64)))
+            recurrent.gated_linear_attention(ctx, y, (0, 16, 32, 48), two(torch.zeros((300, 16))), recurrent.GlaShape(1, 16, 16, 1.0),
+                                             pkg.gpu.GPUBuffer1D(buffer=torch.zeros(16), shape=(16,), size=16), 1e-5, RowSegments(None, 1, 300),
+                                             torch.zeros(300, dtype=torch.int32), torch.zeros((1, 1, 16, 16)), two(torch.zeros((300, 16))), scratch=scratch)
+    assert len(set(seen[:4])) == 4 and seen[4:6] == seen[:2] and len(set(seen)) == 6 and ctx.recurrent_workspace is None
