@@ -24,6 +24,8 @@ from .types import GPUBuffer1D, GPUBuffer2D, GPUContext, KVCache
 
 # Entries of at most this many tokens go row by row through the kernels of a decode step; longer ones are prompt portions.
 SHORT_ENTRY = 16
+# Runs of more rows than this are cut by the fp32 recurrence, which wants scratch memory for them (csrc/gla_run.cu).
+LONG_RUN = 192
 
 
 def buffer1(t: torch.Tensor) -> GPUBuffer1D:
@@ -54,6 +56,17 @@ class RowSegments:
     max_n: int
 
 
+def split_runs(runs: Sequence[Tuple[int, int, int]]) -> Tuple[list, list, int]:
+    """Runs (first row, rows, sequence) that go row by row, as (short ones, long ones, the most rows of a short one to be told).  A table's
+    scratch memory and grids are made for its longest run, so a few long ones among many others get a table of their own; few
+    others go along with them (a launch less)."""
+    long = [r for r in runs if r[1] > LONG_RUN]
+    if not long or len(runs) - len(long) < max(16, 3 * len(long)):
+        return list(runs), [], max((n for _, n, _ in runs), default=0)
+    rest = [r for r in runs if r[1] <= LONG_RUN]
+    return rest, long, max(2, max(n for _, n, _ in rest))  # (2: by the kernel that takes runs, also where all of them are single rows)
+
+
 @dataclass
 class Step:
     """The rows of one step.  The first ``n_single`` go row by row, the rest to the kernels of prompt portions.  Of the former the
@@ -66,8 +79,8 @@ class Step:
     n_few: int
     span: int                        # bounds the tokens that a row of a short entry sees
     plans: Dict[int, PromptPlan]     # prompt portions, by the key the state's prompt_plans chose
-    short: Optional[RowSegments]     # the short entries and
-    long: Optional[RowSegments]      # the prompt portions, as runs of rows
+    short: Optional[RowSegments]     # the short entries (and longer ones, where there is no prompt form) and
+    long: Optional[RowSegments]      # the prompt portions (or a few long ones of the others), as runs of rows
     row_index: Optional[torch.Tensor]  # rows whose logits are wanted (None: all)
     n_out: int
 
@@ -239,6 +252,10 @@ def forward(ctx: GPUContext, state: SequenceState, entries: Sequence[Tuple[int, 
         pos.append(np.arange(start, start + n, dtype=np.int32))
         T += n
         lens[slot] = start + n
+    most = {k: max((n for _, n, _ in r), default=0) for k, r in runs.items()}
+    if most[True] > LONG_RUN:  # (there are no prompt portions then)
+        runs[True], runs[False], most[True] = split_runs(runs[True])
+        most[False] = max((n for _, n, _ in runs[False]), default=0)
     want = [first_row[j] + int(p) for j in range(len(entries)) for p in entries[j][2]]
     n_out = len(want)
     plans = state.prompt_plans(spans) if spans else {}
@@ -249,8 +266,7 @@ def forward(ctx: GPUContext, state: SequenceState, entries: Sequence[Tuple[int, 
     pieces = list(host.to(ctx.device, non_blocking=True).split([len(part) for part in parts]))
     for plan, table, groups in zip(plans.values(), pieces[7:], pieces[7 + len(plans):]):
         plan.table, plan.groups = table, groups if len(groups) else None
-    segments = [RowSegments(table, len(r), max(n for _, n, _ in r)) if r else None
-                for table, r in ((pieces[5], runs[True]), (pieces[6], runs[False]))]
+    segments = [RowSegments(table, len(runs[k]), most[k]) if runs[k] else None for table, k in ((pieces[5], True), (pieces[6], False))]
     batch_begin(ctx)
     state.wait_for_lengths()
     state.run(ctx, Step(ids=pieces[0], places=RowPlaces(pieces[1], pieces[2]), rows=T, n_single=n_single, n_few=n_few, span=span, plans=plans,

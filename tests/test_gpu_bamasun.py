@@ -251,6 +251,19 @@ def test_lengths_set_on_one_stream_and_a_step_on_another(pkg, how):
         assert torch.equal(got, expected) and state.seq_lens.tolist() == [v + 1 for v in n] == state.lengths
 
 
+def test_a_long_run_among_many_single_rows_in_fp32(pkg):
+    """The long run and the single rows have tables of their own: what the oracle says of every one of them, and of the next token."""
+    n, name = 20, "ONLY_GLA"
+    model, cfg = build(pkg, name, F32, batch=n + 1, max_tokens=400)
+    seqs = [U.tokens(cfg, 5 + i % 3, 60 + i) for i in range(n)] + [U.tokens(cfg, 303, 90)]
+    model.forward([(i, seqs[i][:-2], []) for i in range(n)] + [(n, seqs[n][:40], [])])
+    steps = [model.forward([(i, seqs[i][-2:-1], [0]) for i in range(n)] + [(n, seqs[n][40:-1], list(range(262)))]).clone(),
+             model.forward([(i, seqs[i][-1:], [0]) for i in range(n + 1)]).clone()]
+    for i in range(n):
+        U.check_rows(torch.stack([s[i] for s in steps]), oracle(name, seqs[i])[-2:], F32, i)
+    U.check_rows(torch.cat([steps[0][n:], steps[1][n:]]), oracle(name, seqs[n])[-263:], F32, n)
+
+
 def test_a_captured_step_keeps_its_memory(pkg):
     """A captured step of many fp32 sequences, whose products lay their operands out in scratch memory; then a larger step, which needs more of
     everything; then other tensors wherever the memory was.  The graph's step is the same as before, and so are the tensors."""

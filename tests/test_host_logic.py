@@ -280,3 +280,18 @@ def test_memory_of_recurrent_layers_is_not_shared_by_two_models(pkg, ctx, monkey
                                              pkg.gpu.GPUBuffer1D(buffer=torch.zeros(16), shape=(16,), size=16), 1e-5, RowSegments(None, 1, 300),
                                              torch.zeros(300, dtype=torch.int32), torch.zeros((1, 1, 16, 16)), two(torch.zeros((300, 16))), scratch=scratch)
     assert len(set(seen[:4])) == 4 and seen[4:6] == seen[:2] and len(set(seen)) == 6 and ctx.recurrent_workspace is None
+
+
+def test_few_long_runs_have_a_table_of_their_own(pkg):
+    """One long run among many single rows does not make them all reserve its memory; what goes row by row stays with the kernel of runs."""
+    from llm_experiments_b200 import serving
+
+    size = lambda runs, most: pkg._native.lib.b2kv_gla_workspace_bytes(6, 64, 128, len(runs), most, 0, 0) if runs else 0  # noqa: E731
+    singles = [(i, 1, i) for i in range(64)]
+    runs = singles + [(64, 2000, 64), (2064, 192, 65)]
+    rest, long, most = serving.split_runs(runs)
+    assert rest == singles + [(2064, 192, 65)] and long == [(64, 2000, 64)] and most == 192
+    assert size(rest, most) == 0 and 0 < 20 * size(long, 2000) < size(runs, 2000)
+    assert serving.split_runs(singles + [(64, 193, 64)])[1:] == ([(64, 193, 64)], 2)
+    for together in (singles, singles[:15] + [(15, 400, 15)], singles[:20] + [(20 + 300 * i, 300, 20 + i) for i in range(7)], [(0, 5, 1)], []):
+        assert serving.split_runs(together) == (together, [], max((n for _, n, _ in together), default=0))
