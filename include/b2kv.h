@@ -454,8 +454,8 @@ typedef struct b2kv_linear_options {
 } b2kv_linear_options;
 int b2kv_linear_opt(const b2kv_linear_args* args, const b2kv_linear_options* options, int32_t* dev_status, void* stream);
 /*
- * The same with scratch memory of b2kv_linear_workspace_bytes bytes (16-byte aligned; 0: none is of use), in which fp32 products of more
- * than 128 rows lay their operands out once for all tiles of the outputs.  Without it (NULL, or fewer bytes) they do so tile by
+ * The same with scratch memory of b2kv_linear_workspace_bytes bytes (16-byte aligned, 512 MB at most; 0: none is of use), in which fp32
+ * products of more than 256 rows and many tiles lay their operands out once for all tiles of the outputs.  Without it (NULL, or fewer bytes) they do so tile by
  * tile: the same results, later.  It may be used again by the next call on the stream.
  */
 size_t b2kv_linear_workspace_bytes(const b2kv_linear_args* args);

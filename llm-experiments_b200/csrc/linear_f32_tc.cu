@@ -9,8 +9,8 @@
 // against 127 of linear_f32_tile_kernel; 3072 -> 768: 39 and 130; 60 rows, 768 -> 3072: 15 and 25.
 //
 //   * a CTA has 128 x 128 outputs; steps of 64 input features through two stages of 96 KB;
-//   * more than 128 rows, and scratch: the parts are made by a kernel ahead, once for all tiles (b2kv_linear_ws), and warp 8 copies them with
-//     TMA, warp 9 issues the products.  In the same kernel every row of tiles makes the parts of w and every column of tiles those of x
+//   * more than 256 rows, enough tiles and scratch (the rule and its times at parts_bytes): the parts are made by a kernel ahead, once for all
+//     tiles (b2kv_linear_ws), and warp 8 copies them with TMA, warp 9 issues the products.  In the same kernel every row of tiles makes the parts of w and every column of tiles those of x
 //     again, which takes longer than the products (693 rows, 3072 -> 768: 36.8 us, 32.5 with the kernel ahead; 3000 rows, 1024 -> 4096: 205 and 157);
 //   * otherwise warps 8-15 read fp32 rows of x and w, a step ahead in registers, and write the parts as the operands the MMAs want: x K-major,
 //     w as it lies (MN-major), 128-byte swizzle; a thread of warp 0 issues the products;
@@ -46,6 +46,7 @@ constexpr int kSumWarps = 8, kSplitWarps = 8;
 constexpr int kThreads = 32 * (kSumWarps + kSplitWarps);  // 128 registers each
 constexpr int kLdT = kBN + 4;                       // words per row of the tile of sums (over the stages, once they are free)
 constexpr int kMinTileSteps = 900;                  // tiles x steps from which a kernel ahead makes the parts
+constexpr size_t kMaxScratch = size_t{512} << 20;   // bytes of parts at most
 constexpr int kMaxSplits = 8;                       // ranges of input features
 constexpr int kTmemCols = 512;                      // leading sums 2 x 128, the others 128
 constexpr int kColRest = 2 * kBN;
@@ -447,10 +448,15 @@ linear_f32_tc_kernel(const __grid_constant__ b2kv_linear_args a, const __grid_co
 // Scratch of the parts: none where they are made in the products' kernel.
 static size_t parts_bytes(const b2kv_linear_args& a, linf32tc::Parts* p, void* at) {
     using namespace linf32tc;
-    // The tiles make more of the same parts the more of them there are: 36 tiles of 12 steps 16.2 us and 18.6 with the kernel ahead, 60 of 12
-    // 19.9 and 21.3, 78 of 12 29.5 and 26.0, 144 of 12 30.4 and 27.6, 36 of 48 36.8 and 32.5, 96 of 16 37.2 and 31.4, 768 of 16 205 and 157.
-    const long long tiles = static_cast<long long>((a.rows + kBM - 1) / kBM) * ((a.N + kBN - 1) / kBN);
-    if (a.rows <= kBM || a.groups > 1 || tiles * ((a.K + kBK - 1) / kBK) < kMinTileSteps) return 0;
+    // The tiles make more of the same parts the more of them there are (us in the products' kernel, and ahead): 36 tiles of 12 steps 16.2, 18.6;
+    // 60 of 12 19.9, 21.3; 78 of 12 29.5, 26.0; 144 of 12 30.4, 27.6; 36 of 48 36.8, 32.5; 768 of 16 205, 157.  What the kernel ahead costs
+    // is w's bytes, as parts written and read back, and what it saves is one lot of w's parts per row of tiles; by rows of tiles and MB of w's parts:
+    // 2 rows, 25 MB 24.6, 25.4; 100 62, 72; 3 rows, 19 MB 30.4, 27.6; 25 37.7, 32.0; 57 49.1, 50.8; 100 106, 107; 4 rows, 57 MB 126, 116;
+    // 100 151, 119; 144 203, 221; 5 rows, 100 MB 241, 175; 144 277, 273; 6 rows, 144 MB 331, 314; 384 782, 816; 24 rows, 25 MB 214, 164; 100 747, 619.
+    const long long tiles_rows = (a.rows + kBM - 1) / kBM, tiles = tiles_rows * ((a.N + kBN - 1) / kBN);
+    if (tiles_rows < 3 || a.groups > 1 || tiles * ((a.K + kBK - 1) / kBK) < kMinTileSteps) return 0;
+    const size_t parts_w = 6 * static_cast<size_t>(a.K) * a.N;
+    if (parts_w > (tiles_rows == 3 ? size_t{32} << 20 : tiles_rows == 4 ? size_t{112} << 20 : size_t{160} << 20)) return 0;
     const size_t steps = (a.K + kBK - 1) / kBK, tiles_m = (a.rows + kBM - 1) / kBM, tiles_n = (a.N + kBN - 1) / kBN;
     const size_t ldx = pad8(a.K), ldw = pad8(a.N), x = 3 * static_cast<size_t>(a.rows) * ldx, w = 3 * static_cast<size_t>(a.K) * ldw;
     if (p != nullptr) {
@@ -458,7 +464,8 @@ static size_t parts_bytes(const b2kv_linear_args& a, linf32tc::Parts* p, void* a
         p->odd_x = reinterpret_cast<int32_t*>(p->w + w), p->odd_w = p->odd_x + tiles_m * steps;
         p->ldx = static_cast<int>(ldx), p->ldw = static_cast<int>(ldw);
     }
-    return (x + w) * 2 + (tiles_m + tiles_n) * steps * sizeof(int32_t);
+    const size_t bytes = (x + w) * 2 + (tiles_m + tiles_n) * steps * sizeof(int32_t);
+    return bytes <= kMaxScratch ? bytes : 0;
 }
 
 // Three matrices of rows x cols bf16, boxes of box_rows x 64 of one of them, 128-byte swizzle; zero outside.

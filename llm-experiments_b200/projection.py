@@ -142,8 +142,8 @@ def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Se
     the output of a product of more rows, but not of one whose caller said ``ahead``: that none of its outputs is a ``w`` and the
     kernel behind it may start early; nor, right behind it, of a product of at most 128 rows.
 
-    ``scratch`` (of one model's steps, one after the other) keeps the memory in which float32 products of more than 128 rows lay
-    their operands out once; without it they do so tile by tile."""
+    ``scratch`` (of one model's steps, one after the other) keeps the memory, 512 MB at most, in which float32 products of more than 256
+    rows and many tiles lay their operands out once (``b2kv_linear_workspace_bytes``); without it they do so tile by tile."""
     rows, n = x.shape[0] if group_x_rows is None else rows, segments[-1].end
     if rows <= 0 or k <= 0 or n <= 0:
         raise ValueError(f"linear: Invalid dimensions x=({rows}, {k}), w=({k}, {n})")
@@ -170,7 +170,7 @@ def linear(ctx: GPUContext, x: GPUBuffer2D, w: GPUBuffer2D, k: int, segments: Se
     if group_x_rows is not None:
         options = _native.linear_options(group_x_rows.data_ptr(), x.shape[0], _native.LINEAR_AHEAD if ahead else 0)
     ws = None
-    if scratch is not None and rows > 128 and x.buffer.dtype == torch.float32:
+    if scratch is not None and rows > 256 and x.buffer.dtype == torch.float32:
         nbytes = _native.lib.b2kv_linear_workspace_bytes(a)
         if nbytes:
             ws = scratch["linear"] = memory(scratch.get("linear"), nbytes, x.buffer.device)

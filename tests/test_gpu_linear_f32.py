@@ -190,7 +190,7 @@ def test_operands_of_any_size(pkg, rows, K, sx, sw):
     bounded(product(pkg, make_ctx(pkg), x, w), x, w)
 
 
-@pytest.mark.parametrize("rows,K,n", [(693, 768, 3072), (1300, 1040, 644), (130, 16388, 388), (2100, 132, 2500)])
+@pytest.mark.parametrize("rows,K,n", [(693, 768, 3072), (1300, 1040, 644), (130, 16388, 388), (2100, 132, 2500), (257, 6404, 388)])
 def test_parts_made_ahead_have_the_same_bits(pkg, rows, K, n):
     """With scratch memory the operands of large products are laid out by a kernel ahead: the same numbers, also where some have no parts,
     and in a scratch that another product left full of its own."""

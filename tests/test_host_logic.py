@@ -295,3 +295,20 @@ def test_few_long_runs_have_a_table_of_their_own(pkg):
     assert serving.split_runs(singles + [(64, 193, 64)])[1:] == ([(64, 193, 64)], 2)
     for together in (singles, singles[:15] + [(15, 400, 15)], singles[:20] + [(20 + 300 * i, 300, 20 + i) for i in range(7)], [(0, 5, 1)], []):
         assert serving.split_runs(together) == (together, [], max((n for _, n, _ in together), default=0))
+
+
+def test_memory_of_fp32_products_has_a_ceiling(pkg):
+    """Rows and columns around the edges of the rule, and products whose parts would take gigabytes."""
+    native = pkg._native
+
+    def size(rows, k, n, groups=1):
+        return native.lib.b2kv_linear_workspace_bytes(native.linear_args(256, 256, 0, 0, 0, k, 0, n, 0, 0, [(256, n, 0, n, 0)], rows, k, n, groups, 0, 0, 0, 0.0))
+
+    assert size(256, 4096, 4096) == 0 < size(257, 1024, 4096)  # three rows of tiles
+    assert size(384, 1024, 5461 // 4 * 4) > 0 == size(384, 1024, 5464)  # w's parts: 32 MB,
+    assert size(512, 1024, 19112) > 0 == size(512, 1024, 19116)  # 112 MB,
+    assert size(513, 1024, 27304) > 0 == size(513, 1024, 27308)  # 160 MB
+    assert size(257, 64, 384 * 128) == size(693, 64, 64) == size(1000, 4096, 4096, 2) == 0
+    for rows, k, n in ((2048, 2048, 32768), (4096, 4096, 131072), (100000, 4096, 1024), (20000, 4096, 4096)):
+        assert size(rows, k, n) == 0
+    assert max(size(r, k, n) for r in (300, 1000, 5000, 14000) for k in (768, 4096) for n in (768, 4096, 6400)) <= 512 << 20
