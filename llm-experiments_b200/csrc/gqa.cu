@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kAppendThreads) gqa_append_kernel(T* y, T* k_c
 
 // One CTA per (head, query row); its warps take the visible tokens in turn, a few at a time, each with an online softmax of its own, and are
 // merged at the end.  A lane holds kPer elements of the query and of the output.  Few rows are a chain of loads, sums over the warp and
-// exponentials, so tokens that are on their way together share it: three rows of 200 to 600 tokens (12 heads of 64, fp32) 12 us, 25 with four warps
+// exponentials, so tokens that are on their way together share it: three rows of 250 to 310 tokens (12 heads of 64, fp32) 12 us, 25 with four warps
 // and token after token.
 constexpr int kWarps = 8;
 
