@@ -297,8 +297,7 @@ embedding_kernel(const T* __restrict__ table, const T* __restrict__ pos_enc, con
 
 // Index of the largest value of each row (the lowest index among equals, like numpy.argmax).  kVec: rows of whole 16-byte pieces, four of
 // which a thread has on their way together (8 rows of 32768 bf16: 3.2 us behind the product; 7.7 with a value per load and 256 threads).
-constexpr int kArgmaxThreads = 1024;
-template <typename T, bool kVec>
+template <typename T, bool kVec, int kArgmaxThreads>
 __global__ void __launch_bounds__(kArgmaxThreads) argmax_kernel(const T* x, int32_t* out, int V) {
     __shared__ float s_val[kArgmaxThreads / 32];
     __shared__ int s_idx[kArgmaxThreads / 32];
@@ -335,19 +334,27 @@ __global__ void __launch_bounds__(kArgmaxThreads) argmax_kernel(const T* x, int3
     if ((threadIdx.x & 31) == 0) s_val[threadIdx.x >> 5] = best, s_idx[threadIdx.x >> 5] = idx;
     __syncthreads();
     if (threadIdx.x < 32) {
-        best = s_val[threadIdx.x], idx = s_idx[threadIdx.x];
+        constexpr int kWarps = kArgmaxThreads / 32;
+        best = s_val[threadIdx.x % kWarps], idx = s_idx[threadIdx.x % kWarps];
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) merge(__shfl_xor_sync(0xffffffffu, best, off), __shfl_xor_sync(0xffffffffu, idx, off));
+        for (int off = kWarps / 2; off > 0; off >>= 1) merge(__shfl_xor_sync(0xffffffffu, best, off), __shfl_xor_sync(0xffffffffu, idx, off));
         if (threadIdx.x == 0) out[blockIdx.x] = idx == 0x7fffffff ? 0 : idx;  // a row of NaN or -inf only: index 0
     }
 }
 
-template <typename T>
-int launch_argmax(const T* x, int32_t* out, int rows, int size, void* stream) {
+template <typename T, int kArgmaxThreads>
+int launch_argmax_by(const T* x, int32_t* out, int rows, int size, void* stream) {
     const bool vec = aligned16(x) && size % Elt<T>::kPerChunk == 0;
     OverlapLaunch launch(rows, kArgmaxThreads, 0, stream);
-    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, vec ? argmax_kernel<T, true> : argmax_kernel<T, false>, x, out, size));
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, vec ? argmax_kernel<T, true, kArgmaxThreads> : argmax_kernel<T, false, kArgmaxThreads>, x, out, size));
     return B2KV_OK;
+}
+
+// 1024 threads where every row has an SM to itself; with more rows a row's share of threads counts for more than its time (us by 1024 and by 256
+// threads, fp32: 64 rows of 32768 3.0, 6.2; 300 of 512 2.7, 2.2; 1000 of 4096 6.1, 4.1; 4000 of 96 16.8, 4.8).
+template <typename T>
+int launch_argmax(const T* x, int32_t* out, int rows, int size, void* stream) {
+    return rows <= device_sm_count() ? launch_argmax_by<T, 1024>(x, out, rows, size, stream) : launch_argmax_by<T, 256>(x, out, rows, size, stream);
 }
 
 }  // namespace

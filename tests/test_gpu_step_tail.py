@@ -225,3 +225,17 @@ def test_layernorm_of_a_row_does_not_depend_on_the_others(pkg, ctx, dtype, size)
             pkg.gpu.layernorm(ctx, U.buf2d(pkg, ctx, x[r:r + step]), one(g), one(b), U.buf2d(pkg, ctx, y[r:r + step]))
     pkg.gpu.batch_commit(ctx)
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,size", [(148, 96), (149, 96), (149, 1000), (600, 33), (300, 8200)])
+def test_argmax_of_many_rows(pkg, ctx, dtype, rows, size):
+    """Either side of as many rows as there are SMs: fewer threads per row behind it."""
+    x = U.randn((rows, size), dtype, ctx.device, 38)
+    x[1, size // 2:] = 9.0
+    x[rows - 1] = float("-inf")
+    out = torch.full((rows + 1,), -7, dtype=torch.int32, device=ctx.device)
+    pkg.gpu.batch_begin(ctx)
+    pkg.gpu.argmax(ctx, U.buf2d(pkg, ctx, x), pkg.gpu.GPUBuffer1D(buffer=out[:rows], shape=(rows,), size=rows))
+    pkg.gpu.batch_commit(ctx)
+    assert np.array_equal(out[:rows].cpu().numpy(), x.float().cpu().numpy().argmax(1)) and int(out[rows]) == -7
