@@ -137,13 +137,11 @@ __global__ void __launch_bounds__(kAppendThreads) gqa_append_kernel(T* y, T* k_c
     rv.scaled(v_cache + place * nv, v, nullptr, 1.f, nv);
 }
 
-// One CTA per (head, query row); its warps take the visible tokens in turn, a few at a time, each with an online softmax of its own, and are
-// merged at the end.  A lane holds kPer elements of the query and of the output.  Few rows are a chain of loads, sums over the warp and
-// exponentials, so tokens that are on their way together share it: three rows of 250 to 310 tokens (12 heads of 64, fp32) 12 us, 25 with four warps
-// and token after token.
-constexpr int kWarps = 8;
-
-template <typename T, int kPer>
+// One CTA per (head, query row); its warps take the visible tokens in turn, each with an online softmax of its own, and are merged at the end.
+// A lane holds kPer elements of the query and of the output.  Two forms: four warps and token after token, and, where few rows are a chain of loads,
+// sums over the warp and exponentials, eight warps and kTogether tokens at a time, which are on their way together and share the rest
+// (three rows of 250 to 310 tokens, 12 heads of 64, fp32: 25 us and 12; the rule at launch_simt).
+template <typename T, int kPer, int kWarps, int kTogether>
 __global__ void __launch_bounds__(kWarps * 32) gqa_decode_kernel(const GqaDecodeArgs a) {
     extern __shared__ float sm_acc[];  // [kWarps][vdim]
     __shared__ float sm_m[kWarps], sm_l[kWarps];
@@ -166,8 +164,28 @@ __global__ void __launch_bounds__(kWarps * 32) gqa_decode_kernel(const GqaDecode
         acc[c] = 0.f;
     }
     float m = -INFINITY, l = 0.f;
-    constexpr int kTogether = kPer <= 4 ? 4 : 2;
-    for (int t0 = warp * kTogether; t0 <= pos; t0 += kWarps * kTogether) {
+    if constexpr (kTogether == 1) {
+        for (int t = warp; t <= pos; t += kWarps) {
+            const T* key = keys + static_cast<int64_t>(t) * a.G * a.dim;
+            const T* value = values + static_cast<int64_t>(t) * a.G * a.vdim;
+            float v[kPer], s = 0.f;
+#pragma unroll
+            for (int c = 0; c < kPer; ++c) {
+                const int d = c * 32 + lane;
+                v[c] = d < a.vdim ? Elt<T>::to_float(value[d]) : 0.f;
+                s = fmaf(q[c], d < a.dim ? Elt<T>::to_float(key[d]) : 0.f, s);
+            }
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+            s = s * a.scale - slope * static_cast<float>(pos - t);
+            const float mn = fmaxf(m, s), f = expf(m - mn), p = expf(s - mn);
+            l = l * f + p;
+            m = mn;
+#pragma unroll
+            for (int c = 0; c < kPer; ++c) acc[c] = fmaf(acc[c], f, p * v[c]);
+        }
+    }
+    for (int t0 = warp * kTogether; kTogether > 1 && t0 <= pos; t0 += kWarps * kTogether) {
         float v[kTogether][kPer], s[kTogether];
 #pragma unroll
         for (int u = 0; u < kTogether; ++u) {
@@ -476,11 +494,14 @@ int launch_runs(const GqaDecodeArgs& a, void* stream) {
 // For rows that the caller says come in runs, and enough of them (a CTA takes the sequences of its 16 rows one after the other, so that single rows of
 // many sequences would be in line: 16 of them take as long as the one that sees most, times 16).
 int launch_runs_f32(const GqaDecodeArgs& a, void* stream) {
-    // Enough CTAs that the SMs are busy with 64 threads each: below, a CTA's chain of token tiles takes longer than rows one by
-    // one over as many SMs (8 heads of 64 behind 500 tokens: 100 rows 58 us and 47, 160 rows 57 and 69; of 128, with half as many CTAs per SM: 200
-    // rows 111 and 100, 300 rows 132 and 159).
+    // Enough CTAs that the SMs are busy with 64 threads each: below, a CTA's chain of token tiles takes longer than rows one by one over as many SMs;
+    // us row by row and as runs, in the order of CTAs.  Heads of 64 (and 32): 1 prompt of 160 over 8 heads (80) 15.4, 18.6; behind 500 tokens 68, 57;
+    // 1 of 100 over 12 heads (84) 11.7, 13.9; 1 of 200 over 8 (104) 19.0, 23.8; behind 500 92, 65; 1 of 160 over 12 (120) 20.7, 18.8.  Heads of
+    // 128, half as many CTAs per SM: 3 of 100 over 8 (152) 21, 29; behind 500 149, 180; 1 of 300 over 8 (152) 50, 53; behind 500 177, 132; 3 of 300 over
+    // 4 (228) 69, 59.  Prompts mostly begin at their first token, and rows of several sequences in one CTA cost it twice, so the line is where runs
+    // win without a past.
     const long long ctas = static_cast<long long>(a.H) * ((a.rows + kRunRows - 1) / kRunRows), sms = device_sm_count();
-    const bool few = a.rows < 64 || (std::max(a.dim, a.vdim) <= 64 ? 2 * ctas < sms : 4 * ctas < 3 * sms);
+    const bool few = a.rows < 64 || (std::max(a.dim, a.vdim) <= 64 ? 4 * ctas < 3 * sms : 2 * ctas < 3 * sms);
     if ((few && tune_get("gqa_runs") == 0) || (a.rows + kRunRows - 1) / kRunRows > 65535) return B2KV_ERR_UNSUPPORTED;
     const int widest = std::max(a.dim, a.vdim);
     if (widest > 128 || a.dim % 4 || a.vdim % 4 || a.ld_q % 4 || !aligned16(a.q) || !aligned16(a.k_cache) || !aligned16(a.v_cache))
@@ -488,21 +509,29 @@ int launch_runs_f32(const GqaDecodeArgs& a, void* stream) {
     return widest <= 64 ? launch_runs<64, false>(a, stream) : launch_runs<128, false>(a, stream);
 }
 
+template <typename T, int kPer>
+int launch_simt_per(const GqaDecodeArgs& a, bool together, cudaStream_t stream) {
+    constexpr int kTogether = kPer <= 4 ? 4 : 2;
+    const int warps = together ? 8 : 4;
+    const auto kernel = together ? gqa_decode_kernel<T, kPer, 8, kTogether> : gqa_decode_kernel<T, kPer, 4, 1>;
+    kernel<<<dim3(a.H, a.rows), warps * 32, static_cast<size_t>(warps) * a.vdim * sizeof(float), stream>>>(a);
+    B2KV_CUDA_TRY(cudaGetLastError());
+    return B2KV_OK;
+}
+
 template <typename T>
 int launch_simt(const GqaDecodeArgs& a, void* stream) {
     const int widest = a.dim > a.vdim ? a.dim : a.vdim;
     if (widest > 512 || a.rows > 65535) return B2KV_ERR_UNSUPPORTED;
-    const dim3 grid(a.H, a.rows);
-    const size_t smem = static_cast<size_t>(kWarps) * a.vdim * sizeof(float);
+    // Tokens together where a row's time is a chain that other CTAs do not hide, and there are tokens enough for all warps; us token after token and
+    // together, fp32, 12 heads of 64: 3 rows of up to 16 tokens 3.3, 3.2; 100 8.6, 5.2; 2000 131, 57; 40 rows of 16 3.7, 4.2; 100 10.0, 8.1; 150 rows (1800
+    // CTAs) of 100 17.1, 18.8; 400 55.0, 54.2; 2000 380, 301; 400 rows of 100 34.4, 41.7; 400 116, 126; 2000 808, 679.  In bf16 (sizes that the
+    // tensor cores do not take) tokens share less: 12 heads of 60, 3 rows of 100 8.7, 8.4; 2000 133, 121; 150 rows of 400 57, 69.
+    const long long ctas = static_cast<long long>(a.rows) * a.H, sms = device_sm_count();
+    const bool together = sizeof(T) == 4 ? a.span > 32 && (ctas <= 5 * sms || (a.span >= 256 && ctas <= 9 * sms) || a.span >= 1024)
+                                         : a.span >= 256 && ctas <= 4 * sms;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (widest <= 64)
-        gqa_decode_kernel<T, 2><<<grid, kWarps * 32, smem, s>>>(a);
-    else if (widest <= 128)
-        gqa_decode_kernel<T, 4><<<grid, kWarps * 32, smem, s>>>(a);
-    else
-        gqa_decode_kernel<T, 16><<<grid, kWarps * 32, smem, s>>>(a);
-    B2KV_CUDA_TRY(cudaGetLastError());
-    return B2KV_OK;
+    return widest <= 64 ? launch_simt_per<T, 2>(a, together, s) : widest <= 128 ? launch_simt_per<T, 4>(a, together, s) : launch_simt_per<T, 16>(a, together, s);
 }
 
 template <typename T>

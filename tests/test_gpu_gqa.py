@@ -149,6 +149,29 @@ def test_single_rows(pkg, path, dtype, heads, kv, dim, vdim, bias):
     assert (out[len(pos)] == 7).all() and (out[:, heads * vdim:] == 7).all()
 
 
+@pytest.mark.parametrize("dtype,heads,kv,dim,vdim", [(F32, 12, 4, 64, 60), (F32, 3, 1, 128, 130), (BF, 6, 2, 60, 30), (BF, 2, 2, 129, 20)])
+@pytest.mark.parametrize("rows,span", [(1, 32), (1, 33), (2, 255), (2, 256), (40, 90), (250, 40), (250, 300), (400, 90), (400, 300), (420, 1100)])
+def test_tokens_together_and_one_by_one(pkg, dtype, heads, kv, dim, vdim, rows, span):
+    """On CUDA cores, either side of every line between the two forms: few and many rows of short and of long contexts."""
+    from llm_experiments_b200 import gqa
+    from llm_experiments_b200.latent import RowPlaces
+
+    ctx, slots = make_ctx(pkg), 5
+    shape = gqa.GqaShape(heads, kv, dim, vdim, dim ** -0.5)
+    cache = make_cache(pkg, ctx, shape, slots, span, dtype)
+    gen = np.random.default_rng(rows + span)
+    slot, pos = gen.integers(0, slots, rows), np.append(gen.integers(0, span, rows - 1), span - 1)
+    q, out = rnd((rows, heads * dim), dtype, 7), torch.full((rows + 1, heads * vdim), 7.0, dtype=dtype, device="cuda")
+    ints = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")  # noqa: E731
+    in_batch(pkg, ctx, lambda: gqa.gqa_decode(ctx, wrap(pkg, q), shape, None, RowPlaces(ints(slot), ints(pos)), cache, wrap(pkg, out[:rows]), span, path=SIMT))
+    k, v = cache_views(cache, shape)
+    some = sorted({0, rows // 2, rows - 1})
+    want = reference(np64(q[some]).reshape(len(some), heads, dim), np64(k), np64(v), slot[some], pos[some], shape, None)
+    tol = 1e-5 if dtype == F32 else 8e-3
+    np.testing.assert_allclose(np64(out[some]), want, rtol=tol, atol=tol)
+    assert bool((out[rows] == 7).all()) and bool(torch.isfinite(out).all())
+
+
 @pytest.mark.parametrize("heads,kv,dim,vdim", [(3, 1, 4, 8), (4, 2, 64, 64), (2, 1, 72, 128), (2, 2, 128, 20)])
 @pytest.mark.parametrize("runs", [((0, 0, 65),), ((2, 0, 64), (0, 60, 7), (1, 199, 1), (2, 64, 31), (0, 0, 40)), ((1, 130, 96), (0, 3, 33))])
 @pytest.mark.parametrize("singles", [None, 0, 5])
