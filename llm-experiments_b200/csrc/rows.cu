@@ -174,7 +174,16 @@ int launch_rmsnorm(const float* x, int64_t ld_x, const int32_t* row_index, const
     return launch(x, ld_x, row_index, w, w_offset, out, ld_out, rows, size, eps, vec, stream);
 }
 
-template <typename T, int kKeep>
+// A load that stays where it is: the compiler would have the residual's pieces wait until their sums are known.
+__device__ __forceinline__ float4 load_now(const float* p, int i) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p + 4 * i));
+    return v;
+}
+
+// kOne: a CTA per row, all of which are on the device at once; everything that is read is on its way together, with rows of up to 2048
+// elements the weights as well (500 rows of 4096: 5.1 us, 6.2 row after row, for which fewer CTAs fit; 8 of 2048: 2.1 and 2.4).
+template <typename T, int kKeep, bool kOne>
 __global__ void __launch_bounds__(kThreads) layernorm_rows_kernel(const float* y, int64_t ld_y, const int32_t* row_index,
                                                                   const float* w, const float* b, float* x, int64_t ld_x,
                                                                   T* out, int64_t ld_out, int rows, int size, float eps, bool vec) {
@@ -211,12 +220,19 @@ __global__ void __launch_bounds__(kThreads) layernorm_rows_kernel(const float* y
         for (int c = 0; c < kKeep; ++c) {
             const int i = threadIdx.x + c * kThreads;
             if (i < chunks) {
-                next[c] = reinterpret_cast<const float4*>(yr)[i];
-                if (xr != nullptr) next_res[c] = reinterpret_cast<const float4*>(xr)[i];
+                next[c] = kOne ? load_now(yr, i) : reinterpret_cast<const float4*>(yr)[i];
+                if (xr != nullptr) next_res[c] = kOne ? load_now(xr, i) : reinterpret_cast<const float4*>(xr)[i];
             }
         }
     };
     load(blockIdx.x);
+    constexpr bool kWeightsAhead = kOne && kKeep <= 2;
+    float4 w_ahead[kKeep], b_ahead[kKeep];
+#pragma unroll
+    for (int c = 0; c < kKeep && kWeightsAhead; ++c) {
+        const int i = threadIdx.x + c * kThreads;
+        if (i < chunks) w_ahead[c] = load_now(w, i), b_ahead[c] = load_now(b, i);
+    }
     for (int r = blockIdx.x; r < rows; r += row_after_row(kKeep) ? gridDim.x : rows) {
         float* xr = x == nullptr ? nullptr : x + static_cast<int64_t>(r) * ld_x;
         T* outr = out == nullptr ? nullptr : out + static_cast<int64_t>(r) * ld_out;
@@ -227,7 +243,7 @@ __global__ void __launch_bounds__(kThreads) layernorm_rows_kernel(const float* y
             keep[c] = next[c], res[c] = next_res[c];
             if (static_cast<int>(threadIdx.x) + c * kThreads < chunks) sum += (keep[c].x + keep[c].y) + (keep[c].z + keep[c].w);
         }
-        if (row_after_row(kKeep) && r + static_cast<int>(gridDim.x) < rows) load(r + gridDim.x);
+        if (!kOne && row_after_row(kKeep) && r + static_cast<int>(gridDim.x) < rows) load(r + gridDim.x);
         const float mean = block_sum(sum, part[0]) * inv;
 #pragma unroll
         for (int c = 0; c < kKeep; ++c) {
@@ -241,7 +257,8 @@ __global__ void __launch_bounds__(kThreads) layernorm_rows_kernel(const float* y
         for (int c = 0; c < kKeep; ++c) {
             const int i = threadIdx.x + c * kThreads;
             if (i < chunks) {
-                const float4 wv = reinterpret_cast<const float4*>(w)[i], bv = reinterpret_cast<const float4*>(b)[i];
+                const float4 wv = kWeightsAhead ? w_ahead[c] : reinterpret_cast<const float4*>(w)[i];
+                const float4 bv = kWeightsAhead ? b_ahead[c] : reinterpret_cast<const float4*>(b)[i];
                 float4 v = keep[c];
                 v.x = fmaf(v.x * scale, wv.x, bv.x), v.y = fmaf(v.y * scale, wv.y, bv.y);
                 v.z = fmaf(v.z * scale, wv.z, bv.z), v.w = fmaf(v.w * scale, wv.w, bv.w);
@@ -252,15 +269,21 @@ __global__ void __launch_bounds__(kThreads) layernorm_rows_kernel(const float* y
                 if (outr != nullptr) store4(outr + 4 * i, v);
             }
         }
+        if (kOne) break;
     }
 }
 
 template <typename T, int kKeep>
 int launch_layernorm_keep(const float* y, int64_t ld_y, const int32_t* row_index, const float* w, const float* b, float* x,
                           int64_t ld_x, T* out, int64_t ld_out, int rows, int size, float eps, bool vec, void* stream) {
-    static int fit[64] = {0};
-    auto kernel = layernorm_rows_kernel<T, kKeep>;
-    OverlapLaunch launch(row_after_row(kKeep) ? row_ctas(kernel, rows, fit) : rows, kThreads, 0, stream);
+    static int fit[64] = {0}, fit_one[64] = {0};
+    auto kernel = layernorm_rows_kernel<T, kKeep, false>;
+    int ctas = rows;
+    if constexpr (row_after_row(kKeep)) {
+        ctas = row_ctas(kernel, rows, fit);
+        if (row_ctas(layernorm_rows_kernel<T, kKeep, true>, rows, fit_one) == rows) kernel = layernorm_rows_kernel<T, kKeep, true>, ctas = rows;
+    }
+    OverlapLaunch launch(ctas, kThreads, 0, stream);
     B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, kernel, y, ld_y, row_index, w, b, x, ld_x, out, ld_out, rows, size, eps, vec));
     return B2KV_OK;
 }
