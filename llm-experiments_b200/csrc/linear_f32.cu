@@ -265,15 +265,27 @@ int linear_f32(const b2kv_linear_args& a, void* stream) {
                                          a, splits));
         return B2KV_OK;
     }
-    if (a.K <= kThinK && a.groups == 1 && a.group_rows == nullptr) {
-        // rows per CTA: few, unless the columns of w are then read for nothing (more than four CTAs per SM)
-        const long long cols = (a.N / 2 + kThinThreads - 1) / kThinThreads;
-        int row_tile = kThinRows;
-        while (row_tile > 8 && cols * ((a.rows + row_tile - 1) / row_tile) < 4LL * sms) row_tile /= 2;
+    // (many rows of columns that leave a quarter and more of the threads idle: the tiles are better at the same sums, 8000 rows of 384 columns, K = 32,
+    // 9.4 us and 11.9 by threads, 32000 of 96 14.4 and 15.8; fewer rows, 6000 of 96, 6.3 and 5.3)
+    const long long thin_cols = (a.N / 2 + kThinThreads - 1) / kThinThreads;
+    const bool idle = 4LL * a.N <= 3 * thin_cols * 2 * kThinThreads && a.rows * thin_cols >= (a.N <= 2 * kThinThreads ? 32000 : 16000);
+    if (a.K <= kThinK && a.groups == 1 && a.group_rows == nullptr && !idle) {
+        // rows per CTA: as few (eight) as leave all CTAs on the device at once (6000 rows, 16 -> 64: 750 CTAs of 8 rows, of which 740 fit, 4.7 us, 3.5
+        // with 9; 4000 rows, 16 -> 768: 750 of 16 7.4, 6.5 with 17)
+        const long long cols = thin_cols;
+        const auto kernel = a.K <= 16 ? linear_f32_thin_kernel<16> : linear_f32_thin_kernel<32>;
+        static int per_sm[2][64] = {};
+        int dev = 0;
+        B2KV_CUDA_TRY(cudaGetDevice(&dev));
+        if (dev < 0 || dev >= 64) return B2KV_ERR_UNSUPPORTED;
+        int& resident = per_sm[a.K <= 16][dev];
+        if (resident == 0) B2KV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kThinThreads, 0));
+        const long long fit = std::max(resident, 1) * static_cast<long long>(sms);
+        const int row_tile = static_cast<int>(std::min<long long>(std::max<long long>((a.rows * cols + fit - 1) / fit, 8), kThinRows));
         const dim3 grid(static_cast<unsigned>(cols), static_cast<unsigned>((a.rows + row_tile - 1) / row_tile));
         if (grid.y <= 65535u) {
             OverlapLaunch launch(grid, kThinThreads, 0, stream);
-            B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, a.K <= 16 ? linear_f32_thin_kernel<16> : linear_f32_thin_kernel<32>, a, row_tile));
+            B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, kernel, a, row_tile));
             return B2KV_OK;
         }
     }
