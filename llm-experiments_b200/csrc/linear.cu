@@ -157,10 +157,21 @@ static int launch_thin(const b2kv_linear_args& a, void* stream) {
     int row_tile = a.rows > 1024 ? kThinRows : 8;
     const long long cols = (a.N / 2 + kThinThreads - 1) / kThinThreads;
     while (row_tile > 8 && cols * ((a.rows + row_tile - 1) / row_tile) < 6LL * device_sm_count()) row_tile /= 2;
+    const auto kernel = a.K <= 16 ? linear_thin_kernel<16> : linear_thin_kernel<32>;
+    static int per_sm[2][64] = {};
+    int dev = 0;
+    B2KV_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return B2KV_ERR_UNSUPPORTED;
+    int& resident = per_sm[a.K <= 16][dev];
+    if (resident == 0) B2KV_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kThinThreads, 0));
+    // a few CTAs more than fit the device would run behind all others (1056 rows, 16 -> 2048: 1056 of 8 rows, of which 1036 fit, 5.9 us, 5.3 with 9)
+    const long long fit = static_cast<long long>(resident) * device_sm_count(), ctas = cols * ((a.rows + row_tile - 1) / row_tile);
+    if (fit >= cols && ctas > fit && 4 * ctas <= 5 * fit)
+        row_tile = static_cast<int>(std::min<long long>(kThinRows, std::max<long long>(row_tile, (a.rows + fit / cols - 1) / (fit / cols))));
     const dim3 grid(static_cast<unsigned>(cols), (a.rows + row_tile - 1) / row_tile);
     if (grid.y > 65535u) return B2KV_ERR_UNSUPPORTED;
     OverlapLaunch launch(grid, kThinThreads, 0, stream);
-    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, a.K <= 16 ? linear_thin_kernel<16> : linear_thin_kernel<32>, a, row_tile));
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&launch.cfg, kernel, a, row_tile));
     return B2KV_OK;
 }
 
