@@ -406,12 +406,14 @@ latent_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_ql, const __grid_
 
 // One CTA per (head, row): the shares' partial results, each relative to its own reference maximum.  All of it is latency, so the elements of the
 // first shares are on their way with what their weights are made of (64 rows of 32 heads in two shares of 512 elements, behind the
-// products: 4.3 us, 7.7 with the elements asked for when the weights are known).
+// products: 4.3 us, 7.7 with the elements asked for when the weights are known).  kMergeAhead shares at a time: two where there are many
+// rows and so few shares each, 16 or 32 where few rows are cut into many (one row of 8 heads over 8000 tokens, latents of 128, 63 shares: attention and
+// merge 13.2 us, 19.5 by twos).
 constexpr int kMaxSplits = 64;
-constexpr int kMergeThreads = 128, kMergePairs = 2, kMergeAhead = 2;  // kMergePairs: pairs of elements per thread
-__global__ void __launch_bounds__(kMergeThreads, 12)
+constexpr int kMergeThreads = 128;
+template <int kMergeAhead, int kMergePairs>  // kMergePairs: pairs of elements per thread
+__global__ void __launch_bounds__(kMergeThreads, kMergeAhead <= 2 ? 12 : 4)
 latent_merge_kernel(const float* partial, __nv_bfloat16* out, int H, int kv_rank, int splits, bool vec) {
-    static_assert(2 * kMergeThreads * kMergePairs >= 512, "a thread's pairs cover the widest latents");
     __shared__ float w[kMaxSplits];
     grid_launch_dependents();
     if (threadIdx.x == 0) grid_dependency_wait();
@@ -565,8 +567,10 @@ int latent_decode_tc(const LatentDecodeArgs& a, void* workspace, size_t workspac
     const int rc = Hn == 16 ? launch<16>(m, p, static_cast<unsigned>(grid), smem, stream)
                             : launch<32>(m, p, static_cast<unsigned>(grid), smem, stream);
     if (rc != B2KV_OK || p.splits == 1) return rc;
+    static_assert(2 * kMergeThreads * 2 >= 512, "a thread's pairs cover the widest latents");
+    const auto merge = p.splits <= 4 ? latent_merge_kernel<2, 2> : a.kv_rank <= 2 * kMergeThreads ? latent_merge_kernel<32, 1> : latent_merge_kernel<16, 2>;
     OverlapLaunch cfg(dim3(a.H, a.rows), kMergeThreads, 0, stream);
-    B2KV_CUDA_TRY(cudaLaunchKernelEx(&cfg.cfg, latent_merge_kernel, static_cast<const float*>(p.partial), p.out, a.H, a.kv_rank, p.splits,
+    B2KV_CUDA_TRY(cudaLaunchKernelEx(&cfg.cfg, merge, static_cast<const float*>(p.partial), p.out, a.H, a.kv_rank, p.splits,
                                      reinterpret_cast<uintptr_t>(p.partial) % 8 == 0 && reinterpret_cast<uintptr_t>(p.out) % 4 == 0));
     return B2KV_OK;
 }

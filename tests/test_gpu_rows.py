@@ -151,9 +151,9 @@ def test_choices_of_many_rows_are_counted(pkg, rows, experts, groups, keep, top)
 
 
 @pytest.mark.parametrize("rank", [8, 264, 512])
-@pytest.mark.parametrize("span", [300, 700, 3000])
+@pytest.mark.parametrize("span", [300, 700, 3000, 9000])
 def test_shares_of_latent_rows_at_any_place(pkg, rank, span):
-    """Rows in 2 to 12 shares, some of them empty, merged from and to memory by pairs of elements and, one element off, by elements."""
+    """Rows in a few shares and in dozens, some of them empty, merged from and to memory by pairs of elements and, one element off, by elements."""
     native = pkg._native
     g = torch.Generator(device="cuda").manual_seed(rank + span)
     H, dim, rot, n = 20, 16, 8, 4
