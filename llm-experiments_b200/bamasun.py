@@ -302,7 +302,8 @@ def state_create(ctx: GPUContext, cfg: BamasunConfig, weights: BamasunWeights, b
             owned[i].seq_lens = seq_lens
     return BamasunState(cfg=cfg, weights=weights, batch_size=batch_size, max_seq_len=max_seq_len, dtype=dtype, owned=owned,
                         recurrent=states, seq_lens=seq_lens, lengths=[0] * batch_size,
-                        prompt_form=all(gqa.prefill_supported(lc.attention, dtype) for lc in cfg.layers if lc.attention))
+                        prompt_form=all(gqa.prefill_supported(lc.attention, dtype) for lc in cfg.layers if lc.attention),
+                        cuts_runs=any(recurrent.cuts_runs(lc.gla, dtype) for lc in cfg.layers if lc.gla))
 
 
 def _add_normed(ctx, y: GPUBuffer2D, cfg: BamasunConfig, norm: NormWeights, x: GPUBuffer2D, copy: Optional[GPUBuffer2D]) -> None:

@@ -16,7 +16,7 @@ import torch
 from . import _native
 from .batch import batch_op_begin, dev_status_ptr, reference_op, scratch as memory
 from .kv_cache import dtype_code
-from .serving import RowSegments
+from .serving import LONG_RUN, RowSegments
 from .types import GPUBuffer1D, GPUBuffer2D, GPUContext
 
 
@@ -32,6 +32,12 @@ class GlaShape:
 
 def gla_state_create(ctx: GPUContext, shape: GlaShape, batch_size: int) -> torch.Tensor:
     return torch.zeros((batch_size, shape.heads, shape.dim, shape.vdim), dtype=torch.float32, device=ctx.device)
+
+
+def cuts_runs(shape: GlaShape, dtype: torch.dtype) -> bool:
+    """Whether runs of more than ``serving.LONG_RUN`` rows want scratch memory that shorter ones do not (float32)."""
+    size = lambda n: _native.lib.b2kv_gla_workspace_bytes(shape.heads, shape.dim, shape.vdim, 1, n, dtype_code(dtype), 0)  # noqa: E731
+    return dtype == torch.float32 and size(LONG_RUN) == 0 < size(LONG_RUN + 1)
 
 
 @reference_op("gated_linear_attention")

@@ -102,6 +102,7 @@ class SequenceState:
     recurrent: Dict[int, torch.Tensor] = field(default_factory=dict)  # by layer, fp32, first dimension = sequence
     scratch: Dict[str, torch.Tensor] = field(default_factory=dict)
     prompt_form: bool = False        # every layer's sizes have a form for prompt portions
+    cuts_runs: bool = False          # some layer's recurrence cuts long runs that go row by row, in scratch memory
     logits: Optional[GPUBuffer2D] = None  # fp32 rows of the last step
     layer_tap: Optional[list] = None      # debugging: receives a copy of the residual rows after every layer
 
@@ -253,7 +254,7 @@ def forward(ctx: GPUContext, state: SequenceState, entries: Sequence[Tuple[int, 
         T += n
         lens[slot] = start + n
     most = {k: max((n for _, n, _ in r), default=0) for k, r in runs.items()}
-    if most[True] > LONG_RUN:  # (there are no prompt portions then)
+    if state.cuts_runs and most[True] > LONG_RUN:  # (there are no prompt portions then)
         runs[True], runs[False], most[True] = split_runs(runs[True])
         most[False] = max((n for _, n, _ in runs[False]), default=0)
     want = [first_row[j] + int(p) for j in range(len(entries)) for p in entries[j][2]]

@@ -255,6 +255,7 @@ def test_a_long_run_among_many_single_rows_in_fp32(pkg):
     """The long run and the single rows have tables of their own: what the oracle says of every one of them, and of the next token."""
     n, name = 20, "ONLY_GLA"
     model, cfg = build(pkg, name, F32, batch=n + 1, max_tokens=400)
+    assert model.state.cuts_runs
     seqs = [U.tokens(cfg, 5 + i % 3, 60 + i) for i in range(n)] + [U.tokens(cfg, 303, 90)]
     model.forward([(i, seqs[i][:-2], []) for i in range(n)] + [(n, seqs[n][:40], [])])
     steps = [model.forward([(i, seqs[i][-2:-1], [0]) for i in range(n)] + [(n, seqs[n][40:-1], list(range(262)))]).clone(),

@@ -293,6 +293,10 @@ def test_few_long_runs_have_a_table_of_their_own(pkg):
     assert rest == singles + [(2064, 192, 65)] and long == [(64, 2000, 64)] and most == 192
     assert size(rest, most) == 0 and 0 < 20 * size(long, 2000) < size(runs, 2000)
     assert serving.split_runs(singles + [(64, 193, 64)])[1:] == ([(64, 193, 64)], 2)
+    from llm_experiments_b200 import recurrent
+
+    kinds = [((6, 64, 128), torch.float32), ((6, 64, 128), torch.bfloat16), ((4, 128, 256), torch.float32), ((16, 64, 256), torch.float32)]
+    assert [recurrent.cuts_runs(recurrent.GlaShape(*shape, 16.0), dtype) for shape, dtype in kinds] == [True, False, False, False]
     for together in (singles, singles[:15] + [(15, 400, 15)], singles[:20] + [(20 + 300 * i, 300, 20 + i) for i in range(7)], [(0, 5, 1)], []):
         assert serving.split_runs(together) == (together, [], max((n for _, n, _ in together), default=0))
 
